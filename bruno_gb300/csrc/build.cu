@@ -1660,7 +1660,9 @@ __device__ __noinline__ void filter_wide_global(uint64_t *s, uint64_t i, KT key,
   uint32_t all[25];
   int ne = NE;
   for (int q = 0; q < NE; ++q) all[q] = w[q];
-  Probe pr(a.S > 1 ? a.sg[t.sample].g : a.g, i);   /* inside the k-mer's own partition */
+  /* inside the k-mer's own partition, from its first slot on */
+  Probe pr = table_probe(a.S > 1 ? a.sg[t.sample].g : a.g, key_kmer(key), key);
+  pr.i = i;
   for (uint32_t probe = 1; probe < a.max_probe; ++probe) {
     pr.next();
     uint64_t *s2 = a.table + pr.i * SU;
@@ -1849,14 +1851,15 @@ __device__ __forceinline__ uint64_t sm_cas128(uint32_t a, uint64_t cmp_lo, uint6
 
 /* one step of count_in_entries on entry word e (snapshot w): claim it if empty, count if it
  * holds the code; true when the record is counted */
-__device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned code, unsigned long long &claims) {
+__device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned code, uint32_t weight,
+                                              unsigned long long &claims) {
   if (w == 0) {
-    const uint32_t old = atomicCAS(e, 0u, (code << E_CODE_SHIFT) | (1u << E_COUNT_SHIFT));
+    const uint32_t old = atomicCAS(e, 0u, (code << E_CODE_SHIFT) | (weight << E_COUNT_SHIFT));
     if (old == 0) { ++claims; return true; }
     w = old;
   }
   if (entry_code(w) == code) {
-    atomicAdd(e, 1u << E_COUNT_SHIFT);   /* a partition counted here holds fewer than 2^24 records */
+    atomicAdd(e, weight << E_COUNT_SHIFT);   /* a partition counted here holds fewer than 2^24 records */
     return true;
   }
   return false;
@@ -1867,10 +1870,10 @@ __device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned 
  * (most k-mers hold one or two edges); `first` are the words already read */
 template <int NE, int FIRST>
 __device__ __forceinline__ bool sm_count_entries_lazy(uint32_t *e, uint32_t e_addr, const uint32_t *first,
-                                                      unsigned code, unsigned long long &claims) {
+                                                      unsigned code, uint32_t weight, unsigned long long &claims) {
   #pragma unroll
   for (int i = 0; i < FIRST; ++i)
-    if (sm_entry_step(e + i, first[i], code, claims)) return true;
+    if (sm_entry_step(e + i, first[i], code, weight, claims)) return true;
   #pragma unroll
   for (int g = FIRST; g < NE; g += 4) {
     uint64_t w0, w1;
@@ -1878,14 +1881,14 @@ __device__ __forceinline__ bool sm_count_entries_lazy(uint32_t *e, uint32_t e_ad
     const uint32_t s[4] = {(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32)};
     #pragma unroll
     for (int i = 0; i < 4; ++i)
-      if (g + i < NE && sm_entry_step(e + g + i, s[i], code, claims)) return true;
+      if (g + i < NE && sm_entry_step(e + g + i, s[i], code, weight, claims)) return true;
   }
   return false;
 }
 
 /* one record into the partition held in shared memory; false if the region is full */
 __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_t region, uint64_t h, unsigned code,
-                                         uint32_t home, unsigned long long &slot_claims,
+                                         uint32_t home, uint32_t weight, unsigned long long &slot_claims,
                                          unsigned long long &entry_claims) {
   bool seen_primary = false;
   uint32_t j = home;
@@ -1895,7 +1898,7 @@ __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_
     asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(key), "=l"(w01) : "r"(a) : "memory");
     const uint64_t want = h | (seen_primary ? KEY_CONT : 0);
     if (key == KEY_EMPTY) {
-      const uint64_t ne0 = (uint64_t)((code << E_CODE_SHIFT) | (1u << E_COUNT_SHIFT));
+      const uint64_t ne0 = (uint64_t)((code << E_CODE_SHIFT) | (weight << E_COUNT_SHIFT));
       uint64_t ohi;
       const uint64_t olo = sm_cas128(a, KEY_EMPTY, 0ull, want, ne0, ohi);
       if (olo == KEY_EMPTY && ohi == 0) { ++slot_claims; ++entry_claims; return true; }
@@ -1905,7 +1908,7 @@ __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_
     if (key == want) {
       seen_primary = true;
       const uint32_t first[2] = {(uint32_t)w01, (uint32_t)(w01 >> 32)};
-      if (sm_count_entries_lazy<6, 2>((uint32_t *)(sm + (uint64_t)j * 4 + 1), a + 8u, first, code, entry_claims))
+      if (sm_count_entries_lazy<6, 2>((uint32_t *)(sm + (uint64_t)j * 4 + 1), a + 8u, first, code, weight, entry_claims))
         return true;
     }
     j = (j + 1 == region) ? 0u : j + 1;
@@ -1923,6 +1926,67 @@ struct CandArgs {
   unsigned long long *n_cand, *quick_hist;
   uint64_t t[6];
 };
+
+/* The listing over a counted region that has been written back (every thread of the block calls
+ * it): each slot's first key word then holds its place in the block's list (~0: not listed), so
+ * the listing needs no shared memory of its own. */
+template <class KT>
+__device__ __forceinline__ void list_slots(uint64_t *sm, uint32_t region, uint64_t slot0, const CandArgs &ca) {
+  constexpr uint32_t SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW;
+  constexpr int NE = Slot<KT>::ENTRIES;
+  __shared__ unsigned int s_nc, s_qh[4];
+  __shared__ unsigned long long s_base;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t nt = blockDim.x;
+  if (tid < 4) s_qh[tid] = 0;
+  if (tid == 0) s_nc = 0;
+  __syncthreads();
+  /* a quick drop's entries get flags 3 | 8 (k-mer total outside the k bounds) | 4 (entry count
+   * outside the k+2 bounds): four possible values, tallied as 16-bit fields of one word (a thread
+   * sees few enough slots that no field can wrap) */
+  uint64_t qh = 0;
+  for (uint32_t q0 = 0; q0 < region; q0 += nt) {
+    const uint32_t q = q0 + tid;
+    bool listed = false;
+    if (q < region) {
+      const KT key = KOps<KT>::load(sm + q * SU);
+      if (!key_is_empty(key) && !key_cont(key)) {   /* a continuation belongs to its first slot */
+        /* entries fill in order: the first empty one ends them (most slots hold one or two) */
+        const uint32_t *ew = reinterpret_cast<const uint32_t *>(sm + q * SU + KWD);
+        int ne = 0;
+        uint32_t kf = 0;
+        while (ne < NE && ew[ne] != 0) kf += entry_count(ew[ne++]);
+        kf = min(0xFFFFu, kf);
+        listed = ne == NE || kf >= ca.t[2];
+        if (!listed) {
+          const uint32_t kout = (kf < ca.t[0] || kf >= ca.t[1]) ? 2u : 0u;
+          for (int e = 0; e < ne; ++e) {
+            const uint32_t c16 = min(0xFFFFu, entry_count(ew[e]));
+            qh += 1ull << (16 * (kout | ((c16 < ca.t[4] || c16 >= ca.t[5]) ? 1u : 0u)));
+          }
+        }
+      }
+    }
+    const unsigned m = __ballot_sync(~0u, listed);   /* the loop bound is the same for every lane */
+    unsigned base = 0;
+    if (m && lane == __ffs(m) - 1) base = atomicAdd(&s_nc, (unsigned)__popc(m));
+    if (m) base = __shfl_sync(~0u, base, __ffs(m) - 1);
+    if (q < region) sm[q * SU] = listed ? (uint64_t)(base + __popc(m & ((1u << lane) - 1))) : ~0ull;
+  }
+  #pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const unsigned long long h = warp_sum((qh >> (16 * f)) & 0xFFFFull);
+    if (lane == 0 && h) atomicAdd(&s_qh[f], (unsigned)h);
+  }
+  __syncthreads();
+  if (tid == 0) s_base = s_nc ? atomicAdd(ca.n_cand, (unsigned long long)s_nc) : 0;
+  if (tid < 4 && s_qh[tid]) atomicAdd(&ca.quick_hist[3 + 4 * tid], (unsigned long long)s_qh[tid]);
+  __syncthreads();
+  for (uint32_t q = tid; q < region; q += nt) {
+    const uint64_t o = sm[q * SU];
+    if (o != ~0ull && s_base + o < ca.cap) ca.cand[s_base + o] = (uint32_t)(slot0 + q);
+  }
+}
 
 /* One CTA per partition (blockIdx.x counts the partitions of all samples): clear the slots, count
  * the partition's records into them, write the region back.  Partition j of sample s holds the
@@ -1967,7 +2031,7 @@ __global__ void __launch_bounds__(1024) k_count_local(const uint64_t *recs, cons
     if (rec == 0ull) continue;   /* an unused chunk tail, when the buckets are the partitions */
     const uint64_t h = bucket_hi | (rec >> 5);
     const uint32_t home = (uint32_t)__umul64hi(h << (2 + G.g.pbits), G.g.region);
-    if (!sm_count(sm, sm_base, region, h, (unsigned)(rec & 31), home, slots, entries)) full = true;
+    if (!sm_count(sm, sm_base, region, h, (unsigned)(rec & 31), home, 1u, slots, entries)) full = true;
   }
   __syncthreads();
   ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(table + (G.g.base + j * G.g.region) * 4);
@@ -1981,62 +2045,7 @@ __global__ void __launch_bounds__(1024) k_count_local(const uint64_t *recs, cons
       if (s_tally) atomicAdd(&s_tally[(uint64_t)smp * T_NUM + T_ENTRIES], entries);
     }
   }
-  if (ca.cand) {
-    /* the region is written back: each slot's key word now holds its place in the block's list
-     * (~0: not listed), so the listing needs no shared memory of its own */
-    __shared__ unsigned int s_nc, s_qh[4];
-    __shared__ unsigned long long s_base;
-    if (tid < 4) s_qh[tid] = 0;
-    if (tid == 0) s_nc = 0;
-    __syncthreads();
-    /* a quick drop's entries get flags 3 | 8 (k-mer total outside the k bounds) | 4 (entry count
-     * outside the k+2 bounds): four possible values, tallied as 16-bit fields of one word (at
-     * most 12 slots of 6 entries a thread, so no field can wrap) */
-    uint64_t qh = 0;
-    const int lane = tid & 31;
-    for (uint32_t q0 = 0; q0 < region; q0 += nt) {
-      const uint32_t q = q0 + tid;
-      bool listed = false;
-      if (q < region) {
-        const uint64_t key = sm[q * 4];
-        if (key != KEY_EMPTY && !(key & KEY_CONT)) {   /* a continuation belongs to its first slot */
-          /* entries fill in order: the first empty one ends them (most slots hold one or two) */
-          const uint32_t *ew = reinterpret_cast<const uint32_t *>(sm + q * 4 + 1);
-          int ne = 0;
-          uint32_t kf = 0;
-          while (ne < 6 && ew[ne] != 0) kf += entry_count(ew[ne++]);
-          kf = min(0xFFFFu, kf);
-          listed = ne == 6 || kf >= ca.t[2];
-          if (!listed) {
-            const uint32_t kout = (kf < ca.t[0] || kf >= ca.t[1]) ? 2u : 0u;
-            for (int e = 0; e < ne; ++e) {
-              const uint32_t c16 = min(0xFFFFu, entry_count(ew[e]));
-              qh += 1ull << (16 * (kout | ((c16 < ca.t[4] || c16 >= ca.t[5]) ? 1u : 0u)));
-            }
-          }
-        }
-      }
-      const unsigned m = __ballot_sync(~0u, listed);   /* the loop bound is the same for every lane */
-      unsigned base = 0;
-      if (m && lane == __ffs(m) - 1) base = atomicAdd(&s_nc, (unsigned)__popc(m));
-      if (m) base = __shfl_sync(~0u, base, __ffs(m) - 1);
-      if (q < region) sm[q * 4] = listed ? (uint64_t)(base + __popc(m & ((1u << lane) - 1))) : ~0ull;
-    }
-    #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const unsigned long long h = warp_sum((qh >> (16 * f)) & 0xFFFFull);
-      if (lane == 0 && h) atomicAdd(&s_qh[f], (unsigned)h);
-    }
-    __syncthreads();
-    if (tid == 0) s_base = s_nc ? atomicAdd(ca.n_cand, (unsigned long long)s_nc) : 0;
-    if (tid < 4 && s_qh[tid]) atomicAdd(&ca.quick_hist[3 + 4 * tid], (unsigned long long)s_qh[tid]);
-    __syncthreads();
-    const uint64_t slot0 = G.g.base + j * G.g.region;
-    for (uint32_t q = tid; q < region; q += nt) {
-      const uint64_t o = sm[q * 4];
-      if (o != ~0ull && s_base + o < ca.cap) ca.cand[s_base + o] = (uint32_t)(slot0 + q);
-    }
-  }
+  if (ca.cand) list_slots<KW1>(sm, region, G.g.base + j * G.g.region, ca);
   if (full) atomicOr(&ctr->err, (unsigned long long)DERR_TABLE_FULL);
 }
 
@@ -2184,8 +2193,8 @@ void launch_scatter(const typename ScatterRec<KT>::T *records, const unsigned lo
 /* one record into a 64-byte slot region in shared memory (key 2 words, 12 entry words);
  * false if the region is full */
 __device__ __forceinline__ bool sm_count2(uint64_t *sm, uint32_t sm_base, uint32_t region, uint64_t lo, uint64_t hi,
-                                          unsigned code, uint32_t home, unsigned long long &slot_claims,
-                                          unsigned long long &entry_claims) {
+                                          unsigned code, uint32_t home, uint32_t weight,
+                                          unsigned long long &slot_claims, unsigned long long &entry_claims) {
   bool seen_primary = false;
   uint32_t j = home;
   for (uint32_t probe = 0; probe < region; ++probe) {
@@ -2201,7 +2210,7 @@ __device__ __forceinline__ bool sm_count2(uint64_t *sm, uint32_t sm_base, uint32
     }
     if (k0 == lo && k1 == whi) {   /* the entries, four at a time as far as they are needed */
       seen_primary = true;
-      if (sm_count_entries_lazy<12, 0>((uint32_t *)(sm + (uint64_t)j * 8 + 2), a + 16u, nullptr, code, entry_claims))
+      if (sm_count_entries_lazy<12, 0>((uint32_t *)(sm + (uint64_t)j * 8 + 2), a + 16u, nullptr, code, weight, entry_claims))
         return true;
     }
     j = (j + 1 == region) ? 0u : j + 1;
@@ -2237,7 +2246,7 @@ __global__ void __launch_bounds__(PTPB2, 3) k_count_local2(const unsigned long l
     nxt = i + nt < n ? __ldcs(rp + i + nt) : make_ulonglong2(0ull, 0ull);
     const uint64_t h = bucket_hi | (r.x >> 8);   /* the table key is (h, high word) */
     const uint32_t home = (uint32_t)__umul64hi(h << g.pbits, g.region);
-    if (!sm_count2(sm, sm_base, region, h, r.y, (unsigned)(r.x & 31u), home, slots, entries)) full = true;
+    if (!sm_count2(sm, sm_base, region, h, r.y, (unsigned)(r.x & 31u), home, 1u, slots, entries)) full = true;
   }
   __syncthreads();   /* every record is read: the region's memory is free for the slots */
   ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(reg);
@@ -2248,59 +2257,11 @@ __global__ void __launch_bounds__(PTPB2, 3) k_count_local2(const unsigned long l
     if (slots) atomicAdd(&ctr->n_slots_claimed, slots);
     if (entries) atomicAdd(&ctr->n_entries, entries);
   }
-  if (ca.cand) {   /* as in k_count_local, with 12 entries a slot */
-    __shared__ unsigned int s_nc, s_qh[4];
-    __shared__ unsigned long long s_base;
-    if (tid < 4) s_qh[tid] = 0;
-    if (tid == 0) s_nc = 0;
-    __syncthreads();
-    uint64_t qh = 0;
-    const int lane = tid & 31;
-    for (uint32_t q0 = 0; q0 < region; q0 += nt) {
-      const uint32_t q = q0 + tid;
-      bool listed = false;
-      if (q < region) {
-        const uint64_t k0 = sm[q * 8], k1 = sm[q * 8 + 1];
-        if (!(k0 == KEY_EMPTY && k1 == KEY_EMPTY) && !(k1 & KEY_CONT)) {
-          /* entries fill in order: the first empty one ends them (most slots hold one or two) */
-          const uint32_t *ew = reinterpret_cast<const uint32_t *>(sm + q * 8 + 2);
-          int ne = 0;
-          uint32_t kf = 0;
-          while (ne < 12 && ew[ne] != 0) kf += entry_count(ew[ne++]);
-          kf = min(0xFFFFu, kf);
-          listed = ne == 12 || kf >= ca.t[2];
-          if (!listed) {
-            const uint32_t kout = (kf < ca.t[0] || kf >= ca.t[1]) ? 2u : 0u;
-            for (int e = 0; e < ne; ++e) {
-              const uint32_t c16 = min(0xFFFFu, entry_count(ew[e]));
-              qh += 1ull << (16 * (kout | ((c16 < ca.t[4] || c16 >= ca.t[5]) ? 1u : 0u)));
-            }
-          }
-        }
-      }
-      const unsigned m = __ballot_sync(~0u, listed);   /* the loop bound is the same for every lane */
-      unsigned base = 0;
-      if (m && lane == __ffs(m) - 1) base = atomicAdd(&s_nc, (unsigned)__popc(m));
-      if (m) base = __shfl_sync(~0u, base, __ffs(m) - 1);
-      if (q < region) sm[q * 8] = listed ? (uint64_t)(base + __popc(m & ((1u << lane) - 1))) : ~0ull;
-    }
-    #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const unsigned long long h = warp_sum((qh >> (16 * f)) & 0xFFFFull);
-      if (lane == 0 && h) atomicAdd(&s_qh[f], (unsigned)h);
-    }
-    __syncthreads();
-    if (tid == 0) s_base = s_nc ? atomicAdd(ca.n_cand, (unsigned long long)s_nc) : 0;
-    if (tid < 4 && s_qh[tid]) atomicAdd(&ca.quick_hist[3 + 4 * tid], (unsigned long long)s_qh[tid]);
-    __syncthreads();
-    const uint64_t slot0 = g.base + j * g.region;
-    for (uint32_t q = tid; q < region; q += nt) {
-      const uint64_t o = sm[q * 8];
-      if (o != ~0ull && s_base + o < ca.cap) ca.cand[s_base + o] = (uint32_t)(slot0 + q);
-    }
-  }
+  if (ca.cand) list_slots<KW2>(sm, region, g.base + j * g.region, ca);
   if (full) atomicOr(&ctr->err, (unsigned long long)DERR_TABLE_FULL);
 }
+
+#include "superkmer.cuh"
 
 /* table initialisation: every key word EMPTY, every entry 0; written as one flat word
  * array so that every warp store is 256 contiguous bytes */
@@ -2660,6 +2621,9 @@ namespace {
 bruno_status extract_begin(Ctx *c, uint64_t upper, int max_blocks);
 void extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 int wx_blocks(uint64_t nr);
+bool sk_takes(const Ctx *c);
+bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes);
+void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 }  // namespace
 
 /* Indexes every FASTQ segment.  A segment copied from the host in pieces (load_fastq) is
@@ -2677,7 +2641,8 @@ bruno_status run_index_reads(Ctx *c) {
   if ((st = ensure(c, c->tile_base, std::max<uint64_t>(1, total_tiles) * 8)) != BRUNO_OK) return st;
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
-  c->pre_extracted = piped && c->S == 1 && c->W == 1 && !c->cfg.edge_filter && c->force_direct_count != 1;
+  c->sk_on = sk_takes(c);
+  c->pre_extracted = piped && c->S == 1 && !c->cfg.edge_filter && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
   if (c->pre_extracted) {
@@ -2685,7 +2650,8 @@ bruno_status run_index_reads(Ctx *c) {
      * positions of all reads are at most half the bytes */
     int blocks = 0;   /* one launch a segment, bounded as extract_reads bounds it (8 bytes a read at least) */
     for (auto &sg : c->segs) blocks += wx_blocks(sg.n / 8 + 1);
-    if ((st = extract_begin(c, total_bytes / 2 + 1, std::max(1, blocks))) != BRUNO_OK) return st;
+    if ((st = c->sk_on ? sk_begin(c, {total_bytes}) : extract_begin(c, total_bytes / 2 + 1, std::max(1, blocks))) != BRUNO_OK)
+      return st;
     cudaEventRecord(c->kev[0], c->stream);
   }
   /* the read arrays need the record count first; newline counts give an upper bound */
@@ -2727,7 +2693,8 @@ bruno_status run_index_reads(Ctx *c) {
     if (h.bad_line != ~0ull || (lines & 3) != 0)
       return set_err(c, BRUNO_ERR_BAD_INPUT, "malformed FASTQ in file " + std::to_string(si) + " near line " +
                                                  std::to_string(h.bad_line != ~0ull ? h.bad_line : lines));
-    if (c->pre_extracted) extract_reads(c, rcap, rcap + lines / 4);
+    if (c->pre_extracted && c->sk_on) sk_extract_reads(c, rcap, rcap + lines / 4);
+    else if (c->pre_extracted) extract_reads(c, rcap, rcap + lines / 4);
     if (batch_hook && (st = batch_segment(c, si, rcap, rcap + lines / 4)) != BRUNO_OK) return st;
     rcap += lines / 4;
   }
@@ -2753,13 +2720,14 @@ unsigned zeros_word(const void *p) {
   return z;
 }
 
-/* the HyperLogLog estimate of the k-mers sampled into it (1 in 2^HLL_SAMPLE), scaled back to all */
-double hll_sampled_estimate(double sum, unsigned zeros) {
+/* the HyperLogLog estimate of the k-mers sampled into it (1 in 2^q), scaled back to all */
+double hll_estimate(double sum, unsigned zeros, int q) {
   const double m = HLL_M, alpha = 0.7213 / (1.0 + 1.079 / m);
   double est = alpha * m * m / sum;
   if (est <= 2.5 * m && zeros > 0) est = m * std::log(m / zeros);
-  return est * (double)(1u << HLL_SAMPLE);
+  return est * (double)(1u << q);
 }
+double hll_sampled_estimate(double sum, unsigned zeros) { return hll_estimate(sum, zeros, HLL_SAMPLE); }
 
 /* node and chain lists hold 32-bit slot indices: a table is at most 2^32 - 1 slots (137 GB of
  * 32-byte slots, 275 GB of 64-byte ones) */
@@ -3194,6 +3162,324 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
   return set_err(c, BRUNO_ERR_TABLE_FULL, "k-mer table full after regrowth");
 }
 
+/* ------------------------------------------------ counting by super-k-mers, host side */
+
+/* k from 19: below, windows hold fewer than 5 m-mers and a run is hardly longer than a k-mer's own
+ * record; a forced counting path or table size and the (k+1)-mer filter keep the k-mer records, and
+ * so do builds without thresholds: they keep every k-mer, and 3.5M nodes at 12x (13.7M k-mers,
+ * k = 31) took 3.28 ms by super-k-mers against 3.09 */
+bool sk_takes(const Ctx *c) {
+  return c->S == 1 && c->cfg.k >= MZ_M + 4 && c->cfg.thresholding && !c->cfg.edge_filter && c->force_direct_count == 0 &&
+         c->cfg.table_slots == 0;
+}
+
+constexpr uint64_t SK_EST_CAP = 1ull << 20;   /* records the estimate takes (about 2^17 are listed) */
+
+template <class KT, int BL>
+void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+               unsigned long long *s_inst, unsigned long long *s_used) {
+  constexpr size_t smem = sizeof(SkWarp<SkRec<KT>::NW>) * (SK_TPB / 32);
+  static const int occ = [] {
+    cudaFuncSetAttribute(k_sk_extract<KT, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int o = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sk_extract<KT, BL>, SK_TPB, smem) == cudaSuccess && o > 0
+               ? o : 4;
+  }();
+  const uint64_t most = items ? n_items : (nreads + 31) / 32;   /* a few reads a warp at least */
+  const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * occ, most));
+  SkExtract a{};
+  a.rstart = (const uint64_t *)c->rstart.p;
+  a.rend = (const uint64_t *)c->rend.p;
+  a.r0 = r0;
+  a.r1 = r1;
+  a.items = items;
+  a.n_items = n_items;
+  a.k = c->cfg.k;
+  a.chunk = c->sk_chunk;
+  a.samples = (const SkSample *)c->sk_samp.p;
+  a.out = (uint64_t *)c->sk_recs.p;
+  a.cap = c->sk_cap;
+  a.hist = (unsigned long long *)c->sk_hist.p;
+  a.est = (uint32_t *)c->sk_est.p;
+  a.est_cap = SK_EST_CAP;
+  a.s_inst = s_inst;
+  a.s_used = s_used;
+  a.ctr = c->dctr;
+  k_sk_extract<KT, BL><<<(unsigned)grid, SK_TPB, smem, c->stream>>>(a);
+  c->launches += 1;
+}
+template <class KT>
+void sk_launch_k(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+                 unsigned long long *s_inst, unsigned long long *s_used) {
+  const int w1 = c->cfg.k - MZ_M;   /* the window blocks: the largest that no window fits inside */
+  if (w1 >= 16) sk_launch<KT, 16>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
+  else if (w1 >= 8) sk_launch<KT, 8>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
+  else sk_launch<KT, 4>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
+}
+void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+                unsigned long long *s_inst, unsigned long long *s_used) {
+  if (nreads == 0) return;
+  if (c->W == 1) sk_launch_k<KW1>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
+  else sk_launch<KW2, 16>(c, r0, r1, items, n_items, nreads, s_inst, s_used);   /* k > 31: windows of 18 and more */
+}
+void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, r1 - r0, nullptr, nullptr); }
+
+/* Room for the records of samples of the given FASTQ bytes, their bins and their estimates.  A
+ * read's quality line is as long as its sequence, so k-mer positions are at most half the bytes;
+ * runs start at 2 / (w + 1) of them (w m-mers a window) and at every read, and get a quarter
+ * more; input that needs more (it would have to be unlike any sequence) is counted by k-mer
+ * records.  About 512 k-mers a bin: a partition, some thousands of k-mers, is then made up of
+ * enough bins to even out. */
+bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
+  bruno_status st;
+  const uint32_t S = (uint32_t)bytes.size();
+  const int k = c->cfg.k, w = k - MZ_M + 1;
+  uint64_t total = 0;
+  c->sk_bits.assign(S, 0);
+  c->sk_q.assign(S, 0);
+  for (uint32_t q = 0; q < S; ++q) {
+    total += bytes[q];
+    int b = 11, e = 0;
+    while (b < 21 && (bytes[q] >> 10 >> b)) ++b;
+    while (e < 10 && (bytes[q] >> 21 >> (e + 1))) ++e;   /* a sample of about 2^20 k-mers */
+    c->sk_bits[q] = b;
+    c->sk_q[q] = e;
+  }
+  uint64_t bins = 0;
+  for (;;) {
+    bins = 0;
+    for (uint32_t q = 0; q < S; ++q) bins += 1ull << c->sk_bits[q];
+    if (bins <= 1ull << SK_BIN_BITS) break;
+    for (int &b : c->sk_bits) b = std::max(4, b - 1);   /* 2^14 samples of 2^4 bins still fit */
+  }
+  c->sk_bins = (uint32_t)bins;
+  /* a warp reserves output places by the chunk: an eighth of its share of the records, so that the
+   * last chunks' unused places stay few */
+  const double recs = (double)total * 0.5 * 2.5 / (w + 1);
+  const uint64_t warps = (uint64_t)num_sms() * 64;
+  c->sk_chunk = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, (uint64_t)(recs / (8.0 * warps))));
+  /* one extraction launch a segment, each with chunks of its own */
+  c->sk_cap = (uint64_t)recs + total / (2 * k + 9) + 4096 + warps * c->sk_chunk * std::max<size_t>(1, c->segs.size());
+  const size_t rb = c->W == 1 ? 16 : 32;
+  if ((st = ensure(c, c->sk_recs, c->sk_cap * rb)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_hist, bins * 8)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_est, SK_EST_CAP * 4)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_samp, S * sizeof(SkSample))) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->hllreg, (size_t)S * HLL_M * 4)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->hsum, (size_t)S * 16)) != BRUNO_OK) return st;
+  cudaMemsetAsync(c->sk_hist.p, 0, bins * 8, c->stream);
+  cudaMemsetAsync(c->hllreg.p, 0, (size_t)S * HLL_M * 4, c->stream);
+  std::vector<SkSample> xs(S);
+  uint32_t b0 = 0;
+  for (uint32_t q = 0; q < S; ++q) {
+    xs[q] = SkSample{b0, 32u - (unsigned)c->sk_bits[q], (1u << c->sk_q[q]) - 1, 0u};
+    b0 += 1u << c->sk_bits[q];
+  }
+  return cuda_check(c, cudaMemcpyAsync(c->sk_samp.p, xs.data(), S * sizeof(SkSample), cudaMemcpyHostToDevice, c->stream),
+                    "super-k-mer samples");
+}
+
+template <class KT>
+void sk_estimate(Ctx *c, uint32_t S) {
+  k_sk_estimate<KT><<<num_sms() * 4, 128, 0, c->stream>>>(
+      (const uint64_t *)c->sk_recs.p, (const uint32_t *)c->sk_est.p, SK_EST_CAP, c->cfg.k, (const SkSample *)c->sk_samp.p,
+      S, (unsigned int *)c->hllreg.p, c->dctr);
+  c->launches += 1;
+}
+
+/* bins -> partitions (plan: one a sample), records -> partition order */
+template <class KT>
+bruno_status sk_partition(Ctx *c, const std::vector<SkPlan> &plan, uint32_t parts, uint64_t n_rec) {
+  constexpr int NW = SkRec<KT>::NW;
+  bruno_status st;
+  const uint32_t blocks = (c->sk_bins + SK_PLAN_CHUNK - 1) / SK_PLAN_CHUNK;
+  if ((st = ensure(c, c->sk_plan, plan.size() * sizeof(SkPlan))) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_sums, (size_t)blocks * 16)) != BRUNO_OK) return st;
+  if ((st = cuda_check(c, cudaMemcpyAsync(c->sk_plan.p, plan.data(), plan.size() * sizeof(SkPlan), cudaMemcpyHostToDevice,
+                                          c->stream), "partition plan")) != BRUNO_OK)
+    return st;
+  const unsigned long long *hist = (const unsigned long long *)c->sk_hist.p;
+  k_sk_plan_sum<<<blocks, SK_PLAN_TPB, 0, c->stream>>>(hist, c->sk_bins, (ulonglong2 *)c->sk_sums.p, SK_MAX_BIN, c->dctr);
+  k_sk_plan_apply<<<blocks, SK_PLAN_TPB, 0, c->stream>>>(hist, c->sk_bins, (const ulonglong2 *)c->sk_sums.p,
+                                                         (const SkPlan *)c->sk_plan.p, (uint32_t)plan.size(), parts,
+                                                         (uint32_t *)c->sk_part.p, (uint32_t *)c->sk_off.p,
+                                                         (uint32_t *)c->sk_cur.p);
+  const uint64_t per = 256 * SK_SCATTER_U;
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * 8, (n_rec + per - 1) / per));
+  k_sk_scatter<NW><<<grid, 256, 0, c->stream>>>((const uint64_t *)c->sk_recs.p, n_rec, (const uint32_t *)c->sk_part.p,
+                                                (uint32_t *)c->sk_cur.p, (uint64_t *)c->sk_sorted.p, c->dctr);
+  c->launches += 3;
+  return cuda_check(c, cudaGetLastError(), "super-k-mer partitions");
+}
+
+/* Shared memory of a counting block: k-mer slots twice the expected number of a partition and
+ * some (partitions vary by a fifth; the few that need more are counted again with all there is),
+ * rounds that take a typical partition's records at once. */
+template <class KT>
+struct SkShape {
+  static constexpr size_t MOST = 226u << 10;   /* of the 227 KB a block may have */
+  uint32_t slots, round;
+  size_t bytes;
+  SkShape(double kmers, double records) {
+    slots = ((uint32_t)std::min(8000.0, 2.0 * kmers + 64.0 + 100.0 * (kmers < 400.0)) + 31u) & ~31u;
+    round = std::max(128u, std::min(sizeof(KT) == 8 ? 1024u : 512u, ((uint32_t)(1.15 * records) + 63u) & ~63u));
+    while ((bytes = sk_count_bytes<KT>(slots, round)) > MOST) slots -= 32;
+  }
+};
+template <class KT>
+void sk_count_launch(const Ctx *c, const SkCount &a, uint32_t grid, size_t bytes) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(k_sk_count<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
+    return true;
+  }();
+  (void)attr;
+  /* threads: the block's 384 unless the partitions are small or the configured block is */
+  int nt = std::min(SK_COUNT_TPB, count_threads(c));
+  while (nt > 128 && (uint32_t)nt * 2 > a.slots) nt -= 128;
+  k_sk_count<KT><<<grid, nt, bytes, c->stream>>>(a);
+}
+
+/* The partitions counted (records in partition order), those that overflow their block's slots
+ * once more with as many as fit; ok = false if that does not do either. */
+template <class KT>
+bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const SkShape<KT> &shape, bool &ok) {
+  bruno_status st;
+  a.slots = shape.slots;
+  a.round = shape.round;
+  a.hsize = sk_hash_size(a.round);
+  a.late = sk_late_at<KT>(a.slots, a.round);
+  sk_count_launch<KT>(c, a, parts, shape.bytes);
+  c->launches += 1;
+  if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
+  if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  const uint32_t n = (uint32_t)c->hctr->n_over;
+  if (n && !c->hctr->err) {
+    const SkShape<KT> big(8000.0, shape.round);
+    cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
+    a.todo = a.over;
+    a.over += parts;
+    a.slots = big.slots;
+    a.round = big.round;
+    a.hsize = sk_hash_size(a.round);
+    a.late = sk_late_at<KT>(a.slots, a.round);
+    sk_count_launch<KT>(c, a, n, big.bytes);
+    c->launches += 1;
+    if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  }
+  ok = !c->hctr->err && c->hctr->n_over == 0;
+  return BRUNO_OK;
+}
+
+/* The count of one sample by super-k-mers.  used = false (nothing counted, the caller takes the
+ * k-mer records): a bin too large for one CTA, more records than room, or partitions that overflow
+ * at every size tried. */
+template <class KT>
+bruno_status count_superkmers(Ctx *c, bool &used) {
+  constexpr int NW = SkRec<KT>::NW, SU = Slot<KT>::U64;
+  bruno_status st;
+  used = false;
+  if (!c->pre_extracted) {
+    uint64_t bytes = 0;
+    for (auto &sg : c->segs) bytes += sg.n;
+    cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
+    if ((st = sk_begin(c, {bytes})) != BRUNO_OK) return st;
+    cudaEventRecord(c->kev[0], c->stream);
+    sk_extract_reads(c, 0, c->n_reads);
+  }
+  c->pre_extracted = false;   /* what was extracted serves this path alone */
+  sk_estimate<KT>(c, 1);
+  k_hll_sums<<<1, 256, 0, c->stream>>>((const unsigned int *)c->hllreg.p, (double *)c->hsum.p,
+                                       (unsigned int *)((double *)c->hsum.p + 1));
+  c->launches += 1;
+  cudaEventRecord(c->kev[1], c->stream);
+  double hs[2] = {0, 0};
+  cudaMemcpyAsync(hs, c->hsum.p, 16, cudaMemcpyDeviceToHost, c->stream);
+  if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  const uint64_t n_rec = c->hctr->n_sk, inst = c->hctr->n_instances;
+  if (c->hctr->err || n_rec > c->sk_cap || inst >> 32) return BRUNO_OK;
+  c->n_instances = inst;
+  c->n_reads_used = c->hctr->n_reads_used;
+  double distinct = hll_estimate(hs[0], zeros_word(&hs[1]), c->sk_q[0]);
+  for (int attempt = 0; attempt < 3; ++attempt, distinct *= 2) {
+    const uint64_t slots = slots_for(c, distinct);
+    const bruno_table_plan::Plan plan = bruno_table_plan::partitions(slots, part_slots(c) * 4 / SU, MAX_SPLIT_BITS2);
+    if (!plan.fits) return BRUNO_OK;
+    const uint32_t parts = 1u << plan.pbits;
+    const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
+    /* regions are rounded up by two slots each; the rest as the load asks for */
+    const uint64_t cap = slots + 2ull * parts;
+    if ((st = table_room(c, cap)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->table, cap * SU * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->cand, cap * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_sorted, std::max<uint64_t>(1, n_rec) * NW * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_part, (size_t)c->sk_bins * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_off, ((size_t)parts + 1) * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_cur, (size_t)parts * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_info, (size_t)parts * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_over, (size_t)parts * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_bump, 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sgeom, sizeof(SGeom))) != BRUNO_OK) return st;
+    c->geom = TableGeom{cap, 0, plan.pbits, 0, (const uint32_t *)c->sk_part.p, (const uint2 *)c->sk_info.p, 0u,
+                        32 - c->sk_bits[0], c->cfg.k};
+    const SGeom sg{c->geom, 0, 0, 0};
+    cudaMemcpyAsync(c->sgeom.p, &sg, sizeof(sg), cudaMemcpyHostToDevice, c->stream);
+    cudaMemsetAsync(c->sk_bump.p, 0, 8, c->stream);
+    cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
+    cudaMemsetAsync(&c->dctr->n_cand, 0, sizeof(c->dctr->n_cand) + sizeof(c->dctr->quick_hist), c->stream);
+    cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
+    cudaMemsetAsync(&c->dctr->n_slots_claimed, 0, 16, c->stream);
+    cudaMemsetAsync(&c->dctr->n_big, 0, 8, c->stream);
+    cudaEventRecord(c->kev[2], c->stream);
+    if ((st = sk_partition<KT>(c, {SkPlan{0ull, std::max<uint64_t>(1, (inst + parts - 1) / parts), 0u, 0u, parts, 0u}}, parts,
+                               n_rec)) != BRUNO_OK)
+      return st;
+    cudaEventRecord(c->kev[4], c->stream);
+    SkCount a{};
+    a.recs = (const uint64_t *)c->sk_sorted.p;
+    a.off = (const uint32_t *)c->sk_off.p;
+    a.k = c->cfg.k;
+    a.keep_all = !(c->one_call && c->cfg.thresholding && !c->cfg.keep_k2);
+    a.thresholding = c->cfg.thresholding;
+    for (int i = 0; i < 6; ++i) a.t[i] = (uint32_t)std::min<uint64_t>(65536, c->cfg.thresh[i]);
+    a.inv_load = inv_load;
+    a.table = (uint64_t *)c->table.p;
+    a.info = (uint2 *)c->sk_info.p;
+    a.over = (uint32_t *)c->sk_over.p;
+    a.cand = (uint32_t *)c->cand.p;
+    a.sg = (const SGeom *)c->sgeom.p;
+    a.nsamples = 1;
+    a.bump = (unsigned long long *)c->sk_bump.p;
+    a.ctr = c->dctr;
+    bool ok = false;
+    if ((st = sk_count_parts<KT>(c, a, parts, SkShape<KT>(distinct * 1.04 / parts, (double)n_rec / parts), ok)) != BRUNO_OK)
+      return st;
+    cudaEventRecord(c->kev[3], c->stream);
+    if (c->hctr->err & DERR_SKEW) return BRUNO_OK;
+    if (ok) {
+      uint64_t used_slots = 0;
+      cudaMemcpyAsync(&used_slots, c->sk_bump.p, 8, cudaMemcpyDeviceToHost, c->stream);
+      if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "table slots")) != BRUNO_OK) return st;
+      c->nslots = c->geom.nslots = used_slots;
+      float ms[3] = {0, 0, 0};
+      cudaEventElapsedTime(&ms[0], c->kev[0], c->kev[1]);
+      cudaEventElapsedTime(&ms[1], c->kev[2], c->kev[4]);
+      cudaEventElapsedTime(&ms[2], c->kev[2], c->kev[3]);
+      c->phase_ms[6] = ms[0];
+      c->phase_ms[7] = 0;
+      c->phase_ms[8] = ms[2];
+      c->phase_ms[9] = ms[1];
+      c->n_entries = c->hctr->n_entries;
+      c->n_slots_claimed = c->hctr->n_slots_claimed;
+      c->have_cand = true;
+      take_candidates(c);
+      used = true;
+      return BRUNO_OK;
+    }
+  }
+  return BRUNO_OK;
+}
+
 /* The partitioned count for k > 31: exact k-mer positions size 256 buckets of 16-byte records,
  * one extraction fills them (with the distinct estimate), and per attempt the records are
  * scattered into the table's partitions and counted in shared memory.  used = false sends the
@@ -3401,6 +3687,12 @@ bruno_status count_paths(Ctx *c) {
     if ((st = count_partitioned(c, used)) != BRUNO_OK) return st;
     return used ? BRUNO_OK : set_err(c, BRUNO_ERR_TABLE_FULL, "a hash bucket overflowed under the (k+1)-mer filter");
   }
+  if (c->sk_on) {
+    bool used = false;
+    bruno_status st = count_superkmers<KT>(c, used);
+    if (st != BRUNO_OK || used) return st;
+    c->have_cand = false;
+  }
   if (sizeof(KT) == 8 && c->force_direct_count != 1) {
     bool used = false;
     bruno_status st = count_partitioned(c, used);
@@ -3485,8 +3777,8 @@ bruno_status filter_typed(Ctx *c, const uint64_t *thr) {
   /* the count listed the slots that need the full filter (same thresholds): read only those,
    * and add the quick drops the count tallied */
   /* (at most one listed slot a slot: a count past the table's slots would mean a lost list) */
-  const bool use_cand = c->have_cand && c->n_cand <= c->nslots && a.thresholding &&
-                        std::equal(thr, thr + 6, c->cfg.thresh);
+  const bool use_cand = c->have_cand && c->n_cand <= c->nslots &&
+                        (!a.thresholding || std::equal(thr, thr + 6, c->cfg.thresh));
   if (use_cand) {
     a.cand = (const uint32_t *)c->cand.p;
     a.n_cand = c->n_cand;

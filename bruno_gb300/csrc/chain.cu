@@ -111,7 +111,7 @@ __device__ __forceinline__ long long table_find(const uint64_t *table, const Tab
                                                 KT kmer) {
   constexpr int SU = Slot<KT>::U64;
   const KT bare = table_key(kmer), x = as_node(bare);
-  Probe pr(g, table_home(g, bare));
+  Probe pr = table_probe(g, kmer, bare);
   for (uint32_t p = 0; p < max_probe; ++p, pr.next()) {
     const uint64_t *s = table + pr.i * SU;
     KT key = KOps<KT>::load(s);
@@ -123,10 +123,12 @@ __device__ __forceinline__ long long table_find(const uint64_t *table, const Tab
 }
 
 /* Two lookups in lockstep: both first probes are in flight together, and each probe reads
- * the whole slot (key, counters, flags, aux) in 32-byte loads.  found = slot index or -1. */
+ * the whole slot (key, counters, flags, aux) in 32-byte loads.  mz: the k-mers' minimizers, where
+ * the table needs them.  found = slot index or -1.  Every lane of the
+ * warp calls it: the probe loop is the warp's, so that its lanes stay together. */
 template <class KT>
 __device__ __forceinline__ void table_find2(const uint64_t *table, const TableGeom &g, uint32_t max_probe,
-                                            const KT *want, const bool *has, long long *found,
+                                            const KT *want, const uint32_t *mz, const bool *has, long long *found,
                                             uint64_t (*raw)[Slot<KT>::U64]) {
   constexpr int SU = Slot<KT>::U64;
   KT x[2];
@@ -138,20 +140,21 @@ __device__ __forceinline__ void table_find2(const uint64_t *table, const TableGe
     done[q] = !has[q];
     const KT bare = table_key(want[q]);
     x[q] = as_node(bare);
-    const Probe pr(g, table_home(g, bare));
+    const Probe pr = g.bins ? bin_probe(g, mz[q], bare) : Probe(g, table_home(g, bare));
     pos[q] = pr.i; lo[q] = pr.lo; hi[q] = pr.hi;
   }
-  for (uint32_t p = 0; p < max_probe && !(done[0] && done[1]); ++p) {
+  for (uint32_t p = 0; p < max_probe && __any_sync(~0u, !(done[0] && done[1])); ++p) {
     #pragma unroll
     for (int q = 0; q < 2; ++q)
       if (!done[q]) ld_slot<SU>(table + pos[q] * SU, raw[q]);
     #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      if (done[q]) continue;
-      const KT key = KOps<KT>::load(raw[q]);
-      if (KOps<KT>::eq(key, x[q])) { found[q] = (long long)pos[q]; done[q] = true; }
-      else if (key_is_empty(key)) done[q] = true;
-      else if (++pos[q] == hi[q]) pos[q] = lo[q];
+      if (!done[q]) {
+        const KT key = KOps<KT>::load(raw[q]);
+        if (KOps<KT>::eq(key, x[q])) { found[q] = (long long)pos[q]; done[q] = true; }
+        else if (key_is_empty(key)) done[q] = true;
+        else if (++pos[q] == hi[q]) pos[q] = lo[q];
+      }
     }
   }
 }
@@ -166,8 +169,10 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
                                                      ChainState *cs, uint8_t *cedge, uint32_t *csample,
                                                      uint32_t max_probe, DevCounters *ctr) {
   constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t sl = chain_list[i];
+  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < M; i0 += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = i0 + threadIdx.x;
+    const bool live = i < M;   /* the last warps' other lanes go along with slot 0 and write nothing */
+    uint64_t sl = live ? chain_list[i] : 0;
     if (sl >= nslots) {   /* a list entry that was never written: report, never dereference */
       atomicOr(&ctr->err, (unsigned long long)DERR_INVARIANT);
       sl = 0;
@@ -178,10 +183,10 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
     if (nsamples > 1) {   /* a batch: the node's sample (in its flags) has its own partitions */
       const uint32_t smp = (uint32_t)(own[KWD + 2] >> (16 + NF_SAMPLE_SHIFT)) & (MAX_SAMPLES - 1);
       g = sg[smp < nsamples ? smp : 0].g;
-      csample[i] = smp;
+      if (live) csample[i] = smp;
     }
     const KT K = key_kmer(node_key(KOps<KT>::load(own)));
-    KOps<KT>::store(ckey + i * KWD, K);
+    if (live) KOps<KT>::store(ckey + i * KWD, K);
     const uint64_t *pw = own + KWD;
     int inc = -1, outc = -1;
     for (int c = 0; c < 4; ++c) {
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
     }
     /* in neighbour nextReverseFromChar(c), out neighbour nextFromChar(c), canonical */
     KT want[2];
-    bool has[2] = {inc >= 0, outc >= 0}, flip[2] = {false, false};
+    bool has[2] = {live && inc >= 0, live && outc >= 0}, flip[2] = {false, false};
     #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const KT n = q == 0 ? KOps<KT>::prepend((unsigned)max(inc, 0), K, k) : KOps<KT>::append(K, (unsigned)max(outc, 0), k);
@@ -198,9 +203,11 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
       flip[q] = !KOps<KT>::lt(n, y);
       want[q] = flip[q] ? y : n;
     }
+    uint32_t mz[2] = {0, 0};
+    if (g.bins) neighbour_minimizers<KT>(K, k, (unsigned)max(inc, 0), (unsigned)max(outc, 0), mz);
     long long found[2];
     uint64_t raw[2][SU];
-    table_find2<KT>(table, g, max_probe, want, has, found, raw);
+    table_find2<KT>(table, g, max_probe, want, mz, has, found, raw);
     ChainState st;
     st.pad = 0;
     #pragma unroll
@@ -217,6 +224,7 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
       }
       if (q == 0) { st.inP = P; st.inD = D; } else { st.outP = P; st.outD = D; }
     }
+    if (!live) continue;
     cs[i] = st;
     cedge[i] = (uint8_t)((inc >= 0 ? (4 | inc) : 0) | (outc >= 0 ? (32 | (outc << 3)) : 0));
   }

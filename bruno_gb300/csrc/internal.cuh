@@ -19,6 +19,7 @@ constexpr uint32_t DERR_TABLE_FULL = 1u;
 constexpr uint32_t DERR_BAD_INPUT = 2u;
 constexpr uint32_t DERR_INVARIANT = 4u;
 constexpr uint32_t DERR_UNCLEAN_CHAINS = 8u;
+constexpr uint32_t DERR_SKEW = 16u;   /* a minimizer bin the super-k-mer count does not take */
 
 /* Small counters written by kernels, read back by the host between phases. */
 struct DevCounters {
@@ -40,6 +41,8 @@ struct DevCounters {
    * nodes and live branch nodes after an erasure pass */
   unsigned long long cl_term, cl_nonzero, cl_sum, cl_norm, cl_q, cl_found, cl_dead, cl_bub, cl_live, cl_live_branch;
   unsigned long long n_big, n_big_res; /* entries counted past 2^24 (keys in big_key), resolved */
+  unsigned long long n_sk, n_sk_est;   /* super-k-mer record places taken, records listed for the estimate */
+  unsigned long long n_over;           /* partitions whose k-mers overflowed their CTA's slots */
   unsigned long long n_cand;           /* slots the count listed for the filter */
   unsigned long long quick_hist[16];   /* the filter flags of the entries the count dropped */
   unsigned int hll[1 << 12];           /* HyperLogLog registers, p = 12 */
@@ -152,6 +155,16 @@ struct Ctx {
   std::vector<uint64_t> h_rank0, h_head0;  /* first listranked node / chain of each sample (S + 1) */
   std::vector<uint64_t> h_iter;            /* ranking rounds per sample */
   Buf records2, sub_cnt;         /* the same records split per table partition */
+  /* counting by super-k-mers (superkmer.cuh): records as extracted and in partition order, the
+   * minimizer bins' tallies and partitions, the partitions' first records and cursors */
+  Buf sk_recs, sk_sorted, sk_hist, sk_part, sk_off, sk_cur, sk_samp, sk_plan, sk_sums, sk_info, sk_over, sk_bump, sk_est;
+  bool sk_on = false;            /* this build extracts super-k-mers */
+  /* one call builds the whole graph: the thresholds of the configuration are the ones the filter
+   * will use and nobody asks for raw counts, so the count need not keep what the filter drops */
+  bool one_call = false;
+  uint64_t sk_cap = 0;
+  uint32_t sk_bins = 0, sk_chunk = 32;
+  std::vector<int> sk_bits, sk_q; /* per sample: log2 of its bins, of its estimate's sampling */
   bool h2d_pending = false;      /* ev[7] marks the start of the current graph build's host-to-device copies */
   int force_direct_count = 0;    /* cfg.direct_count: 0 automatic, 1 whole table, 2 L2 partitions */
   Buf chain_list, branch_list;   /* slot indices, filled by the filter */

@@ -215,6 +215,13 @@ struct TableGeom {
   uint64_t region;
   int pbits;
   uint64_t base;     /* first slot: a sample's table in a batch of samples starts here (0 otherwise) */
+  /* tables filled by super-k-mers (superkmer.cuh): a k-mer's partition comes from its minimizer,
+   * P = bins[bin0 + (mz_mix(minimizer) >> bin_shift)], and holds info[P].y slots from info[P].x on;
+   * bins == NULL: the partition is the top pbits bits of the key's mix, `region` slots each */
+  const uint32_t *bins = nullptr;
+  const uint2 *info = nullptr;
+  uint32_t bin0 = 0;
+  int bin_shift = 0, k = 0;
 };
 
 /* The table stores a key derived from the canonical k-mer, so that counting records never
@@ -225,6 +232,87 @@ __device__ __forceinline__ KW1 table_key(KW1 x) { return {bj_fwd(x.v)}; }
 __device__ __forceinline__ KW2 table_key(KW2 x) { return {KOps<KW2>::hash(x), x.hi}; }
 __device__ __forceinline__ KW1 key_kmer(KW1 t) { return {bj_inv(t.v)}; }
 __device__ __forceinline__ KW2 key_kmer(KW2 t) { return {kw2_lo(t.hi, t.lo), t.hi}; }
+
+/* ---------------------------------------------------------------- minimizers
+ * The minimizer of a k-mer (Roberts et al., Bioinformatics 20, 2004) is the smallest of its
+ * MZ_M-mers in a fixed order, here a 32-bit mix of the canonical MZ_M-mer, so a k-mer and its
+ * reverse complement have the same one.  MZ_M is odd, so no MZ_M-mer is its own reverse
+ * complement and the order's lowest bit can carry the strand that was the canonical one.  15
+ * bases: the longest odd length whose packed form, canonical choice and mix stay in one 32-bit
+ * register; 4^15 / 2 canonical values keep one value from serving many places of a genome. */
+constexpr int MZ_M = 15;
+constexpr uint32_t MZ_MASK = (1u << (2 * MZ_M)) - 1;
+/* order of an MZ_M-mer from its packed form and its reverse complement's (lowest bit: strand) */
+__device__ __forceinline__ uint32_t mz_order(uint32_t fwd, uint32_t rev) {
+  uint32_t h = (min(fwd, rev) ^ 0x2C9277B5u) * 0x9E3779B1u;
+  h ^= h >> 15;
+  h *= 0x85EBCA6Bu;
+  return (h & ~1u) | (rev < fwd ? 1u : 0u);
+}
+/* a minimizer's bin bits (uniform in the top bits; minimizers themselves crowd the low end) */
+__device__ __forceinline__ uint32_t mz_mix(uint32_t v) {
+  v >>= 1;
+  v *= 0xC2B2AE35u;
+  v ^= v >> 15;
+  v *= 0x27D4EB2Fu;
+  return v ^ (v >> 16);
+}
+__device__ __forceinline__ uint32_t kmer_minimizer(KW1 x, int k) {
+  uint64_t f = x.v, r = KOps<KW1>::rc(x, k).v << (64 - 2 * k);
+  uint32_t best = ~0u;
+  for (int i = k - MZ_M; i >= 0; --i, f >>= 2, r <<= 2)
+    best = min(best, mz_order((uint32_t)f & MZ_MASK, (uint32_t)(r >> (64 - 2 * MZ_M))));
+  return best;
+}
+__device__ __forceinline__ uint32_t kmer_minimizer(KW2 x, int k) {
+  KW2 f = x, r = KOps<KW2>::rc(x, k);
+  const int s = 128 - 2 * k;   /* the reverse complement, first base in the top bits */
+  r = s >= 64 ? KW2{0, r.lo << (s - 64)} : KW2{r.lo << s, (r.hi << s) | (s ? r.lo >> (64 - s) : 0)};
+  uint32_t best = ~0u;
+  for (int i = k - MZ_M; i >= 0; --i) {
+    best = min(best, mz_order((uint32_t)f.lo & MZ_MASK, (uint32_t)(r.hi >> (64 - 2 * MZ_M))));
+    f = {(f.lo >> 2) | (f.hi << 62), f.hi >> 2};
+    r = {r.lo << 2, (r.hi << 2) | (r.lo >> 62)};
+  }
+  return best;
+}
+/* The minimizers of a k-mer's in neighbour (base cin before it) and out neighbour (cout after it):
+ * each shares all its MZ_M-mers but one with the k-mer, so both come from one pass over them. */
+template <class KT>
+__device__ __forceinline__ void neighbour_minimizers(KT x, int k, unsigned cin, unsigned cout, uint32_t *mz) {
+  constexpr int W = KOps<KT>::WORDS;
+  KT f = x, r = KOps<KT>::rc(x, k);
+  const uint32_t r_first = (uint32_t)((const uint64_t *)&r)[0] & MZ_MASK;   /* the first m-mer's complement ends r */
+  uint64_t rt[W];   /* r, its first base in the top bits, high word first */
+  if constexpr (W == 1) {
+    rt[0] = r.v << (64 - 2 * k);
+  } else {
+    const int s = 128 - 2 * k;
+    rt[0] = s >= 64 ? r.lo << (s - 64) : (r.hi << s) | (s ? r.lo >> (64 - s) : 0);
+    rt[1] = s >= 64 ? 0 : r.lo << s;
+  }
+  uint32_t o = 0, in = ~0u, out = ~0u, f_last = 0, r_last = 0, fl = 0;
+  const int w1 = k - MZ_M;
+  for (int i = 0; i <= w1; ++i) {   /* from the last m-mer to the first */
+    fl = (uint32_t)((const uint64_t *)&f)[0] & MZ_MASK;
+    const uint32_t rl = (uint32_t)(rt[0] >> (64 - 2 * MZ_M));
+    o = mz_order(fl, rl);
+    if (i == 0) { f_last = fl; r_last = rl; }
+    else in = min(in, o);
+    if (i < w1) out = min(out, o);
+    if constexpr (W == 1) { f.v >>= 2; rt[0] <<= 2; }
+    else {
+      f = {(f.lo >> 2) | (f.hi << 62), f.hi >> 2};
+      rt[0] = (rt[0] << 2) | (rt[1] >> 62);
+      rt[1] <<= 2;
+    }
+  }
+  mz[0] = min(in, mz_order((fl >> 2) | (cin << (2 * MZ_M - 2)), ((r_first << 2) | (3u - cin)) & MZ_MASK));
+  mz[1] = min(out, mz_order(((f_last << 2) | cout) & MZ_MASK, (r_last >> 2) | ((3u - cout) << (2 * MZ_M - 2))));
+}
+/* a key's place in such a partition: the mix's bits are all free there */
+__device__ __forceinline__ uint32_t bin_home(KW1 t, uint32_t region) { return __umulhi((uint32_t)(t.v >> 30), region); }
+__device__ __forceinline__ uint32_t bin_home(KW2 t, uint32_t region) { return __umulhi((uint32_t)(t.lo >> 32), region); }
 
 /* home slot of a table key */
 __device__ __forceinline__ uint64_t table_home(const TableGeom &g, KW1 t) {
@@ -245,8 +333,20 @@ struct Probe {
     lo = part_lo != ~0ull ? part_lo : (g.pbits ? g.base + ((start - g.base) / g.region) * g.region : g.base);
     hi = lo + g.region;
   }
+  __device__ __forceinline__ Probe(uint64_t first, uint32_t slots, uint32_t at) : i(first + at), lo(first), hi(first + slots) {}
   __device__ __forceinline__ void next() { if (++i == hi) i = lo; }
 };
+/* the probe sequence of a table key with the given minimizer in a table filled by super-k-mers */
+template <class KT>
+__device__ __forceinline__ Probe bin_probe(const TableGeom &g, uint32_t minimizer, KT t) {
+  const uint2 r = __ldg(g.info + __ldg(g.bins + g.bin0 + (mz_mix(minimizer) >> g.bin_shift)));
+  return Probe((uint64_t)r.x, r.y, bin_home(t, r.y));
+}
+/* the probe sequence of canonical k-mer x, whose table key is t */
+template <class KT>
+__device__ __forceinline__ Probe table_probe(const TableGeom &g, KT x, KT t) {
+  return g.bins ? bin_probe(g, kmer_minimizer(x, g.k), t) : Probe(g, table_home(g, t));
+}
 
 /* ---------------------------------------------------------------- table slots */
 template <class KT> struct Slot;

@@ -1,0 +1,1048 @@
+/*
+ * superkmer.cuh -- counting by super-k-mers.
+ *
+ * Consecutive k-mers of a read mostly share their minimizer (kmer.cuh), so a read falls into
+ * runs of k-mers with one minimizer, super-k-mers (Li et al., "Memory efficient minimum
+ * substring partitioning", VLDB 2013; Deorowicz et al., KMC 2, Bioinformatics 31, 2015).  A
+ * run of n k-mers is one record of n + k - 1 bases, the base before it and the base after it,
+ * instead of n records of one k-mer each; every occurrence of a k-mer lands in the partition
+ * of its minimizer.
+ *
+ *   k_sk_extract   reads -> records, unordered, with the records and k-mers of every minimizer
+ *                  bin tallied
+ *   k_sk_estimate  a sample of the minimizers' k-mers -> HyperLogLog registers
+ *   k_sk_plan_*    bins -> partitions of about equal k-mer counts (neighbouring bins share one)
+ *   k_sk_scatter   records -> partition order
+ *   k_sk_count     one CTA a partition: equal records merged into one with a weight, their
+ *                  k-mers counted in shared memory, the k-mers to keep written to the table
+ *
+ * Included by build.cu only, after its helpers (warp_sum, sm_cas128, CandArgs, ...).
+ */
+#pragma once
+
+/* A record: NW 64-bit words, bases from the top of word 0, two bits each: the base before the
+ * first k-mer (0 without one), the n + k - 1 bases of the k-mers, the base after the last (0
+ * without one).  At most k - MZ_M + 1 k-mers share one occurrence of a minimizer, so 2k - 13 bases
+ * (49 for k = 31, 113 for k = 63) leave the last word's low 30 bits for
+ * [bin:22 | has right:1 | has left:1 | n - 1:6].  The record is on the strand its minimizer is
+ * canonical on, so both strands of a place give the same record. */
+template <class KT> struct SkRec;
+template <> struct SkRec<KW1> { static constexpr int NW = 2; };
+template <> struct SkRec<KW2> { static constexpr int NW = 4; };
+constexpr uint64_t SK_LEFT = 1ull << 6, SK_RIGHT = 1ull << 7;
+constexpr int SK_BIN_SHIFT = 8, SK_BIN_BITS = 22;
+constexpr uint64_t SK_BIN_MASK = (1ull << SK_BIN_BITS) - 1;
+__device__ __forceinline__ unsigned sk_n(uint64_t last) { return (unsigned)(last & 63u) + 1u; }
+
+/* a sample's minimizer bins: bin0 + (mz_mix >> shift); the k-mers of records whose mix has no
+ * bit of smask feed the estimate */
+struct SkSample { unsigned int bin0, shift, smask, pad; };
+
+constexpr int SK_TPB = 256;      /* extraction: 8 warps a block, each on its own tiles */
+constexpr int SK_WORDS = 32;     /* a tile: one word of 16 bases a lane */
+constexpr int SK_HALO = 4;       /* words past the tile that a window of 49 m-mers may touch */
+constexpr int SK_READS = 16;     /* reads of a tile at most (the shortest that count take two words) */
+
+template <int NW>
+struct SkWarp {
+  uint32_t pmin[16][SK_WORDS + SK_HALO];     /* prefix minima inside blocks; then the runs' minimizers */
+  uint32_t bases[1 + SK_WORDS + 2 * NW + 3]; /* 16 bases a word, first base on top; word t at t + 1 */
+  uint32_t marks[SK_WORDS + 1];              /* bit i: a run starts, or the read's k-mers end, at base i */
+  uint16_t starts[16 * SK_WORDS];            /* run starts of the tile */
+  unsigned long long addr[SK_READS];
+  int len[SK_READS], nk[SK_READS];           /* bases, k-mers */
+};
+
+/* bases (j >= 0) of a record */
+template <int NW>
+__device__ __forceinline__ unsigned sk_base(const uint64_t *w, int j) {
+  return (unsigned)(w[j >> 5] >> (62 - 2 * (j & 31))) & 3u;
+}
+
+/* the n bases (1..16) at device address s, packed from the top; .y nonzero: one is not A, C, G, T */
+__device__ __forceinline__ uint2 sk_pack(uintptr_t s, int n) {
+  const uintptr_t e = s + n, s4 = s & ~(uintptr_t)3;
+  uint32_t v[5];
+  #pragma unroll
+  for (int q = 0; q < 5; ++q) v[q] = s4 + 4 * q < e ? __ldg((const uint32_t *)(s4 + 4 * q)) : 0u;
+  const unsigned sh = 8u * (unsigned)(s & 3);
+  uint32_t packed = 0, err = 0;
+  #pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t w = __funnelshift_r(v[q], v[q + 1], sh);
+    const uint32_t c = ((w >> 1) ^ (w >> 2)) & 0x03030303u;   /* A0 C1 G2 T3, either case */
+    /* the four codes as selector nibbles give back the letters they stand for */
+    const uint32_t y = c | (c >> 4);
+    const uint32_t want = __byte_perm(0x54474341u, 0u, (y & 0xFFu) | ((y >> 8) & 0xFF00u));
+    uint32_t d = (w & 0xDFDFDFDFu) ^ want;
+    const int left = n - 4 * q;   /* bytes of the read in this word */
+    if (left < 4) d &= left <= 0 ? 0u : (1u << (8 * left)) - 1;
+    err |= d;
+    packed = (packed << 8) | ((c * 0x40100401u) >> 24);
+  }
+  return make_uint2(packed, err);
+}
+
+/* left shift of an NW-word number (word 0 the most significant) by s < 64 * NW bits */
+template <int NW>
+__device__ __forceinline__ void sk_shl(uint64_t *w, unsigned s) {
+  if (NW == 4 && (s & 128u)) { w[0] = w[2]; w[1] = w[3]; w[2] = 0; w[3] = 0; }
+  if (s & 64u) {
+    #pragma unroll
+    for (int i = 0; i < NW - 1; ++i) w[i] = w[i + 1];
+    w[NW - 1] = 0;
+  }
+  const unsigned r = s & 63u;
+  if (r) {
+    #pragma unroll
+    for (int i = 0; i < NW - 1; ++i) w[i] = (w[i] << r) | (w[i + 1] >> (64 - r));
+    w[NW - 1] <<= r;
+  }
+}
+/* the top `bits` bits of word i of an NW-word number kept by a mask of the top `n` bits overall */
+__device__ __forceinline__ uint64_t sk_top_mask(int n, int i) {
+  const int b = n - 64 * i;
+  return b <= 0 ? 0ull : b >= 64 ? ~0ull : ~0ull << (64 - b);
+}
+
+/* no record: the unused end of a chunk that a warp reserved (n - 1 is at most 48) */
+constexpr uint64_t SK_NONE = 63;
+
+/* HyperLogLog registers fed with the k-mers of the records listed; registers are read before they
+ * are raised, since most updates raise nothing */
+template <class KT>
+__global__ void __launch_bounds__(128) k_sk_estimate(const uint64_t *recs, const uint32_t *list, uint64_t cap, int k,
+                                                     const SkSample *samples, uint32_t S, unsigned int *hll,
+                                                     const DevCounters *ctr) {
+  constexpr int NW = SkRec<KT>::NW;
+  const uint64_t n_list = min((unsigned long long)cap, ctr->n_sk_est);
+  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n_list; x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t *rec = recs + (uint64_t)list[x] * NW;
+    const uint64_t last = rec[NW - 1];
+    const uint32_t bin = (uint32_t)((last >> SK_BIN_SHIFT) & SK_BIN_MASK);
+    uint32_t lo = 0, hi = S;
+    while (hi - lo > 1) { const uint32_t m = (lo + hi) >> 1; if (samples[m].bin0 <= bin) lo = m; else hi = m; }
+    unsigned int *reg = hll + (uint64_t)lo * HLL_M;
+    const int n = (int)sk_n(last);
+    KT f{}, r{};
+    for (int j = 1; j < n + k; ++j) {
+      const unsigned c = sk_base<NW>(rec, j);
+      f = KOps<KT>::append(f, c, k);
+      r = KOps<KT>::prepend(3u - c, r, k);
+      if (j < k) continue;
+      const KT t = table_key(KOps<KT>::lt(f, r) ? f : r);
+      const uint64_t h = sizeof(KT) == 8 ? ((const uint64_t *)&t)[0] << 2 : ((const uint64_t *)&t)[0];
+      const unsigned idx = (unsigned)(h >> (64 - HLL_P));
+      const unsigned rho = (unsigned)__clzll((h << HLL_P) | (1ull << (HLL_P - 1))) + 1u;
+      if (rho > *(volatile unsigned int *)&reg[idx]) atomicMax(&reg[idx], rho);
+    }
+  }
+}
+
+struct SkExtract {
+  const uint64_t *rstart, *rend;
+  uint64_t r0, r1;                  /* reads, when there are no items */
+  const XItem *items;
+  uint64_t n_items;
+  int k;
+  uint32_t chunk;                   /* output records a warp reserves at once */
+  const SkSample *samples;
+  uint64_t *out;
+  uint64_t cap;
+  unsigned long long *hist;         /* per bin: k-mers << 32 | records */
+  uint32_t *est;                    /* records for the estimate */
+  uint64_t est_cap;
+  unsigned long long *s_inst, *s_used;
+  DevCounters *ctr;
+};
+
+/* Reads -> records.  A warp takes tiles of whole reads, 32 words of 16 bases at most (of a longer
+ * read, a piece whose k-mers fit).  Each lane packs one word (a read with a base other than A, C,
+ * G, T is dropped), orders the 16 m-mers that start in it, and finds the minimum of every window
+ * of k - MZ_M + 1 m-mers from block prefix and suffix minima (van Herk 1992): a window that starts
+ * in block a and ends in block b is a's suffix from the start, the whole blocks between, and b's
+ * prefix up to the end.  BL (16, 8 or 4) is the block, at most k - MZ_M, so that no window lies
+ * inside one block.  Where the minimum changes a run starts; the tile's runs are listed, and each
+ * lane builds the records of every 32nd run from the packed words.  Everything stays inside the
+ * warp: with one tile a block of 256 threads the block's barriers cost half its time (6.4 ms at
+ * 1.2G k-mers).  Output places come in chunks that a warp reserves (one counter cannot take an
+ * atomic per tile); a chunk's unused end is marked SK_NONE. */
+template <class KT, int BL>
+__global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
+  constexpr int NW = SkRec<KT>::NW, NB = 16 / BL;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SkWarp<NW> &S = reinterpret_cast<SkWarp<NW> *>(smem_raw)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, k = a.k;
+  const unsigned le = ~0u >> (31 - lane);   /* this lane and the ones below */
+  const int w1 = k - MZ_M;                  /* a window's last m-mer, from its first */
+  const int cw = w1 % BL, qw = w1 / BL;
+  const int piece = (16 * SK_WORDS - k - 1) & ~15;   /* k-mers of a long read's piece */
+  for (int i = lane; i < 16 * SK_HALO; i += 32) S.pmin[i / SK_HALO][SK_WORDS + i % SK_HALO] = ~0u;
+  if (lane == 0) S.marks[SK_WORDS] = 0;
+  const uint64_t warp = (uint64_t)blockIdx.x * (SK_TPB / 32) + (threadIdx.x >> 5), warps = (uint64_t)gridDim.x * (SK_TPB / 32);
+  unsigned long long inst_all = 0, used_all = 0;
+  unsigned long long cpos = 0, cend = 0;   /* the warp's chunk of the output */
+  bool over = false;
+  /* items of one sample each, or (one sample) an even share of the reads */
+  const uint64_t it0 = a.items ? warp * a.n_items / warps : 0, it1 = a.items ? (warp + 1) * a.n_items / warps : 1;
+  for (uint64_t it = it0; it < it1; ++it) {
+    uint64_t ra, rb;
+    unsigned smp = 0;
+    if (a.items) { ra = a.items[it].a; rb = a.items[it].b; smp = a.items[it].s; }
+    else { ra = a.r0 + (a.r1 - a.r0) * warp / warps; rb = a.r0 + (a.r1 - a.r0) * (warp + 1) / warps; }
+    const SkSample X = a.samples[smp];
+    unsigned inst = 0, used = 0;
+    uint64_t sp = 0, ep = 0;   /* the read ra + lane */
+    if (ra + lane < rb) { sp = a.rstart[ra + lane]; ep = a.rend[ra + lane]; }
+    uint64_t q0 = 0;           /* first k-mer of the long read's next piece */
+    bool long_ok = false;
+    while (ra < rb) {
+      /* (1) the tile's reads: as many as fit the words, or a piece of a long one */
+      __syncwarp();   /* the tile before has been read */
+      const uint64_t L64 = ep - sp, L0 = __shfl_sync(~0u, L64, 0);
+      unsigned first;
+      uint32_t n_words, reads = 1;
+      bool pre = false, post = false;
+      if (L0 > 16 * SK_WORDS) {
+        const uint64_t s0 = __shfl_sync(~0u, sp, 0), nk = L0 - k + 1;
+        if (q0 == 0) {   /* the whole read's bases checked before its first piece */
+          unsigned bad = 0;
+          for (uint64_t p = 16 * lane; p < L0; p += 16 * SK_WORDS) bad |= sk_pack(s0 + p, (int)min((uint64_t)16, L0 - p)).y;
+          long_ok = !__any_sync(~0u, bad);
+        }
+        const int n = (int)min((uint64_t)piece, nk - q0);
+        pre = q0 > 0;
+        post = q0 + n < nk;
+        if (lane == 0) {
+          S.addr[0] = s0 + q0;
+          S.nk[0] = n;
+          S.len[0] = n + k - 1 + (post ? 1 : 0);
+          S.bases[0] = pre ? sk_pack(s0 + q0 - 1, 1).x >> 30 : 0u;
+        }
+        first = long_ok ? 1u : 0u;
+        n_words = long_ok ? (uint32_t)(n + k - 1 + (post ? 1 : 0) + 15) >> 4 : 0u;
+        q0 += n;
+        if (!long_ok || q0 >= nk) q0 = 0; else reads = 0;
+      } else {
+        const uint32_t L = L64 >= (uint64_t)k + 2 ? (uint32_t)min(L64, (uint64_t)16 * SK_WORDS + 1) : 0u;
+        const uint32_t nw = (L + 15) >> 4;
+        uint32_t x = nw;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(~0u, x, o);
+          if (lane >= o) x += y;
+        }
+        /* x never falls, so the reads that fit come first */
+        const bool fits = ra + lane < rb && x <= SK_WORDS, kept = fits && nw;
+        const unsigned mf = __ballot_sync(~0u, fits), mk = __ballot_sync(~0u, kept);
+        reads = __popc(mf);
+        n_words = mf ? __shfl_sync(~0u, x, 31 - __clz(mf)) : 0u;
+        if (kept) {
+          const int d = __popc(mk & (le >> 1));
+          S.addr[d] = sp; S.len[d] = (int)L; S.nk[d] = (int)L - k + 1;
+        }
+        first = __reduce_or_sync(~0u, kept ? 1u << (x - nw) : 0u);
+        if (lane == 0) S.bases[0] = 0;
+      }
+      ra += reads;
+      if (reads && ra + lane < rb) { sp = a.rstart[ra + lane]; ep = a.rend[ra + lane]; }   /* the next tile's */
+      if (reads && ra + lane >= rb) { sp = 0; ep = 0; }
+      if (n_words == 0) continue;
+      __syncwarp();
+      /* (2) the lane's word: 16 bases packed and checked */
+      const bool mine = (uint32_t)lane < n_words;
+      const int rd = __popc(first & le) - 1, w0 = 31 - __clz(first & le), p0 = 16 * (lane - w0);
+      const unsigned above = first & ~le;
+      const int w2 = above ? __ffs(above) - 1 : (int)n_words;
+      uint2 pk = make_uint2(0u, 0u);
+      int L = 0;
+      if (mine) {
+        L = S.len[rd];
+        pk = sk_pack(S.addr[rd] + p0, min(16, L - p0));
+      }
+      S.bases[lane + 1] = pk.x;
+      if (lane < 2 * NW + 3) S.bases[SK_WORDS + 1 + lane] = 0;
+      const unsigned bad = __ballot_sync(~0u, pk.y != 0);
+      const bool good = mine && (bad & (~0u >> (32 - w2)) & (~0u << w0)) == 0;
+      /* (3) the orders of the 16 m-mers that start in the word, then block minima */
+      const uint32_t nextw = __shfl_down_sync(~0u, pk.x, 1);
+      uint32_t h[16];
+      {
+        const uint64_t W = ((uint64_t)pk.x << 32) | (lane < 31 ? nextw : 0u), R = rev_pairs(~W);
+        const int last = good ? L - MZ_M - p0 : -1;   /* m-mers past the read's last take no part */
+        #pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t o = mz_order((uint32_t)(W >> (64 - 2 * MZ_M - 2 * i)) & MZ_MASK, (uint32_t)(R >> (2 * i)) & MZ_MASK);
+          h[i] = i <= last ? o : ~0u;
+        }
+        uint32_t m = ~0u;
+        #pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          m = i % BL == 0 ? h[i] : min(m, h[i]);
+          S.pmin[i][lane] = m;
+        }
+        #pragma unroll
+        for (int i = 14; i >= 0; --i)
+          if (i % BL != BL - 1) h[i] = min(h[i], h[i + 1]);
+      }
+      __syncwarp();
+      #pragma unroll
+      for (int bb = 0; bb < NB; ++bb) {
+        /* whole blocks inside the windows of this block: qw - 1 of them, or qw once the end has
+         * crossed into the next block */
+        uint32_t mid = ~0u;
+        for (int q = 1; q < qw; ++q) {
+          const int g = bb + q;
+          mid = min(mid, S.pmin[(g % NB) * BL + BL - 1][lane + g / NB]);
+        }
+        const int g = bb + qw;
+        const uint32_t mid2 = min(mid, S.pmin[(g % NB) * BL + BL - 1][lane + g / NB]);
+        #pragma unroll
+        for (int i = 0; i < BL; ++i) {
+          const int e = bb * BL + i + w1;   /* the window's last m-mer, in positions from this word */
+          h[bb * BL + i] = min(h[bb * BL + i], min(i < BL - cw ? mid : mid2, S.pmin[e & 15][lane + (e >> 4)]));
+        }
+      }
+      /* (4) run starts, and the end of the read's k-mers */
+      uint32_t prev = __shfl_up_sync(~0u, h[15], 1);
+      uint32_t st = 0, marks = 0;
+      if (good) {
+        const int nk = S.nk[rd] - p0;   /* k-mer positions from the word on */
+        #pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          st |= h[i] != prev ? 1u << i : 0u;
+          prev = h[i];
+        }
+        if (p0 == 0) { st |= 1u; used += !pre; }
+        st &= nk >= 16 ? 0xFFFFu : nk > 0 ? (1u << nk) - 1 : 0u;
+        marks = st;
+        if (nk >= 0 && nk < 16) marks |= 1u << nk;
+        inst += (unsigned)max(0, min(16, nk));
+      }
+      S.marks[lane] = marks;
+      const uint32_t cnt = __popc(st);
+      uint32_t x = cnt;
+      #pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(~0u, x, o);
+        if (lane >= o) x += y;
+      }
+      const uint32_t total = __shfl_sync(~0u, x, 31);
+      uint32_t at = x - cnt;
+      __syncwarp();   /* every window has been read: the runs' minimizers instead */
+      #pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (st & (1u << i)) {
+          S.starts[at++] = (uint16_t)(16 * lane + i);
+          S.pmin[i][lane] = h[i];
+        }
+      /* the tile's places: the rest of the chunk, then a new one */
+      const uint32_t rest = (uint32_t)min((unsigned long long)total, cend - cpos);
+      const unsigned long long o1 = cpos;
+      unsigned long long o2 = 0;
+      cpos += rest;
+      if (rest < total) {
+        const unsigned long long ch = max(a.chunk, total - rest);
+        if (lane == 0) o2 = atomicAdd(&a.ctr->n_sk, ch);
+        o2 = __shfl_sync(~0u, o2, 0);
+        cpos = o2 + (total - rest);
+        cend = o2 + ch;
+      }
+      __syncwarp();
+      /* (5) the records */
+      for (uint32_t y = lane; y < total; y += 32) {
+        const int t = S.starts[y] >> 4, i = S.starts[y] & 15;
+        const uint32_t mz = S.pmin[i][t];
+        const unsigned ft = first & (~0u >> (31 - t));
+        const int r = __popc(ft) - 1, wr = 31 - __clz(ft), p = 16 * (t - wr) + i, nk = S.nk[r];
+        int run;   /* to the next mark: there is one, the end of the read's k-mers */
+        const uint32_t m = S.marks[t] >> i >> 1;
+        if (m) run = __ffs(m);
+        else {
+          run = 16 - i;
+          int u = t + 1;
+          while (u < SK_WORDS && S.marks[u] == 0) { run += 16; ++u; }
+          run += __ffs(S.marks[u]) - 1;   /* (marks[SK_WORDS] exists and is never reached) */
+        }
+        const uint32_t mix = mz_mix(mz), bin = X.bin0 + (mix >> X.shift);
+        unsigned long long o = y < rest ? o1 + y : o2 + (y - rest);
+        for (int d = 0; d < run; ) {   /* a minimizer that recurs may run on: cut at what a record holds */
+          const int n = min(run - d, k - MZ_M + 1), q = p + d - 1;   /* the base before the first k-mer */
+          const int tw = wr + 1 + (q >> 4);
+          const unsigned sh = 2u * (unsigned)(q & 15);
+          uint64_t w[NW];
+          uint32_t cur = S.bases[tw];
+          #pragma unroll
+          for (int u = 0; u < NW; ++u) {
+            const uint32_t b1 = S.bases[tw + 2 * u + 1], b2 = S.bases[tw + 2 * u + 2];
+            w[u] = ((uint64_t)__funnelshift_l(b1, cur, sh) << 32) | __funnelshift_l(b2, b1, sh);
+            cur = b2;
+          }
+          bool hl = q >= 0 || pre, hr = p + d + n < nk || post;
+          const int nb = n + k + 1;
+          if (mz & 1u) {   /* the other strand: its first base is the complement of our last */
+            uint64_t z[NW];
+            #pragma unroll
+            for (int u = 0; u < NW; ++u) z[u] = rev_pairs(~w[NW - 1 - u]);
+            sk_shl<NW>(z, 64u * NW - 2u * (unsigned)nb);
+            #pragma unroll
+            for (int u = 0; u < NW; ++u) w[u] = z[u];
+            const bool s = hl; hl = hr; hr = s;
+          }
+          const int bits = 2 * (hr ? nb : nb - 1);
+          #pragma unroll
+          for (int u = 0; u < NW; ++u) w[u] &= sk_top_mask(bits, u);
+          if (!hl) w[0] &= ~0ull >> 2;
+          w[NW - 1] |= ((uint64_t)bin << SK_BIN_SHIFT) | (hr ? SK_RIGHT : 0ull) | (hl ? SK_LEFT : 0ull) | (uint64_t)(n - 1);
+          if (o < a.cap) {
+            ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(a.out + o * NW);
+            #pragma unroll
+            for (int u = 0; u < NW; u += 2) __stcs(dst + u / 2, make_ulonglong2(w[u], w[u + 1]));
+          } else over = true;
+          atomicAdd(&a.hist[bin], ((unsigned long long)n << 32) | 1ull);
+          if ((mix & X.smask) == 0) {
+            const unsigned long long e = atomicAdd(&a.ctr->n_sk_est, 1ull);
+            if (e < a.est_cap) a.est[e] = (uint32_t)o;
+          }
+          d += n;
+          if (d < run) o = atomicAdd(&a.ctr->n_sk, 1ull);
+        }
+      }
+    }
+    const unsigned long long iw = warp_sum(inst), uw = warp_sum(used);
+    if (lane == 0) {
+      inst_all += iw; used_all += uw;
+      if (a.s_inst && iw) atomicAdd(&a.s_inst[smp], iw);
+      if (a.s_used && uw) atomicAdd(&a.s_used[smp], uw);
+    }
+  }
+  for (unsigned long long o = cpos + lane; o < cend; o += 32)
+    if (o < a.cap) a.out[o * NW + NW - 1] = SK_NONE;
+  if (lane == 0) {
+    if (inst_all) atomicAdd(&a.ctr->n_instances, inst_all);
+    if (used_all) atomicAdd(&a.ctr->n_reads_used, used_all);
+  }
+  if (over) atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
+}
+
+/* ------------------------------------------------------------ bins -> partitions
+ * Partition of a bin = (k-mers of its sample's bins before it) / T, T = the sample's k-mers over
+ * its partitions: neighbouring bins share a partition of T k-mers give or take a bin, so a
+ * partition's size does not depend on how evenly minimizers spread. */
+struct SkPlan {   /* a sample */
+  unsigned long long inst0, T;        /* k-mers of the samples before, k-mers a partition */
+  unsigned int bin0, pbase, parts, pad;   /* first bin, first partition, partitions */
+};
+/* k-mers of one bin at most: one CTA counts it, and a count in shared memory must stay below 2^24 */
+constexpr unsigned long long SK_MAX_BIN = 1ull << 22;
+constexpr int SK_PLAN_TPB = 256, SK_PLAN_PER = 16, SK_PLAN_CHUNK = SK_PLAN_TPB * SK_PLAN_PER;
+
+__global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_sum(const unsigned long long *hist, uint32_t nbins,
+                                                             ulonglong2 *sums, unsigned long long max_bin,
+                                                             DevCounters *ctr) {
+  unsigned long long inst = 0, rec = 0;
+  bool big = false;
+  for (uint32_t j = threadIdx.x; j < SK_PLAN_CHUNK; j += SK_PLAN_TPB) {
+    const uint32_t b = blockIdx.x * SK_PLAN_CHUNK + j;
+    if (b >= nbins) break;
+    const unsigned long long v = hist[b];
+    inst += v >> 32; rec += v & 0xFFFFFFFFull;
+    big |= (v >> 32) > max_bin;
+  }
+  inst = warp_sum(inst); rec = warp_sum(rec);
+  __shared__ unsigned long long si[SK_PLAN_TPB / 32], sr[SK_PLAN_TPB / 32];
+  if ((threadIdx.x & 31) == 0) { si[threadIdx.x >> 5] = inst; sr[threadIdx.x >> 5] = rec; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < SK_PLAN_TPB / 32; ++q) { inst += si[q]; rec += sr[q]; }
+    sums[blockIdx.x] = make_ulonglong2(inst, rec);
+  }
+  if (big) atomicOr(&ctr->err, (unsigned long long)DERR_SKEW);   /* a bin too large for one CTA */
+}
+
+/* part[b] = partition of bin b (over all samples); off[P], cur[P] = first record of partition P
+ * (nparts + 1 and nparts of them) */
+__global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_apply(const unsigned long long *hist, uint32_t nbins,
+                                                               const ulonglong2 *sums, const SkPlan *plan, uint32_t S,
+                                                               uint32_t nparts, uint32_t *part, uint32_t *off,
+                                                               uint32_t *cur) {
+  __shared__ unsigned long long si[SK_PLAN_TPB], sr[SK_PLAN_TPB];
+  const int tid = threadIdx.x;
+  unsigned long long bi = 0, br = 0;   /* sums of the blocks before */
+  for (uint32_t q = tid; q < blockIdx.x; q += SK_PLAN_TPB) { bi += sums[q].x; br += sums[q].y; }
+  const uint32_t b0 = blockIdx.x * SK_PLAN_CHUNK + tid * SK_PLAN_PER, b1 = min(nbins, b0 + SK_PLAN_PER);
+  unsigned long long ti = 0, tr = 0;
+  for (uint32_t b = b0; b < b1; ++b) { const unsigned long long v = hist[b]; ti += v >> 32; tr += v & 0xFFFFFFFFull; }
+  /* the block's base: every thread's share of the earlier sums; then the threads' exclusive scan */
+  si[tid] = bi; sr[tid] = br;
+  __syncthreads();
+  for (int o = SK_PLAN_TPB / 2; o > 0; o >>= 1) {
+    if (tid < o) { si[tid] += si[tid + o]; sr[tid] += sr[tid + o]; }
+    __syncthreads();
+  }
+  bi = si[0]; br = sr[0];
+  __syncthreads();
+  si[tid] = ti; sr[tid] = tr;
+  __syncthreads();
+  for (int o = 1; o < SK_PLAN_TPB; o <<= 1) {
+    const unsigned long long vi = tid >= o ? si[tid - o] : 0, vr = tid >= o ? sr[tid - o] : 0;
+    __syncthreads();
+    si[tid] += vi; sr[tid] += vr;
+    __syncthreads();
+  }
+  unsigned long long inst = bi + si[tid] - ti, rec = br + sr[tid] - tr;
+  if (b0 >= nbins) return;
+  /* the sample of a bin, and the bin's partition from the k-mers before it */
+  auto sample_of_bin = [&](uint32_t b) {
+    uint32_t lo = 0, hi = S;
+    while (hi - lo > 1) { const uint32_t m = (lo + hi) >> 1; if (plan[m].bin0 <= b) lo = m; else hi = m; }
+    return lo;
+  };
+  auto part_of = [&](const SkPlan &X, unsigned long long before) {
+    return X.pbase + (uint32_t)min((before - X.inst0) / X.T, (unsigned long long)(X.parts - 1));
+  };
+  uint32_t s = sample_of_bin(b0);
+  SkPlan X = plan[s];
+  /* the partition of the bin before b0: partitions after it, up to b0's own, start at b0 */
+  uint32_t next;   /* first partition whose start is not yet known */
+  if (b0 == 0) next = 0;
+  else {
+    const uint32_t sp = b0 > X.bin0 ? s : sample_of_bin(b0 - 1);
+    const SkPlan Y = sp == s ? X : plan[sp];
+    next = part_of(Y, inst - (hist[b0 - 1] >> 32)) + 1;
+  }
+  for (uint32_t b = b0; b < b1; ++b) {
+    while (s + 1 < S && plan[s + 1].bin0 <= b) X = plan[++s];
+    const uint32_t P = part_of(X, inst);
+    part[b] = P;
+    for (; next <= P; ++next) { off[next] = (uint32_t)rec; cur[next] = (uint32_t)rec; }
+    const unsigned long long v = hist[b];
+    inst += v >> 32; rec += v & 0xFFFFFFFFull;
+  }
+  if (b1 == nbins) {
+    for (; next < nparts; ++next) { off[next] = (uint32_t)rec; cur[next] = (uint32_t)rec; }
+    off[nparts] = (uint32_t)rec;
+  }
+}
+
+/* Records -> partition order: one returning atomic on the partition's cursor and one store a
+ * record.  A partition's open line stays in L2 until its records have filled it (2^18 open
+ * 128-byte lines are 32 MB of the 129 MB), so the scattered stores leave as whole lines. */
+constexpr int SK_SCATTER_U = 4;
+template <int NW>
+__global__ void __launch_bounds__(256) k_sk_scatter(const uint64_t *rec, uint64_t n, const uint32_t *part,
+                                                    uint32_t *cur, uint64_t *out, const DevCounters *ctr) {
+  if (ctr->err) return;   /* the bins cannot be counted this way: the caller falls back */
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * SK_SCATTER_U) {
+    ulonglong2 r[SK_SCATTER_U][NW / 2];
+    uint32_t P[SK_SCATTER_U], o[SK_SCATTER_U];
+    #pragma unroll
+    for (int u = 0; u < SK_SCATTER_U; ++u) {
+      const uint64_t i = i0 + u * stride;
+      if (i >= n) continue;
+      #pragma unroll
+      for (int q = 0; q < NW / 2; ++q) r[u][q] = __ldcs(reinterpret_cast<const ulonglong2 *>(rec + i * NW) + q);
+    }
+    bool has[SK_SCATTER_U];
+    #pragma unroll
+    for (int u = 0; u < SK_SCATTER_U; ++u) has[u] = i0 + u * stride < n && (r[u][NW / 2 - 1].y & 63u) != SK_NONE;
+    #pragma unroll
+    for (int u = 0; u < SK_SCATTER_U; ++u)
+      if (has[u]) P[u] = __ldg(part + ((r[u][NW / 2 - 1].y >> SK_BIN_SHIFT) & SK_BIN_MASK));
+    #pragma unroll
+    for (int u = 0; u < SK_SCATTER_U; ++u)
+      if (has[u]) o[u] = atomicAdd(&cur[P[u]], 1u);
+    #pragma unroll
+    for (int u = 0; u < SK_SCATTER_U; ++u) {
+      if (!has[u]) continue;
+      #pragma unroll
+      for (int q = 0; q < NW / 2; ++q) reinterpret_cast<ulonglong2 *>(out + (uint64_t)o[u] * NW)[q] = r[u][q];
+    }
+  }
+}
+
+/* ------------------------------------------------------------ counting
+ * One CTA a partition.  Its records come in rounds; equal records (the same place read without
+ * an error, from either strand: two thirds of them at 30x) are merged in a small hash of record
+ * numbers, then the distinct ones' k-mers, cut into items of SK_ITEM k-mers so that every thread
+ * has work, are counted with the record's weight in a hash of k-mers in shared memory: per slot
+ * the k-mer and two entry words, in two arrays (a k-mer with more biedges goes on in later slots
+ * keyed k-mer | CONT).  The k-mers to keep are then placed in a region of the table of their own
+ * number over the load, in the table's slot format, and listed for the filter.
+ *
+ * keep_all: every k-mer is kept (the raw counts or other thresholds may still be asked for);
+ * otherwise a k-mer that the filter's quick rule drops (its total below the (k+1)-mer lower bound;
+ * filter_quick) is tallied and left out: at 30x and 0.5% errors three k-mers of four. */
+constexpr int SK_COUNT_TPB = 384;
+constexpr int SK_ITEM = 4;
+constexpr double SK_MAX_INV_LOAD = 4.0;
+constexpr uint32_t SK_LATE = 256;
+struct SkCount {
+  const uint64_t *recs;
+  const uint32_t *off;              /* first record of every partition */
+  const uint32_t *todo;             /* NULL: partition blockIdx.x; else the partitions to count */
+  uint32_t slots;                   /* k-mer slots in shared memory */
+  uint32_t late;                    /* where the late k-mers wait, in shared-memory words */
+  uint32_t round, hsize;            /* records a round (at most 1024), entries of their hash (a power of two) */
+  int k;
+  int keep_all, thresholding;
+  uint32_t t[6];                    /* the filter's bounds, clamped to 65536 (counts end at 65535) */
+  double inv_load;                  /* table slots a kept slot */
+  uint64_t *table;
+  uint64_t cap;                     /* table slots of the sample(s) */
+  uint2 *info;                      /* per partition: its first slot, its slots */
+  uint32_t *over;                   /* partitions that overflowed the shared-memory slots */
+  uint32_t *cand;                   /* the slots the filter must read */
+  unsigned long long *s_tally;
+  const SGeom *sg;
+  uint32_t nsamples;
+  unsigned long long *bump;         /* per sample: table slots taken so far */
+  DevCounters *ctr;
+};
+
+/* entries of the record hash: a power of two, a third of them free at least */
+__host__ __device__ constexpr uint32_t sk_hash_size(uint32_t round) {
+  uint32_t h = 64;
+  while (2 * h < 3 * round) h *= 2;
+  return h;
+}
+/* Shared memory: slots (key, two entries); then a round's records, weights, record hash (its memory
+ * then holds the item list, at most 5 or 13 items a record of 2 bytes each) and late k-mers, or the
+ * list of kept slots and the bitmap of a region of at most SK_MAX_INV_LOAD slots a kept one */
+template <class KT>
+__host__ __device__ constexpr uint32_t sk_late_at(uint32_t slots, uint32_t round) {   /* in 8-byte words, even */
+  const size_t items = (size_t)round * (sizeof(KT) == 8 ? 10 : 26), hash = (size_t)sk_hash_size(round) * 4;
+  const size_t b = (size_t)slots * (Slot<KT>::KEYW * 8 + 8) + (size_t)round * (SkRec<KT>::NW * 8 + 4) +
+                   (items > hash ? items : hash);
+  return (uint32_t)((b + 15) / 16 * 2);
+}
+template <class KT>
+__host__ __device__ constexpr size_t sk_count_bytes(uint32_t slots, uint32_t round) {
+  const size_t r = (size_t)sk_late_at<KT>(slots, round) * 8 + SK_LATE * (Slot<KT>::KEYW * 8 + 8);
+  const size_t l = (size_t)slots * (Slot<KT>::KEYW * 8 + 8 + 2) + 8 + (size_t)(slots * SK_MAX_INV_LOAD) / 8 + 8;
+  return r > l ? r : l;
+}
+
+__device__ __forceinline__ uint32_t sk_home(KW1 x, uint32_t slots) {
+  uint32_t h = (uint32_t)x.v * 0x9E3779B1u ^ (uint32_t)(x.v >> 32) * 0x85EBCA6Bu;
+  h ^= h >> 16;
+  return __umulhi(h * 0xC2B2AE35u, slots);
+}
+__device__ __forceinline__ uint32_t sk_home(KW2 x, uint32_t slots) {
+  uint32_t h = (uint32_t)x.lo * 0x9E3779B1u ^ (uint32_t)(x.lo >> 32) * 0x85EBCA6Bu;
+  h ^= (uint32_t)x.hi * 0x27D4EB2Fu ^ (uint32_t)(x.hi >> 32) * 0x165667B1u;
+  h ^= h >> 16;
+  return __umulhi(h * 0xC2B2AE35u, slots);
+}
+/* The shared-memory slots: k <= 31 one 16-byte (key, entries 0-1), read at once and claimed with its
+ * first entry by one 128-bit CAS; k > 31 keys and entry pairs in two arrays. */
+template <class KT> struct SkSlots;
+template <> struct SkSlots<KW1> {
+  uint64_t *p;
+  uint32_t n;
+  __device__ __forceinline__ SkSlots(uint64_t *mem, uint32_t slots) : p(mem), n(slots) {}
+  __device__ __forceinline__ void clear(uint32_t i) const { reinterpret_cast<ulonglong2 *>(p)[i] = make_ulonglong2(KEY_EMPTY, 0ull); }
+  __device__ __forceinline__ uint32_t *entries(uint32_t j) const { return reinterpret_cast<uint32_t *>(p + 2 * j + 1); }
+  __device__ __forceinline__ KW1 key(uint32_t j) const { return {p[2 * j]}; }
+  __device__ __forceinline__ uint64_t pair(uint32_t j) const { return p[2 * j + 1]; }
+  /* slot j's key and entries as they are, or after claiming it for `want` with `fresh` (claimed) */
+  __device__ __forceinline__ KW1 visit(uint32_t j, KW1 want, uint32_t fresh, uint64_t &e, bool &claimed) const {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p + 2 * j);
+    KW1 x;
+    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x.v), "=l"(e) : "r"(a) : "memory");
+    if ((int64_t)x.v < 0) {   /* empty: no key has its top bit set */
+      x.v = sm_cas128(a, KEY_EMPTY, 0ull, want.v, (uint64_t)fresh, e);
+      claimed = (int64_t)x.v < 0;
+    }
+    return x;
+  }
+};
+template <> struct SkSlots<KW2> {
+  uint64_t *p, *q;
+  uint32_t n;
+  __device__ __forceinline__ SkSlots(uint64_t *mem, uint32_t slots) : p(mem), q(mem + 2 * slots), n(slots) {}
+  __device__ __forceinline__ void clear(uint32_t i) const {
+    reinterpret_cast<ulonglong2 *>(p)[i] = make_ulonglong2(KEY_EMPTY, KEY_EMPTY);
+    q[i] = 0;
+  }
+  __device__ __forceinline__ uint32_t *entries(uint32_t j) const { return reinterpret_cast<uint32_t *>(q + j); }
+  __device__ __forceinline__ KW2 key(uint32_t j) const { return {p[2 * j], p[2 * j + 1]}; }
+  __device__ __forceinline__ uint64_t pair(uint32_t j) const { return q[j]; }
+  __device__ __forceinline__ KW2 visit(uint32_t j, KW2 want, uint32_t, uint64_t &e, bool &) const {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p + 2 * j);
+    KW2 x;
+    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x.lo), "=l"(x.hi) : "r"(a) : "memory");
+    if (key_is_empty(x)) {
+      KW2 o;
+      o.lo = sm_cas128(a, KEY_EMPTY, KEY_EMPTY, want.lo, want.hi, o.hi);
+      x = key_is_empty(o) ? want : o;
+    }
+    e = *(volatile const uint64_t *)(q + j);
+    return x;
+  }
+};
+
+constexpr uint32_t SK_MAX_PROBE = 512;   /* a longer run: the partition is too full */
+
+/* A slot's second entry word carries SK_MORE (its E_BIG bit: no count here reaches 2^24) once the
+ * k-mer goes on in a continuation slot. */
+constexpr uint32_t SK_MORE = E_BIG;
+__device__ __forceinline__ uint32_t sk_count_of(uint32_t w) { return w >> E_COUNT_SHIFT; }
+
+/* `fresh` is an entry word: a code and the occurrences to count.  One entry word of a slot tried for
+ * it; `w` is what the word was seen to hold */
+__device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t fresh, unsigned &claims) {
+  if (w == 0) {
+    w = atomicCAS(e, 0u, fresh);
+    if (w == 0) { ++claims; return true; }
+  }
+  if (entry_code(w) != entry_code(fresh)) return false;
+  atomicAdd(e, fresh & ~((1u << E_COUNT_SHIFT) - 1));
+  return true;
+}
+
+/* an entry word's occurrences into the shared-memory slots of a k-mer, continuation slots and all
+ * (any lanes may call it); false if the slots are full */
+template <class KT>
+__device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, unsigned &claims) {
+  uint32_t j = sk_home(want, sl.n);
+  for (uint32_t probe = 0; probe < SK_MAX_PROBE; ++probe) {
+    uint64_t seen;
+    bool claimed = false;
+    const KT key = sl.visit(j, want, fresh, seen, claimed);
+    if (claimed) { ++claims; return true; }
+    if (KOps<KT>::eq(key, want)) {
+      uint32_t *e = sl.entries(j);
+      if (sk_try_entry(e, *(volatile uint32_t *)e, fresh, claims)) return true;
+      if (sk_try_entry(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims)) return true;
+      atomicOr(e + 1, SK_MORE);
+      ((uint64_t *)&want)[KOps<KT>::WORDS - 1] |= KEY_CONT;
+    }
+    if (++j == sl.n) j = 0;
+  }
+  return false;
+}
+
+/* fn(entry words 0 and 1) for the k-mer of slot q, then for its continuation slots, in order */
+template <class KT, class F>
+__device__ __forceinline__ void sk_entries(const SkSlots<KT> &sl, uint32_t q, KT key, F fn) {
+  uint64_t e = sl.pair(q);
+  fn(e & ~((uint64_t)SK_MORE << 32));
+  ((uint64_t *)&key)[KOps<KT>::WORDS - 1] |= KEY_CONT;
+  uint32_t j = q;
+  while ((e >> 32) & SK_MORE) {   /* its next slot lies further on */
+    KT x;
+    do {
+      if (++j == sl.n) j = 0;
+      x = sl.key(j);
+    } while (!KOps<KT>::eq(x, key) && !key_is_empty(x));
+    if (key_is_empty(x)) return;
+    e = sl.pair(j);
+    fn(e & ~((uint64_t)SK_MORE << 32));
+  }
+}
+
+/* a k-mer with a longer probe run, or whose slot's two entries are taken, waits here until the
+ * round's others are counted: its warp's other lanes would wait for it */
+template <class KT> struct SkLate { KT key; uint64_t fresh; };
+
+template <class KT>
+__global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_count(SkCount a) {
+  constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW, NE = Slot<KT>::ENTRIES, NW = SkRec<KT>::NW;
+  extern __shared__ __align__(16) uint64_t sm[];
+  __shared__ uint32_t s_items, s_full, s_listed, s_other, s_conts, s_wide, s_base, s_slots, s_late_n;
+  __shared__ unsigned int s_qh[4], s_claims;
+  __shared__ unsigned long long s_cand;
+  if (a.ctr->err & DERR_SKEW) return;
+  const uint32_t part = a.todo ? a.todo[blockIdx.x] : blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, k = a.k;
+  const uint32_t nt = blockDim.x, slots = a.slots, round = a.round;
+  const SkSlots<KT> sl(sm, slots);
+  uint64_t *s_rec = sm + (size_t)slots * (KWD + 1);
+  uint32_t *s_wt = reinterpret_cast<uint32_t *>(s_rec + (size_t)round * NW), *s_hash = s_wt + round;
+  uint16_t *s_list = reinterpret_cast<uint16_t *>(s_hash);
+  SkLate<KT> *s_late = reinterpret_cast<SkLate<KT> *>(sm + a.late);
+  for (uint32_t i = tid; i < slots; i += nt) sl.clear(i);
+  if (tid < 4) s_qh[tid] = 0;
+  if (tid == 0) { s_full = 0; s_listed = 0; s_other = 0; s_conts = 0; s_wide = 0; s_claims = 0; }
+  const uint32_t hmask = a.hsize - 1;
+  unsigned claims = 0;
+  const uint32_t r1 = a.off[part + 1];
+  for (uint32_t r0 = a.off[part]; r0 < r1; r0 += round) {
+    const uint32_t nr = min(round, r1 - r0);
+    for (uint32_t i = tid; i < nr * (NW / 2); i += nt)
+      reinterpret_cast<ulonglong2 *>(s_rec)[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(a.recs + (uint64_t)r0 * NW) + i);
+    for (uint32_t i = tid; i < nr; i += nt) s_wt[i] = 0;
+    for (uint32_t i = tid; i <= hmask; i += nt) s_hash[i] = ~0u;
+    if (tid == 0) { s_items = 0; s_late_n = 0; }
+    __syncthreads();
+    /* equal records merge into the first that claimed a hash entry */
+    for (uint32_t i = tid; i < nr; i += nt) {
+      ulonglong2 rec[NW / 2];
+      uint64_t z = 0;
+      #pragma unroll
+      for (int q = 0; q < NW / 2; ++q) {
+        rec[q] = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)i * NW)[q];
+        z = (z ^ rec[q].x) * 0x9E3779B97F4A7C15ull ^ rec[q].y ^ (z >> 29);
+      }
+      z *= 0xD6E8FEB86659FD93ull;
+      uint32_t h = (uint32_t)(z >> 52) & hmask;
+      for (;;) {   /* a third of the entries stays free */
+        const uint32_t o = atomicCAS(&s_hash[h], ~0u, i);
+        if (o == ~0u) { atomicAdd(&s_wt[i], 1u); break; }
+        bool same = true;
+        #pragma unroll
+        for (int q = 0; q < NW / 2; ++q) {
+          const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)o * NW)[q];
+          same &= v.x == rec[q].x && v.y == rec[q].y;
+        }
+        if (same) { atomicAdd(&s_wt[o], 1u); break; }
+        h = (h + 1) & hmask;
+      }
+    }
+    __syncthreads();
+    /* the distinct records' k-mers as items of SK_ITEM */
+    for (uint32_t i0 = 0; i0 < nr; i0 += nt) {
+      const uint32_t i = i0 + tid;
+      const unsigned n = i < nr && s_wt[i] ? sk_n(s_rec[(size_t)i * NW + NW - 1]) : 0u;
+      const uint32_t ni = (n + SK_ITEM - 1) / SK_ITEM;
+      uint32_t x = ni;
+      #pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(~0u, x, o);
+        if (lane >= o) x += y;
+      }
+      uint32_t at = 0;
+      if (lane == 31 && x) at = atomicAdd(&s_items, x);
+      at = __shfl_sync(~0u, at, 31) + x - ni;
+      for (uint32_t q = 0; q < ni; ++q) s_list[at + q] = (uint16_t)(i | (q << 10));
+    }
+    __syncthreads();
+    const uint32_t items = s_items;
+    /* the warp's lanes stay together: every loop's bound is the warp's or fixed */
+    for (uint32_t y0 = tid & ~31u; y0 < items; y0 += nt) {
+      const bool has = y0 + lane < items;
+      const uint32_t it = has ? s_list[y0 + lane] : 0u, id = it & 1023u;
+      const int o0 = SK_ITEM * (int)(it >> 10);
+      const uint64_t *w = s_rec + (size_t)id * NW;
+      const uint64_t last = w[NW - 1];
+      const int nk = (int)sk_n(last), n = has ? min(nk - o0, SK_ITEM) : 0;
+      const uint32_t weight = s_wt[id] << E_COUNT_SHIFT;
+      KT f = KOps<KT>::extract(w, o0 + 1, k), r = KOps<KT>::rc(f, k);
+      /* in5, out5 of the k-mers: the base before (0: none), then the bases after from the top of `next` */
+      unsigned in5 = o0 > 0 || (last & SK_LEFT) ? sk_base<NW>(w, o0) + 1u : 0u;
+      const int b = o0 + k + 1;
+      const uint64_t n0 = w[b >> 5] << (2 * (b & 31)), n1 = (b >> 5) + 1 < NW ? w[(b >> 5) + 1] : 0ull;
+      uint32_t next = (uint32_t)((n0 | ((b & 31) ? n1 >> (64 - 2 * (b & 31)) : 0ull)) >> 32);
+      const int n_out = nk - o0 - ((last & SK_RIGHT) ? 0 : 1);   /* k-mers of the item that have a base after */
+      for (int d = 0; __any_sync(~0u, d < n); ++d) {
+        bool todo = d < n;
+        const unsigned c = next >> 30, out5 = d < n_out ? c + 1u : 0u;
+        next <<= 2;
+        /* lex_less: the smaller strand, with the biedge reverse-complemented on a flip */
+        const bool fwd = KOps<KT>::lt(f, r);
+        const KT key = fwd ? f : r;
+        const unsigned code = fwd ? biedge_code(in5, out5) : biedge_code(out5 ? 5u - out5 : 0u, in5 ? 5u - in5 : 0u);
+        const uint32_t fresh = (code << E_CODE_SHIFT) | weight;
+        in5 = KOps<KT>::first(f, k) + 1u;
+        f = KOps<KT>::append(f, c, k);
+        r = KOps<KT>::prepend(3u - c, r, k);
+        /* the k-mer's slot within three probes (nine in ten), then its entry among the slot's two */
+        uint32_t j = sk_home(key, slots);
+        uint64_t seen = 0;
+        bool seek = todo;
+        #pragma unroll
+        for (int probe = 0; probe < 3; ++probe) {
+          if (seek) {
+            bool claimed = false;
+            const KT x = sl.visit(j, key, fresh, seen, claimed);
+            if (claimed) { ++claims; todo = false; }
+            seek = !claimed && !KOps<KT>::eq(x, key);
+            if (seek && ++j == slots) j = 0;
+          }
+        }
+        if (todo && !seek) {
+          uint32_t *e = sl.entries(j);
+          uint32_t cur = (uint32_t)seen;
+          if (cur != 0 && entry_code(cur) != code) { cur = (uint32_t)(seen >> 32); ++e; }
+          todo = !sk_try_entry(e, cur, fresh, claims);
+        }
+        if (todo) {   /* the rest, later */
+          const uint32_t at = atomicAdd(&s_late_n, 1u);
+          if (at < SK_LATE) s_late[at] = SkLate<KT>{key, fresh};
+          else if (!sk_insert<KT>(sl, key, fresh, claims)) s_full = 1;
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    const uint32_t late = min(s_late_n, SK_LATE);
+    for (uint32_t y = tid; y < late; y += nt)
+      if (!sk_insert<KT>(sl, s_late[y].key, (uint32_t)s_late[y].fresh, claims)) s_full = 1;
+    __syncthreads();
+    if (s_full) break;
+  }
+  __syncthreads();
+  if (s_full) {   /* counted again with more slots: nothing of it is tallied or written */
+    if (tid == 0) a.over[atomicAdd(&a.ctr->n_over, 1ull)] = part;
+    return;
+  }
+  /* which k-mers to keep, by slot: the listed ones from the front of the list, others (keep_all) from
+   * its back (the list and the region's bitmap take the memory of the records and all behind it) */
+  uint16_t *kept = reinterpret_cast<uint16_t *>(s_rec);
+  uint64_t qh = 0;   /* quick drops' flags 3 | 8 | 4 as 16-bit fields (a thread sees under 2^11 slots) */
+  uint32_t my_conts = 0;
+  const uint32_t t_low = a.thresholding ? a.t[2] : 0u;
+  const bool no_bounds = a.t[0] == 0 && a.t[1] > 0xFFFFu && a.t[4] == 0 && a.t[5] > 0xFFFFu;   /* flags 3 only */
+  for (uint32_t q0 = tid & ~31u; q0 < slots; q0 += nt) {
+    const uint32_t q = q0 + lane;   /* slots are a multiple of 32 */
+    const KT key = sl.key(q);
+    bool listed = false, keep = false;
+    if (!key_is_empty(key)) {
+      if (key_cont(key)) {
+        ++my_conts;
+      } else {
+        const uint64_t e = sl.pair(q);
+        const uint32_t c0 = sk_count_of((uint32_t)e), c1 = sk_count_of((uint32_t)(e >> 32));
+        const bool more = ((e >> 32) & SK_MORE) != 0;
+        uint32_t kf = c0 + c1;
+        if (more && kf < t_low) {   /* the total needs the continuation slots */
+          kf = 0;
+          sk_entries<KT>(sl, q, key, [&](uint64_t x) { kf += sk_count_of((uint32_t)x) + sk_count_of((uint32_t)(x >> 32)); });
+        }
+        kf = min(0xFFFFu, kf);
+        listed = kf >= t_low;
+        keep = listed || a.keep_all;
+        if (!listed) {
+          if (no_bounds && !more) {
+            qh += 1 + (c1 != 0);
+          } else {
+            const uint32_t kout = (kf < a.t[0] || kf >= a.t[1]) ? 2u : 0u;
+            sk_entries<KT>(sl, q, key, [&](uint64_t x) {
+              #pragma unroll
+              for (int z = 0; z < 2; ++z) {
+                const uint32_t c16 = min(0xFFFFu, sk_count_of((uint32_t)(x >> (32 * z))));
+                if (c16) qh += 1ull << (16 * (kout | ((c16 < a.t[4] || c16 >= a.t[5]) ? 1u : 0u)));
+              }
+            });
+          }
+        }
+      }
+    }
+    const unsigned ml = __ballot_sync(~0u, listed), below = (1u << lane) - 1;
+    uint32_t at = 0;
+    if (ml) {
+      if (lane == 0) at = atomicAdd(&s_listed, (uint32_t)__popc(ml));
+      at = __shfl_sync(~0u, at, 0);
+      if (listed) kept[at + __popc(ml & below)] = (uint16_t)q;
+    }
+    if (a.keep_all) {
+      const unsigned mo = __ballot_sync(~0u, keep && !listed);
+      if (lane == 0 && mo) at = atomicAdd(&s_other, (uint32_t)__popc(mo));
+      at = __shfl_sync(~0u, at, 0);
+      if (keep && !listed) kept[slots - 1 - (at + __popc(mo & below))] = (uint16_t)q;
+    }
+  }
+  my_conts = (uint32_t)warp_sum(my_conts);
+  claims = (unsigned)warp_sum(claims);
+  if (lane == 0) {
+    if (my_conts) atomicAdd(&s_conts, my_conts);
+    if (claims) atomicAdd(&s_claims, claims);
+  }
+  #pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const unsigned long long h = warp_sum((qh >> (16 * f)) & 0xFFFFull);
+    if (lane == 0 && h) atomicAdd(&s_qh[f], (unsigned)h);
+  }
+  __syncthreads();
+  const uint32_t listed = s_listed, nkept = listed + s_other;
+  /* table slots: one a kept k-mer, and a k-mer of more entries than that holds has three continuation
+   * slots here for every one it takes there.  Two slots at least of the region stay empty, which
+   * ends every probe run. */
+  const uint32_t tslots = nkept + s_conts / (NE / 2), want_R = (uint32_t)(tslots * a.inv_load) + 2u;
+  if (tid == 0) {
+    const uint32_t R = want_R;
+    const uint32_t smp = sample_of_part(a.sg, a.nsamples, part);
+    const TableGeom &g = a.sg[smp].g;
+    const unsigned long long lo = atomicAdd(&a.bump[smp], (unsigned long long)R);
+    const unsigned long long c0 = atomicAdd(&a.ctr->n_cand, (unsigned long long)listed);
+    s_cand = c0;
+    const bool fits = lo + R <= g.nslots;
+    if (!fits) atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
+    s_slots = fits ? R : 0;
+    s_base = (uint32_t)(g.base + lo);
+    a.info[part] = make_uint2((uint32_t)(g.base + lo), R);
+    if (tslots) atomicAdd(&a.ctr->n_slots_claimed, (unsigned long long)tslots);
+    if (s_claims) atomicAdd(&a.ctr->n_entries, (unsigned long long)s_claims);
+    if (a.s_tally && s_claims) atomicAdd(&a.s_tally[(uint64_t)smp * T_NUM + T_ENTRIES], (unsigned long long)s_claims);
+  }
+  if (tid < 4 && s_qh[tid]) atomicAdd(&a.ctr->quick_hist[3 + 4 * tid], (unsigned long long)s_qh[tid]);
+  /* the places taken in the region, a bit each, behind the list */
+  uint32_t *taken = reinterpret_cast<uint32_t *>(kept) + (slots + 1) / 2;
+  for (uint32_t i = tid; i < (want_R + 31u) / 32; i += nt) taken[i] = 0;
+  __syncthreads();
+  const uint32_t R = s_slots;
+  if (R == 0) return;
+  uint64_t *dst = a.table + (uint64_t)s_base * SU;
+  auto place = [&](uint32_t pos) {   /* the first free place from pos on */
+    for (;;) {
+      const uint32_t bit = 1u << (pos & 31);
+      if (!(atomicOr(&taken[pos >> 5], bit) & bit)) return pos;
+      if (++pos == R) pos = 0;
+    }
+  };
+  for (uint32_t x = tid; x < nkept; x += nt) {
+    const uint32_t q = x < listed ? kept[x] : kept[slots - 1 - (x - listed)];
+    const KT key = sl.key(q), t = table_key(key);
+    const uint32_t pos = place(bin_home(t, R));
+    ulonglong2 *to = reinterpret_cast<ulonglong2 *>(dst + (uint64_t)pos * SU);
+    const uint64_t e = sl.pair(q);
+    #pragma unroll
+    for (int i = 0; i < SU; i += 2) {
+      uint64_t v[2] = {0, 0};
+      #pragma unroll
+      for (int z = 0; z < 2; ++z)
+        if (i + z < KWD) v[z] = ((const uint64_t *)&t)[i + z];
+        else if (i + z == KWD) v[z] = e & ~((uint64_t)SK_MORE << 32);
+      to[i / 2] = make_ulonglong2(v[0], v[1]);
+    }
+    if ((e >> 32) & SK_MORE) {
+      int n = KWD;
+      sk_entries<KT>(sl, q, key, [&](uint64_t x) {
+        if (n > KWD && n < SU) dst[(uint64_t)pos * SU + n] = x;
+        if (n == SU) s_wide = 1;
+        ++n;
+      });
+    }
+    if (x < listed) a.cand[s_cand + x] = s_base + pos;
+  }
+  __syncthreads();
+  if (s_wide)   /* k-mers of more entries than a table slot holds: continuation slots behind the first */
+    for (uint32_t x = tid; x < nkept; x += nt) {
+      const uint32_t q = x < listed ? kept[x] : kept[slots - 1 - (x - listed)];
+      const KT key = sl.key(q);
+      KT t = table_key(key);
+      ((uint64_t *)&t)[KWD - 1] |= KEY_CONT;
+      uint64_t *to = nullptr;
+      int n = 0;
+      sk_entries<KT>(sl, q, key, [&](uint64_t e) {
+        const int i = n % (SU - KWD);
+        if (n >= SU - KWD && i == 0) {
+          to = dst + (uint64_t)place(bin_home(table_key(key), R)) * SU;
+          KOps<KT>::store(to, t);
+          for (int z = KWD; z < SU; ++z) to[z] = 0;
+        }
+        if (to) to[KWD + i] = e;
+        ++n;
+      });
+    }
+  __syncthreads();
+  for (uint32_t pos = tid; pos < R; pos += nt) {
+    if (taken[pos >> 5] >> (pos & 31) & 1u) continue;
+    #pragma unroll
+    for (int i = 0; i < SU; i += 2)
+      reinterpret_cast<ulonglong2 *>(dst + (uint64_t)pos * SU)[i / 2] =
+          make_ulonglong2(i < KWD ? KEY_EMPTY : 0ull, i + 1 < KWD ? KEY_EMPTY : 0ull);
+  }
+}
