@@ -2624,6 +2624,7 @@ int wx_blocks(uint64_t nr);
 bool sk_takes(const Ctx *c);
 bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes);
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
+bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f);
 }  // namespace
 
 /* Indexes every FASTQ segment.  A segment copied from the host in pieces (load_fastq) is
@@ -2641,7 +2642,7 @@ bruno_status run_index_reads(Ctx *c) {
   if ((st = ensure(c, c->tile_base, std::max<uint64_t>(1, total_tiles) * 8)) != BRUNO_OK) return st;
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
-  c->sk_on = sk_takes(c);
+  c->sk_on = sk_takes(c) && (c->S == 1 || !c->samp_off.empty());
   c->pre_extracted = piped && c->S == 1 && !c->cfg.edge_filter && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
@@ -3169,11 +3170,9 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
  * so do builds without thresholds: they keep every k-mer, and 3.5M nodes at 12x (13.7M k-mers,
  * k = 31) took 3.28 ms by super-k-mers against 3.09 */
 bool sk_takes(const Ctx *c) {
-  return c->S == 1 && c->cfg.k >= MZ_M + 4 && c->cfg.thresholding && !c->cfg.edge_filter && c->force_direct_count == 0 &&
+  return c->cfg.k >= MZ_M + 4 && c->cfg.thresholding && !c->cfg.edge_filter && c->force_direct_count == 0 &&
          c->cfg.table_slots == 0;
 }
-
-constexpr uint64_t SK_EST_CAP = 1ull << 20;   /* records the estimate takes (about 2^17 are listed) */
 
 template <class KT, int BL>
 void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
@@ -3201,7 +3200,7 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_
   a.cap = c->sk_cap;
   a.hist = (unsigned long long *)c->sk_hist.p;
   a.est = (uint32_t *)c->sk_est.p;
-  a.est_cap = SK_EST_CAP;
+  a.est_cap = c->sk_est_cap;
   a.s_inst = s_inst;
   a.s_used = s_used;
   a.ctr = c->dctr;
@@ -3235,13 +3234,15 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
   const uint32_t S = (uint32_t)bytes.size();
   const int k = c->cfg.k, w = k - MZ_M + 1;
   uint64_t total = 0;
+  /* the estimate is made from about 2^20 k-mers, in a batch 2^17 each */
+  const int sample_bits = S == 1 ? 21 : 18;
   c->sk_bits.assign(S, 0);
   c->sk_q.assign(S, 0);
   for (uint32_t q = 0; q < S; ++q) {
     total += bytes[q];
     int b = 11, e = 0;
     while (b < 21 && (bytes[q] >> 10 >> b)) ++b;
-    while (e < 10 && (bytes[q] >> 21 >> (e + 1))) ++e;   /* a sample of about 2^20 k-mers */
+    while (e < 13 && (bytes[q] >> sample_bits >> (e + 1))) ++e;
     c->sk_bits[q] = b;
     c->sk_q[q] = e;
   }
@@ -3263,7 +3264,8 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
   const size_t rb = c->W == 1 ? 16 : 32;
   if ((st = ensure(c, c->sk_recs, c->sk_cap * rb)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->sk_hist, bins * 8)) != BRUNO_OK) return st;
-  if ((st = ensure(c, c->sk_est, SK_EST_CAP * 4)) != BRUNO_OK) return st;
+  c->sk_est_cap = std::min<uint64_t>(c->sk_cap, std::max<uint64_t>(1ull << 20, (uint64_t)S << 16));
+  if ((st = ensure(c, c->sk_est, c->sk_est_cap * 4)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->sk_samp, S * sizeof(SkSample))) != BRUNO_OK) return st;
   if ((st = ensure(c, c->hllreg, (size_t)S * HLL_M * 4)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->hsum, (size_t)S * 16)) != BRUNO_OK) return st;
@@ -3277,14 +3279,6 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
   }
   return cuda_check(c, cudaMemcpyAsync(c->sk_samp.p, xs.data(), S * sizeof(SkSample), cudaMemcpyHostToDevice, c->stream),
                     "super-k-mer samples");
-}
-
-template <class KT>
-void sk_estimate(Ctx *c, uint32_t S) {
-  k_sk_estimate<KT><<<num_sms() * 4, 128, 0, c->stream>>>(
-      (const uint64_t *)c->sk_recs.p, (const uint32_t *)c->sk_est.p, SK_EST_CAP, c->cfg.k, (const SkSample *)c->sk_samp.p,
-      S, (unsigned int *)c->hllreg.p, c->dctr);
-  c->launches += 1;
 }
 
 /* bins -> partitions (plan: one a sample), records -> partition order */
@@ -3339,29 +3333,44 @@ void sk_count_launch(const Ctx *c, const SkCount &a, uint32_t grid, size_t bytes
   k_sk_count<KT><<<grid, nt, bytes, c->stream>>>(a);
 }
 
+/* One launch's partitions (all, or a size class of a batch's) and its blocks' shape */
+template <class KT>
+struct SkLaunch {
+  uint32_t parts;
+  SkShape<KT> shape;
+  const ClassRun *cls;
+  uint32_t ncls;
+};
+
 /* The partitions counted (records in partition order), those that overflow their block's slots
  * once more with as many as fit; ok = false if that does not do either. */
 template <class KT>
-bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const SkShape<KT> &shape, bool &ok) {
+bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector<SkLaunch<KT>> &launches, bool &ok) {
   bruno_status st;
-  a.slots = shape.slots;
-  a.round = shape.round;
-  a.hsize = sk_hash_size(a.round);
-  a.late = sk_late_at<KT>(a.slots, a.round);
-  sk_count_launch<KT>(c, a, parts, shape.bytes);
-  c->launches += 1;
+  uint32_t round = 128;
+  auto shaped = [&](const SkShape<KT> &s) {
+    a.slots = s.slots;
+    a.round = s.round;
+    a.hsize = sk_hash_size(s.round);
+    a.late = sk_late_at<KT>(s.slots, s.round);
+  };
+  for (const SkLaunch<KT> &l : launches) {
+    shaped(l.shape);
+    a.cls = l.cls;
+    a.ncls = l.ncls;
+    round = std::max(round, l.shape.round);
+    sk_count_launch<KT>(c, a, l.parts, l.shape.bytes);
+    c->launches += 1;
+  }
   if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
   const uint32_t n = (uint32_t)c->hctr->n_over;
   if (n && !c->hctr->err) {
-    const SkShape<KT> big(8000.0, shape.round);
+    const SkShape<KT> big(8000.0, round);
     cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
     a.todo = a.over;
     a.over += parts;
-    a.slots = big.slots;
-    a.round = big.round;
-    a.hsize = sk_hash_size(a.round);
-    a.late = sk_late_at<KT>(a.slots, a.round);
+    shaped(big);
     sk_count_launch<KT>(c, a, n, big.bytes);
     c->launches += 1;
     if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
@@ -3371,69 +3380,90 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const SkShape<KT>
   return BRUNO_OK;
 }
 
-/* The count of one sample by super-k-mers.  used = false (nothing counted, the caller takes the
- * k-mer records): a bin too large for one CTA, more records than room, or partitions that overflow
- * at every size tried. */
+/* The count by super-k-mers of the extracted records (one sample, or a batch's), kev[0] recorded
+ * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): a
+ * bin too large for one CTA, more records than room, or partitions that overflow at every size
+ * tried.  max_split: the partition plan's split bits. */
 template <class KT>
-bruno_status count_superkmers(Ctx *c, bool &used) {
+bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
   constexpr int NW = SkRec<KT>::NW, SU = Slot<KT>::U64;
   bruno_status st;
   used = false;
-  if (!c->pre_extracted) {
-    uint64_t bytes = 0;
-    for (auto &sg : c->segs) bytes += sg.n;
-    cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
-    if ((st = sk_begin(c, {bytes})) != BRUNO_OK) return st;
-    cudaEventRecord(c->kev[0], c->stream);
-    sk_extract_reads(c, 0, c->n_reads);
-  }
-  c->pre_extracted = false;   /* what was extracted serves this path alone */
-  sk_estimate<KT>(c, 1);
-  k_hll_sums<<<1, 256, 0, c->stream>>>((const unsigned int *)c->hllreg.p, (double *)c->hsum.p,
-                                       (unsigned int *)((double *)c->hsum.p + 1));
-  c->launches += 1;
+  const uint32_t S = c->S;
+  k_sk_estimate<KT><<<num_sms() * 4, 128, 0, c->stream>>>(
+      (const uint64_t *)c->sk_recs.p, (const uint32_t *)c->sk_est.p, c->sk_est_cap, c->cfg.k,
+      (const SkSample *)c->sk_samp.p, S, (unsigned int *)c->hllreg.p, c->dctr);
+  k_hll_sums<<<S, 256, 0, c->stream>>>((const unsigned int *)c->hllreg.p, (double *)c->hsum.p,
+                                       (unsigned int *)((double *)c->hsum.p + S));
+  c->launches += 2;
   cudaEventRecord(c->kev[1], c->stream);
-  double hs[2] = {0, 0};
-  cudaMemcpyAsync(hs, c->hsum.p, 16, cudaMemcpyDeviceToHost, c->stream);
+  std::vector<double> hs(2 * S), distinct(S);
+  cudaMemcpyAsync(hs.data(), c->hsum.p, (size_t)S * 16, cudaMemcpyDeviceToHost, c->stream);
+  if (S > 1) {
+    c->h_inst.assign(S, 0);
+    c->h_used.assign(S, 0);
+    cudaMemcpyAsync(c->h_inst.data(), c->s_inst.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(c->h_used.data(), c->s_used.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
+  }
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
   const uint64_t n_rec = c->hctr->n_sk, inst = c->hctr->n_instances;
-  if (c->hctr->err || n_rec > c->sk_cap || inst >> 32) return BRUNO_OK;
+  if (c->hctr->err || n_rec > c->sk_cap || inst >> 32 || n_rec >> 32) return BRUNO_OK;
   c->n_instances = inst;
   c->n_reads_used = c->hctr->n_reads_used;
-  double distinct = hll_estimate(hs[0], zeros_word(&hs[1]), c->sk_q[0]);
-  for (int attempt = 0; attempt < 3; ++attempt, distinct *= 2) {
-    const uint64_t slots = slots_for(c, distinct);
-    const bruno_table_plan::Plan plan = bruno_table_plan::partitions(slots, part_slots(c) * 4 / SU, MAX_SPLIT_BITS2);
-    if (!plan.fits) return BRUNO_OK;
-    const uint32_t parts = 1u << plan.pbits;
-    const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
-    /* regions are rounded up by two slots each; the rest as the load asks for */
-    const uint64_t cap = slots + 2ull * parts;
-    if ((st = table_room(c, cap)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->table, cap * SU * 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->cand, cap * 4)) != BRUNO_OK) return st;
+  const unsigned char *zeros = (const unsigned char *)(hs.data() + S);   /* S 32-bit words after the sums */
+  for (uint32_t q = 0; q < S; ++q) distinct[q] = hll_estimate(hs[q], zeros_word(zeros + 4 * q), c->sk_q[q]);
+  const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
+  const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
+  for (int attempt = 0; attempt < 3; ++attempt) {
+    std::vector<SGeom> sg(S);
+    std::vector<SkPlan> plan(S);
+    std::vector<uint64_t> region(S), caps(S);
+    uint64_t base = 0, parts = 0, before = 0;
+    uint32_t bin0 = 0;
+    for (uint32_t q = 0; q < S; ++q) {
+      const uint64_t slots = slots_for(c, distinct[q]), n_inst = S > 1 ? c->h_inst[q] : inst;
+      const bruno_table_plan::Plan pl = bruno_table_plan::partitions(slots, part_slots(c) * 4 / SU, max_split);
+      if (!pl.fits) return BRUNO_OK;
+      const uint64_t n = 1ull << pl.pbits;
+      caps[q] = slots + 2 * n;   /* a partition's slots are rounded up by two */
+      sg[q].g = TableGeom{caps[q], 0, pl.pbits, base, nullptr, nullptr, bin0, 32 - c->sk_bits[q], c->cfg.k};
+      sg[q].pbase = parts;
+      sg[q].rec2_base = sg[q].cap2 = 0;
+      plan[q] = SkPlan{before, std::max<uint64_t>(1, (n_inst + n - 1) / n), bin0, (uint32_t)parts, (uint32_t)n, 0u};
+      region[q] = pl.region;
+      before += n_inst;
+      base += caps[q];
+      parts += n;
+      bin0 += 1u << c->sk_bits[q];
+    }
+    if (parts >> 31) return BRUNO_OK;
+    if ((st = table_room(c, base)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->table, base * SU * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->cand, base * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_sorted, std::max<uint64_t>(1, n_rec) * NW * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_part, (size_t)c->sk_bins * 4)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_off, ((size_t)parts + 1) * 4)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_cur, (size_t)parts * 4)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_info, (size_t)parts * 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_over, (size_t)parts * 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_bump, 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sgeom, sizeof(SGeom))) != BRUNO_OK) return st;
-    c->geom = TableGeom{cap, 0, plan.pbits, 0, (const uint32_t *)c->sk_part.p, (const uint2 *)c->sk_info.p, 0u,
-                        32 - c->sk_bits[0], c->cfg.k};
-    const SGeom sg{c->geom, 0, 0, 0};
-    cudaMemcpyAsync(c->sgeom.p, &sg, sizeof(sg), cudaMemcpyHostToDevice, c->stream);
-    cudaMemsetAsync(c->sk_bump.p, 0, 8, c->stream);
+    if ((st = ensure(c, c->sk_off, (parts + 1) * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_cur, parts * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_info, parts * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_over, parts * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_bump, (size_t)S * 8)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sgeom, S * sizeof(SGeom))) != BRUNO_OK) return st;
+    for (SGeom &x : sg) {
+      x.g.bins = (const uint32_t *)c->sk_part.p;
+      x.g.info = (const uint2 *)c->sk_info.p;
+    }
+    if ((st = cuda_check(c, cudaMemcpyAsync(c->sgeom.p, sg.data(), S * sizeof(SGeom), cudaMemcpyHostToDevice, c->stream),
+                         "sample geometry")) != BRUNO_OK)
+      return st;
+    cudaMemsetAsync(c->sk_bump.p, 0, (size_t)S * 8, c->stream);
     cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
     cudaMemsetAsync(&c->dctr->n_cand, 0, sizeof(c->dctr->n_cand) + sizeof(c->dctr->quick_hist), c->stream);
     cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
     cudaMemsetAsync(&c->dctr->n_slots_claimed, 0, 16, c->stream);
     cudaMemsetAsync(&c->dctr->n_big, 0, 8, c->stream);
+    if (S > 1) cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
     cudaEventRecord(c->kev[2], c->stream);
-    if ((st = sk_partition<KT>(c, {SkPlan{0ull, std::max<uint64_t>(1, (inst + parts - 1) / parts), 0u, 0u, parts, 0u}}, parts,
-                               n_rec)) != BRUNO_OK)
-      return st;
+    if ((st = sk_partition<KT>(c, plan, (uint32_t)parts, n_rec)) != BRUNO_OK) return st;
     cudaEventRecord(c->kev[4], c->stream);
     SkCount a{};
     a.recs = (const uint64_t *)c->sk_sorted.p;
@@ -3447,20 +3477,56 @@ bruno_status count_superkmers(Ctx *c, bool &used) {
     a.info = (uint2 *)c->sk_info.p;
     a.over = (uint32_t *)c->sk_over.p;
     a.cand = (uint32_t *)c->cand.p;
+    a.s_tally = S > 1 ? (unsigned long long *)c->s_tally.p : nullptr;
     a.sg = (const SGeom *)c->sgeom.p;
-    a.nsamples = 1;
+    a.nsamples = S;
     a.bump = (unsigned long long *)c->sk_bump.p;
     a.ctr = c->dctr;
+    std::vector<SkLaunch<KT>> launches;
+    std::vector<ClassRun> runs;
+    if (S == 1) {
+      launches.push_back({(uint32_t)parts, SkShape<KT>(distinct[0] * 1.04 / parts, (double)n_rec / parts), nullptr, 0u});
+    } else {
+      /* a launch per region class (classes a factor of about 1.5 apart), its blocks shaped by the
+       * class's largest partitions */
+      std::vector<size_t> at;
+      for (int cl = 0; cl < bruno_table_plan::REGION_CLASSES; ++cl) {
+        const size_t first = runs.size();
+        uint32_t n = 0;
+        double kmers = 0, recs = 0;
+        for (uint32_t q = 0; q < S; ++q) {
+          if (bruno_table_plan::region_class(region[q]) != cl) continue;
+          runs.push_back(ClassRun{n, (uint32_t)sg[q].pbase});
+          n += plan[q].parts;
+          kmers = std::max(kmers, distinct[q] * 1.04 / plan[q].parts);
+          recs = std::max(recs, recs_per_kmer * (double)c->h_inst[q] / plan[q].parts);
+        }
+        if (!n) continue;
+        launches.push_back({n, SkShape<KT>(kmers, recs), nullptr, (uint32_t)(runs.size() - first)});
+        at.push_back(first);
+      }
+      if ((st = ensure(c, c->grp_tmp, runs.size() * sizeof(ClassRun) + 16)) != BRUNO_OK) return st;
+      if ((st = cuda_check(c, cudaMemcpyAsync(c->grp_tmp.p, runs.data(), runs.size() * sizeof(ClassRun),
+                                              cudaMemcpyHostToDevice, c->stream), "partition classes")) != BRUNO_OK)
+        return st;
+      for (size_t l = 0; l < launches.size(); ++l) launches[l].cls = (const ClassRun *)c->grp_tmp.p + at[l];
+    }
     bool ok = false;
-    if ((st = sk_count_parts<KT>(c, a, parts, SkShape<KT>(distinct * 1.04 / parts, (double)n_rec / parts), ok)) != BRUNO_OK)
-      return st;
+    if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, ok)) != BRUNO_OK) return st;
     cudaEventRecord(c->kev[3], c->stream);
     if (c->hctr->err & DERR_SKEW) return BRUNO_OK;
     if (ok) {
-      uint64_t used_slots = 0;
-      cudaMemcpyAsync(&used_slots, c->sk_bump.p, 8, cudaMemcpyDeviceToHost, c->stream);
+      std::vector<uint64_t> taken(S);
+      cudaMemcpyAsync(taken.data(), c->sk_bump.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
       if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "table slots")) != BRUNO_OK) return st;
-      c->nslots = c->geom.nslots = used_slots;
+      for (uint32_t q = 0; q < S; ++q) sg[q].g.nslots = taken[q];
+      c->geom = sg[0].g;
+      c->nslots = S == 1 ? taken[0] : base;
+      c->sk_gaps.clear();
+      if (S > 1) {
+        c->h_sgeom = sg;
+        c->sk_gaps = caps;
+      }
       float ms[3] = {0, 0, 0};
       cudaEventElapsedTime(&ms[0], c->kev[0], c->kev[1]);
       cudaEventElapsedTime(&ms[1], c->kev[2], c->kev[4]);
@@ -3471,13 +3537,31 @@ bruno_status count_superkmers(Ctx *c, bool &used) {
       c->phase_ms[9] = ms[1];
       c->n_entries = c->hctr->n_entries;
       c->n_slots_claimed = c->hctr->n_slots_claimed;
+      c->n_big = 0;
       c->have_cand = true;
       take_candidates(c);
       used = true;
       return BRUNO_OK;
     }
+    for (double &d : distinct) d *= 2;
   }
   return BRUNO_OK;
+}
+
+/* one sample: extraction, unless the read index did it as the pieces landed, and the count */
+template <class KT>
+bruno_status count_one_superkmers(Ctx *c, bool &used) {
+  if (!c->pre_extracted) {
+    uint64_t bytes = 0;
+    for (auto &sg : c->segs) bytes += sg.n;
+    cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
+    bruno_status st = sk_begin(c, {bytes});
+    if (st != BRUNO_OK) return st;
+    cudaEventRecord(c->kev[0], c->stream);
+    sk_extract_reads(c, 0, c->n_reads);
+  }
+  c->pre_extracted = false;   /* what was extracted serves this path alone */
+  return count_superkmers<KT>(c, MAX_SPLIT_BITS2, used);
 }
 
 /* The partitioned count for k > 31: exact k-mer positions size 256 buckets of 16-byte records,
@@ -3689,7 +3773,7 @@ bruno_status count_paths(Ctx *c) {
   }
   if (c->sk_on) {
     bool used = false;
-    bruno_status st = count_superkmers<KT>(c, used);
+    bruno_status st = count_one_superkmers<KT>(c, used);
     if (st != BRUNO_OK || used) return st;
     c->have_cand = false;
   }
@@ -3876,12 +3960,34 @@ bruno_status extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector
 }
 }  // namespace
 
+/* the same by super-k-mers: items of one sample's reads, several a warp so that the warps even out */
+namespace {
+bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f) {
+  bruno_status st;
+  const uint64_t nr = f.back() - f.front(), warps = (uint64_t)num_sms() * 32;
+  const uint64_t per = std::max<uint64_t>(32, std::min<uint64_t>(512, nr / (8 * warps)));
+  std::vector<XItem> items;
+  for (uint32_t q = q0; q < q1; ++q)
+    for (uint64_t a = f[q - q0]; a < f[q - q0 + 1]; a += per)
+      items.push_back(XItem{a, std::min<uint64_t>(f[q - q0 + 1], a + per), q, 0u});
+  if (items.empty()) return BRUNO_OK;
+  if ((st = ensure(c, c->xitems, items.size() * sizeof(XItem))) != BRUNO_OK) return st;
+  if ((st = cuda_check(c, cudaMemcpyAsync(c->xitems.p, items.data(), items.size() * sizeof(XItem), cudaMemcpyHostToDevice,
+                                          c->stream), "extraction items")) != BRUNO_OK)
+    return st;
+  sk_extract(c, 0, 0, (const XItem *)c->xitems.p, items.size(), nr, (unsigned long long *)c->s_inst.p,
+             (unsigned long long *)c->s_used.p);
+  return cuda_check(c, cudaGetLastError(), "k_sk_extract");
+}
+}  // namespace
+
 /* the read index's hook for a batch copied in groups: segment si (reads [r0, r1)) has landed */
 bruno_status batch_segment(Ctx *c, size_t si, uint64_t r0, uint64_t r1) {
   std::vector<uint64_t> f;
   const uint32_t q0 = c->seg_samp[si], q1 = c->seg_samp[si + 1];
   bruno_status st = first_reads(c, q0, q1, r0, r1, f);
-  return st != BRUNO_OK ? st : extract_samples(c, q0, q1, f);
+  if (st != BRUNO_OK) return st;
+  return c->sk_on ? sk_extract_samples(c, q0, q1, f) : extract_samples(c, q0, q1, f);
 }
 
 /* The batched form's count: S samples, concatenated in one device copy, each counted into
@@ -3891,6 +3997,33 @@ bruno_status run_count_samples(Ctx *c) {
   bruno_status st;
   c->have_cand = false;
   const uint32_t S = c->S;
+  if ((st = ensure(c, c->s_inst, (size_t)S * 8)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->s_used, (size_t)S * 8)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->s_tally, (size_t)S * T_NUM * 8)) != BRUNO_OK) return st;
+  cudaMemsetAsync(c->s_inst.p, 0, (size_t)S * 8, c->stream);
+  cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
+  cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
+  bool indexed = false;
+  if (S > 1 && sk_takes(c)) {   /* by super-k-mers, if the samples' minimizers allow it */
+    std::vector<uint64_t> bytes(S);
+    for (uint32_t q = 0; q < S; ++q) bytes[q] = c->samp_off[q + 1] - c->samp_off[q];
+    if ((st = sk_begin(c, bytes)) != BRUNO_OK) return st;
+    if (c->batch_piped) cudaEventRecord(c->kev[0], c->stream);
+    if ((st = run_index_reads(c)) != BRUNO_OK) return st;
+    indexed = true;
+    if ((st = first_reads(c, 0, S, 0, c->n_reads, c->samp_r0)) != BRUNO_OK) return st;
+    if (!c->batch_piped) {
+      cudaEventRecord(c->kev[0], c->stream);
+      if ((st = sk_extract_samples(c, 0, S, c->samp_r0)) != BRUNO_OK) return st;
+    }
+    bool used = false;
+    if ((st = count_superkmers<KW1>(c, MAX_SPLIT_BITS, used)) != BRUNO_OK || used) return st;
+    cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
+    cudaMemsetAsync(c->s_inst.p, 0, (size_t)S * 8, c->stream);
+    cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
+  }
+  c->sk_on = false;
+  c->sk_gaps.clear();
   const int sms = num_sms();
   /* per sample its buckets: capacities from its bytes, so they are known before any read is */
   c->x_cap.assign(S, 0);
@@ -3907,15 +4040,9 @@ bruno_status run_count_samples(Ctx *c) {
   if ((st = ensure(c, c->bucket_cnt, (size_t)S * NBUCKET * 8)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->xsamp, S * sizeof(XSample))) != BRUNO_OK) return st;
   if ((st = ensure(c, c->hllreg, (size_t)S * HLL_M * 4)) != BRUNO_OK) return st;
-  if ((st = ensure(c, c->s_inst, (size_t)S * 8)) != BRUNO_OK) return st;
-  if ((st = ensure(c, c->s_used, (size_t)S * 8)) != BRUNO_OK) return st;
-  if ((st = ensure(c, c->s_tally, (size_t)S * T_NUM * 8)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->hsum, (size_t)S * 16)) != BRUNO_OK) return st;
   cudaMemsetAsync(c->bucket_cnt.p, 0, (size_t)S * NBUCKET * 8, c->stream);
   cudaMemsetAsync(c->hllreg.p, 0, (size_t)S * HLL_M * 4, c->stream);
-  cudaMemsetAsync(c->s_inst.p, 0, (size_t)S * 8, c->stream);
-  cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
-  cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
   static const bool wattr = [] {
     cudaFuncSetAttribute(k_extract_s<KW1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(ExtractSmemT<KW1>));
@@ -3926,11 +4053,12 @@ bruno_status run_count_samples(Ctx *c) {
   (void)wattr;
   /* the read index (its counters reset first); a batch copied in groups extracts each group
    * as it lands (batch_segment), otherwise one launch over every sample follows */
-  if (c->batch_piped) cudaEventRecord(c->kev[0], c->stream);
-  if ((st = run_index_reads(c)) != BRUNO_OK) return st;
-  const uint64_t nreads = c->n_reads;
-  if ((st = first_reads(c, 0, S, 0, nreads, c->samp_r0)) != BRUNO_OK) return st;
-  if (!c->batch_piped) {
+  if (c->batch_piped && !indexed) cudaEventRecord(c->kev[0], c->stream);
+  if (!indexed) {
+    if ((st = run_index_reads(c)) != BRUNO_OK) return st;
+    if ((st = first_reads(c, 0, S, 0, c->n_reads, c->samp_r0)) != BRUNO_OK) return st;
+  }
+  if (!c->batch_piped || indexed) {
     cudaEventRecord(c->kev[0], c->stream);
     if ((st = extract_samples(c, 0, S, c->samp_r0)) != BRUNO_OK) return st;
   }
@@ -4006,7 +4134,30 @@ bruno_status run_filter(Ctx *c, const uint64_t *thresh) {
   return c->W == 1 ? filter_typed<KW1>(c, thresh) : filter_typed<KW2>(c, thresh);
 }
 
+bruno_status run_fill_gaps(Ctx *c) {
+  if (c->S <= 1 || c->sk_gaps.empty()) return BRUNO_OK;
+  const uint32_t S = c->S;
+  bruno_status st = ensure(c, c->fr_tmp, (size_t)S * 8);
+  if (st != BRUNO_OK) return st;
+  /* the samples' geometry with the slots they took (the device's copy has their whole shares) */
+  st = cuda_check(c, cudaMemcpyAsync(c->sgeom.p, c->h_sgeom.data(), S * sizeof(SGeom), cudaMemcpyHostToDevice, c->stream),
+                  "sample geometry");
+  if (st == BRUNO_OK)
+    st = cuda_check(c, cudaMemcpyAsync(c->fr_tmp.p, c->sk_gaps.data(), (size_t)S * 8, cudaMemcpyHostToDevice, c->stream),
+                    "sample shares");
+  if (st != BRUNO_OK) return st;
+  k_sk_fill_gaps<<<dim3(16, std::min<uint32_t>(S, 1024)), 256, 0, c->stream>>>(
+      (uint64_t *)c->table.p, (const SGeom *)c->sgeom.p, (const uint64_t *)c->fr_tmp.p, S);
+  c->launches += 1;
+  c->sk_gaps.clear();
+  return cuda_check(c, cudaGetLastError(), "k_sk_fill_gaps");
+}
+
 bruno_status run_copy_nodes(Ctx *c, uint64_t *keys, uint16_t *counts, uint8_t *flags, size_t cap, size_t *n) {
+  if (keys || counts || flags) {
+    bruno_status st = run_fill_gaps(c);
+    if (st != BRUNO_OK) return st;
+  }
   return run_copy_nodes_range(c, 0, c->nslots, c->n_nodes, keys, counts, flags, cap, n);
 }
 

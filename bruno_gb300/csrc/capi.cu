@@ -199,6 +199,7 @@ bruno_status bruno_reset(bruno_ctx *c) {
   c->samp_r0.clear();
   c->batch_piped = false;
   c->seg_samp.clear();
+  c->sk_gaps.clear();
   c->n_reads = c->n_reads_used = c->n_instances = c->n_entries = 0;
   c->n_k2 = c->n_filtered = 0;
   c->k2_dumped = false;
@@ -711,7 +712,10 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
   c->S = (uint32_t)n_samples;
   c->stage = 1;
   record(c, 0);
-  if ((st = run_count_samples(c)) != BRUNO_OK) return st;
+  c->one_call = true;
+  st = run_count_samples(c);
+  c->one_call = false;
+  if (st != BRUNO_OK) return st;
   record(c, 1);
   cudaEventSynchronize(c->ev[1]);
   if (c->batch_piped) {

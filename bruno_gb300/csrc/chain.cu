@@ -2577,15 +2577,21 @@ bruno_status run_chain_summaries(Ctx *c) {
 
 bruno_status run_node_query(Ctx *c, int filter, bool erase, uint64_t *keys, uint16_t *counts, uint8_t *flags,
                             size_t cap, size_t *n) {
+  const bruno_status gaps = run_fill_gaps(c);   /* they scan the whole table */
+  if (gaps != BRUNO_OK) return gaps;
   bruno_status st = c->W == 1 ? node_query_typed<KW1>(c, filter, erase, keys, counts, flags, cap, n)
                               : node_query_typed<KW2>(c, filter, erase, keys, counts, flags, cap, n);
   if (st != BRUNO_OK || !erase) return st;
   return c->W == 1 ? node_recount_typed<KW1>(c) : node_recount_typed<KW2>(c);
 }
 bruno_status run_check_index(Ctx *c, bruno_index_check *out) {
+  const bruno_status gaps = run_fill_gaps(c);   /* they scan the whole table */
+  if (gaps != BRUNO_OK) return gaps;
   return c->W == 1 ? check_index_typed<KW1>(c, out) : check_index_typed<KW2>(c, out);
 }
 bruno_status run_erase_nodes(Ctx *c, const uint64_t *kmers, size_t n) {
+  const bruno_status gaps = run_fill_gaps(c);   /* they scan the whole table */
+  if (gaps != BRUNO_OK) return gaps;
   return c->W == 1 ? erase_nodes_typed<KW1>(c, kmers, n) : erase_nodes_typed<KW2>(c, kmers, n);
 }
 bruno_status run_chain_query(Ctx *c, int filter, int which, uint64_t *kmers, uint64_t *inK, uint64_t *outK,

@@ -162,7 +162,8 @@ struct Ctx {
   /* one call builds the whole graph: the thresholds of the configuration are the ones the filter
    * will use and nobody asks for raw counts, so the count need not keep what the filter drops */
   bool one_call = false;
-  uint64_t sk_cap = 0;
+  uint64_t sk_cap = 0, sk_est_cap = 0;
+  std::vector<uint64_t> sk_gaps; /* a batch whose samples left table slots unwritten: their shares' sizes */
   uint32_t sk_bins = 0, sk_chunk = 32;
   std::vector<int> sk_bits, sk_q; /* per sample: log2 of its bins, of its estimate's sampling */
   bool h2d_pending = false;      /* ev[7] marks the start of the current graph build's host-to-device copies */
@@ -253,6 +254,8 @@ bruno_status run_chain_summaries(Ctx *c);
 bruno_status run_clean(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t *bubbles, uint64_t *edges,
                        int32_t *status);
 bruno_status run_copy_nodes(Ctx *c, uint64_t *keys, uint16_t *counts, uint8_t *flags, size_t cap, size_t *n);
+/* empties what a batch's samples left of their table shares, for a scan over the whole table */
+bruno_status run_fill_gaps(Ctx *c);
 /* the nodes of table slots [base, base + nslots), of which there are nn */
 bruno_status run_copy_nodes_range(Ctx *c, uint64_t base, uint64_t nslots, uint64_t nn, uint64_t *keys, uint16_t *counts,
                                   uint8_t *flags, size_t cap, size_t *n);

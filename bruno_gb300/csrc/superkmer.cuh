@@ -43,10 +43,13 @@ constexpr int SK_WORDS = 32;     /* a tile: one word of 16 bases a lane */
 constexpr int SK_HALO = 4;       /* words past the tile that a window of 49 m-mers may touch */
 constexpr int SK_READS = 16;     /* reads of a tile at most (the shortest that count take two words) */
 
+/* word t of a tile is bases[sk_pad + t]: a record of the other strand is cut out from its end, up to
+ * 2 * NW words before */
+template <int NW> constexpr int sk_pad = 2 * NW + 1;
 template <int NW>
 struct SkWarp {
   uint32_t pmin[16][SK_WORDS + SK_HALO];     /* prefix minima inside blocks; then the runs' minimizers */
-  uint32_t bases[1 + SK_WORDS + 2 * NW + 3]; /* 16 bases a word, first base on top; word t at t + 1 */
+  uint32_t bases[2 * NW + 1 + SK_WORDS + 2 * NW + 3]; /* 16 bases a word, first base on top; word t at sk_pad + t */
   uint32_t marks[SK_WORDS + 1];              /* bit i: a run starts, or the read's k-mers end, at base i */
   uint16_t starts[16 * SK_WORDS];            /* run starts of the tile */
   unsigned long long addr[SK_READS];
@@ -83,26 +86,10 @@ __device__ __forceinline__ uint2 sk_pack(uintptr_t s, int n) {
   return make_uint2(packed, err);
 }
 
-/* left shift of an NW-word number (word 0 the most significant) by s < 64 * NW bits */
-template <int NW>
-__device__ __forceinline__ void sk_shl(uint64_t *w, unsigned s) {
-  if (NW == 4 && (s & 128u)) { w[0] = w[2]; w[1] = w[3]; w[2] = 0; w[3] = 0; }
-  if (s & 64u) {
-    #pragma unroll
-    for (int i = 0; i < NW - 1; ++i) w[i] = w[i + 1];
-    w[NW - 1] = 0;
-  }
-  const unsigned r = s & 63u;
-  if (r) {
-    #pragma unroll
-    for (int i = 0; i < NW - 1; ++i) w[i] = (w[i] << r) | (w[i + 1] >> (64 - r));
-    w[NW - 1] <<= r;
-  }
-}
-/* the top `bits` bits of word i of an NW-word number kept by a mask of the top `n` bits overall */
-__device__ __forceinline__ uint64_t sk_top_mask(int n, int i) {
-  const int b = n - 64 * i;
-  return b <= 0 ? 0ull : b >= 64 ? ~0ull : ~0ull << (64 - b);
+/* 16 bases reversed */
+__device__ __forceinline__ uint32_t rev_pairs32(uint32_t x) {
+  x = __brev(x);
+  return ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
 }
 
 /* no record: the unused end of a chunk that a warp reserved (n - 1 is at most 48) */
@@ -168,8 +155,8 @@ struct SkExtract {
  * 1.2G k-mers).  Output places come in chunks that a warp reserves (one counter cannot take an
  * atomic per tile); a chunk's unused end is marked SK_NONE. */
 template <class KT, int BL>
-__global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
-  constexpr int NW = SkRec<KT>::NW, NB = 16 / BL;
+__global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
+  constexpr int NW = SkRec<KT>::NW, NB = 16 / BL, PAD = sk_pad<NW>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SkWarp<NW> &S = reinterpret_cast<SkWarp<NW> *>(smem_raw)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31, k = a.k;
@@ -179,52 +166,65 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
   const int piece = (16 * SK_WORDS - k - 1) & ~15;   /* k-mers of a long read's piece */
   for (int i = lane; i < 16 * SK_HALO; i += 32) S.pmin[i / SK_HALO][SK_WORDS + i % SK_HALO] = ~0u;
   if (lane == 0) S.marks[SK_WORDS] = 0;
-  const uint64_t warp = (uint64_t)blockIdx.x * (SK_TPB / 32) + (threadIdx.x >> 5), warps = (uint64_t)gridDim.x * (SK_TPB / 32);
-  unsigned long long inst_all = 0, used_all = 0;
-  unsigned long long cpos = 0, cend = 0;   /* the warp's chunk of the output */
-  bool over = false;
+  if (lane < PAD) S.bases[lane] = 0;   /* (what a record cuts from there is masked off) */
+  uint32_t cpos = 0, cend = 0;   /* the warp's chunk of the output (fewer than 2^32 records) */
   /* items of one sample each, or (one sample) an even share of the reads */
-  const uint64_t it0 = a.items ? warp * a.n_items / warps : 0, it1 = a.items ? (warp + 1) * a.n_items / warps : 1;
-  for (uint64_t it = it0; it < it1; ++it) {
-    uint64_t ra, rb;
+  uint32_t it, it1;
+  {
+    const uint32_t warp = blockIdx.x * (SK_TPB / 32) + (threadIdx.x >> 5), warps = gridDim.x * (SK_TPB / 32);
+    const uint64_t n = a.items ? a.n_items : warps;
+    it = (uint32_t)(warp * n / warps);
+    it1 = (uint32_t)((warp + 1) * n / warps);
+  }
+  for (; it < it1; ++it) {
+    uint64_t ra;
+    uint32_t n_reads;   /* reads of the item not yet taken */
     unsigned smp = 0;
-    if (a.items) { ra = a.items[it].a; rb = a.items[it].b; smp = a.items[it].s; }
-    else { ra = a.r0 + (a.r1 - a.r0) * warp / warps; rb = a.r0 + (a.r1 - a.r0) * (warp + 1) / warps; }
-    const SkSample X = a.samples[smp];
+    if (a.items) {
+      ra = a.items[it].a;
+      n_reads = (uint32_t)(a.items[it].b - ra);
+      smp = a.items[it].s;
+    } else {
+      const uint32_t warps = gridDim.x * (SK_TPB / 32);
+      ra = a.r0 + (a.r1 - a.r0) * it / warps;
+      n_reads = (uint32_t)(a.r0 + (a.r1 - a.r0) * (it + 1) / warps - ra);
+    }
     unsigned inst = 0, used = 0;
-    uint64_t sp = 0, ep = 0;   /* the read ra + lane */
-    if (ra + lane < rb) { sp = a.rstart[ra + lane]; ep = a.rend[ra + lane]; }
-    uint64_t q0 = 0;           /* first k-mer of the long read's next piece */
+    uint64_t sp = 0;           /* the read ra + lane */
+    uint32_t len = 0;
+    if (lane < n_reads) { sp = a.rstart[ra + lane]; len = (uint32_t)(a.rend[ra + lane] - sp); }
+    uint32_t q0 = 0;           /* first k-mer of the long read's next piece */
     bool long_ok = false;
-    while (ra < rb) {
+    while (n_reads) {
       /* (1) the tile's reads: as many as fit the words, or a piece of a long one */
       __syncwarp();   /* the tile before has been read */
-      const uint64_t L64 = ep - sp, L0 = __shfl_sync(~0u, L64, 0);
+      const uint32_t L0 = __shfl_sync(~0u, len, 0);
       unsigned first;
       uint32_t n_words, reads = 1;
       bool pre = false, post = false;
       if (L0 > 16 * SK_WORDS) {
-        const uint64_t s0 = __shfl_sync(~0u, sp, 0), nk = L0 - k + 1;
+        const uint64_t s0 = __shfl_sync(~0u, sp, 0);
+        const uint32_t nk = L0 - k + 1;
         if (q0 == 0) {   /* the whole read's bases checked before its first piece */
           unsigned bad = 0;
-          for (uint64_t p = 16 * lane; p < L0; p += 16 * SK_WORDS) bad |= sk_pack(s0 + p, (int)min((uint64_t)16, L0 - p)).y;
+          for (uint32_t p = 16 * lane; p < L0; p += 16 * SK_WORDS) bad |= sk_pack(s0 + p, (int)min(16u, L0 - p)).y;
           long_ok = !__any_sync(~0u, bad);
         }
-        const int n = (int)min((uint64_t)piece, nk - q0);
+        const int n = (int)min((uint32_t)piece, nk - q0);
         pre = q0 > 0;
         post = q0 + n < nk;
         if (lane == 0) {
           S.addr[0] = s0 + q0;
           S.nk[0] = n;
           S.len[0] = n + k - 1 + (post ? 1 : 0);
-          S.bases[0] = pre ? sk_pack(s0 + q0 - 1, 1).x >> 30 : 0u;
+          S.bases[PAD - 1] = pre ? sk_pack(s0 + q0 - 1, 1).x >> 30 : 0u;
         }
         first = long_ok ? 1u : 0u;
         n_words = long_ok ? (uint32_t)(n + k - 1 + (post ? 1 : 0) + 15) >> 4 : 0u;
         q0 += n;
         if (!long_ok || q0 >= nk) q0 = 0; else reads = 0;
       } else {
-        const uint32_t L = L64 >= (uint64_t)k + 2 ? (uint32_t)min(L64, (uint64_t)16 * SK_WORDS + 1) : 0u;
+        const uint32_t L = len >= (uint32_t)k + 2 ? min(len, 16u * SK_WORDS + 1) : 0u;
         const uint32_t nw = (L + 15) >> 4;
         uint32_t x = nw;
         #pragma unroll
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
           if (lane >= o) x += y;
         }
         /* x never falls, so the reads that fit come first */
-        const bool fits = ra + lane < rb && x <= SK_WORDS, kept = fits && nw;
+        const bool fits = lane < n_reads && x <= SK_WORDS, kept = fits && nw;
         const unsigned mf = __ballot_sync(~0u, fits), mk = __ballot_sync(~0u, kept);
         reads = __popc(mf);
         n_words = mf ? __shfl_sync(~0u, x, 31 - __clz(mf)) : 0u;
@@ -242,11 +242,13 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
           S.addr[d] = sp; S.len[d] = (int)L; S.nk[d] = (int)L - k + 1;
         }
         first = __reduce_or_sync(~0u, kept ? 1u << (x - nw) : 0u);
-        if (lane == 0) S.bases[0] = 0;
       }
       ra += reads;
-      if (reads && ra + lane < rb) { sp = a.rstart[ra + lane]; ep = a.rend[ra + lane]; }   /* the next tile's */
-      if (reads && ra + lane >= rb) { sp = 0; ep = 0; }
+      n_reads -= reads;
+      if (reads) {   /* the next tile's reads */
+        len = 0;
+        if (lane < n_reads) { sp = a.rstart[ra + lane]; len = (uint32_t)(a.rend[ra + lane] - sp); }
+      }
       if (n_words == 0) continue;
       __syncwarp();
       /* (2) the lane's word: 16 bases packed and checked */
@@ -260,8 +262,8 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
         L = S.len[rd];
         pk = sk_pack(S.addr[rd] + p0, min(16, L - p0));
       }
-      S.bases[lane + 1] = pk.x;
-      if (lane < 2 * NW + 3) S.bases[SK_WORDS + 1 + lane] = 0;
+      S.bases[PAD + lane] = pk.x;
+      if (lane < 2 * NW + 3) S.bases[PAD + SK_WORDS + lane] = 0;
       const unsigned bad = __ballot_sync(~0u, pk.y != 0);
       const bool good = mine && (bad & (~0u >> (32 - w2)) & (~0u << w0)) == 0;
       /* (3) the orders of the 16 m-mers that start in the word, then block minima */
@@ -269,12 +271,10 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
       uint32_t h[16];
       {
         const uint64_t W = ((uint64_t)pk.x << 32) | (lane < 31 ? nextw : 0u), R = rev_pairs(~W);
-        const int last = good ? L - MZ_M - p0 : -1;   /* m-mers past the read's last take no part */
+        /* (m-mers past the read's last are in no window of its k-mers) */
         #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const uint32_t o = mz_order((uint32_t)(W >> (64 - 2 * MZ_M - 2 * i)) & MZ_MASK, (uint32_t)(R >> (2 * i)) & MZ_MASK);
-          h[i] = i <= last ? o : ~0u;
-        }
+        for (int i = 0; i < 16; ++i)
+          h[i] = mz_order((uint32_t)(W >> (64 - 2 * MZ_M - 2 * i)) & MZ_MASK, (uint32_t)(R >> (2 * i)) & MZ_MASK);
         uint32_t m = ~0u;
         #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -297,10 +297,13 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
         }
         const int g = bb + qw;
         const uint32_t mid2 = min(mid, S.pmin[(g % NB) * BL + BL - 1][lane + g / NB]);
+        /* the windows' ends: BL - cw of them in the block qw further on, cw in the one after that */
+        const uint32_t *e1 = &S.pmin[(g % NB) * BL + cw][lane + g / NB];
+        const uint32_t *e2 = &S.pmin[((g + 1) % NB) * BL][lane + (g + 1) / NB] - (BL - cw) * (SK_WORDS + SK_HALO);
         #pragma unroll
         for (int i = 0; i < BL; ++i) {
-          const int e = bb * BL + i + w1;   /* the window's last m-mer, in positions from this word */
-          h[bb * BL + i] = min(h[bb * BL + i], min(i < BL - cw ? mid : mid2, S.pmin[e & 15][lane + (e >> 4)]));
+          const bool same = i < BL - cw;
+          h[bb * BL + i] = min(h[bb * BL + i], min(same ? mid : mid2, (same ? e1 : e2)[i * (SK_WORDS + SK_HALO)]));
         }
       }
       /* (4) run starts, and the end of the read's k-mers */
@@ -331,25 +334,22 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
       uint32_t at = x - cnt;
       __syncwarp();   /* every window has been read: the runs' minimizers instead */
       #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (st & (1u << i)) {
-          S.starts[at++] = (uint16_t)(16 * lane + i);
-          S.pmin[i][lane] = h[i];
-        }
+      for (int i = 0; i < 16; ++i) S.pmin[i][lane] = h[i];
+      for (uint32_t b = st; b; b &= b - 1) S.starts[at++] = (uint16_t)(16 * lane + __ffs(b) - 1);
       /* the tile's places: the rest of the chunk, then a new one */
-      const uint32_t rest = (uint32_t)min((unsigned long long)total, cend - cpos);
-      const unsigned long long o1 = cpos;
-      unsigned long long o2 = 0;
+      const uint32_t rest = min(total, cend - cpos), o1 = cpos;
+      uint32_t o2 = 0;
       cpos += rest;
       if (rest < total) {
-        const unsigned long long ch = max(a.chunk, total - rest);
-        if (lane == 0) o2 = atomicAdd(&a.ctr->n_sk, ch);
+        const uint32_t ch = max(a.chunk, total - rest);
+        if (lane == 0) o2 = (uint32_t)atomicAdd(&a.ctr->n_sk, (unsigned long long)ch);
         o2 = __shfl_sync(~0u, o2, 0);
         cpos = o2 + (total - rest);
         cend = o2 + ch;
       }
       __syncwarp();
       /* (5) the records */
+      const SkSample X = a.samples[smp];
       for (uint32_t y = lane; y < total; y += 32) {
         const int t = S.starts[y] >> 4, i = S.starts[y] & 15;
         const uint32_t mz = S.pmin[i][t];
@@ -365,64 +365,64 @@ __global__ void __launch_bounds__(SK_TPB, 4) k_sk_extract(SkExtract a) {
           run += __ffs(S.marks[u]) - 1;   /* (marks[SK_WORDS] exists and is never reached) */
         }
         const uint32_t mix = mz_mix(mz), bin = X.bin0 + (mix >> X.shift);
-        unsigned long long o = y < rest ? o1 + y : o2 + (y - rest);
+        uint32_t o = y < rest ? o1 + y : o2 + (y - rest);
         for (int d = 0; d < run; ) {   /* a minimizer that recurs may run on: cut at what a record holds */
-          const int n = min(run - d, k - MZ_M + 1), q = p + d - 1;   /* the base before the first k-mer */
-          const int tw = wr + 1 + (q >> 4);
-          const unsigned sh = 2u * (unsigned)(q & 15);
-          uint64_t w[NW];
+          const int n = min(run - d, k - MZ_M + 1), nb = n + k + 1, q = p + d - 1;   /* q: the base before the first k-mer */
+          bool hl = q >= 0 || pre, hr = p + d + n < nk || post;
+          const bool other = mz & 1u;   /* on the other strand: cut out from the end, then reversed */
+          const int b0 = 16 * (PAD + wr) + (other ? q + nb - 32 * NW : q), tw = b0 >> 4;
+          const unsigned sh = 2u * (unsigned)(b0 & 15);
+          uint32_t v[2 * NW];
           uint32_t cur = S.bases[tw];
           #pragma unroll
-          for (int u = 0; u < NW; ++u) {
-            const uint32_t b1 = S.bases[tw + 2 * u + 1], b2 = S.bases[tw + 2 * u + 2];
-            w[u] = ((uint64_t)__funnelshift_l(b1, cur, sh) << 32) | __funnelshift_l(b2, b1, sh);
-            cur = b2;
+          for (int u = 0; u < 2 * NW; ++u) {
+            const uint32_t nxt = S.bases[tw + u + 1];
+            v[u] = __funnelshift_l(nxt, cur, sh);
+            cur = nxt;
           }
-          bool hl = q >= 0 || pre, hr = p + d + n < nk || post;
-          const int nb = n + k + 1;
-          if (mz & 1u) {   /* the other strand: its first base is the complement of our last */
-            uint64_t z[NW];
+          if (other) {
             #pragma unroll
-            for (int u = 0; u < NW; ++u) z[u] = rev_pairs(~w[NW - 1 - u]);
-            sk_shl<NW>(z, 64u * NW - 2u * (unsigned)nb);
-            #pragma unroll
-            for (int u = 0; u < NW; ++u) w[u] = z[u];
+            for (int u = 0; u < NW; ++u) {
+              const uint32_t x = rev_pairs32(~v[u]);
+              v[u] = rev_pairs32(~v[2 * NW - 1 - u]);
+              v[2 * NW - 1 - u] = x;
+            }
             const bool s = hl; hl = hr; hr = s;
           }
-          const int bits = 2 * (hr ? nb : nb - 1);
+          const int bits = 2 * (hr ? nb : nb - 1);   /* past the last base, and the absent base before: zero */
           #pragma unroll
-          for (int u = 0; u < NW; ++u) w[u] &= sk_top_mask(bits, u);
-          if (!hl) w[0] &= ~0ull >> 2;
-          w[NW - 1] |= ((uint64_t)bin << SK_BIN_SHIFT) | (hr ? SK_RIGHT : 0ull) | (hl ? SK_LEFT : 0ull) | (uint64_t)(n - 1);
+          for (int u = 0; u < 2 * NW; ++u) v[u] &= __funnelshift_lc(0u, ~0u, (unsigned)max(0, 32 * (u + 1) - bits));
+          if (!hl) v[0] &= ~0u >> 2;
+          v[2 * NW - 1] |= (bin << SK_BIN_SHIFT) | (hr ? (uint32_t)SK_RIGHT : 0u) | (hl ? (uint32_t)SK_LEFT : 0u) | (uint32_t)(n - 1);
           if (o < a.cap) {
-            ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(a.out + o * NW);
+            ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(a.out + (uint64_t)o * NW);
             #pragma unroll
-            for (int u = 0; u < NW; u += 2) __stcs(dst + u / 2, make_ulonglong2(w[u], w[u + 1]));
-          } else over = true;
+            for (int u = 0; u < NW; u += 2)
+              __stcs(dst + u / 2, make_ulonglong2(((uint64_t)v[2 * u] << 32) | v[2 * u + 1],
+                                                  ((uint64_t)v[2 * u + 2] << 32) | v[2 * u + 3]));
+          } else {
+            atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
+          }
           atomicAdd(&a.hist[bin], ((unsigned long long)n << 32) | 1ull);
           if ((mix & X.smask) == 0) {
             const unsigned long long e = atomicAdd(&a.ctr->n_sk_est, 1ull);
-            if (e < a.est_cap) a.est[e] = (uint32_t)o;
+            if (e < a.est_cap) a.est[e] = o;
           }
           d += n;
-          if (d < run) o = atomicAdd(&a.ctr->n_sk, 1ull);
+          if (d < run) o = (uint32_t)atomicAdd(&a.ctr->n_sk, 1ull);
         }
       }
     }
     const unsigned long long iw = warp_sum(inst), uw = warp_sum(used);
     if (lane == 0) {
-      inst_all += iw; used_all += uw;
+      if (iw) atomicAdd(&a.ctr->n_instances, iw);
+      if (uw) atomicAdd(&a.ctr->n_reads_used, uw);
       if (a.s_inst && iw) atomicAdd(&a.s_inst[smp], iw);
       if (a.s_used && uw) atomicAdd(&a.s_used[smp], uw);
     }
   }
-  for (unsigned long long o = cpos + lane; o < cend; o += 32)
-    if (o < a.cap) a.out[o * NW + NW - 1] = SK_NONE;
-  if (lane == 0) {
-    if (inst_all) atomicAdd(&a.ctr->n_instances, inst_all);
-    if (used_all) atomicAdd(&a.ctr->n_reads_used, used_all);
-  }
-  if (over) atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
+  for (uint32_t o = cpos + lane; o < cend; o += 32)
+    if (o < a.cap) a.out[(uint64_t)o * NW + NW - 1] = SK_NONE;
 }
 
 /* ------------------------------------------------------------ bins -> partitions
@@ -581,7 +581,9 @@ constexpr uint32_t SK_LATE = 256;
 struct SkCount {
   const uint64_t *recs;
   const uint32_t *off;              /* first record of every partition */
-  const uint32_t *todo;             /* NULL: partition blockIdx.x; else the partitions to count */
+  const uint32_t *todo;             /* the partitions to count; NULL: those of `cls`, or all */
+  const ClassRun *cls;              /* a batch's partitions of one size class, as runs of samples */
+  uint32_t ncls;
   uint32_t slots;                   /* k-mer slots in shared memory */
   uint32_t late;                    /* where the late k-mers wait, in shared-memory words */
   uint32_t round, hsize;            /* records a round (at most 1024), entries of their hash (a power of two) */
@@ -755,7 +757,12 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   __shared__ unsigned int s_qh[4], s_claims;
   __shared__ unsigned long long s_cand;
   if (a.ctr->err & DERR_SKEW) return;
-  const uint32_t part = a.todo ? a.todo[blockIdx.x] : blockIdx.x;
+  uint32_t part = a.todo ? a.todo[blockIdx.x] : blockIdx.x;
+  if (a.cls && !a.todo) {
+    uint32_t lo = 0, hi = a.ncls;
+    while (hi - lo > 1) { const uint32_t m = (lo + hi) >> 1; if (__ldg(&a.cls[m].run) <= blockIdx.x) lo = m; else hi = m; }
+    part = a.cls[lo].pbase + (blockIdx.x - a.cls[lo].run);
+  }
   const int tid = threadIdx.x, lane = tid & 31, k = a.k;
   const uint32_t nt = blockDim.x, slots = a.slots, round = a.round;
   const SkSlots<KT> sl(sm, slots);
@@ -1044,5 +1051,15 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     for (int i = 0; i < SU; i += 2)
       reinterpret_cast<ulonglong2 *>(dst + (uint64_t)pos * SU)[i / 2] =
           make_ulonglong2(i < KWD ? KEY_EMPTY : 0ull, i + 1 < KWD ? KEY_EMPTY : 0ull);
+  }
+}
+
+/* the slots of every sample's share of the table past the ones its regions took, for calls that
+ * scan a batch's table (used: per sample, the slots taken) */
+__global__ void k_sk_fill_gaps(uint64_t *table, const SGeom *sg, const uint64_t *cap, uint32_t S) {
+  for (uint32_t q = blockIdx.y; q < S; q += gridDim.y) {
+    const uint64_t lo = (sg[q].g.base + sg[q].g.nslots) * 4, hi = (sg[q].g.base + cap[q]) * 4;
+    for (uint64_t i = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (uint64_t)gridDim.x * blockDim.x)
+      table[i] = (i & 3) == 0 ? KEY_EMPTY : 0ull;
   }
 }

@@ -66,8 +66,6 @@ def low_mmer(seed):
         y >>= np.uint64(2)
     m = np.uint64(0xFFFFFFFF)
     h = ((np.minimum(x, r) ^ np.uint64(0x2C9277B5)) * np.uint64(0x9E3779B1)) & m
-    h ^= h >> np.uint64(15)
-    h = (h * np.uint64(0x85EBCA6B)) & m
     v = int(x[np.argmin(h)])
     return "".join("ACGT"[(v >> (2 * (M - 1 - i))) & 3] for i in range(M))
 
