@@ -395,7 +395,31 @@ __global__ void __launch_bounds__(TPB) k_lr_apply(ChainState *cs, const uint32_t
  * neighbouring rulers, the ruler lists are ranked by pointer jumping, and every node adds
  * its offset to its ruler's ranks. */
 constexpr uint32_t RULER_SAMPLE = 32;
-struct Jump { uint32_t t; uint32_t fd; uint64_t d; }; /* ruler ordinal; flip | done << 1; distance */
+/* A link of the ruler lists in one word, so that the lists can be jumped in place (a side reads a
+ * neighbour's link while that one moves on: either is a valid link): ruler ordinal, flip, done,
+ * distance (the caller checks that the chain nodes are fewer than 2^30). */
+struct Jump {
+  uint64_t w;   /* [done:1 | flip:1 | ordinal:31 | distance:31] */
+  __device__ __forceinline__ Jump() : w(0) {}
+  __device__ __forceinline__ Jump(uint32_t t, uint32_t fd, uint64_t d)
+      : w(((uint64_t)(fd >> 1) << 63) | ((uint64_t)(fd & 1u) << 62) | ((uint64_t)t << 31) | (d < 0x7FFFFFFFull ? d : 0x7FFFFFFFull)) {}
+  __device__ __forceinline__ uint32_t t() const { return (uint32_t)(w >> 31) & 0x7FFFFFFFu; }
+  __device__ __forceinline__ uint32_t flip() const { return (uint32_t)(w >> 62) & 1u; }
+  __device__ __forceinline__ bool done() const { return (w >> 63) != 0; }
+  __device__ __forceinline__ uint64_t d() const { return w & 0x7FFFFFFFull; }
+};
+
+/* The ranking works on the chain nodes, or on segments of them: maximal runs whose nodes lie in one
+ * block of SEG_N consecutive chain indices.  In a table filled by super-k-mers neighbours mostly
+ * share a partition, so a segment holds the k-mers of a minimizer's run (8.5 nodes at k = 31, 20 at
+ * k = 63) and ranking the segments takes that share of the random reads.  A segment is a node
+ * of the same kind: side 0 leads out of its left end, side 1 out of its right end, and it
+ * counts for `n` nodes; the weight of a node or segment is the upper half of its state's
+ * spare word (the lower half: its ruler ordinal). */
+constexpr int SEG_N = 2048;
+struct SegInfo { uint32_t L, R, n, pad; };   /* left and right ends as node << 1 | side that leads out; nodes */
+constexpr uint32_t SEG_OFF = 1;              /* a node's place: segment, steps from its left end << 1 | reversed */
+__device__ __forceinline__ uint32_t weight_of(const ChainState &s) { return (uint32_t)(s.pad >> 32); }
 
 __device__ __forceinline__ bool side_terminal(uint32_t D) { return (D & DM) == 0; }
 __device__ __forceinline__ uint64_t side_ptr(const ChainState &s, int side) { return side ? s.outP : s.inP; }
@@ -407,7 +431,10 @@ __device__ __forceinline__ uint32_t side_dist(const ChainState &s, int side) { r
  * read that gives it the next pointer.  The other half -- every chain pointer is answered by
  * the facing side of its target -- is checked by the first walk for every node it passes and
  * by the marking pass for the nodes no walk reaches. */
-__global__ void __launch_bounds__(TPB) k_fast_check(ChainState *cs, uint64_t M, uint32_t *rnode, DevCounters *ctr) {
+/* n_dev: the number of nodes in device memory (segments), or NULL */
+__global__ void __launch_bounds__(TPB) k_fast_check(ChainState *cs, uint64_t M, const unsigned long long *n_dev,
+                                                    const SegInfo *seg, uint32_t *rnode, DevCounters *ctr) {
+  if (n_dev) M = *n_dev;
   unsigned long long bad = 0;
   for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < M; i0 += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t v = i0 + threadIdx.x;
@@ -423,7 +450,7 @@ __global__ void __launch_bounds__(TPB) k_fast_check(ChainState *cs, uint64_t M, 
       ruler = term_side || (mix64(v * 0x9e3779b97f4a7c15ull + 0x632be59bd9b4e019ull) % RULER_SAMPLE) == 0;
     }
     const unsigned long long o = block_append(ruler, &ctr->lr_remaining);
-    if (v < M) cs[v].pad = ruler ? o : (uint64_t)NONE32;
+    if (v < M) cs[v].pad = (ruler ? o : (uint64_t)NONE32) | ((uint64_t)(seg ? seg[v].n : 1u) << 32);
     if (ruler) rnode[o] = (uint32_t)v;
   }
   bad = warp_sum(bad);
@@ -438,23 +465,133 @@ __device__ __forceinline__ bool answers(const ChainState &t, int facing, uint32_
          (((back & PF_FLIP) ? 1u : 0u) == f);
 }
 
+/* Chain nodes -> segments (SEG_N nodes a block).  A side is a state (node, side); a state whose
+ * pointer leads to another node of the block goes on at the state that pointer arrives at, any
+ * other stops.  Pointer jumping in shared memory finds both stops of every node; the node whose
+ * side is the smaller stop opens the segment.  Pointers inside the block are checked both ways
+ * here, pointers between segments in k_seg_link.  Nodes of a cycle inside the block get no
+ * segment.
+ *
+ * Bound: 32 bytes read and 8 written a node, and about 6 rounds over 16 KB of shared memory. */
+constexpr int SEG_STOP = 12;   /* a state word: next state, steps to it from this bit on (0: it stops) */
+__global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_t M, uint2 *place, SegInfo *seg,
+                                                   DevCounters *ctr) {
+  __shared__ uint32_t nx[2 * SEG_N];
+  __shared__ uint16_t ord[2 * SEG_N];
+  __shared__ uint32_t s_n, s_base;
+  const uint64_t base = (uint64_t)blockIdx.x * SEG_N;
+  const int n = (int)min((uint64_t)SEG_N, M - base), tid = threadIdx.x;
+  unsigned long long bad = 0;
+  for (int i = tid; i < n; i += TPB) {
+    const ChainState st = cs[base + i];
+    #pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const uint64_t P = side_ptr(st, s);
+      const uint32_t D = side_dist(st, s), x = 2u * i + s;
+      uint32_t w = x;
+      if (!side_terminal(D)) {
+        const uint64_t u = (uint64_t)(uint32_t)P - base;
+        if (D != 1 || (P & (PF_EXT | PF_BLANK))) ++bad;
+        else if (u < (uint64_t)n && u != (uint64_t)i) w = (2u * (uint32_t)u + (s ^ ((P & PF_FLIP) ? 1u : 0u))) | (1u << SEG_STOP);
+      }
+      nx[x] = w;
+    }
+  }
+  if (tid == 0) s_n = 0;
+  __syncthreads();
+  constexpr uint32_t IDX = (1u << SEG_STOP) - 1;
+  static_assert(2 * SEG_N == 1 << SEG_STOP, "a state fits its bits");
+  for (int x = tid; x < 2 * n; x += TPB)   /* arriving at state y, the other side of its node points back */
+    if (nx[x] >> SEG_STOP && nx[(nx[x] & IDX) ^ 1u] != ((uint32_t)(x ^ 1) | (1u << SEG_STOP))) ++bad;
+  __syncthreads();
+  for (int round = 0; round < SEG_STOP; ++round) {   /* 2^12 steps cover any path of the block */
+    bool moved = false;
+    for (int x = tid; x < 2 * n; x += TPB) {
+      const uint32_t w = nx[x], t = nx[w & IDX];
+      if ((w >> SEG_STOP) && (t >> SEG_STOP)) {
+        nx[x] = (t & IDX) | (((w >> SEG_STOP) + (t >> SEG_STOP)) << SEG_STOP);
+        moved = true;
+      }
+    }
+    if (!__syncthreads_or(moved)) break;
+  }
+  /* (a node on a cycle: its states never come to a stop) */
+  for (int i = tid; i < n; i += TPB) {
+    const uint32_t e0 = nx[2 * i] & IDX, e1 = nx[2 * i + 1] & IDX, l = min(e0, e1);
+    if ((l >> 1) == (uint32_t)i && !(nx[e0] >> SEG_STOP) && !(nx[e1] >> SEG_STOP)) ord[l] = (uint16_t)atomicAdd(&s_n, 1u);
+  }
+  __syncthreads();
+  if (tid == 0) s_base = s_n ? (uint32_t)atomicAdd(&ctr->n_seg, (unsigned long long)s_n) : 0u;
+  __syncthreads();
+  for (int i = tid; i < n; i += TPB) {
+    const uint32_t w0 = nx[2 * i], w1 = nx[2 * i + 1], e0 = w0 & IDX, e1 = w1 & IDX;
+    uint2 pl = make_uint2(NONE32, 0u);
+    if (!(nx[e0] >> SEG_STOP) && !(nx[e1] >> SEG_STOP)) {
+      const uint32_t l = min(e0, e1), rev = e0 > e1, off = (rev ? w1 : w0) >> SEG_STOP;
+      pl = make_uint2(s_base + ord[l], (off << SEG_OFF) | rev);
+      if ((l >> 1) == (uint32_t)i)
+        seg[pl.x] = SegInfo{(uint32_t)(2 * base) + l, (uint32_t)(2 * base) + max(e0, e1),
+                            (w0 >> SEG_STOP) + (w1 >> SEG_STOP) + 1u, 0u};
+    }
+    place[base + i] = pl;
+  }
+  bad = warp_sum(bad);
+  if ((tid & 31) == 0 && bad) atomicAdd(&ctr->lr_multi, bad);
+}
+
+/* a segment's state: each end's pointer out, to the segment of the node it names, or the end's own
+ * terminal side */
+__global__ void __launch_bounds__(TPB) k_seg_link(const ChainState *cs, const uint2 *place, const SegInfo *seg,
+                                                  ChainState *rs, DevCounters *ctr) {
+  const uint64_t n = ctr->n_seg;
+  unsigned long long bad = 0;
+  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
+    const SegInfo si = seg[g];
+    ChainState r;
+    r.pad = 0;
+    #pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const uint32_t end = s ? si.R : si.L, a = end >> 1, sa = end & 1u;
+      const ChainState st = cs[a];
+      uint64_t P = side_ptr(st, sa);
+      uint32_t D = side_dist(st, sa);
+      if (!side_terminal(D)) {
+        const uint32_t u = (uint32_t)P, f = (P & PF_FLIP) ? 1u : 0u, dir = sa ^ f;   /* dir: the side that leads on at u */
+        const uint2 pl = place[u];
+        if (!answers(cs[u], 1 - (int)dir, a, f) || pl.x == NONE32) ++bad;
+        const uint32_t F = (uint32_t)s ^ dir ^ (pl.y & 1u);
+        P = (uint64_t)(pl.x == NONE32 ? 0u : pl.x) | (F ? PF_FLIP : 0ull);
+        D = 1;
+      }
+      if (s) { r.outP = P; r.outD = D; } else { r.inP = P; r.inD = D; }
+    }
+    rs[g] = r;
+  }
+  bad = warp_sum(bad);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&ctr->lr_multi, bad);
+}
+
 /* Walk 1: every non-terminal ruler side walks to the next ruler and records (that ruler,
  * flip parity, gap) -- the first pointer-jumping link.  A terminal side is a finished link
  * to itself.  One read per step, which also checks that the node stepped to points back; the
  * grid is one resident wave, so each thread walks several sides and the geometric walk
- * lengths average out. */
-__global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const uint32_t *rnode, uint64_t R, uint64_t M,
-                                                    Jump *E0, uint64_t *place, DevCounters *ctr) {
+ * lengths average out.  (R: read from the counters, as the host does not wait for it.) */
+__global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const uint32_t *rnode, uint64_t M,
+                                                    const unsigned long long *n_dev, Jump *E0, uint64_t *place,
+                                                    DevCounters *ctr) {
   unsigned long long bad = 0;
+  const uint64_t R = ctr->lr_remaining;
+  if (n_dev) M = *n_dev;
   for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * R; q += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t ord = (uint32_t)(q >> 1), r = rnode[ord];
     const int s0 = (int)(q & 1);
     ChainState st = cs[r];
-    if (side_terminal(side_dist(st, s0))) { E0[q] = Jump{ord, 2u, 0}; continue; }
+    if (side_terminal(side_dist(st, s0))) { E0[q] = Jump(ord, 2u, 0); continue; }
     uint32_t flip = 0, cur = r;
     int dir = s0;
-    Jump out{ord, 0u, 0};   /* unreachable in a consistent map: every walk meets a ruler */
-    for (uint64_t dist = 1; dist <= M; ++dist) {
+    uint64_t d = 0;
+    Jump out(ord, 0u, 0);   /* unreachable in a consistent map: every walk meets a ruler */
+    for (uint64_t step = 1; step <= M; ++step) {
       const uint64_t P = side_ptr(st, dir);
       if (side_dist(st, dir) != 1 || (P & (PF_EXT | PF_BLANK))) { ++bad; break; }
       const uint32_t f = (P & PF_FLIP) ? 1u : 0u, nxt = (uint32_t)P;
@@ -463,9 +600,10 @@ __global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const u
       st = cs[nxt];
       if (!answers(st, 1 - dir, cur, f)) { ++bad; break; }
       cur = nxt;
-      if ((uint32_t)st.pad != NONE32) { out = Jump{(uint32_t)st.pad, flip, dist}; break; }
+      d += weight_of(st);
+      if ((uint32_t)st.pad != NONE32) { out = Jump((uint32_t)st.pad, flip, d); break; }
       /* the node's place on the segment, in the slot of the direction this walk crosses it */
-      if (place) place[2ull * nxt + dir] = ((uint64_t)q << 32) | (dist << 1) | flip;
+      if (place) place[2ull * nxt + dir] = ((uint64_t)q << 32) | (step << 1) | flip;
     }
     E0[q] = out;
   }
@@ -473,19 +611,25 @@ __global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const u
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&ctr->lr_multi, bad);
 }
 
-__global__ void __launch_bounds__(TPB) k_fast_jump(const Jump *E, Jump *F, uint64_t R, DevCounters *ctr) {
+/* one round of pointer jumping, in place but for the first (F = E0's copy to be); undone: the sides
+ * that have not reached an end.  A side whose neighbour is done is done after the round, so a
+ * round that leaves as many undone as the one before has only ruler cycles left. */
+__global__ void __launch_bounds__(TPB) k_fast_jump(const Jump *E, Jump *F, DevCounters *ctr, int round) {
   unsigned long long undone = 0;
+  const uint64_t R = ctr->lr_remaining;
+  if (round > 0 && ctr->lr_round[round - 1] == 0) return;
   for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * R; q += (uint64_t)gridDim.x * blockDim.x) {
-    Jump e = E[q];
-    if (!(e.fd & 2u)) {
+    Jump e;
+    e.w = *(volatile const uint64_t *)&E[q].w;
+    if (!e.done()) {
       const int s = (int)(q & 1);
-      const uint32_t f = e.fd & 1u;
-      const Jump n = E[2ull * e.t + (f ? 1 - s : s)];   /* continue in the same travel direction */
-      const uint64_t sum = e.d + n.d;   /* saturate: only ruler cycles keep growing */
-      e = Jump{n.t, (f ^ (n.fd & 1u)) | (n.fd & 2u), sum > 0xFFFFFFFFFFFFull ? 0xFFFFFFFFFFFFull : sum};
+      const uint32_t f = e.flip();
+      Jump n;   /* continue in the same travel direction */
+      n.w = *(volatile const uint64_t *)&E[2ull * e.t() + (f ? 1 - s : s)].w;
+      e = Jump(n.t(), (f ^ n.flip()) | (n.done() ? 2u : 0u), e.d() + n.d());   /* (saturates on ruler cycles) */
     }
-    undone += !(e.fd & 2u);
-    F[q] = e;
+    undone += !e.done();
+    *(volatile uint64_t *)&F[q].w = e.w;
   }
   undone = warp_sum(undone);
   __shared__ unsigned long long s_undone;
@@ -493,26 +637,27 @@ __global__ void __launch_bounds__(TPB) k_fast_jump(const Jump *E, Jump *F, uint6
   __syncthreads();
   if ((threadIdx.x & 31) == 0 && undone) atomicAdd(&s_undone, undone);
   __syncthreads();
-  if (threadIdx.x == 0 && s_undone) atomicAdd(&ctr->lr_applied, s_undone);
+  if (threadIdx.x == 0 && s_undone) atomicAdd(&ctr->lr_round[round], s_undone);
 }
 
 /* final state of one side: the path end in that direction, its flip, the distance */
 __device__ __forceinline__ void fast_side(const uint32_t *rnode, const Jump &e, uint32_t flip, uint64_t d,
                                           uint64_t &P, uint32_t &D) {
-  P = (uint64_t)rnode[e.t] | (((flip ^ (e.fd & 1u)) != 0) ? PF_FLIP : 0ull);
+  P = (uint64_t)rnode[e.t()] | (((flip ^ e.flip()) != 0) ? PF_FLIP : 0ull);
   D = (uint32_t)d | TM;
 }
 
 /* rulers on paths: both non-terminal sides point at their path ends */
 __global__ void __launch_bounds__(TPB) k_fast_rulers(const ChainState *cs, ChainState *cs2, const uint32_t *rnode,
-                                                      uint64_t R, const Jump *E) {
+                                                      const Jump *E, const DevCounters *ctr) {
+  const uint64_t R = ctr->lr_remaining;
   for (uint64_t a = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; a < R; a += (uint64_t)gridDim.x * blockDim.x) {
     const Jump e0 = E[2 * a], e1 = E[2 * a + 1];
-    if (!(e0.fd & 2u) || !(e1.fd & 2u)) continue;   /* a ruler cycle: left for the cycle pass */
+    if (!e0.done() || !e1.done()) continue;   /* a ruler cycle: left for the cycle pass */
     const uint32_t v = rnode[a];
     ChainState st = cs[v];
-    if (!side_terminal(st.inD)) fast_side(rnode, e0, 0, e0.d, st.inP, st.inD);
-    if (!side_terminal(st.outD)) fast_side(rnode, e1, 0, e1.d, st.outP, st.outD);
+    if (!side_terminal(st.inD)) fast_side(rnode, e0, 0, e0.d(), st.inP, st.inD);
+    if (!side_terminal(st.outD)) fast_side(rnode, e1, 0, e1.d(), st.outP, st.outD);
     cs2[v] = st;
   }
 }
@@ -522,34 +667,41 @@ __global__ void __launch_bounds__(TPB) k_fast_rulers(const ChainState *cs, Chain
  * gets its final state: the side facing the walk's start leads past the start ruler to the
  * end E[start side'] and the other side past the far ruler to E[start side].  The walk reads
  * the chain map and writes the final states into a second array, so no step waits behind a
- * store to the array it reads. */
+ * store to the array it reads.  Distances run from the end of a node's (segment's) side: forward
+ * from the far end of the node at j steps it is the start's less j, back from its near end it
+ * is the j steps without its own weight, the start's weight, and the start's other distance. */
 __global__ void __launch_bounds__(TPB) k_fast_fill(const ChainState *cs, ChainState *cs2, const uint32_t *rnode,
-                                                    uint64_t R, const Jump *E0, const Jump *E) {
+                                                    const Jump *E0, const Jump *E, const DevCounters *ctr) {
+  const uint64_t R = ctr->lr_remaining;
   for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * R; q += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t ord = (uint32_t)(q >> 1);
     const int s0 = (int)(q & 1);
     const Jump link = E0[q];
-    if (link.fd & 2u) continue;                                   /* terminal side */
-    if (!(link.t > ord || (link.t == ord && s0 == 1))) continue;  /* walked from the other end */
+    if (link.done()) continue;                                            /* terminal side */
+    if (!(link.t() > ord || (link.t() == ord && s0 == 1))) continue;      /* walked from the other end */
     const Jump ef = E[q], eb = E[q ^ 1];
-    if (!(ef.fd & 2u) || !(eb.fd & 2u)) continue;                 /* a ruler cycle */
-    const uint64_t Pb_t = rnode[eb.t], Pf_t = rnode[ef.t];
+    if (!ef.done() || !eb.done()) continue;                               /* a ruler cycle */
+    const uint64_t Pb_t = rnode[eb.t()], Pf_t = rnode[ef.t()];
     ChainState st = cs[rnode[ord]];
+    const uint64_t back = eb.d() + weight_of(st);
     uint32_t flip = 0;
     int dir = s0;
-    for (uint64_t j = 1; j < link.d; ++j) {
+    for (uint64_t j = 0; ; ) {
       const uint64_t P = side_ptr(st, dir);
       const uint32_t v = (uint32_t)P;
       const uint32_t f = (P & PF_FLIP) ? 1u : 0u;
       flip ^= f;
       dir = f ? 1 - dir : dir;
       st = cs[v];
+      const uint64_t wt = weight_of(st);
+      j += wt;
+      if (j >= link.d()) break;   /* the far ruler */
       ChainState w;
       w.pad = st.pad;
       /* side 1-dir faces the walk's start ruler, side dir leads on to the far ruler */
-      const uint64_t Pb = Pb_t | (((flip ^ (eb.fd & 1u)) != 0) ? PF_FLIP : 0ull);
-      const uint64_t Pf = Pf_t | (((flip ^ (ef.fd & 1u)) != 0) ? PF_FLIP : 0ull);
-      const uint32_t Db = (uint32_t)(j + eb.d) | TM, Df = (uint32_t)(ef.d - j) | TM;
+      const uint64_t Pb = Pb_t | (((flip ^ eb.flip()) != 0) ? PF_FLIP : 0ull);
+      const uint64_t Pf = Pf_t | (((flip ^ ef.flip()) != 0) ? PF_FLIP : 0ull);
+      const uint32_t Db = (uint32_t)(j - wt + back) | TM, Df = (uint32_t)(ef.d() - j) | TM;
       if (dir) { w.inP = Pb; w.inD = Db; w.outP = Pf; w.outD = Df; }
       else { w.outP = Pb; w.outD = Db; w.inP = Pf; w.inD = Df; }
       cs2[v] = w;
@@ -573,12 +725,12 @@ __global__ void __launch_bounds__(TPB) k_fast_place(const ChainState *cs, ChainS
     const uint64_t q = p >> 32, j = (p >> 1) & 0x7FFFFFFFull;
     const uint32_t flip = (uint32_t)(p & 1u);
     const Jump ef = E[q], eb = E[q ^ 1];
-    if (!(ef.fd & 2u) || !(eb.fd & 2u)) continue;                 /* a ruler cycle */
+    if (!ef.done() || !eb.done()) continue;                 /* a ruler cycle */
     ChainState w;
     w.pad = cs[v].pad;
-    const uint64_t Pb = (uint64_t)rnode[eb.t] | (((flip ^ (eb.fd & 1u)) != 0) ? PF_FLIP : 0ull);
-    const uint64_t Pf = (uint64_t)rnode[ef.t] | (((flip ^ (ef.fd & 1u)) != 0) ? PF_FLIP : 0ull);
-    const uint32_t Db = (uint32_t)(j + eb.d) | TM, Df = (uint32_t)(ef.d - j) | TM;
+    const uint64_t Pb = (uint64_t)rnode[eb.t()] | (((flip ^ eb.flip()) != 0) ? PF_FLIP : 0ull);
+    const uint64_t Pf = (uint64_t)rnode[ef.t()] | (((flip ^ ef.flip()) != 0) ? PF_FLIP : 0ull);
+    const uint32_t Db = (uint32_t)(j + eb.d()) | TM, Df = (uint32_t)(ef.d() - j) | TM;
     if (dir) { w.inP = Pb; w.inD = Db; w.outP = Pf; w.outD = Df; }
     else { w.outP = Pb; w.outD = Db; w.inP = Pf; w.inD = Df; }
     cs2[v] = w;
@@ -588,7 +740,46 @@ __global__ void __launch_bounds__(TPB) k_fast_place(const ChainState *cs, ChainS
 /* removed[] (1 = cycle: the node got no final state, 2 = isolated: both sides terminal), the
  * counts, and the longest path in nodes.  cs2 starts as all ones, which no final state is. */
 constexpr uint32_t CS2_UNSET = 0xFFFFFFFFu;
-__global__ void __launch_bounds__(TPB) k_fast_mark(const ChainState *cs, const ChainState *cs2, uint64_t M,
+
+/* the final state of node v from its segment's: on from the segment's ends by its place in it, or to
+ * the segment's own end where that is the path's (unset for nodes of cycles) */
+__device__ __forceinline__ ChainState expand_node(const ChainState *cs, uint64_t v, uint2 pl, const SegInfo *seg,
+                                                  const ChainState *rs2) {
+  ChainState st;
+  st.inP = st.outP = st.pad = ~0ull;
+  st.inD = st.outD = CS2_UNSET;
+  if (pl.x == NONE32) return st;
+  const ChainState g = rs2[pl.x];
+  if (g.inD == CS2_UNSET) return st;
+  const SegInfo si = seg[pl.x];
+  const ChainState own = cs[v];
+  const uint32_t rev = pl.y & 1u, off = pl.y >> SEG_OFF;
+  uint64_t P[2];
+  uint32_t D[2];
+  #pragma unroll
+  for (int s = 0; s < 2; ++s) {   /* the segment's side s, which the node's side s ^ rev leads to */
+    const uint32_t mine = (uint32_t)s ^ rev, steps = s ? si.n - 1u - off : off, Dg = side_dist(g, s);
+    if (side_terminal(Dg)) {
+      const uint32_t end = s ? si.R : si.L;
+      P[s] = steps ? (uint64_t)(end >> 1) | (((end & 1u) != mine) ? PF_FLIP : 0ull) : side_ptr(own, (int)mine);
+      D[s] = steps ? steps | TM : side_dist(own, (int)mine);
+    } else {
+      const uint64_t Pg = side_ptr(g, s);
+      const SegInfo e = seg[(uint32_t)Pg];
+      const uint32_t end = ((uint32_t)s ^ ((Pg & PF_FLIP) ? 1u : 0u)) ? e.R : e.L;
+      P[s] = (uint64_t)(end >> 1) | (((end & 1u) != mine) ? PF_FLIP : 0ull);
+      D[s] = (steps + (Dg & DM)) | TM;
+    }
+  }
+  st.inP = rev ? P[1] : P[0]; st.inD = rev ? D[1] : D[0];
+  st.outP = rev ? P[0] : P[1]; st.outD = rev ? D[0] : D[1];
+  st.pad = 0;
+  return st;
+}
+
+/* place != NULL: the nodes' final states are made here from their segments' (written to cs2) */
+__global__ void __launch_bounds__(TPB) k_fast_mark(const ChainState *cs, ChainState *cs2, uint64_t M, const uint2 *place,
+                                                    const SegInfo *seg, const ChainState *rs2,
                                                     uint8_t *removed, unsigned long long *nmax,
                                                     const uint32_t *csample, unsigned long long *s_tally,
                                                     DevCounters *ctr) {
@@ -598,7 +789,13 @@ __global__ void __launch_bounds__(TPB) k_fast_mark(const ChainState *cs, const C
     const uint64_t v = v0 + threadIdx.x;
     uint32_t cyc_v = 0, iso_v = 0, mx_v = 0;
     if (v < M) {
-      const ChainState st = cs2[v];
+      ChainState st;
+      if (place) {
+        st = expand_node(cs, v, place[v], seg, rs2);
+        cs2[v] = st;
+      } else {
+        st = cs2[v];
+      }
       const bool cyc = st.inD == CS2_UNSET;
       uint8_t r = 0;
       if (cyc) {
@@ -2427,7 +2624,12 @@ bruno_status clean_typed(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t 
 bruno_status run_extract_chains(Ctx *c) { return c->W == 1 ? extract_typed<KW1>(c) : extract_typed<KW2>(c); }
 
 /* The ruling-set ranking; returns false (and changes nothing) if the chain map is not
- * mutually consistent, in which case the round-synchronous path runs. */
+ * mutually consistent, in which case the round-synchronous path runs.  Over segments where the
+ * chain indices follow the table's minimizer partitions (50M nodes, k = 31: 8.1 ms over the
+ * nodes); over the nodes themselves where they follow a hash, or with rank_fill = 1.  The host
+ * waits once for the first rounds of pointer jumping (and before that for the number of segments
+ * where it sizes gigabytes): what the kernels find inconsistent is looked at then, every
+ * index being in range whatever the pointers say. */
 static bruno_status fast_list_rank(Ctx *c, bool &used) {
   bruno_status st;
   used = false;
@@ -2439,18 +2641,49 @@ static bruno_status fast_list_rank(Ctx *c, bool &used) {
   if ((st = ensure(c, c->removed, Mb)) != BRUNO_OK) return st;
   uint32_t *rnode = (uint32_t *)c->unf1.p;
   cudaMemsetAsync(&c->dctr->lr_applied, 0, 32, c->stream);   /* applied, remaining, cycles, multi */
-  k_fast_check<<<sms * 8, TPB, 0, c->stream>>>(cs, M, rnode, c->dctr);
+  cudaMemsetAsync(&c->dctr->n_seg, 0, 8 + sizeof(c->dctr->lr_round), c->stream);
+  const bool over_segs = c->geom.bins && c->cfg.rank_fill != 1 && M > 0;
+  constexpr uint64_t WAIT = 4ull << 20;   /* from here on sizes are worth waiting for */
+  auto blocks = [&](uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (n + TPB - 1) / TPB)); };
+  uint64_t N = M;                          /* nodes or segments ranked (segments: at most) */
+  ChainState *rs = cs, *rs2 = nullptr;
+  const unsigned long long *n_dev = nullptr;
+  uint2 *in_seg = nullptr;
+  SegInfo *seg = nullptr;
+  if (over_segs) {
+    if ((st = ensure(c, c->seg_place, Mb * sizeof(uint2))) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->seg_info, Mb * sizeof(SegInfo))) != BRUNO_OK) return st;
+    in_seg = (uint2 *)c->seg_place.p;
+    seg = (SegInfo *)c->seg_info.p;
+    k_seg_local<<<(unsigned)((M + SEG_N - 1) / SEG_N), TPB, 0, c->stream>>>(cs, M, in_seg, seg, c->dctr);
+    c->launches += 2;   /* and k_seg_link */
+    if (M > WAIT) {
+      if ((st = sync_counters(c)) != BRUNO_OK) return st;
+      if (c->hctr->lr_multi != 0) return BRUNO_OK;            /* inconsistent pointers */
+      N = c->hctr->n_seg;
+    }
+    const uint64_t Nb = std::max<uint64_t>(1, N);
+    if ((st = ensure(c, c->seg_state, Nb * 2 * sizeof(ChainState))) != BRUNO_OK) return st;
+    rs = (ChainState *)c->seg_state.p;
+    rs2 = rs + Nb;
+    n_dev = &c->dctr->n_seg;
+    k_seg_link<<<blocks(N), TPB, 0, c->stream>>>(cs, in_seg, seg, rs, c->dctr);
+  }
+  k_fast_check<<<blocks(N), TPB, 0, c->stream>>>(rs, N, n_dev, seg, rnode, c->dctr);
   c->launches += 1;
-  if ((st = sync_counters(c)) != BRUNO_OK) return st;
-  if (c->hctr->lr_multi != 0) return BRUNO_OK;                /* inconsistent pointers */
-  const uint64_t R = c->hctr->lr_remaining, Rb = std::max<uint64_t>(1, R);
-  if ((st = ensure(c, c->pay, Rb * 2 * sizeof(Jump) * 3)) != BRUNO_OK) return st;
-  Jump *E0 = (Jump *)c->pay.p, *E = E0 + 2 * Rb, *F = E + 2 * Rb;
+  uint64_t Rb = std::max<uint64_t>(1, N);   /* rulers at most */
+  if (N > WAIT) {
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    if (c->hctr->lr_multi != 0) return BRUNO_OK;
+    Rb = std::max<uint64_t>(1, c->hctr->lr_remaining);
+  }
+  if ((st = ensure(c, c->pay, Rb * 2 * sizeof(Jump) * 2)) != BRUNO_OK) return st;
+  Jump *E0 = (Jump *)c->pay.p, *E = E0 + 2 * Rb;
   static const int walk_occ = [] {   /* resident walk blocks per SM: the walks run as one wave */
     int o = 0;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_fast_walk, TPB, 0) == cudaSuccess && o > 0 ? o : 4;
   }();
-  const int gw = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * walk_occ, (2 * R + TPB - 1) / TPB));
+  const int gw = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * walk_occ, (2 * Rb + TPB - 1) / TPB));
   uint64_t *place = nullptr;
   Buf place_buf;
   struct FreeOnExit {   /* the places go back to the pool on every way out */
@@ -2462,38 +2695,33 @@ static bruno_status fast_list_rank(Ctx *c, bool &used) {
     place = (uint64_t *)place_buf.p;
     cudaMemsetAsync(place, 0xFF, M * 16, c->stream);
   }
-  k_fast_walk<<<gw, TPB, 0, c->stream>>>(cs, rnode, R, M, E0, place, c->dctr);
+  k_fast_walk<<<gw, TPB, 0, c->stream>>>(rs, rnode, N, n_dev, E0, place, c->dctr);
   c->launches += 1;
-  if ((st = sync_counters(c)) != BRUNO_OK) return st;
-  if (c->hctr->lr_multi != 0) return BRUNO_OK;                /* a pointer not answered by its target */
-  const Jump *src = E0;
-  uint64_t prev = ~0ull;
-  for (int round = 0; round < 64; ++round) {
-    cudaMemsetAsync(&c->dctr->lr_applied, 0, 8, c->stream);
-    k_fast_jump<<<gw, TPB, 0, c->stream>>>(src, E, R, c->dctr);
-    c->launches += 1;
-    src = E;
-    std::swap(E, F);
+  constexpr int BATCH = 8, ROUNDS = 64;   /* rounds queued at once; a finished one costs a launch */
+  for (int round = 0; round < ROUNDS; ) {
+    for (int i = 0; i < BATCH; ++i, ++round)
+      k_fast_jump<<<gw, TPB, 0, c->stream>>>(round ? E : E0, E, c->dctr, round);
+    c->launches += BATCH;
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
-    const uint64_t undone = c->hctr->lr_applied;
-    if (undone == 0 || undone == prev) break;   /* only ruler cycles keep sides undone */
-    prev = undone;
+    if (c->hctr->lr_multi != 0) return BRUNO_OK;   /* inconsistent, or a pointer not answered by its target */
+    const unsigned long long *u = c->hctr->lr_round;
+    if (u[round - 1] == 0 || u[round - 1] == u[round - 2]) break;   /* only ruler cycles keep sides undone */
   }
   /* final states go to a second chain-state array (all ones = unset), which then becomes
    * the chain map; a node left unset is a cycle node, whose state nothing reads again */
   if ((st = ensure(c, c->cstate2, Mb * sizeof(ChainState))) != BRUNO_OK) return st;
   ChainState *cs2 = (ChainState *)c->cstate2.p;
-  cudaMemsetAsync(cs2, 0xFF, M * sizeof(ChainState), c->stream);
+  if (!over_segs) rs2 = cs2;
+  cudaMemsetAsync(rs2, 0xFF, N * sizeof(ChainState), c->stream);
   if (place) {
-    k_fast_place<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, rnode, M, src, place);
+    k_fast_place<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, rnode, M, E, place);
   } else {
-    k_fast_fill<<<gw, TPB, 0, c->stream>>>(cs, cs2, rnode, R, E0, src);
+    k_fast_fill<<<gw, TPB, 0, c->stream>>>(rs, rs2, rnode, E0, E, c->dctr);
   }
-  k_fast_rulers<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (R + TPB - 1) / TPB)), TPB, 0,
-                  c->stream>>>(cs, cs2, rnode, R, src);
+  k_fast_rulers<<<blocks(Rb), TPB, 0, c->stream>>>(rs, rs2, rnode, E, c->dctr);
   cudaMemsetAsync(&c->dctr->n_cycle, 0, 16, c->stream);
   cudaMemsetAsync(&c->dctr->n_heads, 0, 8, c->stream);        /* longest path, in nodes */
-  k_fast_mark<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, M, (uint8_t *)c->removed.p, &c->dctr->n_heads,
+  k_fast_mark<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, M, in_seg, seg, rs2, (uint8_t *)c->removed.p, &c->dctr->n_heads,
                                                c->S > 1 ? (const uint32_t *)c->csample.p : nullptr,
                                                c->S > 1 ? (unsigned long long *)c->s_tally.p : nullptr, c->dctr);
   c->launches += 3;

@@ -33,6 +33,8 @@ struct DevCounters {
   unsigned long long flag_hist[16];
   unsigned long long lr_applied, lr_remaining, lr_cycles, lr_multi;
   unsigned long long n_cycle, n_isolated, n_ranked, n_heads, n_chain_chars;
+  unsigned long long n_seg;            /* segments of chain nodes */
+  unsigned long long lr_round[64];     /* ranking: sides not at their end after each round of jumping */
   unsigned long long n_upper;          /* k-mer positions of all reads long enough */
   unsigned long long n_chain_edges;    /* chain-end records appended */
   unsigned long long n_groups, n_hist; /* general emission: representative groups, histogram bins */
@@ -194,6 +196,7 @@ struct Ctx {
   Buf blk_cnt, blk_base;
 
   /* chains */
+  Buf seg_place, seg_info, seg_state;   /* ranking over segments of chain nodes */
   Buf ckey, cedge, cstate, cstate2, pend, pay, unf0, unf1, removed;
   uint64_t iterations = 0, n_cycle = 0, n_isolated = 0, multi = 0;
   bool exact_ranking = false;    /* force the round-synchronous ranking (tests) */
