@@ -1778,19 +1778,24 @@ __global__ void __launch_bounds__(TPB) k_cl_isolated(uint64_t *table, uint64_t n
   }
 }
 
+constexpr int CL_TILE = 2048;
 /* IsBranchPoint / IsChainNode again for every node (the filter's rule, debruijn_graph_filters.hpp
  * :57-220), with the chain and branch lists and each chain node's index rebuilt */
 template <class KT>
 __global__ void __launch_bounds__(TPB) k_cl_classify(uint64_t *table, uint64_t nslots, int k, uint32_t *chain_list,
                                                       uint32_t *branch_list, uint64_t cap, DevCounters *ctr) {
   constexpr int KWD = Slot<KT>::KEYW, SU = Slot<KT>::U64;
+  /* a block lists CL_TILE consecutive slots at a time, so that chain indices follow the table: the
+   * ranking contracts neighbours whose indices are near */
+  __shared__ uint32_t s_list[CL_TILE], s_nc, s_nb;
+  __shared__ unsigned long long s_base_c, s_base_b;
   bool over = false;
-  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < nslots; i0 += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = i0 + threadIdx.x;
-    uint64_t *s = table + (i < nslots ? i : 0) * SU;
-    const bool node = i < nslots && key_is_node(KOps<KT>::load(s));
-    bool branch = false;
-    if (node) {
+  for (uint64_t i0 = (uint64_t)blockIdx.x * CL_TILE; i0 < nslots; i0 += (uint64_t)gridDim.x * CL_TILE) {
+    if (threadIdx.x == 0) { s_nc = 0; s_nb = 0; }
+    __syncthreads();
+    for (uint64_t i = i0 + threadIdx.x; i < min(nslots, i0 + CL_TILE); i += TPB) {
+      const uint64_t *s = table + i * SU;
+      if (!key_is_node(KOps<KT>::load(s))) continue;
       const KT key = key_kmer(node_key(KOps<KT>::load(s)));
       const bool kpal = k_palindrome(key, k);
       const bool high = km1_high_palindrome(key, k), low = km1_low_palindrome(key, k);
@@ -1805,17 +1810,28 @@ __global__ void __launch_bounds__(TPB) k_cl_classify(uint64_t *table, uint64_t n
         if (oddk && o && low && (first == 3u - c || first == c)) k1pal = true;
         if (oddk && n && high && (last == 3u - c || last == c)) k1pal = true;
       }
-      branch = din >= 2 || dout >= 2 || kpal || k1pal;
+      /* chain nodes from the front of the list, branch nodes from its back */
+      if (din >= 2 || dout >= 2 || kpal || k1pal) s_list[CL_TILE - 1 - atomicAdd(&s_nb, 1u)] = (uint32_t)i;
+      else s_list[atomicAdd(&s_nc, 1u)] = (uint32_t)i;
     }
-    const unsigned long long oc = block_append(node && !branch, &ctr->n_chain);
-    const unsigned long long ob = block_append(node && branch, &ctr->n_branch);
-    if (node) {
-      const unsigned long long o = branch ? ob : oc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_base_c = s_nc ? atomicAdd(&ctr->n_chain, (unsigned long long)s_nc) : 0ull;
+      s_base_b = s_nb ? atomicAdd(&ctr->n_branch, (unsigned long long)s_nb) : 0ull;
+    }
+    __syncthreads();
+    const uint32_t nc = s_nc, n = nc + s_nb;
+    for (uint32_t x = threadIdx.x; x < n; x += TPB) {
+      const bool branch = x >= nc;
+      const uint32_t i = s_list[branch ? CL_TILE - 1 - (x - nc) : x];
+      const unsigned long long o = branch ? s_base_b + (x - nc) : s_base_c + x;
       if (o >= cap) { over = true; continue; }
+      uint64_t *s = table + (uint64_t)i * SU;
       const uint64_t aux = branch ? 0xFFFFFFFFull : o;
       s[KWD + 2] = (s[KWD + 2] & 0xFFFFull) | ((uint64_t)(branch ? NF_BRANCH : NF_CHAIN) << 16) | (aux << 32);
-      (branch ? branch_list : chain_list)[o] = (uint32_t)i;
+      (branch ? branch_list : chain_list)[o] = i;
     }
+    __syncthreads();   /* the list and its counts have been read */
   }
   if (over) atomicOr(&ctr->err, (unsigned long long)DERR_INVARIANT);
 }
@@ -1824,8 +1840,8 @@ __global__ void __launch_bounds__(TPB) k_cl_classify(uint64_t *table, uint64_t n
  * chain end (IsTerminusOrIsolated), oriented so that the 5' terminus is the representative,
  * with the end node's total in- or out-edge frequency.  tslot: record index per chain node. */
 template <class KT>
-__global__ void __launch_bounds__(TPB) k_cl_termini(EmitArgs a, const uint64_t *table, TableGeom g, FSum<KT> *trec,
-                                                     uint32_t *tslot, DevCounters *ctr) {
+__global__ void __launch_bounds__(TPB) k_cl_termini(EmitArgs a, const uint64_t *table, const uint32_t *chain_list,
+                                                     FSum<KT> *trec, uint32_t *tslot, DevCounters *ctr) {
   constexpr int KWD = KOps<KT>::WORDS, SU = Slot<KT>::U64;
   unsigned long long nz = 0;
   bool bad = false, missing = false;
@@ -1841,9 +1857,9 @@ __global__ void __launch_bounds__(TPB) k_cl_termini(EmitArgs a, const uint64_t *
         const KT K = KOps<KT>::load(a.ckey + i * KWD);
         const KT inK = side_kmer<KT>(st.inP, a), outK = side_kmer<KT>(st.outP, a);
         uint16_t fin = 0, fout = 0;
-        const long long s = table_find<KT>(table, g, 4096u, K);
-        if (s < 0) missing = true;
-        else { fout = total_of(table[(uint64_t)s * SU + KWD]); fin = total_of(table[(uint64_t)s * SU + KWD + 1]); }
+        const uint64_t *s = table + (uint64_t)chain_list[i] * SU;   /* the node's slot, unless it was cleared */
+        if (!key_is_node(KOps<KT>::load(s))) missing = true;
+        else { fout = total_of(s[KWD]); fin = total_of(s[KWD + 1]); }
         const KT Z{};
         r.len = (st.inD & DM) + (st.outD & DM);
         r.node = (uint32_t)i;
@@ -2531,7 +2547,8 @@ bruno_status clean_typed(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t 
     FSum<KT> *trec = (FSum<KT> *)c->cl_trec.p;
     cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
     cudaMemsetAsync(&c->dctr->cl_term, 0, 8 * 8, c->stream);   /* cl_term .. cl_bub */
-    if (M) k_cl_termini<KT><<<sms * 8, TPB, 0, c->stream>>>(a, table, c->geom, trec, (uint32_t *)c->cl_tslot.p, c->dctr);
+    if (M) k_cl_termini<KT><<<sms * 8, TPB, 0, c->stream>>>(
+        a, table, (const uint32_t *)c->chain_list.p, trec, (uint32_t *)c->cl_tslot.p, c->dctr);
     c->launches += 1;
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     const uint64_t nt = c->hctr->cl_term, ntb = std::max<uint64_t>(1, nt);
