@@ -3170,7 +3170,7 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
  * so do builds without thresholds: they keep every k-mer, and 3.5M nodes at 12x (13.7M k-mers,
  * k = 31) took 3.28 ms by super-k-mers against 3.09 */
 bool sk_takes(const Ctx *c) {
-  return c->cfg.k >= MZ_M + 4 && c->cfg.thresholding && !c->cfg.edge_filter && c->force_direct_count == 0 &&
+  return c->cfg.k >= MZ_M + 4 && !c->cfg.edge_filter && c->force_direct_count == 0 &&
          c->cfg.table_slots == 0;
 }
 
@@ -3315,7 +3315,7 @@ struct SkShape {
   uint32_t slots, round;
   size_t bytes;
   SkShape(double kmers, double records) {
-    slots = ((uint32_t)std::min(8000.0, 2.0 * kmers + 64.0 + 100.0 * (kmers < 400.0)) + 31u) & ~31u;
+    slots = ((uint32_t)std::min(8000.0, 1.8 * kmers + 64.0 + 100.0 * (kmers < 400.0)) + 31u) & ~31u;
     round = std::max(128u, std::min(sizeof(KT) == 8 ? 1024u : 512u, ((uint32_t)(1.15 * records) + 63u) & ~63u));
     while ((bytes = sk_count_bytes<KT>(slots, round)) > MOST) slots -= 32;
   }
@@ -3439,7 +3439,15 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if (parts >> 31) return BRUNO_OK;
     if ((st = table_room(c, base)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->table, base * SU * 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->cand, base * 4)) != BRUNO_OK) return st;
+    /* one call: the count makes the nodes, and lists them; a kept k-mer takes inv_load slots */
+    const bool nodes = c->one_call && !c->cfg.keep_k2 && !c->cfg.keep_filtered;
+    const uint64_t list_cap = (uint64_t)((double)base / inv_load) + 1;
+    if (nodes) {
+      if ((st = ensure(c, c->chain_list, list_cap * 4)) != BRUNO_OK) return st;
+      if ((st = ensure(c, c->branch_list, list_cap * 4)) != BRUNO_OK) return st;
+    } else if ((st = ensure(c, c->cand, base * 4)) != BRUNO_OK) {
+      return st;
+    }
     if ((st = ensure(c, c->sk_sorted, std::max<uint64_t>(1, n_rec) * NW * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_part, (size_t)c->sk_bins * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_off, (parts + 1) * 4)) != BRUNO_OK) return st;
@@ -3460,6 +3468,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     cudaMemsetAsync(&c->dctr->n_cand, 0, sizeof(c->dctr->n_cand) + sizeof(c->dctr->quick_hist), c->stream);
     cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
     cudaMemsetAsync(&c->dctr->n_slots_claimed, 0, 16, c->stream);
+    cudaMemsetAsync(&c->dctr->n_nodes, 0, offsetof(DevCounters, lr_applied) - offsetof(DevCounters, n_nodes), c->stream);
     cudaMemsetAsync(&c->dctr->n_big, 0, 8, c->stream);
     if (S > 1) cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
     cudaEventRecord(c->kev[2], c->stream);
@@ -3469,14 +3478,18 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     a.recs = (const uint64_t *)c->sk_sorted.p;
     a.off = (const uint32_t *)c->sk_off.p;
     a.k = c->cfg.k;
-    a.keep_all = !(c->one_call && c->cfg.thresholding && !c->cfg.keep_k2);
+    a.keep_all = !nodes && !(c->one_call && c->cfg.thresholding && !c->cfg.keep_k2);
     a.thresholding = c->cfg.thresholding;
     for (int i = 0; i < 6; ++i) a.t[i] = (uint32_t)std::min<uint64_t>(65536, c->cfg.thresh[i]);
     a.inv_load = inv_load;
     a.table = (uint64_t *)c->table.p;
     a.info = (uint2 *)c->sk_info.p;
     a.over = (uint32_t *)c->sk_over.p;
-    a.cand = (uint32_t *)c->cand.p;
+    a.cand = nodes ? nullptr : (uint32_t *)c->cand.p;
+    a.nodes = nodes;
+    a.chain_list = (uint32_t *)c->chain_list.p;
+    a.branch_list = (uint32_t *)c->branch_list.p;
+    a.list_cap = list_cap;
     a.s_tally = S > 1 ? (unsigned long long *)c->s_tally.p : nullptr;
     a.sg = (const SGeom *)c->sgeom.p;
     a.nsamples = S;
@@ -3538,8 +3551,16 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
       c->n_entries = c->hctr->n_entries;
       c->n_slots_claimed = c->hctr->n_slots_claimed;
       c->n_big = 0;
-      c->have_cand = true;
+      c->have_cand = !nodes;
       take_candidates(c);
+      c->nodes_made = nodes;
+      if (nodes) {
+        c->n_chain = c->hctr->n_chain;
+        c->n_branch = c->hctr->n_branch;
+        c->n_nodes = c->n_chain + c->n_branch;
+        for (int f = 0; f < 16; ++f) c->flag_hist[f] = c->hctr->flag_hist[f] + c->hctr->quick_hist[f];
+        c->filter_read = c->hctr->n_cand;
+      }
       used = true;
       return BRUNO_OK;
     }
@@ -3794,7 +3815,7 @@ bruno_status count_paths(Ctx *c) {
 /* counting, then the entries counted past 2^24 (if any) resolved for the filter */
 template <class KT>
 bruno_status count_typed(Ctx *c) {
-  c->have_cand = false;
+  c->have_cand = c->nodes_made = false;
   bruno_status st = count_paths<KT>(c);
   if (st != BRUNO_OK) return st;
   c->n_big = c->hctr->n_big;
@@ -3829,6 +3850,11 @@ bruno_status dump_k2_typed(Ctx *c) {
 template <class KT>
 bruno_status filter_typed(Ctx *c, const uint64_t *thr) {
   bruno_status st;
+  if (c->nodes_made) {   /* the count made the nodes (one call: its thresholds are these) */
+    c->nodes_made = false;
+    c->n_filtered = 0;
+    return cuda_check(c, cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream), "counters");
+  }
   FilterArgs a{};
   a.table = (uint64_t *)c->table.p;
   a.nslots = c->nslots;
@@ -3995,7 +4021,7 @@ bruno_status batch_segment(Ctx *c, size_t si, uint64_t r0, uint64_t r1) {
  * plain build is a batch of one).  Needs k <= 31 and the shared-memory partitions. */
 bruno_status run_count_samples(Ctx *c) {
   bruno_status st;
-  c->have_cand = false;
+  c->have_cand = c->nodes_made = false;
   const uint32_t S = c->S;
   if ((st = ensure(c, c->s_inst, (size_t)S * 8)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->s_used, (size_t)S * 8)) != BRUNO_OK) return st;

@@ -164,6 +164,7 @@ struct Ctx {
   /* one call builds the whole graph: the thresholds of the configuration are the ones the filter
    * will use and nobody asks for raw counts, so the count need not keep what the filter drops */
   bool one_call = false;
+  bool nodes_made = false;       /* ... and the count made the nodes */
   uint64_t sk_cap = 0, sk_est_cap = 0;
   std::vector<uint64_t> sk_gaps; /* a batch whose samples left table slots unwritten: their shares' sizes */
   uint32_t sk_bins = 0, sk_chunk = 32;

@@ -575,7 +575,8 @@ __global__ void __launch_bounds__(256) k_sk_scatter(const uint64_t *rec, uint64_
  * otherwise a k-mer that the filter's quick rule drops (its total below the (k+1)-mer lower bound;
  * filter_quick) is tallied and left out: at 30x and 0.5% errors three k-mers of four. */
 constexpr int SK_COUNT_TPB = 384;
-constexpr int SK_ITEM = 4;
+constexpr int SK_ITEM = 3;
+template <class KT> constexpr int SK_ITEMS = ((sizeof(KT) == 8 ? 17 : 49) + SK_ITEM - 1) / SK_ITEM;   /* items a record at most */
 constexpr double SK_MAX_INV_LOAD = 4.0;
 constexpr uint32_t SK_LATE = 256;
 struct SkCount {
@@ -595,7 +596,10 @@ struct SkCount {
   uint64_t cap;                     /* table slots of the sample(s) */
   uint2 *info;                      /* per partition: its first slot, its slots */
   uint32_t *over;                   /* partitions that overflowed the shared-memory slots */
-  uint32_t *cand;                   /* the slots the filter must read */
+  uint32_t *cand;                   /* the slots the filter must read (not with nodes) */
+  int nodes;                        /* local_insert_by_freqencies is done here, on the kept k-mers */
+  uint32_t *chain_list, *branch_list;   /* slots of the chain and branch nodes */
+  uint64_t list_cap;
   unsigned long long *s_tally;
   const SGeom *sg;
   uint32_t nsamples;
@@ -610,11 +614,11 @@ __host__ __device__ constexpr uint32_t sk_hash_size(uint32_t round) {
   return h;
 }
 /* Shared memory: slots (key, two entries); then a round's records, weights, record hash (its memory
- * then holds the item list, at most 5 or 13 items a record of 2 bytes each) and late k-mers, or the
+ * then holds the item list, 2 bytes an item) and late k-mers, or the
  * list of kept slots and the bitmap of a region of at most SK_MAX_INV_LOAD slots a kept one */
 template <class KT>
 __host__ __device__ constexpr uint32_t sk_late_at(uint32_t slots, uint32_t round) {   /* in 8-byte words, even */
-  const size_t items = (size_t)round * (sizeof(KT) == 8 ? 10 : 26), hash = (size_t)sk_hash_size(round) * 4;
+  const size_t items = (size_t)round * SK_ITEMS<KT> * 2, hash = (size_t)sk_hash_size(round) * 4;
   const size_t b = (size_t)slots * (Slot<KT>::KEYW * 8 + 8) + (size_t)round * (SkRec<KT>::NW * 8 + 4) +
                    (items > hash ? items : hash);
   return (uint32_t)((b + 15) / 16 * 2);
@@ -626,17 +630,27 @@ __host__ __device__ constexpr size_t sk_count_bytes(uint32_t slots, uint32_t rou
   return r > l ? r : l;
 }
 
-__device__ __forceinline__ uint32_t sk_home(KW1 x, uint32_t slots) {
-  uint32_t h = (uint32_t)x.v * 0x9E3779B1u ^ (uint32_t)(x.v >> 32) * 0x85EBCA6Bu;
-  h ^= h >> 16;
-  return __umulhi(h * 0xC2B2AE35u, slots);
-}
-__device__ __forceinline__ uint32_t sk_home(KW2 x, uint32_t slots) {
-  uint32_t h = (uint32_t)x.lo * 0x9E3779B1u ^ (uint32_t)(x.lo >> 32) * 0x85EBCA6Bu;
-  h ^= (uint32_t)x.hi * 0x27D4EB2Fu ^ (uint32_t)(x.hi >> 32) * 0x165667B1u;
-  h ^= h >> 16;
-  return __umulhi(h * 0xC2B2AE35u, slots);
-}
+/* A k-mer's probe sequence in the shared-memory slots: an odd step of its own, so that runs do not
+ * cluster (a lane with a long run holds up its warp, and the last late k-mer its block) */
+struct SkSeq {
+  uint32_t j, step;
+  __device__ __forceinline__ SkSeq(uint32_t h, uint32_t slots) {
+    h ^= h >> 16;
+    h *= 0xC2B2AE35u;
+    j = __umulhi(h, slots);
+    step = (h & 30u) | 1u;
+  }
+  __device__ __forceinline__ SkSeq(KW1 x, uint32_t slots)
+      : SkSeq((uint32_t)x.v * 0x9E3779B1u ^ (uint32_t)(x.v >> 32) * 0x85EBCA6Bu, slots) {}
+  __device__ __forceinline__ SkSeq(KW2 x, uint32_t slots)
+      : SkSeq((uint32_t)x.lo * 0x9E3779B1u ^ (uint32_t)(x.lo >> 32) * 0x85EBCA6Bu ^ (uint32_t)x.hi * 0x27D4EB2Fu ^
+                  (uint32_t)(x.hi >> 32) * 0x165667B1u, slots) {}
+  __device__ __forceinline__ void next(uint32_t slots) {
+    j += step;
+    if (j >= slots) j -= slots;
+  }
+};
+
 /* The shared-memory slots: k <= 31 one 16-byte (key, entries 0-1), read at once and claimed with its
  * first entry by one 128-bit CAS; k > 31 keys and entry pairs in two arrays. */
 template <class KT> struct SkSlots;
@@ -708,20 +722,19 @@ __device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t f
  * (any lanes may call it); false if the slots are full */
 template <class KT>
 __device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, unsigned &claims) {
-  uint32_t j = sk_home(want, sl.n);
-  for (uint32_t probe = 0; probe < SK_MAX_PROBE; ++probe) {
+  SkSeq p(want, sl.n);
+  for (uint32_t probe = 0; probe < SK_MAX_PROBE; ++probe, p.next(sl.n)) {
     uint64_t seen;
     bool claimed = false;
-    const KT key = sl.visit(j, want, fresh, seen, claimed);
+    const KT key = sl.visit(p.j, want, fresh, seen, claimed);
     if (claimed) { ++claims; return true; }
     if (KOps<KT>::eq(key, want)) {
-      uint32_t *e = sl.entries(j);
+      uint32_t *e = sl.entries(p.j);
       if (sk_try_entry(e, *(volatile uint32_t *)e, fresh, claims)) return true;
       if (sk_try_entry(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims)) return true;
       atomicOr(e + 1, SK_MORE);
       ((uint64_t *)&want)[KOps<KT>::WORDS - 1] |= KEY_CONT;
     }
-    if (++j == sl.n) j = 0;
   }
   return false;
 }
@@ -731,30 +744,130 @@ template <class KT, class F>
 __device__ __forceinline__ void sk_entries(const SkSlots<KT> &sl, uint32_t q, KT key, F fn) {
   uint64_t e = sl.pair(q);
   fn(e & ~((uint64_t)SK_MORE << 32));
+  if (!((e >> 32) & SK_MORE)) return;
+  SkSeq p(key, sl.n);   /* the k-mer's own sequence, from slot q on */
   ((uint64_t *)&key)[KOps<KT>::WORDS - 1] |= KEY_CONT;
-  uint32_t j = q;
-  while ((e >> 32) & SK_MORE) {   /* its next slot lies further on */
+  p.j = q;
+  do {   /* its next slot lies further on */
     KT x;
     do {
-      if (++j == sl.n) j = 0;
-      x = sl.key(j);
+      p.next(sl.n);
+      x = sl.key(p.j);
     } while (!KOps<KT>::eq(x, key) && !key_is_empty(x));
     if (key_is_empty(x)) return;
-    e = sl.pair(j);
+    e = sl.pair(p.j);
     fn(e & ~((uint64_t)SK_MORE << 32));
-  }
+  } while ((e >> 32) & SK_MORE);
 }
 
 /* a k-mer with a longer probe run, or whose slot's two entries are taken, waits here until the
  * round's others are counted: its warp's other lanes would wait for it */
 template <class KT> struct SkLate { KT key; uint64_t fresh; };
 
+/* the first ten bases of a k-mer */
+__device__ __forceinline__ uint32_t sk_top20(KW1 x, int k) { return (uint32_t)(x.v >> (2 * k - 20)) & 0xFFFFFu; }
+__device__ __forceinline__ uint32_t sk_top20(KW2 x, int k) { return (uint32_t)KOps<KW2>::shr(x, 2 * k - 20).lo & 0xFFFFFu; }
+
+/* local_insert_by_freqencies for one k-mer (filter_kmer's steps over entries in shared memory): the
+ * node's counters, 0 if no entry is kept, 1 for a chain node, 2 for a branch node.  The entries'
+ * flags 0..3 are tallied in the bytes of `few`, others in hist. */
+template <class KT>
+__device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key, const SkCount &a, uint64_t *pw,
+                                       uint32_t &few, unsigned int *hist) {
+  const int k = a.k;
+  const unsigned first = KOps<KT>::first(key, k), last = KOps<KT>::last(key);
+  /* a palindrome's ends are complements: eight bases at the ends of the k-mer and of its two
+   * (k-1)-mers rule all but one in 2^16 out before the whole is compared */
+  const uint32_t tail = (uint32_t)((const uint64_t *)&key)[0], head = sk_top20(key, k), rt = rev_pairs32(~tail);
+  bool oddk = (k & 1) != 0, kpal = false, high = false, low = false;
+  if (oddk) {
+    if ((head >> 4) == rev_pairs32(~(tail >> 2)) >> 16) high = km1_high_palindrome(key, k);
+    if (((head >> 2) & 0xFFFFu) == rt >> 16) low = km1_low_palindrome(key, k);
+  } else if ((head >> 4) == rt >> 16) {
+    kpal = k_palindrome(key, k);
+  }
+  uint32_t kf = 0, ok = 0;   /* ok: bit c (4 + c): the (k+1)-mers over in (out) base c are kept */
+  if (a.thresholding) {
+    uint32_t k1[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    sk_entries<KT>(sl, q, key, [&](uint64_t x) {
+      #pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        const uint32_t w = (uint32_t)(x >> (32 * z));
+        if (w == 0) continue;
+        const uint32_t c = sk_count_of(w), half = (c + 1) >> 1;
+        const unsigned code = entry_code(w), in5 = code_in5(code), out5 = code_out5(code);
+        kf += c;
+        const uint32_t vi = oddk && high && !kpal && last == 4u - in5 ? half : c;
+        const uint32_t vo = oddk && low && !kpal && first == 4u - out5 ? half : c;
+        #pragma unroll
+        for (unsigned b = 0; b < 4; ++b) {
+          k1[b] += in5 == b + 1 ? vi : 0u;
+          k1[4 + b] += out5 == b + 1 ? vo : 0u;
+        }
+      }
+    });
+    kf = min(0xFFFFu, kf);
+    #pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint32_t v = min(0xFFFFu, k1[b]);
+      ok |= v >= a.t[2] && v < a.t[3] ? 1u << b : 0u;
+    }
+  }
+  uint32_t nc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  bool any = false;
+  sk_entries<KT>(sl, q, key, [&](uint64_t x) {
+    #pragma unroll
+    for (int z = 0; z < 2; ++z) {
+      const uint32_t w = (uint32_t)(x >> (32 * z));
+      if (w == 0) continue;
+      const uint32_t c16 = min(0xFFFFu, sk_count_of(w));
+      const unsigned code = entry_code(w);
+      unsigned in5 = code_in5(code), out5 = code_out5(code), f = 0;
+      if (a.thresholding) {   /* an absent base counts as a (k+1)-mer outside the bounds */
+        if (c16 < a.t[4] || c16 >= a.t[5]) f |= 4;
+        if (kf < a.t[0] || kf >= a.t[1]) f |= 8;
+        if (!((ok << 1) >> in5 & 1u) || !in5) f |= 2;
+        if (!((ok >> 3) >> out5 & 1u) || !out5) f |= 1;
+      }
+      if (f < 4) few += 1u << (8 * f);   /* (at most 25 entries a k-mer) */
+      else atomicAdd(&hist[f], 1u);
+      if (f >= 3) continue;
+      if (f == 1) out5 = 0;
+      if (f == 2) in5 = 0;
+      any = true;
+      #pragma unroll
+      for (unsigned b = 0; b < 4; ++b) {
+        nc[b] += out5 == b + 1 ? c16 : 0u;
+        nc[4 + b] += in5 == b + 1 ? c16 : 0u;
+      }
+      nc[8] += c16;
+    }
+  });
+  if (!any) return 0;
+  unsigned din = 0, dout = 0;   /* IsBranchPoint / IsChainNode (debruijn_graph_filters.hpp:57-220) */
+  bool k1pal = false;
+  #pragma unroll
+  for (unsigned b = 0; b < 4; ++b) {
+    dout += nc[b] > 0;
+    din += nc[4 + b] > 0;
+    if (oddk && nc[b] > 0 && low && (first == 3u - b || first == b)) k1pal = true;
+    if (oddk && nc[4 + b] > 0 && high && (last == 3u - b || last == b)) k1pal = true;
+  }
+  #pragma unroll
+  for (int b = 0; b < 9; ++b) nc[b] = min(0xFFFFu, nc[b]);
+  pw[0] = (uint64_t)(nc[0] | (nc[1] << 16)) | ((uint64_t)(nc[2] | (nc[3] << 16)) << 32);
+  pw[1] = (uint64_t)(nc[4] | (nc[5] << 16)) | ((uint64_t)(nc[6] | (nc[7] << 16)) << 32);
+  pw[2] = nc[8];
+  return din >= 2 || dout >= 2 || kpal || k1pal ? 2 : 1;
+}
+
 template <class KT>
 __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_count(SkCount a) {
   constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW, NE = Slot<KT>::ENTRIES, NW = SkRec<KT>::NW;
   extern __shared__ __align__(16) uint64_t sm[];
-  __shared__ uint32_t s_items, s_full, s_listed, s_other, s_conts, s_wide, s_base, s_slots, s_late_n;
-  __shared__ unsigned int s_qh[4], s_claims;
+  __shared__ uint32_t s_items, s_full, s_listed, s_other, s_conts, s_wide, s_base, s_slots, s_late_n, s_smp;
+  __shared__ unsigned int s_qh[4], s_claims, s_hist[16], s_nc[2];
+  __shared__ unsigned long long s_nbase[2];
   __shared__ unsigned long long s_cand;
   if (a.ctr->err & DERR_SKEW) return;
   uint32_t part = a.todo ? a.todo[blockIdx.x] : blockIdx.x;
@@ -772,6 +885,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   SkLate<KT> *s_late = reinterpret_cast<SkLate<KT> *>(sm + a.late);
   for (uint32_t i = tid; i < slots; i += nt) sl.clear(i);
   if (tid < 4) s_qh[tid] = 0;
+  if (tid < 16) s_hist[tid] = 0;
+  if (tid < 2) s_nc[tid] = 0;
   if (tid == 0) { s_full = 0; s_listed = 0; s_other = 0; s_conts = 0; s_wide = 0; s_claims = 0; }
   const uint32_t hmask = a.hsize - 1;
   unsigned claims = 0;
@@ -856,21 +971,21 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         f = KOps<KT>::append(f, c, k);
         r = KOps<KT>::prepend(3u - c, r, k);
         /* the k-mer's slot within three probes (nine in ten), then its entry among the slot's two */
-        uint32_t j = sk_home(key, slots);
+        SkSeq p(key, slots);
         uint64_t seen = 0;
         bool seek = todo;
         #pragma unroll
         for (int probe = 0; probe < 3; ++probe) {
           if (seek) {
             bool claimed = false;
-            const KT x = sl.visit(j, key, fresh, seen, claimed);
+            const KT x = sl.visit(p.j, key, fresh, seen, claimed);
             if (claimed) { ++claims; todo = false; }
             seek = !claimed && !KOps<KT>::eq(x, key);
-            if (seek && ++j == slots) j = 0;
+            if (seek) p.next(slots);
           }
         }
         if (todo && !seek) {
-          uint32_t *e = sl.entries(j);
+          uint32_t *e = sl.entries(p.j);
           uint32_t cur = (uint32_t)seen;
           if (cur != 0 && entry_code(cur) != code) { cur = (uint32_t)(seen >> 32); ++e; }
           todo = !sk_try_entry(e, cur, fresh, claims);
@@ -968,18 +1083,60 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
    * slots here for every one it takes there.  Two slots at least of the region stay empty, which
    * ends every probe run. */
   const uint32_t tslots = nkept + s_conts / (NE / 2), want_R = (uint32_t)(tslots * a.inv_load) + 2u;
+  /* the first nodes, one a thread, before the reservations: region, chain and branch indices are
+   * then taken at once, by three warps */
+  int kind = 0;
+  KT t{};
+  uint64_t pw[3] = {0, 0, 0};
+  uint32_t few = 0, at = 0;
+  auto make_node = [&](uint32_t x) {   /* every thread of the block */
+    kind = 0;
+    if (x < nkept) {
+      const KT key = sl.key(kept[x]);
+      kind = sk_node<KT>(sl, kept[x], key, a, pw, few, s_hist);
+      t = table_key(key);
+    }
+    const unsigned mc = __ballot_sync(~0u, kind == 1), mb = __ballot_sync(~0u, kind == 2);
+    uint32_t oc = 0, ob = 0;
+    if (lane == 0) {
+      oc = mc ? atomicAdd(&s_nc[0], (unsigned)__popc(mc)) : 0u;
+      ob = mb ? atomicAdd(&s_nc[1], (unsigned)__popc(mb)) : 0u;
+    }
+    oc = __shfl_sync(~0u, oc, 0) + __popc(mc & ((1u << lane) - 1));
+    ob = __shfl_sync(~0u, ob, 0) + __popc(mb & ((1u << lane) - 1));
+    at = kind == 2 ? ob : oc;
+    /* the flags' bytes, summed over the warp in 16-bit halves */
+    const uint32_t f02 = __reduce_add_sync(~0u, few & 0x00FF00FFu), f13 = __reduce_add_sync(~0u, (few >> 8) & 0x00FF00FFu);
+    few = 0;
+    if (lane < 4) {
+      const uint32_t f = ((lane & 1 ? f13 : f02) >> (lane & 2 ? 16 : 0)) & 0xFFFFu;
+      if (f) atomicAdd(&s_hist[lane], f);
+    }
+  };
+  auto reserve = [&](int list, uint32_t smp) {   /* one thread: the block's chain (0) or branch (1) indices */
+    const uint32_t n = s_nc[list];
+    if (!n) return;
+    s_nbase[list] = atomicAdd(list ? &a.ctr->n_branch : &a.ctr->n_chain, (unsigned long long)n);
+    if (a.s_tally) atomicAdd(&a.s_tally[(uint64_t)smp * T_NUM + (list ? T_BRANCH : T_CHAIN)], (unsigned long long)n);
+  };
+  if (a.nodes) {
+    make_node(tid);
+    __syncthreads();
+  }
+  if (a.nodes && (tid == 32 || tid == 64)) reserve(tid / 32 - 1, sample_of_part(a.sg, a.nsamples, part));
   if (tid == 0) {
     const uint32_t R = want_R;
     const uint32_t smp = sample_of_part(a.sg, a.nsamples, part);
     const TableGeom &g = a.sg[smp].g;
     const unsigned long long lo = atomicAdd(&a.bump[smp], (unsigned long long)R);
-    const unsigned long long c0 = atomicAdd(&a.ctr->n_cand, (unsigned long long)listed);
-    s_cand = c0;
+    s_cand = a.cand ? atomicAdd(&a.ctr->n_cand, (unsigned long long)listed) : 0ull;
     const bool fits = lo + R <= g.nslots;
     if (!fits) atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
     s_slots = fits ? R : 0;
+    s_smp = smp;
     s_base = (uint32_t)(g.base + lo);
     a.info[part] = make_uint2((uint32_t)(g.base + lo), R);
+    if (!a.cand) atomicAdd(&a.ctr->n_cand, (unsigned long long)listed);
     if (tslots) atomicAdd(&a.ctr->n_slots_claimed, (unsigned long long)tslots);
     if (s_claims) atomicAdd(&a.ctr->n_entries, (unsigned long long)s_claims);
     if (a.s_tally && s_claims) atomicAdd(&a.s_tally[(uint64_t)smp * T_NUM + T_ENTRIES], (unsigned long long)s_claims);
@@ -999,7 +1156,39 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
       if (++pos == R) pos = 0;
     }
   };
-  for (uint32_t x = tid; x < nkept; x += nt) {
+  if (a.nodes) {   /* the nodes themselves */
+    for (uint32_t x0 = 0;;) {
+      if (kind) {
+        const unsigned long long o = s_nbase[kind - 1] + at;
+        const uint32_t pos = place(bin_home(t, R));
+        const uint64_t aux = kind == 1 ? o : 0xFFFFFFFFull;
+        pw[2] |= (uint64_t)((kind == 1 ? NF_CHAIN : NF_BRANCH) | (s_smp << NF_SAMPLE_SHIFT)) << 16 | aux << 32;
+        t = as_node(t);
+        ulonglong2 *to = reinterpret_cast<ulonglong2 *>(dst + (uint64_t)pos * SU);
+        if constexpr (KWD == 1) {
+          to[0] = make_ulonglong2(((const uint64_t *)&t)[0], pw[0]);
+          to[1] = make_ulonglong2(pw[1], pw[2]);
+        } else {
+          to[0] = make_ulonglong2(((const uint64_t *)&t)[0], ((const uint64_t *)&t)[KWD - 1]);
+          to[1] = make_ulonglong2(pw[0], pw[1]);
+          to[2] = make_ulonglong2(pw[2], 0ull);
+          to[3] = make_ulonglong2(0ull, 0ull);
+        }
+        if (o < a.list_cap) (kind == 1 ? a.chain_list : a.branch_list)[o] = s_base + pos;
+        else atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
+      }
+      x0 += nt;
+      if (x0 >= nkept) break;
+      __syncthreads();
+      if (tid < 2) s_nc[tid] = 0;
+      __syncthreads();
+      make_node(x0 + tid);
+      __syncthreads();
+      if (tid == 32 || tid == 64) reserve(tid / 32 - 1, s_smp);
+      __syncthreads();
+    }
+  }
+  for (uint32_t x = tid; x < (a.nodes ? 0u : nkept); x += nt) {
     const uint32_t q = x < listed ? kept[x] : kept[slots - 1 - (x - listed)];
     const KT key = sl.key(q), t = table_key(key);
     const uint32_t pos = place(bin_home(t, R));
@@ -1025,6 +1214,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     if (x < listed) a.cand[s_cand + x] = s_base + pos;
   }
   __syncthreads();
+  if (tid < 16 && s_hist[tid]) atomicAdd(&a.ctr->flag_hist[tid], (unsigned long long)s_hist[tid]);
   if (s_wide)   /* k-mers of more entries than a table slot holds: continuation slots behind the first */
     for (uint32_t x = tid; x < nkept; x += nt) {
       const uint32_t q = x < listed ? kept[x] : kept[slots - 1 - (x - listed)];
