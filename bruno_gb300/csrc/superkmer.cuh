@@ -970,12 +970,12 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         in5 = KOps<KT>::first(f, k) + 1u;
         f = KOps<KT>::append(f, c, k);
         r = KOps<KT>::prepend(3u - c, r, k);
-        /* the k-mer's slot within three probes (nine in ten), then its entry among the slot's two */
+        /* the k-mer's slot within two probes, then its entry among the slot's two */
         SkSeq p(key, slots);
         uint64_t seen = 0;
         bool seek = todo;
         #pragma unroll
-        for (int probe = 0; probe < 3; ++probe) {
+        for (int probe = 0; probe < 2; ++probe) {
           if (seek) {
             bool claimed = false;
             const KT x = sl.visit(p.j, key, fresh, seen, claimed);
