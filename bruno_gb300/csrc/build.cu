@@ -2632,6 +2632,7 @@ bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vec
  * right away, so parsing and extraction run under the remaining copies. */
 bruno_status run_index_reads(Ctx *c) {
   bruno_status st;
+  constexpr uint64_t SMALL_SEGMENT = 16ull << 20;   /* 64 MB of read spans at most */
   /* first pass: sizes for every segment */
   uint64_t total_tiles = 0, total_bytes = 0;
   for (auto &sg : c->segs) {
@@ -2663,10 +2664,7 @@ bruno_status run_index_reads(Ctx *c) {
     if (sg.ev >= 0) cudaStreamWaitEvent(c->stream, c->seg_ev[sg.ev], 0);
     const uint64_t tiles = (sg.n + TILE - 1) / TILE;
     cudaMemsetAsync(&c->dctr->n_newlines_eff, 0, 8, c->stream);   /* the extraction's tallies stay */
-    long long neg = -1;
-    unsigned long long nb = ~0ull;
-    cudaMemcpyAsync(&c->dctr->last_nonws, &neg, sizeof(neg), cudaMemcpyHostToDevice, c->stream);
-    cudaMemcpyAsync(&c->dctr->bad_line, &nb, sizeof(nb), cudaMemcpyHostToDevice, c->stream);
+    cudaMemsetAsync(&c->dctr->last_nonws, 0xFF, 16, c->stream);   /* and bad_line: none */
     c->launches += 2;   /* k_tile_stats, k_index_lines; the scan counts its own */
     const bool aligned = ((uintptr_t)sg.ptr & 15) == 0;
     k_tile_stats<<<(unsigned)tiles, TPB, 0, c->stream>>>((const unsigned char *)sg.ptr, sg.n, (uint64_t *)c->tile_cnt.p,
@@ -2674,9 +2672,13 @@ bruno_status run_index_reads(Ctx *c) {
     if ((st = scan_ctx(c, (const uint64_t *)c->tile_cnt.p, (uint64_t *)c->tile_base.p, tiles, &c->dctr->n_records)) !=
         BRUNO_OK)
       return st;
-    if ((st = sync_counters(c)) != BRUNO_OK) return st;
-    /* n_records temporarily holds the total newline count: records <= newlines / 4 + 1 */
-    uint64_t upper = c->hctr->n_records / 4 + 1;
+    /* records: a small segment's at most its bytes over the four newlines of each; a larger one's
+     * newlines are waited for (n_records temporarily holds their count) */
+    uint64_t upper = sg.n / 4 + 1;
+    if (sg.n > SMALL_SEGMENT || c->segs.size() > 1) {
+      if ((st = sync_counters(c)) != BRUNO_OK) return st;
+      upper = c->hctr->n_records / 4 + 1;
+    }
     /* grow keeping the spans of earlier files; pieces of one input grow once, for all pieces
      * at the first piece's records per byte */
     if ((c->pre_extracted || batch_hook) && si == 0 && sg.n > 0)
@@ -3363,6 +3365,7 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
     c->launches += 1;
   }
   if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
+  cudaEventRecord(c->kev[3], c->stream);
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
   const uint32_t n = (uint32_t)c->hctr->n_over;
   if (n && !c->hctr->err) {
@@ -3374,6 +3377,7 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
     sk_count_launch<KT>(c, a, n, big.bytes);
     c->launches += 1;
     if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
+    cudaEventRecord(c->kev[3], c->stream);
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
   }
   ok = !c->hctr->err && c->hctr->n_over == 0;
@@ -3393,13 +3397,14 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
   k_sk_estimate<KT><<<num_sms() * 4, 128, 0, c->stream>>>(
       (const uint64_t *)c->sk_recs.p, (const uint32_t *)c->sk_est.p, c->sk_est_cap, c->cfg.k,
       (const SkSample *)c->sk_samp.p, S, (unsigned int *)c->hllreg.p, c->dctr);
-  k_hll_sums<<<S, 256, 0, c->stream>>>((const unsigned int *)c->hllreg.p, (double *)c->hsum.p,
-                                       (unsigned int *)((double *)c->hsum.p + S));
+  double *sums = S > 1 ? (double *)c->hsum.p : &c->dctr->hll_sum;
+  k_hll_sums<<<S, 256, 0, c->stream>>>((const unsigned int *)c->hllreg.p, sums,
+                                       S > 1 ? (unsigned int *)(sums + S) : &c->dctr->hll_zeros);
   c->launches += 2;
   cudaEventRecord(c->kev[1], c->stream);
   std::vector<double> hs(2 * S), distinct(S);
-  cudaMemcpyAsync(hs.data(), c->hsum.p, (size_t)S * 16, cudaMemcpyDeviceToHost, c->stream);
   if (S > 1) {
+    cudaMemcpyAsync(hs.data(), sums, (size_t)S * 16, cudaMemcpyDeviceToHost, c->stream);
     c->h_inst.assign(S, 0);
     c->h_used.assign(S, 0);
     cudaMemcpyAsync(c->h_inst.data(), c->s_inst.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
@@ -3411,7 +3416,9 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
   c->n_instances = inst;
   c->n_reads_used = c->hctr->n_reads_used;
   const unsigned char *zeros = (const unsigned char *)(hs.data() + S);   /* S 32-bit words after the sums */
-  for (uint32_t q = 0; q < S; ++q) distinct[q] = hll_estimate(hs[q], zeros_word(zeros + 4 * q), c->sk_q[q]);
+  for (uint32_t q = 0; q < S; ++q)
+    distinct[q] = S > 1 ? hll_estimate(hs[q], zeros_word(zeros + 4 * q), c->sk_q[q])
+                        : hll_estimate(c->hctr->hll_sum, c->hctr->hll_zeros, c->sk_q[0]);
   const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
   const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
   for (int attempt = 0; attempt < 3; ++attempt) {
@@ -3454,7 +3461,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if ((st = ensure(c, c->sk_cur, parts * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_info, parts * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_over, parts * 8)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_bump, (size_t)S * 8)) != BRUNO_OK) return st;
+    if (S > 1 && (st = ensure(c, c->sk_bump, (size_t)S * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sgeom, S * sizeof(SGeom))) != BRUNO_OK) return st;
     for (SGeom &x : sg) {
       x.g.bins = (const uint32_t *)c->sk_part.p;
@@ -3463,13 +3470,9 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if ((st = cuda_check(c, cudaMemcpyAsync(c->sgeom.p, sg.data(), S * sizeof(SGeom), cudaMemcpyHostToDevice, c->stream),
                          "sample geometry")) != BRUNO_OK)
       return st;
-    cudaMemsetAsync(c->sk_bump.p, 0, (size_t)S * 8, c->stream);
-    cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
-    cudaMemsetAsync(&c->dctr->n_cand, 0, sizeof(c->dctr->n_cand) + sizeof(c->dctr->quick_hist), c->stream);
     cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
-    cudaMemsetAsync(&c->dctr->n_slots_claimed, 0, 16, c->stream);
-    cudaMemsetAsync(&c->dctr->n_nodes, 0, offsetof(DevCounters, lr_applied) - offsetof(DevCounters, n_nodes), c->stream);
-    cudaMemsetAsync(&c->dctr->n_big, 0, 8, c->stream);
+    cudaMemsetAsync(&c->dctr->n_slots_claimed, 0, offsetof(DevCounters, hll) - offsetof(DevCounters, n_slots_claimed), c->stream);
+    if (S > 1) cudaMemsetAsync(c->sk_bump.p, 0, (size_t)S * 8, c->stream);
     if (S > 1) cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
     cudaEventRecord(c->kev[2], c->stream);
     if ((st = sk_partition<KT>(c, plan, (uint32_t)parts, n_rec)) != BRUNO_OK) return st;
@@ -3493,7 +3496,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     a.s_tally = S > 1 ? (unsigned long long *)c->s_tally.p : nullptr;
     a.sg = (const SGeom *)c->sgeom.p;
     a.nsamples = S;
-    a.bump = (unsigned long long *)c->sk_bump.p;
+    a.bump = S > 1 ? (unsigned long long *)c->sk_bump.p : &c->dctr->sk_bump;
     a.ctr = c->dctr;
     std::vector<SkLaunch<KT>> launches;
     std::vector<ClassRun> runs;
@@ -3526,12 +3529,13 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     }
     bool ok = false;
     if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, ok)) != BRUNO_OK) return st;
-    cudaEventRecord(c->kev[3], c->stream);
     if (c->hctr->err & DERR_SKEW) return BRUNO_OK;
     if (ok) {
-      std::vector<uint64_t> taken(S);
-      cudaMemcpyAsync(taken.data(), c->sk_bump.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
-      if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "table slots")) != BRUNO_OK) return st;
+      std::vector<uint64_t> taken(S, c->hctr->sk_bump);
+      if (S > 1) {
+        cudaMemcpyAsync(taken.data(), c->sk_bump.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
+        if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "table slots")) != BRUNO_OK) return st;
+      }
       for (uint32_t q = 0; q < S; ++q) sg[q].g.nslots = taken[q];
       c->geom = sg[0].g;
       c->nslots = S == 1 ? taken[0] : base;

@@ -86,11 +86,17 @@ bruno_status sync_counters(Ctx *c, bool with_hll) {
   return cuda_check(c, e, "device phase");
 }
 
-static void record(Ctx *c, int i) { cudaEventRecord(c->ev[i], c->stream); }
+/* a phase's first and last event; the time between is taken when somebody asks for it
+ * (bruno_phase_ms), so that no phase waits for its last event */
+static void phase_begin(Ctx *c, int phase) { cudaEventRecord(c->pev[phase][0], c->stream); }
+static void phase_end(Ctx *c, int phase) {
+  cudaEventRecord(c->pev[phase][1], c->stream);
+  c->ptimed |= 1u << phase;
+}
 
-static double elapsed(Ctx *c, int a, int b) {
+static double elapsed(cudaEvent_t a, cudaEvent_t b) {
   float ms = 0;
-  if (cudaEventElapsedTime(&ms, c->ev[a], c->ev[b]) != cudaSuccess) { cudaGetLastError(); return 0; }
+  if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&ms, a, b) != cudaSuccess) { cudaGetLastError(); return 0; }
   return ms;
 }
 
@@ -124,7 +130,8 @@ bruno_status bruno_ctx_create(const bruno_cfg *cfg, bruno_ctx **out) {
   if (st == BRUNO_OK) { cudaDeviceSetLimit(cudaLimitMaxL2FetchGranularity, 32); cudaGetLastError(); }
   if (st == BRUNO_OK) st = cuda_check(c, cudaMalloc(&c->dctr, sizeof(DevCounters)), "counters");
   if (st == BRUNO_OK) st = cuda_check(c, cudaMallocHost(&c->hctr, sizeof(DevCounters)), "pinned counters");
-  for (int i = 0; i < 8 && st == BRUNO_OK; ++i) st = cuda_check(c, cudaEventCreate(&c->ev[i]), "event");
+  for (int i = 0; i < 12 && st == BRUNO_OK; ++i) st = cuda_check(c, cudaEventCreate(&c->pev[i / 2][i % 2]), "event");
+  if (st == BRUNO_OK) st = cuda_check(c, cudaEventCreate(&c->h2d_begin), "event");
   for (int i = 0; i < 5 && st == BRUNO_OK; ++i) st = cuda_check(c, cudaEventCreate(&c->kev[i]), "event");
   if (st == BRUNO_OK) st = cuda_check(c, cudaEventCreate(&c->h2d_end), "event");
   if (st == BRUNO_OK) st = cuda_check(c, cudaEventCreateWithFlags(&c->order_ev, cudaEventDisableTiming), "event");
@@ -158,7 +165,8 @@ bruno_status bruno_ctx_destroy(bruno_ctx *c) {
   for (Buf &b : c->seg_bufs) release(b);
   if (c->dctr) cudaFree(c->dctr);
   if (c->hctr) cudaFreeHost(c->hctr);
-  for (int i = 0; i < 8; ++i) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
+  for (auto &p : c->pev) for (cudaEvent_t e : p) if (e) cudaEventDestroy(e);
+  if (c->h2d_begin) cudaEventDestroy(c->h2d_begin);
   for (int i = 0; i < 5; ++i) if (c->kev[i]) cudaEventDestroy(c->kev[i]);
   for (cudaEvent_t e : c->seg_ev) cudaEventDestroy(e);
   if (c->h2d_end) cudaEventDestroy(c->h2d_end);
@@ -230,6 +238,8 @@ bruno_status bruno_reset(bruno_ctx *c) {
   c->launches = 0;
   std::memset(c->flag_hist, 0, sizeof(c->flag_hist));
   std::memset(c->phase_ms, 0, sizeof(c->phase_ms));
+  c->ptimed = 0;
+  c->h2d_timed = 0;
   c->err.clear();
   return BRUNO_OK;
 }
@@ -248,7 +258,7 @@ bruno_status bruno_load_fastq(bruno_ctx *c, const char *buf, size_t nbytes, int3
     if (st != BRUNO_OK) return st;
     char *dst = (char *)c->seg_bufs[i].p;
     if (cuts.size() < 2 && !c->h2d_piped) {   /* one piece: copied on the context's stream */
-      if (!c->h2d_pending) { record(c, 7); c->h2d_pending = true; }   /* before the first host copy */
+      if (!c->h2d_pending) { cudaEventRecord(c->h2d_begin, c->stream); c->h2d_pending = true; }   /* before the first host copy */
       st = cuda_check(c, cudaMemcpyAsync(dst, buf, nbytes, cudaMemcpyHostToDevice, c->stream), "H2D FASTQ");
       if (st != BRUNO_OK) return st;
       c->segs.push_back({dst, nbytes});
@@ -259,7 +269,7 @@ bruno_status bruno_load_fastq(bruno_ctx *c, const char *buf, size_t nbytes, int3
       cudaEventRecord(c->order_ev, c->stream);
       cudaStreamWaitEvent(c->copy_stream, c->order_ev, 0);
       for (int i = 0; i + 1 < c->n_copy; ++i) cudaStreamWaitEvent(c->copy_more[i], c->order_ev, 0);
-      if (!c->h2d_pending) { cudaEventRecord(c->ev[7], c->copy_stream); c->h2d_pending = true; }
+      if (!c->h2d_pending) { cudaEventRecord(c->h2d_begin, c->copy_stream); c->h2d_pending = true; }
       uint64_t at = 0;   /* where the piece goes in the device copy */
       for (size_t j = 0; j < cuts.size(); ++j) {
         const uint64_t off = cuts[j], len = (j + 1 < cuts.size() ? cuts[j + 1] : nbytes) - off;
@@ -293,28 +303,19 @@ bruno_status bruno_load_fastq(bruno_ctx *c, const char *buf, size_t nbytes, int3
 bruno_status bruno_compute_biedge_freqencies(bruno_ctx *c) {
   if (!c) return BRUNO_ERR_ARG;
   if (c->stage != 1) return set_err(c, BRUNO_ERR_ARG, "compute_biedge_freqencies needs loaded FASTQ");
-  record(c, 0);
+  phase_begin(c, 0);
   bruno_status st = run_index_reads(c);
   if (st != BRUNO_OK) return st;
-  record(c, 1);
+  phase_end(c, 0);
+  phase_begin(c, 1);
   st = run_count(c);
   if (st != BRUNO_OK) return st;
-  record(c, 2);
+  phase_end(c, 1);
   if (c->cfg.keep_k2 && (st = run_dump_k2(c)) != BRUNO_OK) return st;
-  cudaEventSynchronize(c->ev[2]);
-  c->phase_ms[0] = elapsed(c, 0, 1);
-  if (c->h2d_pending) {   /* the copies: back to back right before this call's start event, or
-                            on the copy stream beneath the read index */
-    if (c->h2d_piped) {
-      float ms = 0;
-      if (cudaEventElapsedTime(&ms, c->ev[7], c->h2d_end) != cudaSuccess) { cudaGetLastError(); ms = 0; }
-      c->phase_ms[10] = ms;
-    } else {
-      c->phase_ms[10] = elapsed(c, 7, 0);
-    }
-    c->h2d_pending = false;
-  }
-  c->phase_ms[1] = elapsed(c, 1, 2);
+  /* the copies: back to back right before this call's first event, or on the copy stream beneath
+   * the read index */
+  if (c->h2d_pending) c->h2d_timed = c->h2d_piped ? 1 : 2;
+  c->h2d_pending = false;
   c->stage = 2;
   return BRUNO_OK;
 }
@@ -322,13 +323,11 @@ bruno_status bruno_compute_biedge_freqencies(bruno_ctx *c) {
 bruno_status bruno_local_insert_by_freqencies(bruno_ctx *c, const uint64_t *thresh) {
   if (!c) return BRUNO_ERR_ARG;
   if (c->stage != 2) return set_err(c, BRUNO_ERR_ARG, "local_insert_by_freqencies needs counted (k+2)-mers");
-  record(c, 2);
+  phase_begin(c, 2);
   std::memcpy(c->thr_used, thresh ? thresh : c->cfg.thresh, sizeof(c->thr_used));
   bruno_status st = run_filter(c, c->thr_used);
   if (st != BRUNO_OK) return st;
-  record(c, 3);
-  cudaEventSynchronize(c->ev[3]);
-  c->phase_ms[2] = elapsed(c, 2, 3);
+  phase_end(c, 2);
   c->stage = 3;
   return BRUNO_OK;
 }
@@ -336,12 +335,10 @@ bruno_status bruno_local_insert_by_freqencies(bruno_ctx *c, const uint64_t *thre
 bruno_status bruno_extract_chains(bruno_ctx *c) {
   if (!c) return BRUNO_ERR_ARG;
   if (c->stage != 3) return set_err(c, BRUNO_ERR_ARG, "extract_chains needs the filtered graph");
-  record(c, 3);
+  phase_begin(c, 3);
   bruno_status st = run_extract_chains(c);
   if (st != BRUNO_OK) return st;
-  record(c, 4);
-  cudaEventSynchronize(c->ev[4]);
-  c->phase_ms[3] = elapsed(c, 3, 4);
+  phase_end(c, 3);
   c->stage = 4;
   return BRUNO_OK;
 }
@@ -349,12 +346,10 @@ bruno_status bruno_extract_chains(bruno_ctx *c) {
 bruno_status bruno_list_rank(bruno_ctx *c, int32_t min_update, uint64_t *iterations) {
   if (!c) return BRUNO_ERR_ARG;
   if (c->stage != 4) return set_err(c, BRUNO_ERR_ARG, "list_rank needs extracted chains");
-  record(c, 4);
+  phase_begin(c, 4);
   bruno_status st = run_list_rank(c, min_update);
   if (st != BRUNO_OK) return st;
-  record(c, 5);
-  cudaEventSynchronize(c->ev[5]);
-  c->phase_ms[4] = elapsed(c, 4, 5);
+  phase_end(c, 4);
   if (iterations) *iterations = c->iterations;
   c->stage = 5;
   return BRUNO_OK;
@@ -363,12 +358,10 @@ bruno_status bruno_list_rank(bruno_ctx *c, int32_t min_update, uint64_t *iterati
 bruno_status bruno_to_compressed_chains(bruno_ctx *c) {
   if (!c) return BRUNO_ERR_ARG;
   if (c->stage != 5) return set_err(c, BRUNO_ERR_ARG, "to_compressed_chains needs ranked chains");
-  record(c, 5);
+  phase_begin(c, 5);
   bruno_status st = run_compress(c);
   if (st != BRUNO_OK) return st;
-  record(c, 6);
-  cudaEventSynchronize(c->ev[6]);
-  c->phase_ms[5] = elapsed(c, 5, 6);
+  phase_end(c, 5);
   c->stage = 6;
   if (!c->chains_clean)
     return set_err(c, BRUNO_ERR_INVARIANT,
@@ -383,13 +376,11 @@ bruno_status bruno_clean_deadend_and_bubbles_naive(bruno_ctx *c, bruno_clean_sta
   if (c->stage < 5) return set_err(c, BRUNO_ERR_ARG, "cleaning needs ranked chains");
   if (c->cleaned) return set_err(c, BRUNO_ERR_ARG, "the graph is cleaned already; call bruno_reset first");
   bruno_clean_stats s{};
-  record(c, 5);
+  phase_begin(c, 5);
   bruno_status st = run_clean(c, &s.rounds, &s.deadends, &s.bubbles, &s.edges, &s.status);
   if (stats) *stats = s;
   if (st != BRUNO_OK) return st;
-  record(c, 6);
-  cudaEventSynchronize(c->ev[6]);
-  c->phase_ms[5] = elapsed(c, 5, 6);
+  phase_end(c, 5);
   c->cleaned = true;
   c->stage = 6;
   if (!c->chains_clean)
@@ -407,7 +398,9 @@ bruno_status bruno_build_and_compact(bruno_ctx *c, const char *buf, size_t nbyte
   if (st == BRUNO_OK) st = bruno_compute_biedge_freqencies(c);
   c->one_call = false;
   if (st == BRUNO_OK) st = bruno_local_insert_by_freqencies(c, nullptr);
+  c->one_call = true;   /* (the ranking's wait will do for the chain map) */
   if (st == BRUNO_OK) st = bruno_extract_chains(c);
+  c->one_call = false;
   if (st == BRUNO_OK) st = bruno_list_rank(c, c->cfg.min_update, nullptr);
   if (st == BRUNO_OK) st = bruno_to_compressed_chains(c);
   return st;
@@ -667,7 +660,7 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
   static const char nl = '\n';
   c->batch_piped = ngroups > 1;
   if (!c->batch_piped) {   /* one copy after another on the context's stream, one segment */
-    record(c, 7);
+    cudaEventRecord(c->h2d_begin, c->stream);
     for (size_t q = 0; q < n_samples && st == BRUNO_OK; ++q) {
       if (!nbytes[q]) continue;
       st = cuda_check(c, cudaMemcpyAsync(dst + c->samp_off[q], bufs[q], nbytes[q],
@@ -683,7 +676,7 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
     /* after whatever the context's stream has queued (the buffer's allocation) */
     cudaEventRecord(c->order_ev, c->stream);
     cudaStreamWaitEvent(c->copy_stream, c->order_ev, 0);
-    cudaEventRecord(c->ev[7], c->copy_stream);
+    cudaEventRecord(c->h2d_begin, c->copy_stream);
     for (size_t gi = 0; gi < ngroups && st == BRUNO_OK; ++gi) {
       const uint32_t q0 = c->seg_samp[gi], q1 = c->seg_samp[gi + 1];
       for (uint32_t q = q0; q < q1 && st == BRUNO_OK; ++q) {
@@ -711,21 +704,13 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
   }
   c->S = (uint32_t)n_samples;
   c->stage = 1;
-  record(c, 0);
+  phase_begin(c, 1);
   c->one_call = true;
   st = run_count_samples(c);
   c->one_call = false;
   if (st != BRUNO_OK) return st;
-  record(c, 1);
-  cudaEventSynchronize(c->ev[1]);
-  if (c->batch_piped) {
-    float ms = 0;
-    if (cudaEventElapsedTime(&ms, c->ev[7], c->h2d_end) != cudaSuccess) { cudaGetLastError(); ms = 0; }
-    c->phase_ms[10] = ms;
-  } else {
-    c->phase_ms[10] = elapsed(c, 7, 0);
-  }
-  c->phase_ms[1] = elapsed(c, 0, 1);
+  phase_end(c, 1);
+  c->h2d_timed = c->batch_piped ? 1 : 3;   /* (the copies end where the count begins) */
   c->stage = 2;
   if ((st = bruno_local_insert_by_freqencies(c, nullptr)) != BRUNO_OK) return st;
   if ((st = bruno_extract_chains(c)) != BRUNO_OK) return st;
@@ -884,6 +869,11 @@ bruno_status bruno_host_free(void *p) {
 
 bruno_status bruno_phase_ms(bruno_ctx *c, double *ms, size_t n) {
   if (!c || !ms) return BRUNO_ERR_ARG;
+  for (int p = 0; p < 6; ++p)
+    if (c->ptimed >> p & 1u) c->phase_ms[p] = elapsed(c->pev[p][0], c->pev[p][1]);
+  c->ptimed = 0;
+  if (c->h2d_timed) c->phase_ms[10] = elapsed(c->h2d_begin, c->h2d_timed == 1 ? c->h2d_end : c->pev[c->h2d_timed == 2 ? 0 : 1][0]);
+  c->h2d_timed = 0;
   for (size_t i = 0; i < n && i < 11; ++i) ms[i] = c->phase_ms[i];
   return BRUNO_OK;
 }

@@ -945,7 +945,8 @@ __global__ void __launch_bounds__(TPB) k_ranked(EmitArgs a) {
 }
 
 template <class KT>
-__global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off, char *chars) {
+__global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off, char *chars, uint64_t room) {
+  if (a.ctr->n_chain_chars > room) return;   /* (the host makes room and comes again) */
   constexpr int KWD = KOps<KT>::WORDS;
   const char ACGT[4] = {'A', 'C', 'G', 'T'};
   bool bad = false;
@@ -978,7 +979,9 @@ __global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off
  * they are covered once exactly when the live nodes are as many as the positions -- one per
  * chain for the representative's k bases plus one per further base -- which the host checks:
  * n_ranked == n_chain_chars - n_chains * (k - 1). */
-__global__ void k_check_chains(const char *chars, uint64_t nchars, DevCounters *ctr) {
+__global__ void k_check_chains(const char *chars, uint64_t room, DevCounters *ctr) {
+  const uint64_t nchars = ctr->n_chain_chars;
+  if (nchars > room) return;
   bool bad = false;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nchars; i += (uint64_t)gridDim.x * blockDim.x)
     if (chars[i] == 0) bad = true;
@@ -1318,6 +1321,7 @@ bruno_status extract_typed(Ctx *c) {
                     c->stream>>>((const uint64_t *)c->table.p, c->geom, (const SGeom *)c->sgeom.p, c->S, c->cfg.k,
                                  (ChainState *)c->cstate.p, M, 4096u, (const uint32_t *)c->branch_list.p, c->n_branch);
   c->launches += 2;
+  if (c->one_call) return cuda_check(c, cudaGetLastError(), "chain map");   /* the ranking looks at what went wrong */
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
   if (c->hctr->err & DERR_INVARIANT) return set_err(c, BRUNO_ERR_INVARIANT, "chain list incomplete");
   return BRUNO_OK;
@@ -1553,29 +1557,45 @@ bruno_status compress_typed(Ctx *c) {
     a.h_samp = (uint32_t *)c->h_samp.p;
   }
   const int sms = sms_count();
+  /* a small graph's chains are at most as many as its nodes, of k bases a node at most: nothing is
+   * waited for before the end (chains past the last have length 0) */
+  const bool small = c->S == 1 && M <= (1ull << 18);
+  if (small) cudaMemsetAsync(a.head_len, 0, (M + 1) * 8, c->stream);
   k_ranked<KT><<<sms * 8, TPB, 0, c->stream>>>(a);
-  if ((st = sync_counters(c)) != BRUNO_OK) return st;
-  c->n_ranked = c->hctr->n_ranked;
-  c->n_heads = c->hctr->n_heads;
-  const uint64_t nh = c->n_heads;
-  if (c->S > 1) {
-    if ((st = group_by_sample<KT>(c)) != BRUNO_OK) return st;
-    a.rK = (uint64_t *)c->r_K.p; a.rrep = (uint64_t *)c->r_rep.p; a.rdist = (int32_t *)c->r_dist.p;
-    a.heads = (uint32_t *)c->heads.p; a.head_len = (uint64_t *)c->head_len.p; a.ch_rep = (uint64_t *)c->ch_rep.p;
+  uint64_t nh = M, nchars = M * (uint64_t)c->cfg.k;
+  if (!small) {
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    c->n_ranked = c->hctr->n_ranked;
+    nh = c->n_heads = c->hctr->n_heads;
+    if (c->S > 1) {
+      if ((st = group_by_sample<KT>(c)) != BRUNO_OK) return st;
+      a.rK = (uint64_t *)c->r_K.p; a.rrep = (uint64_t *)c->r_rep.p; a.rdist = (int32_t *)c->r_dist.p;
+      a.heads = (uint32_t *)c->heads.p; a.head_len = (uint64_t *)c->head_len.p; a.ch_rep = (uint64_t *)c->ch_rep.p;
+    }
+    cudaMemsetAsync((uint64_t *)c->head_len.p + nh, 0, 8, c->stream);
   }
   /* offsets: exclusive scan of per-chain lengths, total into n_chain_chars */
-  cudaMemsetAsync((uint64_t *)c->head_len.p + nh, 0, 8, c->stream);
   if ((st = scan_ctx(c, (const uint64_t *)c->head_len.p, (uint64_t *)c->head_off.p, nh + 1,
                      &c->dctr->n_chain_chars)) != BRUNO_OK)
     return st;
-  if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  if (!small) {
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    nchars = c->hctr->n_chain_chars;
+  }
+  for (;;) {
+    if ((st = ensure(c, c->ch_chars, std::max<uint64_t>(1, nchars))) != BRUNO_OK) return st;
+    cudaMemsetAsync(c->ch_chars.p, 0, nchars, c->stream);
+    k_fill<KT><<<sms * 8, TPB, 0, c->stream>>>(a, (const uint64_t *)c->head_off.p, (char *)c->ch_chars.p, nchars);
+    k_check_chains<<<sms * 4, TPB, 0, c->stream>>>((const char *)c->ch_chars.p, nchars, c->dctr);
+    c->launches += 2;
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    if (c->hctr->n_chain_chars <= nchars) break;
+    nchars = c->hctr->n_chain_chars;   /* chain pointers that disagree: chains that share nodes */
+  }
+  c->launches += 1;   /* k_ranked (the scan counts its own) */
+  c->n_ranked = c->hctr->n_ranked;
+  nh = c->n_heads = c->hctr->n_heads;
   c->n_chain_chars = c->hctr->n_chain_chars;
-  if ((st = ensure(c, c->ch_chars, std::max<uint64_t>(1, c->n_chain_chars))) != BRUNO_OK) return st;
-  cudaMemsetAsync(c->ch_chars.p, 0, c->n_chain_chars, c->stream);
-  k_fill<KT><<<sms * 8, TPB, 0, c->stream>>>(a, (const uint64_t *)c->head_off.p, (char *)c->ch_chars.p);
-  c->launches += 3;  /* k_ranked, k_fill, k_check_chains (the scan counts its own) */
-  k_check_chains<<<sms * 4, TPB, 0, c->stream>>>((const char *)c->ch_chars.p, c->n_chain_chars, c->dctr);
-  if ((st = sync_counters(c)) != BRUNO_OK) return st;
   c->chains_clean = !(c->hctr->err & DERR_UNCLEAN_CHAINS) &&
                     c->n_ranked + nh * (uint64_t)(c->cfg.k - 1) == c->n_chain_chars;
   if (!c->chains_clean) return general_emission<KT>(c, a);
@@ -2764,6 +2784,7 @@ bruno_status run_list_rank(Ctx *c, int min_update) {
     bool used = false;
     if ((st = fast_list_rank(c, used)) != BRUNO_OK) return st;
     c->fast_ranked = used;
+    if (used && (c->hctr->err & DERR_INVARIANT)) return set_err(c, BRUNO_ERR_INVARIANT, "chain list incomplete");
     if (used) return BRUNO_OK;
   }
   const uint64_t M = c->n_chain, Mb = std::max<uint64_t>(1, M);
@@ -2781,6 +2802,7 @@ bruno_status run_list_rank(Ctx *c, int min_update) {
   k_lr_init<<<sms * 8, TPB, 0, c->stream>>>(cs, M, cur, &c->dctr->lr_remaining);
   c->launches += 2;  /* k_lr_init, k_separate */
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  if (c->hctr->err & DERR_INVARIANT) return set_err(c, BRUNO_ERR_INVARIANT, "chain list incomplete");
   uint64_t remaining = c->hctr->lr_remaining;
   bool all_compacted = remaining == 0;
   uint64_t iterations = 0;

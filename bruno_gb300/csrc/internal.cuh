@@ -28,7 +28,12 @@ struct DevCounters {
   long long last_nonws;                /* index of the last byte that is not \n or \r, -1 if none */
   unsigned long long bad_line;         /* first malformed line, ~0 if none */
   unsigned long long n_records;
-  unsigned long long n_instances, n_reads_used, n_slots_claimed, n_entries;
+  unsigned long long n_sk, n_sk_est;   /* super-k-mer record places taken, records listed for the estimate */
+  unsigned long long n_instances, n_reads_used;
+  double hll_sum;                      /* one sample's HyperLogLog registers: sum of 2^-register, ... */
+  unsigned int hll_zeros, hll_pad;     /* ... registers at zero */
+  /* from here to hll: cleared by every counting attempt */
+  unsigned long long n_slots_claimed, n_entries;
   unsigned long long n_nodes, n_branch, n_chain, n_filtered, n_k2_dump;
   unsigned long long flag_hist[16];
   unsigned long long lr_applied, lr_remaining, lr_cycles, lr_multi;
@@ -43,7 +48,7 @@ struct DevCounters {
    * nodes and live branch nodes after an erasure pass */
   unsigned long long cl_term, cl_nonzero, cl_sum, cl_norm, cl_q, cl_found, cl_dead, cl_bub, cl_live, cl_live_branch;
   unsigned long long n_big, n_big_res; /* entries counted past 2^24 (keys in big_key), resolved */
-  unsigned long long n_sk, n_sk_est;   /* super-k-mer record places taken, records listed for the estimate */
+  unsigned long long sk_bump;          /* table slots taken by the one sample's regions */
   unsigned long long n_over;           /* partitions whose k-mers overflowed their CTA's slots */
   unsigned long long n_cand;           /* slots the count listed for the filter */
   unsigned long long quick_hist[16];   /* the filter flags of the entries the count dropped */
@@ -169,7 +174,7 @@ struct Ctx {
   std::vector<uint64_t> sk_gaps; /* a batch whose samples left table slots unwritten: their shares' sizes */
   uint32_t sk_bins = 0, sk_chunk = 32;
   std::vector<int> sk_bits, sk_q; /* per sample: log2 of its bins, of its estimate's sampling */
-  bool h2d_pending = false;      /* ev[7] marks the start of the current graph build's host-to-device copies */
+  bool h2d_pending = false;      /* h2d_begin marks the start of the current graph build's host-to-device copies */
   int force_direct_count = 0;    /* cfg.direct_count: 0 automatic, 1 whole table, 2 L2 partitions */
   Buf chain_list, branch_list;   /* slot indices, filled by the filter */
   Buf scan_tmp;                  /* block offsets of the multi-block scan */
@@ -220,7 +225,10 @@ struct Ctx {
   bool cleaned = false;
   uint64_t thr_used[6] = {0, 0, 0, 0, 0, 0};   /* the thresholds local_insert_by_freqencies used */
 
-  cudaEvent_t ev[8] = {nullptr};
+  cudaEvent_t pev[6][2] = {};      /* first and last event of the six phases */
+  unsigned ptimed = 0;             /* phases whose events are newer than phase_ms */
+  cudaEvent_t h2d_begin = nullptr; /* before the current graph build's first host-to-device copy */
+  int h2d_timed = 0;               /* that copy's end: 1 h2d_end, 2 the parse's, 3 the count's first event; 0 not newer */
   cudaEvent_t kev[5] = {nullptr};  /* counting sub-steps */
   double phase_ms[11] = {0};       /* 6 phases, then estimate/extract, table init, count, split,
                                       and the host-to-device copies of the FASTQ input */
