@@ -2644,7 +2644,7 @@ bruno_status run_index_reads(Ctx *c) {
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
   c->sk_on = sk_takes(c) && (c->S == 1 || !c->samp_off.empty());
-  c->pre_extracted = piped && c->S == 1 && !c->cfg.edge_filter && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
+  c->pre_extracted = piped && c->S == 1 && (!c->cfg.edge_filter || c->sk_on) && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
   if (c->pre_extracted) {
@@ -3167,12 +3167,17 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
 
 /* ------------------------------------------------ counting by super-k-mers, host side */
 
+/* One call: the count makes the nodes and nobody asks for what was counted */
+bool sk_makes_nodes(const Ctx *c) { return c->one_call && !c->cfg.keep_k2 && !c->cfg.keep_filtered; }
+
 /* k from 19: below, windows hold fewer than 5 m-mers and a run is hardly longer than a k-mer's own
- * record; a forced counting path or table size and the (k+1)-mer filter keep the k-mer records, and
- * so do builds without thresholds: they keep every k-mer, and 3.5M nodes at 12x (13.7M k-mers,
- * k = 31) took 3.28 ms by super-k-mers against 3.09 */
+ * record; a forced counting path or table size keeps the k-mer records.  The (k+1)-mer filter drops
+ * edges before anything is counted, so only a count that makes the nodes can do without them in the
+ * table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33 by
+ * a table of (k+1)-mers); a read of exactly k + 1 bases has a (k+1)-mer and no k-mer, and such an
+ * input goes by the table. */
 bool sk_takes(const Ctx *c) {
-  return c->cfg.k >= MZ_M + 4 && !c->cfg.edge_filter && c->force_direct_count == 0 &&
+  return c->cfg.k >= MZ_M + 4 && (!c->cfg.edge_filter || sk_makes_nodes(c)) && c->force_direct_count == 0 &&
          c->cfg.table_slots == 0;
 }
 
@@ -3196,6 +3201,7 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_
   a.items = items;
   a.n_items = n_items;
   a.k = c->cfg.k;
+  a.skew_len = c->cfg.edge_filter ? (uint32_t)c->cfg.k + 1 : ~0u;
   a.chunk = c->sk_chunk;
   a.samples = (const SkSample *)c->sk_samp.p;
   a.out = (uint64_t *)c->sk_recs.p;
@@ -3325,14 +3331,16 @@ struct SkShape {
 template <class KT>
 void sk_count_launch(const Ctx *c, const SkCount &a, uint32_t grid, size_t bytes) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_sk_count<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
+    cudaFuncSetAttribute(k_sk_count<KT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
+    cudaFuncSetAttribute(k_sk_count<KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
     return true;
   }();
   (void)attr;
   /* threads: the block's 384 unless the partitions are small or the configured block is */
   int nt = std::min(SK_COUNT_TPB, count_threads(c));
   while (nt > 128 && (uint32_t)nt * 2 > a.slots) nt -= 128;
-  k_sk_count<KT><<<grid, nt, bytes, c->stream>>>(a);
+  if (c->cfg.edge_filter) k_sk_count<KT, true><<<grid, nt, bytes, c->stream>>>(a);
+  else k_sk_count<KT, false><<<grid, nt, bytes, c->stream>>>(a);
 }
 
 /* One launch's partitions (all, or a size class of a batch's) and its blocks' shape */
@@ -3447,7 +3455,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if ((st = table_room(c, base)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->table, base * SU * 8)) != BRUNO_OK) return st;
     /* one call: the count makes the nodes, and lists them; a kept k-mer takes inv_load slots */
-    const bool nodes = c->one_call && !c->cfg.keep_k2 && !c->cfg.keep_filtered;
+    const bool nodes = sk_makes_nodes(c);
     const uint64_t list_cap = (uint64_t)((double)base / inv_load) + 1;
     if (nodes) {
       if ((st = ensure(c, c->chain_list, list_cap * 4)) != BRUNO_OK) return st;
@@ -3564,6 +3572,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
         c->n_nodes = c->n_chain + c->n_branch;
         for (int f = 0; f < 16; ++f) c->flag_hist[f] = c->hctr->flag_hist[f] + c->hctr->quick_hist[f];
         c->filter_read = c->hctr->n_cand;
+        if (c->cfg.edge_filter) c->n_entries = c->flag_hist[0];   /* the entries that are left */
       }
       used = true;
       return BRUNO_OK;
@@ -3782,6 +3791,12 @@ bruno_status build_k1w_table(Ctx *c) {
 
 template <class KT>
 bruno_status count_paths(Ctx *c) {
+  if (c->sk_on) {
+    bool used = false;
+    bruno_status st = count_one_superkmers<KT>(c, used);
+    if (st != BRUNO_OK || used) return st;
+    c->have_cand = false;
+  }
   if (c->cfg.edge_filter && sizeof(KT) == 16) {   /* k > 31: the 128-bit (k+1)-mer table, partitioned count */
     bruno_status st = build_k1w_table(c);
     if (st != BRUNO_OK) return st;
@@ -3795,12 +3810,6 @@ bruno_status count_paths(Ctx *c) {
     bool used = false;
     if ((st = count_partitioned(c, used)) != BRUNO_OK) return st;
     return used ? BRUNO_OK : set_err(c, BRUNO_ERR_TABLE_FULL, "a hash bucket overflowed under the (k+1)-mer filter");
-  }
-  if (c->sk_on) {
-    bool used = false;
-    bruno_status st = count_one_superkmers<KT>(c, used);
-    if (st != BRUNO_OK || used) return st;
-    c->have_cand = false;
   }
   if (sizeof(KT) == 8 && c->force_direct_count != 1) {
     bool used = false;

@@ -132,6 +132,7 @@ struct SkExtract {
   const XItem *items;
   uint64_t n_items;
   int k;
+  uint32_t skew_len;                /* a read of this length: the input is counted another way (~0: none) */
   uint32_t chunk;                   /* output records a warp reserves at once */
   const SkSample *samples;
   uint64_t *out;
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
         /* x never falls, so the reads that fit come first */
         const bool fits = lane < n_reads && x <= SK_WORDS, kept = fits && nw;
         const unsigned mf = __ballot_sync(~0u, fits), mk = __ballot_sync(~0u, kept);
+        if (fits && len == a.skew_len) atomicOr(&a.ctr->err, (unsigned long long)DERR_SKEW);
         reads = __popc(mf);
         n_words = mf ? __shfl_sync(~0u, x, 31 - __clz(mf)) : 0u;
         if (kept) {
@@ -770,8 +772,15 @@ __device__ __forceinline__ uint32_t sk_top20(KW2 x, int k) { return (uint32_t)KO
 
 /* local_insert_by_freqencies for one k-mer (filter_kmer's steps over entries in shared memory): the
  * node's counters, 0 if no entry is kept, 1 for a chain node, 2 for a branch node.  The entries'
- * flags 0..3 are tallied in the bytes of `few`, others in hist. */
-template <class KT>
+ * flags 0..3 are tallied in the bytes of `few`, others in hist.
+ *
+ * EF: the blocked driver's (k+1)-mer filter instead.  Every (k+1)-mer of a read is an out edge of its
+ * first k-mer and an in edge of its second, so an edge's occurrences over the k-mer's entries are
+ * those of its (k+1)-mer: no table of (k+1)-mers.  Twice those where the (k+1)-mer is its own reverse
+ * complement (both its k-mers are this one); and where the k-mer is, its out edge in b is its in edge
+ * in the complement of b, seen from the other strand.  Edges outside the bounds leave the entries;
+ * entries then alike are one, entries without edges none (flag 0 tallies what is left). */
+template <class KT, bool EF>
 __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key, const SkCount &a, uint64_t *pw,
                                        uint32_t &few, unsigned int *hist) {
   const int k = a.k;
@@ -787,7 +796,7 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
     kpal = k_palindrome(key, k);
   }
   uint32_t kf = 0, ok = 0;   /* ok: bit c (4 + c): the (k+1)-mers over in (out) base c are kept */
-  if (a.thresholding) {
+  if (EF || a.thresholding) {
     uint32_t k1[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     sk_entries<KT>(sl, q, key, [&](uint64_t x) {
       #pragma unroll
@@ -797,8 +806,8 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
         const uint32_t c = sk_count_of(w), half = (c + 1) >> 1;
         const unsigned code = entry_code(w), in5 = code_in5(code), out5 = code_out5(code);
         kf += c;
-        const uint32_t vi = oddk && high && !kpal && last == 4u - in5 ? half : c;
-        const uint32_t vo = oddk && low && !kpal && first == 4u - out5 ? half : c;
+        const uint32_t vi = !EF && oddk && high && !kpal && last == 4u - in5 ? half : c;
+        const uint32_t vo = !EF && oddk && low && !kpal && first == 4u - out5 ? half : c;
         #pragma unroll
         for (unsigned b = 0; b < 4; ++b) {
           k1[b] += in5 == b + 1 ? vi : 0u;
@@ -809,12 +818,16 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
     kf = min(0xFFFFu, kf);
     #pragma unroll
     for (int b = 0; b < 8; ++b) {
-      const uint32_t v = min(0xFFFFu, k1[b]);
+      uint32_t v = k1[b];
+      if (EF && kpal) v += k1[7 - b];
+      if (EF && (b < 4 ? high && last == 3u - b : low && first == 7u - b)) v >>= 1;
+      v = min(0xFFFFu, v);
       ok |= v >= a.t[2] && v < a.t[3] ? 1u << b : 0u;
     }
   }
   uint32_t nc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   bool any = false;
+  uint32_t left = 0;   /* EF: the codes of the entries that are left */
   sk_entries<KT>(sl, q, key, [&](uint64_t x) {
     #pragma unroll
     for (int z = 0; z < 2; ++z) {
@@ -823,13 +836,19 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
       const uint32_t c16 = min(0xFFFFu, sk_count_of(w));
       const unsigned code = entry_code(w);
       unsigned in5 = code_in5(code), out5 = code_out5(code), f = 0;
-      if (a.thresholding) {   /* an absent base counts as a (k+1)-mer outside the bounds */
+      if (EF) {
+        if (!((ok << 1) >> in5 & 1u)) in5 = 0;
+        if (!((ok >> 3) >> out5 & 1u)) out5 = 0;
+        if (in5 == 0 && out5 == 0) continue;
+        left |= 1u << biedge_code(in5, out5);
+      } else if (a.thresholding) {   /* an absent base counts as a (k+1)-mer outside the bounds */
         if (c16 < a.t[4] || c16 >= a.t[5]) f |= 4;
         if (kf < a.t[0] || kf >= a.t[1]) f |= 8;
         if (!((ok << 1) >> in5 & 1u) || !in5) f |= 2;
         if (!((ok >> 3) >> out5 & 1u) || !out5) f |= 1;
       }
-      if (f < 4) few += 1u << (8 * f);   /* (at most 25 entries a k-mer) */
+      if (EF) ;
+      else if (f < 4) few += 1u << (8 * f);   /* (at most 25 entries a k-mer) */
       else atomicAdd(&hist[f], 1u);
       if (f >= 3) continue;
       if (f == 1) out5 = 0;
@@ -844,6 +863,7 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
     }
   });
   if (!any) return 0;
+  if (EF) few += __popc(left);
   unsigned din = 0, dout = 0;   /* IsBranchPoint / IsChainNode (debruijn_graph_filters.hpp:57-220) */
   bool k1pal = false;
   #pragma unroll
@@ -861,7 +881,7 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
   return din >= 2 || dout >= 2 || kpal || k1pal ? 2 : 1;
 }
 
-template <class KT>
+template <class KT, bool EF>
 __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_count(SkCount a) {
   constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW, NE = Slot<KT>::ENTRIES, NW = SkRec<KT>::NW;
   extern __shared__ __align__(16) uint64_t sm[];
@@ -1015,7 +1035,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   uint16_t *kept = reinterpret_cast<uint16_t *>(s_rec);
   uint64_t qh = 0;   /* quick drops' flags 3 | 8 | 4 as 16-bit fields (a thread sees under 2^11 slots) */
   uint32_t my_conts = 0;
-  const uint32_t t_low = a.thresholding ? a.t[2] : 0u;
+  uint32_t t_low = a.thresholding ? a.t[2] : 0u;
+  if (EF && !(k & 1)) t_low = (t_low + 1) / 2;   /* (a palindrome's edges occur up to twice as often as it) */
   const bool no_bounds = a.t[0] == 0 && a.t[1] > 0xFFFFu && a.t[4] == 0 && a.t[5] > 0xFFFFu;   /* flags 3 only */
   for (uint32_t q0 = tid & ~31u; q0 < slots; q0 += nt) {
     const uint32_t q = q0 + lane;   /* slots are a multiple of 32 */
@@ -1036,7 +1057,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         kf = min(0xFFFFu, kf);
         listed = kf >= t_low;
         keep = listed || a.keep_all;
-        if (!listed) {
+        if (!EF && !listed) {
           if (no_bounds && !more) {
             qh += 1 + (c1 != 0);
           } else {
@@ -1093,7 +1114,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     kind = 0;
     if (x < nkept) {
       const KT key = sl.key(kept[x]);
-      kind = sk_node<KT>(sl, kept[x], key, a, pw, few, s_hist);
+      kind = sk_node<KT, EF>(sl, kept[x], key, a, pw, few, s_hist);
       t = table_key(key);
     }
     const unsigned mc = __ballot_sync(~0u, kind == 1), mb = __ballot_sync(~0u, kind == 2);
@@ -1119,11 +1140,11 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     s_nbase[list] = atomicAdd(list ? &a.ctr->n_branch : &a.ctr->n_chain, (unsigned long long)n);
     if (a.s_tally) atomicAdd(&a.s_tally[(uint64_t)smp * T_NUM + (list ? T_BRANCH : T_CHAIN)], (unsigned long long)n);
   };
-  if (a.nodes) {
+  if (EF || a.nodes) {
     make_node(tid);
     __syncthreads();
   }
-  if (a.nodes && (tid == 32 || tid == 64)) reserve(tid / 32 - 1, sample_of_part(a.sg, a.nsamples, part));
+  if ((EF || a.nodes) && (tid == 32 || tid == 64)) reserve(tid / 32 - 1, sample_of_part(a.sg, a.nsamples, part));
   if (tid == 0) {
     const uint32_t R = want_R;
     const uint32_t smp = sample_of_part(a.sg, a.nsamples, part);
@@ -1138,7 +1159,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     a.info[part] = make_uint2((uint32_t)(g.base + lo), R);
     if (!a.cand) atomicAdd(&a.ctr->n_cand, (unsigned long long)listed);
     if (tslots) atomicAdd(&a.ctr->n_slots_claimed, (unsigned long long)tslots);
-    if (s_claims) atomicAdd(&a.ctr->n_entries, (unsigned long long)s_claims);
+    if (!EF && s_claims) atomicAdd(&a.ctr->n_entries, (unsigned long long)s_claims);
     if (a.s_tally && s_claims) atomicAdd(&a.s_tally[(uint64_t)smp * T_NUM + T_ENTRIES], (unsigned long long)s_claims);
   }
   if (tid < 4 && s_qh[tid]) atomicAdd(&a.ctr->quick_hist[3 + 4 * tid], (unsigned long long)s_qh[tid]);
@@ -1156,7 +1177,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
       if (++pos == R) pos = 0;
     }
   };
-  if (a.nodes) {   /* the nodes themselves */
+  if (EF || a.nodes) {   /* the nodes themselves */
     for (uint32_t x0 = 0;;) {
       if (kind) {
         const unsigned long long o = s_nbase[kind - 1] + at;
@@ -1188,7 +1209,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
       __syncthreads();
     }
   }
-  for (uint32_t x = tid; x < (a.nodes ? 0u : nkept); x += nt) {
+  for (uint32_t x = tid; x < (EF || a.nodes ? 0u : nkept); x += nt) {
     const uint32_t q = x < listed ? kept[x] : kept[slots - 1 - (x - listed)];
     const KT key = sl.key(q), t = table_key(key);
     const uint32_t pos = place(bin_home(t, R));

@@ -8,7 +8,7 @@ import pytest
 import bruno_gb300 as bg
 from helpers import assert_same, chain_set, sort_nodes, sort_ranked
 from oracle import oracle
-from test_gpu_parity import compare, gpu_run
+from test_gpu_parity import compare, compare_one_call, gpu_run, one_call_run
 
 pytestmark = pytest.mark.gpu
 
@@ -108,3 +108,25 @@ def test_one_call_keeps_what_the_filter_keeps(k, lower):
         assert_same(sort_nodes(*g.nodes()), ref["nodes"], "graph nodes")
         assert_same(sort_ranked(*g.ranked()), ref["ranked"], "listranked chain nodes")
         assert chain_set(*g.chains()) == chain_set(*ref["chains"])
+
+
+@pytest.mark.parametrize("with_k1", [False, True])
+@pytest.mark.parametrize("k", [20, 21, 31, 32, 45, 62, 63])
+def test_edge_filter_from_the_entries(k, with_k1):
+    """the (k+1)-mer filter of a one-call build: (k+1)-mers and (even k) k-mers that are their own
+    reverse complements, homopolymers and k-mers between every pair of bases, with bounds around their
+    counts; a read of k + 1 bases has a (k+1)-mer and no k-mer"""
+    rng = np.random.default_rng(k)
+    rand = lambda n: "".join("ACGT"[c] for c in rng.integers(0, 4, n))
+    core, half = rand(k), rand((k + 1) // 2)
+    wide = [rand(40) + a + core + b + rand(40) for a in "ACGT" for b in "ACGT"]
+    pal = [rand(50) + half + rc(half) + rand(50) for _ in range(3)]
+    reads = [r for r in edge_reads(k, 3) if with_k1 or len(r) != k + 1]
+    reads += wide * 2 + pal * 2 + [rc(x) for x in pal] + [core + w[60:] for w in wide] + [half + rc(half) + "A", "A" * (k + 2)]
+    if with_k1:
+        reads += [(half + rc(half))[:k + 1], core + "A"] * 2
+    data = fastq(reads)
+    for lo, hi in ((1, 65536), (2, 65536), (5, 65536), (2, 9)):
+        thr = np.array([0, 65536, lo, hi, 0, 65536], dtype=np.uint64)
+        ref = oracle.run(data, k=k, thresh=thr, min_update=True, keep_k2=True, keep_filtered=True, edge_filter=True)
+        compare_one_call(one_call_run(data, k, True, thr, True, edge_filter=True), ref)
