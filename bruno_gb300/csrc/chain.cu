@@ -230,6 +230,183 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
   }
 }
 
+/* The same for a table in minimizer partitions, a partition a block: its nodes' k-mers and chain
+ * indices in shared memory, chained from a hash of their own, where eight neighbours of nine are
+ * found (k = 31: a window's minimizer changes at 2 / 18 of the positions) without their minimizer,
+ * their table key or a read of the table; the sides left over are listed and looked up in the table
+ * with every lane at work.  Bound by instructions, of which k_chain_init spends a thousand a node, on
+ * the neighbours' minimizers and keys and on lanes that wait for the longest of 64 probe runs (49M
+ * nodes: 3.05 ms, now 2.18; with the table's own probe runs in shared memory 2.84).  A partition of
+ * more than `cap` nodes goes through by the piece, with every side looked up in the table. */
+constexpr int CI_NODES = 4096;   /* `cap` at most: a node and a side in 16 bits */
+template <class KT>
+__host__ __device__ constexpr size_t ci_bytes(uint32_t cap) { return (size_t)cap * (KOps<KT>::WORDS * 8 + 4 + 4 + 2 + 2 + 4); }
+__device__ __forceinline__ uint32_t ci_hash(KW1 x, uint32_t n) {
+  return __umulhi(((uint32_t)x.v ^ (uint32_t)(x.v >> 32) * 0x85EBCA6Bu) * 0x9E3779B1u, n);
+}
+__device__ __forceinline__ uint32_t ci_hash(KW2 x, uint32_t n) {
+  const uint64_t y = x.lo ^ x.hi * 0xD6E8FEB86659FD93ull;
+  return ci_hash(KW1{y}, n);
+}
+template <class KT>
+__global__ void __launch_bounds__(TPB, sizeof(KT) == 8 ? 6 : 4) k_chain_local(const uint64_t *table, TableGeom g0, const SGeom *sg,
+                                                      uint32_t nsamples, int k, uint64_t M, uint32_t cap, uint64_t *ckey,
+                                                      ChainState *cs, uint8_t *cedge, uint32_t *csample,
+                                                      uint32_t max_probe, DevCounters *ctr) {
+  constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW;
+  constexpr uint16_t END = 0xFFFFu;
+  extern __shared__ __align__(16) uint64_t s_kmer[];
+  uint32_t *s_aux = reinterpret_cast<uint32_t *>(s_kmer + (size_t)cap * KWD);   /* chain index, NONE32: a branch node */
+  uint32_t *s_head = s_aux + cap;                       /* first node of each of `cap` hash chains */
+  uint16_t *s_next = reinterpret_cast<uint16_t *>(s_head + cap), *s_todo = s_next + cap;
+  uint16_t *s_edge = s_todo + 2 * cap;                  /* a node's slot, then its edge byte */
+  __shared__ uint32_t s_n, s_left;
+  const uint2 reg = g0.info[blockIdx.x];
+  const uint32_t R = reg.y, nt = blockDim.x, lane = threadIdx.x & 31, below = (1u << lane) - 1;
+  bool bad = false;
+  auto append = [&](bool want, uint32_t *n) -> uint32_t {   /* the warp's places in a list of the block */
+    const unsigned m = __ballot_sync(~0u, want);
+    uint32_t at = 0;
+    if (lane == 0 && m) at = atomicAdd(n, (uint32_t)__popc(m));
+    return __shfl_sync(~0u, at, 0) + __popc(m & below);
+  };
+  /* the neighbour over base c at one side (0 in: nextReverseFromChar, 1 out: nextFromChar), canonical */
+  auto neighbour = [&](KT K, KT rK, unsigned c, int side, bool &flip) -> KT {
+    const KT n = side ? KOps<KT>::append(K, c, k) : KOps<KT>::prepend(c, K, k);
+    const KT y = side ? KOps<KT>::prepend(3u - c, rK, k) : KOps<KT>::append(rK, 3u - c, k);
+    flip = !KOps<KT>::lt(n, y);
+    return flip ? y : n;
+  };
+  /* 4 | the last base with a count, 0 if none has one */
+  auto edge = [](uint64_t counts) { return counts ? 4u | (unsigned)(63 - __clzll(counts)) >> 4 : 0u; };
+  const uint32_t smp = nsamples > 1 ? sample_of_part(sg, nsamples, blockIdx.x) : 0u;
+  bool local = true;
+  for (uint32_t t0 = 0; t0 < R; ) {
+    const uint32_t n = local ? R : min(cap, R - t0);
+    const uint64_t *slots = table + ((uint64_t)reg.x + t0) * SU;
+    if (threadIdx.x == 0) { s_n = 0; s_left = 0; }
+    for (uint32_t i = threadIdx.x; i < cap; i += nt) s_head[i] = END;
+    __syncthreads();
+    constexpr int U = 4;   /* loads in flight a thread */
+    for (uint32_t i0 = threadIdx.x & ~31u; i0 < n; i0 += U * nt) {
+      bool node[U];
+      #pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t i = i0 + u * nt + lane;
+        node[u] = i < n && key_is_node(KOps<KT>::load(slots + (uint64_t)i * SU));
+      }
+      #pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t at = append(node[u], &s_n);
+        if (node[u] && at < cap) s_edge[at] = (uint16_t)(i0 + u * nt + lane);
+      }
+    }
+    __syncthreads();
+    const uint32_t nodes = s_n;
+    if (nodes > cap) {   /* (of the whole partition; a piece has as many slots) */
+      __syncthreads();
+      local = false;
+      continue;
+    }
+    for (uint32_t x = threadIdx.x; x < nodes; x += nt) {
+      const uint64_t *w = slots + (uint64_t)s_edge[x] * SU;
+      const uint64_t f = w[KWD + 2];
+      const unsigned out = edge(w[KWD]), in = edge(w[KWD + 1]);
+      uint32_t a = NONE32;
+      if ((f >> 16) & NF_CHAIN) {
+        a = (uint32_t)(f >> 32);
+        if (a >= M) { bad = true; a = NONE32; }
+      }
+      const KT K = key_kmer(node_key(KOps<KT>::load(w)));
+      KOps<KT>::store(s_kmer + (size_t)x * KWD, K);
+      s_aux[x] = a;
+      s_edge[x] = (uint16_t)(in | (out << 3));
+      if (local) s_next[x] = (uint16_t)atomicExch(&s_head[ci_hash(K, cap)], x);
+    }
+    __syncthreads();
+    for (uint32_t y0 = threadIdx.x & ~31u; y0 < nodes; y0 += nt) {
+      const uint32_t i = min(y0 + lane, nodes - 1), a = s_aux[i];
+      const bool live = y0 + lane < nodes && a != NONE32;
+      const unsigned edges = s_edge[i];
+      const KT K = KOps<KT>::load(s_kmer + (size_t)i * KWD), rK = KOps<KT>::rc(K, k);
+      uint64_t P[2];
+      uint32_t D[2], at[2] = {END, END};
+      bool left[2], flip[2];
+      KT want[2];
+      #pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const unsigned e = edges >> (3 * q) & 7u;
+        left[q] = live && e;
+        P[q] = left[q] ? PF_EXT | (q ? PF_EXTOUT : 0) | a : PF_BLANK;
+        D[q] = left[q] ? 1 : TM;
+        want[q] = neighbour(K, rK, e & 3u, q, flip[q]);
+        if (local && left[q]) at[q] = s_head[ci_hash(want[q], cap)];
+      }
+      while (__any_sync(~0u, (at[0] & at[1]) != END)) {   /* both sides' chains; each ends */
+        #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (at[q] == END) continue;
+          if (KOps<KT>::eq(KOps<KT>::load(s_kmer + (size_t)at[q] * KWD), want[q])) {
+            const uint32_t to = s_aux[at[q]];
+            if (to != NONE32) P[q] = (uint64_t)to | (flip[q] ? PF_FLIP : 0);
+            left[q] = false;
+            at[q] = END;
+          } else {
+            at[q] = s_next[at[q]];
+          }
+        }
+      }
+      #pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t o = append(left[q], &s_left);
+        if (left[q]) s_todo[o] = (uint16_t)(i | (q << 15));
+      }
+      if (!live) continue;
+      KOps<KT>::store(ckey + (uint64_t)a * KWD, K);
+      ChainState st;
+      st.inP = P[0]; st.outP = P[1]; st.inD = D[0]; st.outD = D[1]; st.pad = 0;
+      cs[a] = st;
+      cedge[a] = (uint8_t)edges;
+      if (nsamples > 1) csample[a] = smp;
+    }
+    __syncthreads();
+    /* neighbours in other partitions, or in none */
+    const uint32_t todo = s_left;
+    for (uint32_t y0 = threadIdx.x & ~31u; y0 < todo; y0 += nt) {
+      const bool live = y0 + lane < todo;
+      const uint32_t e = s_todo[live ? y0 + lane : 0], i = e & 0x7FFFu;
+      const int q = (int)(e >> 15);
+      const KT K = KOps<KT>::load(s_kmer + (size_t)i * KWD);
+      bool flip;
+      const KT want = neighbour(K, KOps<KT>::rc(K, k), s_edge[i] >> (3 * q) & 3u, q, flip), bare = table_key(want), x = as_node(bare);
+      Probe pr = bin_probe(nsamples > 1 ? sg[smp].g : g0, kmer_minimizer(want, k), bare);
+      bool seek = live;
+      for (uint32_t p = 0; p < max_probe && __any_sync(~0u, seek); ++p) {
+        if (!seek) continue;
+        uint64_t raw[SU];
+        ld_slot<SU>(table + pr.i * SU, raw);
+        const KT key = KOps<KT>::load(raw);
+        if (KOps<KT>::eq(key, x)) {
+          const uint32_t to = (uint32_t)(raw[KWD + 2] >> 32);
+          if (((raw[KWD + 2] >> 16) & NF_CHAIN) && to < M) {
+            const uint64_t P = (uint64_t)to | (flip ? PF_FLIP : 0);
+            ChainState &st = cs[s_aux[i]];
+            if (q) st.outP = P; else st.inP = P;
+          }
+          seek = false;
+        } else if (key_is_empty(key)) {
+          seek = false;
+        } else {
+          pr.next();
+        }
+      }
+    }
+    __syncthreads();   /* the lists are the next piece's */
+    t0 += n;
+  }
+  if (bad) atomicOr(&ctr->err, (unsigned long long)DERR_INVARIANT);
+}
+
 /* neighbours of branch nodes get their facing side set to branch_neighbor (0) */
 template <class KT>
 __global__ void __launch_bounds__(TPB) k_termini(const uint64_t *table, TableGeom g0, const SGeom *sg,
@@ -1311,11 +1488,29 @@ bruno_status extract_typed(Ctx *c) {
   const int sms = sms_count();
   cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
   if (c->S > 1 && (st = ensure(c, c->csample, Mb * 4)) != BRUNO_OK) return st;
-  k_chain_init<KT><<<sms * 8, TPB, 0, c->stream>>>((const uint64_t *)c->table.p, c->nslots, c->geom,
-                                                   (const SGeom *)c->sgeom.p, c->S, c->cfg.k,
-                                                   (const uint32_t *)c->chain_list.p, M, (uint64_t *)c->ckey.p,
-                                                   (ChainState *)c->cstate.p, (uint8_t *)c->cedge.p,
-                                                   (uint32_t *)c->csample.p, 4096u, c->dctr);
+  /* by partitions where the table has them and its chain nodes are the listed ones (nodes erased
+   * since the lists were made stay in the chain map, without neighbours) */
+  if (c->geom.bins && !c->nodes_erased) {
+    static const bool attr = cudaFuncSetAttribute(k_chain_local<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)ci_bytes<KT>(CI_NODES)) == cudaSuccess;
+    (void)attr;
+    /* half as much again as a typical partition's nodes; a thread for about two to four of them: more
+     * threads wait longer at the barriers, fewer go round more often (k = 31, 188 nodes: 2.18 ms with
+     * 128 threads, 2.36 with 64, 2.39 with 32; 300 nodes: 0.46 with 128, 0.60 with 256, 0.54 with 64;
+     * 900 nodes: 0.24 with 256, 0.27 with 128; k = 63, 150 nodes: 1.39 with 64, 1.60 with 128) */
+    const double mean = (double)(M + c->n_branch) / c->sk_parts;
+    const uint32_t cap = (uint32_t)std::max(128.0, std::min((double)CI_NODES, 1.5 * mean + 64.0)) & ~31u;
+    const int nt = KWD == 1 ? (mean > 500 ? TPB : mean > 120 ? TPB / 2 : TPB / 4) : mean > 300 ? TPB / 2 : TPB / 4;
+    k_chain_local<KT><<<c->sk_parts, nt, ci_bytes<KT>(cap), c->stream>>>(
+        (const uint64_t *)c->table.p, c->geom, (const SGeom *)c->sgeom.p, c->S, c->cfg.k, M, cap, (uint64_t *)c->ckey.p,
+        (ChainState *)c->cstate.p, (uint8_t *)c->cedge.p, (uint32_t *)c->csample.p, 4096u, c->dctr);
+  } else {
+    k_chain_init<KT><<<sms * 8, TPB, 0, c->stream>>>((const uint64_t *)c->table.p, c->nslots, c->geom,
+                                                     (const SGeom *)c->sgeom.p, c->S, c->cfg.k,
+                                                     (const uint32_t *)c->chain_list.p, M, (uint64_t *)c->ckey.p,
+                                                     (ChainState *)c->cstate.p, (uint8_t *)c->cedge.p,
+                                                     (uint32_t *)c->csample.p, 4096u, c->dctr);
+  }
   if (c->n_branch)
     k_termini<KT><<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(sms * 8, (c->n_branch + TPB - 1) / TPB)), TPB, 0,
                     c->stream>>>((const uint64_t *)c->table.p, c->geom, (const SGeom *)c->sgeom.p, c->S, c->cfg.k,
@@ -2641,6 +2836,7 @@ bruno_status clean_typed(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t 
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     if (c->hctr->err & DERR_INVARIANT) return set_err(c, BRUNO_ERR_INVARIANT, "cleaning: node lists overflowed");
     c->n_chain = c->hctr->n_chain;
+    c->nodes_erased = false;
     c->n_branch = c->hctr->n_branch;
     c->n_nodes = c->n_chain + c->n_branch;
     if ((st = extract_typed<KT>(c)) != BRUNO_OK) return st;
@@ -2848,6 +3044,7 @@ bruno_status run_node_query(Ctx *c, int filter, bool erase, uint64_t *keys, uint
   if (gaps != BRUNO_OK) return gaps;
   bruno_status st = c->W == 1 ? node_query_typed<KW1>(c, filter, erase, keys, counts, flags, cap, n)
                               : node_query_typed<KW2>(c, filter, erase, keys, counts, flags, cap, n);
+  c->nodes_erased |= erase;
   if (st != BRUNO_OK || !erase) return st;
   return c->W == 1 ? node_recount_typed<KW1>(c) : node_recount_typed<KW2>(c);
 }
@@ -2859,6 +3056,7 @@ bruno_status run_check_index(Ctx *c, bruno_index_check *out) {
 bruno_status run_erase_nodes(Ctx *c, const uint64_t *kmers, size_t n) {
   const bruno_status gaps = run_fill_gaps(c);   /* they scan the whole table */
   if (gaps != BRUNO_OK) return gaps;
+  c->nodes_erased = true;
   return c->W == 1 ? erase_nodes_typed<KW1>(c, kmers, n) : erase_nodes_typed<KW2>(c, kmers, n);
 }
 bruno_status run_chain_query(Ctx *c, int filter, int which, uint64_t *kmers, uint64_t *inK, uint64_t *outK,

@@ -170,6 +170,9 @@ struct Ctx {
    * will use and nobody asks for raw counts, so the count need not keep what the filter drops */
   bool one_call = false;
   bool nodes_made = false;       /* ... and the count made the nodes */
+  bool nodes_erased = false;     /* nodes have left the graph since their lists were made */
+  uint32_t sk_parts = 0;         /* minimizer partitions of the table, ... */
+  uint64_t sk_taken = 0;         /* ... and the slots in them */
   uint64_t sk_cap = 0, sk_est_cap = 0;
   std::vector<uint64_t> sk_gaps; /* a batch whose samples left table slots unwritten: their shares' sizes */
   uint32_t sk_bins = 0, sk_chunk = 32;
