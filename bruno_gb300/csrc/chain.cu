@@ -1058,6 +1058,7 @@ __device__ __forceinline__ KT ptr_kmer(uint64_t P, const uint64_t *ckey, const u
   return (P & PF_FLIP) ? KOps<KT>::rc(base, k) : base;
 }
 
+constexpr uint32_t SENSE = 0x80000000u;
 struct EmitArgs {
   const uint64_t *ckey;
   const uint8_t *cedge;
@@ -1068,7 +1069,7 @@ struct EmitArgs {
   uint64_t *rK, *rrep;
   int32_t *rdist;
   uint32_t *rep_idx;   /* per chain node: chain index of its representative, NONE32 if external */
-  int32_t *dist_of;    /* per chain node: rank distance */
+  int32_t *dist_of;    /* per chain node: rank distance, SENSE if the k-mer is on its chain's strand */
   uint32_t *head_of;   /* per chain node: chain ordinal if it is a head */
   uint32_t *heads;     /* per chain ordinal: head node */
   uint64_t *head_len;  /* per chain ordinal: k - 1 + nodes */
@@ -1099,7 +1100,7 @@ __global__ void __launch_bounds__(TPB) k_ranked(EmitArgs a) {
       const uint32_t sd = sense ? st.inD : st.outD;
       const uint64_t sp = sense ? st.inP : st.outP;
       a.rep_idx[i] = term(sd) ? (uint32_t)i : ((sp & (PF_EXT | PF_BLANK)) ? NONE32 : (uint32_t)sp);
-      a.dist_of[i] = dist;
+      a.dist_of[i] = (int32_t)((uint32_t)dist | (sense ? SENSE : 0u));
       head = dist == 0;
     }
     const unsigned long long o = block_append(live, &a.ctr->n_ranked);
@@ -1121,6 +1122,9 @@ __global__ void __launch_bounds__(TPB) k_ranked(EmitArgs a) {
   }
 }
 
+/* The chains' characters.  A node's strand comes from k_ranked, which has its ends' k-mers at hand:
+ * working it out again took the node's chain-map record and two scattered k-mers more, 1.6 ms of
+ * 49M nodes, now 0.6.  Bound by what is left of the scattered reads (head, offsets). */
 template <class KT>
 __global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off, char *chars, uint64_t room) {
   if (a.ctr->n_chain_chars > room) return;   /* (the host makes room and comes again) */
@@ -1133,19 +1137,16 @@ __global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off
     const uint32_t h = (ri == NONE32) ? NONE32 : a.head_of[ri];
     if (h == NONE32) { bad = true; continue; }
     const uint64_t off = ch_off[h], len = ch_off[h + 1] - off;
-    const int32_t d = a.dist_of[i];
-    const ChainState st = a.cs[i];
+    const uint32_t d = (uint32_t)a.dist_of[i] & DM;
+    const bool sense = (uint32_t)a.dist_of[i] & SENSE;
     const KT key = KOps<KT>::load(a.ckey + i * KWD);
-    const KT L = term(st.inD) ? key : ptr_kmer<KT>(st.inP, a.ckey, a.cedge, a.k);
-    const KT R = KOps<KT>::rc(term(st.outD) ? key : ptr_kmer<KT>(st.outP, a.ckey, a.cedge, a.k), a.k);
-    const bool sense = KOps<KT>::le(L, R);
-    const KT K = sense ? key : KOps<KT>::rc(key, a.k);
     if (d == 0) {   /* the representative itself: all k bases */
+      const KT K = sense ? key : KOps<KT>::rc(key, a.k);
       for (int q = 0; q < a.k; ++q) chars[off + q] = ACGT[KOps<KT>::base_lsb(K, a.k - 1 - q)];
     } else {        /* one base per node: the last base of K on the representative's strand */
       const uint64_t pos = (uint64_t)(a.k - 1) + (uint64_t)d;
       if (pos >= len) { bad = true; continue; }
-      chars[off + pos] = ACGT[KOps<KT>::last(K)];
+      chars[off + pos] = ACGT[sense ? KOps<KT>::last(key) : 3u - KOps<KT>::first(key, a.k)];
     }
   }
   if (bad) atomicOr(&a.ctr->err, (unsigned long long)DERR_UNCLEAN_CHAINS);
@@ -1248,7 +1249,7 @@ __global__ void __launch_bounds__(TPB) k_gen_resolve(const uint8_t *removed, con
     uint32_t g = gid[i];
     if (g & GID_OWNER) g = own_gid[g & ~GID_OWNER];
     gid[i] = g;
-    atomicMax(gmax + g, (uint32_t)abs(dist_of[i]));
+    atomicMax(gmax + g, ((uint32_t)dist_of[i] & DM));
   }
 }
 
@@ -1263,7 +1264,7 @@ __global__ void __launch_bounds__(TPB) k_gen_hist(const uint8_t *removed, const 
                                                    uint64_t *wcnt) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (uint64_t)gridDim.x * blockDim.x) {
     if (removed[i]) continue;
-    const uint32_t d = (uint32_t)abs(dist_of[i]);
+    const uint32_t d = ((uint32_t)dist_of[i] & DM);
     const uint64_t x = hoff[gid[i]] + d;
     atomicAdd((unsigned long long *)(ncnt + x), 1ull);
     atomicAdd((unsigned long long *)(wcnt + x), d == 0 ? (unsigned long long)k : 1ull);
@@ -1275,7 +1276,7 @@ __global__ void __launch_bounds__(TPB) k_gen_place(const uint8_t *removed, const
                                                     uint32_t *cur, uint32_t *members) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (uint64_t)gridDim.x * blockDim.x) {
     if (removed[i]) continue;
-    const uint64_t x = hoff[gid[i]] + (uint32_t)abs(dist_of[i]);
+    const uint64_t x = hoff[gid[i]] + ((uint32_t)dist_of[i] & DM);
     members[noff[x] + atomicAdd(cur + x, 1u)] = (uint32_t)i;
   }
 }
