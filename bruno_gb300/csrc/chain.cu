@@ -1123,8 +1123,8 @@ __global__ void __launch_bounds__(TPB) k_ranked(EmitArgs a) {
 }
 
 /* The chains' characters.  A node's strand comes from k_ranked, which has its ends' k-mers at hand:
- * working it out again took the node's chain-map record and two scattered k-mers more, 1.6 ms of
- * 49M nodes, now 0.6.  Bound by what is left of the scattered reads (head, offsets). */
+ * working it out again took the node's chain-map record and two scattered k-mers more: 49M nodes 1.6 ms,
+ * now 0.4.  Bound by what is left of the scattered reads (head, offsets). */
 template <class KT>
 __global__ void __launch_bounds__(TPB) k_fill(EmitArgs a, const uint64_t *ch_off, char *chars, uint64_t room) {
   if (a.ctr->n_chain_chars > room) return;   /* (the host makes room and comes again) */
@@ -1489,9 +1489,11 @@ bruno_status extract_typed(Ctx *c) {
   const int sms = sms_count();
   cudaMemsetAsync(&c->dctr->err, 0, 8, c->stream);
   if (c->S > 1 && (st = ensure(c, c->csample, Mb * 4)) != BRUNO_OK) return st;
-  /* by partitions where the table has them and its chain nodes are the listed ones (nodes erased
-   * since the lists were made stay in the chain map, without neighbours) */
-  if (c->geom.bins && !c->nodes_erased) {
+  /* by partitions where the table has them, its chain nodes are the listed ones (nodes erased since
+   * the lists were made stay in the chain map, without neighbours) and a slot in four at least is a
+   * node (one in two of a one-call build; in a table of all k-mers one in 13, k = 45, 18M slots: 0.31
+   * ms against the list's 0.20) */
+  if (c->geom.bins && !c->nodes_erased && 4 * (M + c->n_branch) >= c->sk_taken) {
     static const bool attr = cudaFuncSetAttribute(k_chain_local<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)ci_bytes<KT>(CI_NODES)) == cudaSuccess;
     (void)attr;
