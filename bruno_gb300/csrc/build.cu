@@ -3316,9 +3316,15 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
                     "super-k-mer samples");
 }
 
-/* bins -> partitions (plan: one a sample), records -> partition order */
+/* bins -> partitions (plan: one a sample), records -> partition order: in two passes from a million
+ * 16-byte records and 2^12 partitions on, where the scatter's single stores and atomics cost more
+ * than another read and write of the records (2^12 partitions: 2.2M records 0.080 ms against 0.105,
+ * 5M 0.28 against 0.46; 2^15, 27M 0.64 against 0.67; 2^18, 133M 2.80 against 3.55).  32-byte records,
+ * of which a tile holds half as many, are scattered (2^17 partitions: 0.81 ms against 0.89). */
+constexpr uint64_t SK_SPLIT_RECORDS = 1ull << 20;
+constexpr uint32_t SK_SPLIT_PARTS = 1u << 12;
 template <class KT>
-bruno_status sk_partition(Ctx *c, const std::vector<SkPlan> &plan, uint32_t parts, uint64_t n_rec) {
+bruno_status sk_partition(Ctx *c, const std::vector<SkPlan> &plan, uint32_t parts, uint64_t n_rec, const uint64_t *&sorted) {
   constexpr int NW = SkRec<KT>::NW;
   bruno_status st;
   const uint32_t blocks = (c->sk_bins + SK_PLAN_CHUNK - 1) / SK_PLAN_CHUNK;
@@ -3333,11 +3339,29 @@ bruno_status sk_partition(Ctx *c, const std::vector<SkPlan> &plan, uint32_t part
                                                          (const SkPlan *)c->sk_plan.p, (uint32_t)plan.size(), parts,
                                                          (uint32_t *)c->sk_part.p, (uint32_t *)c->sk_off.p,
                                                          (uint32_t *)c->sk_cur.p);
-  const uint64_t per = 256 * SK_SCATTER_U;
-  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * 8, (n_rec + per - 1) / per));
-  k_sk_scatter<NW><<<grid, 256, 0, c->stream>>>((const uint64_t *)c->sk_recs.p, n_rec, (const uint32_t *)c->sk_part.p,
-                                                (uint32_t *)c->sk_cur.p, (uint64_t *)c->sk_sorted.p, c->dctr);
-  c->launches += 3;
+  uint64_t *recs = (uint64_t *)c->sk_recs.p, *other = (uint64_t *)c->sk_sorted.p;
+  const uint32_t *part = (const uint32_t *)c->sk_part.p, *off = (const uint32_t *)c->sk_off.p;
+  uint32_t *cur = (uint32_t *)c->sk_cur.p, *groups = cur + parts;
+  const int lg = parts > SK_SPLIT_N * (SK_SPLIT_N / 2) ? 10 : 9;   /* two groups' partitions in a tile's counters, if it goes */
+  if (NW == 2 && n_rec >= SK_SPLIT_RECORDS && parts >= SK_SPLIT_PARTS && (parts - 1) >> lg < SK_SPLIT_N) {
+    static const bool attr = cudaFuncSetAttribute(k_sk_split<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)SK_SPLIT_BYTES<NW>) == cudaSuccess;
+    (void)attr;
+    const unsigned grid = (unsigned)((n_rec + SK_SPLIT_TILE<NW> - 1) / SK_SPLIT_TILE<NW>);
+    k_sk_groups<<<SK_SPLIT_N / 256, 256, 0, c->stream>>>(off, parts, lg, groups);
+    k_sk_split<NW><<<grid, SK_SPLIT_TPB, SK_SPLIT_BYTES<NW>, c->stream>>>(recs, n_rec, nullptr, part, lg, 0, groups, other,
+                                                                          n_rec, c->dctr);
+    k_sk_split<NW><<<grid, SK_SPLIT_TPB, SK_SPLIT_BYTES<NW>, c->stream>>>(other, n_rec, off + parts, part, lg, 1, cur, recs,
+                                                                          n_rec, c->dctr);
+    c->launches += 5;
+    sorted = recs;
+  } else {
+    const uint64_t per = 256 * SK_SCATTER_U;
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * 8, (n_rec + per - 1) / per));
+    k_sk_scatter<NW><<<grid, 256, 0, c->stream>>>(recs, n_rec, part, cur, other, c->dctr);
+    c->launches += 3;
+    sorted = other;
+  }
   return cuda_check(c, cudaGetLastError(), "super-k-mer partitions");
 }
 
@@ -3493,7 +3517,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if ((st = ensure(c, c->sk_sorted, std::max<uint64_t>(1, n_rec) * NW * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_part, (size_t)c->sk_bins * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_off, (parts + 1) * 4)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_cur, parts * 4)) != BRUNO_OK) return st;
+    if ((st = ensure(c, c->sk_cur, (parts + SK_SPLIT_N) * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_info, parts * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_over, parts * 8)) != BRUNO_OK) return st;
     if (S > 1 && (st = ensure(c, c->sk_bump, (size_t)S * 8)) != BRUNO_OK) return st;
@@ -3510,10 +3534,11 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     if (S > 1) cudaMemsetAsync(c->sk_bump.p, 0, (size_t)S * 8, c->stream);
     if (S > 1) cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
     cudaEventRecord(c->kev[2], c->stream);
-    if ((st = sk_partition<KT>(c, plan, (uint32_t)parts, n_rec)) != BRUNO_OK) return st;
+    const uint64_t *sorted = nullptr;
+    if ((st = sk_partition<KT>(c, plan, (uint32_t)parts, n_rec, sorted)) != BRUNO_OK) return st;
     cudaEventRecord(c->kev[4], c->stream);
     SkCount a{};
-    a.recs = (const uint64_t *)c->sk_sorted.p;
+    a.recs = sorted;
     a.off = (const uint32_t *)c->sk_off.p;
     a.k = c->cfg.k;
     a.keep_all = !nodes && !(c->one_call && c->cfg.thresholding && !c->cfg.keep_k2);

@@ -564,6 +564,111 @@ __global__ void __launch_bounds__(256) k_sk_scatter(const uint64_t *rec, uint64_
   }
 }
 
+/* The same in two passes, to groups of 2^lg partitions and from these to partitions: a block orders a
+ * tile of records by group (partition) in shared memory and writes a run of its own to each, one
+ * atomic a run.  Bound by its phases: a block of a tile in registers and in shared memory leaves two
+ * to an SM (133M records, 2^18 partitions, both passes: 2.80 ms; tiles of 2048 records, whose runs
+ * are half as long, 3.41; of 8192, one block an SM, 3.10; 1024 threads a tile of 4096 3.14). */
+constexpr int SK_SPLIT_TPB = 512, SK_SPLIT_N = 1024;   /* groups, and partitions of a group, at most */
+template <int NW> constexpr int SK_SPLIT_TILE = 16384 / (2 * NW);
+template <int NW> constexpr size_t SK_SPLIT_BYTES = (size_t)SK_SPLIT_TILE<NW> * (NW * 8 + 2) + SK_SPLIT_N * 8;
+template <int NW>
+__global__ void __launch_bounds__(SK_SPLIT_TPB, 2) k_sk_split(const uint64_t *rec, uint64_t n, const uint32_t *n_dev,
+                                                           const uint32_t *part, int lg, int fine, uint32_t *cur,
+                                                           uint64_t *out, uint64_t room, const DevCounters *ctr) {
+  constexpr int TILE = SK_SPLIT_TILE<NW>, U = TILE / SK_SPLIT_TPB;
+  extern __shared__ __align__(16) uint64_t s_rec[];
+  uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_rec + (size_t)TILE * NW), *s_dst = s_cnt + SK_SPLIT_N;
+  uint16_t *s_d = reinterpret_cast<uint16_t *>(s_dst + SK_SPLIT_N);
+  __shared__ uint32_t s_warp[SK_SPLIT_TPB / 32];
+  if (ctr->err) return;   /* the bins cannot be counted this way: the caller falls back */
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint64_t total = n_dev ? *n_dev : n;   /* (the second pass: no unused places) */
+  const uint64_t i0 = (uint64_t)blockIdx.x * TILE;
+  if (n_dev)   /* unused places behind, as the extraction leaves them: the records may be ordered again */
+    for (uint64_t i = max(total, i0) + tid; i < min(room, i0 + TILE); i += SK_SPLIT_TPB) out[i * NW + NW - 1] = SK_NONE;
+  if (i0 >= total) return;
+  for (int i = tid; i < SK_SPLIT_N; i += SK_SPLIT_TPB) s_cnt[i] = 0;
+  /* the second pass: partitions counted from the first of the tile's first group */
+  uint32_t p0 = 0;
+  if (fine) p0 = __ldg(part + ((rec[i0 * NW + NW - 1] >> SK_BIN_SHIFT) & SK_BIN_MASK)) >> lg << lg;
+  __syncthreads();
+  ulonglong2 r[U][NW / 2];
+  uint32_t d[U], at[U];
+  #pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint64_t i = i0 + u * SK_SPLIT_TPB + tid;
+    d[u] = ~0u;
+    if (i >= total) continue;
+    #pragma unroll
+    for (int q = 0; q < NW / 2; ++q) r[u][q] = __ldcs(reinterpret_cast<const ulonglong2 *>(rec + i * NW) + q);
+  }
+  #pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (i0 + u * SK_SPLIT_TPB + tid >= total || (r[u][NW / 2 - 1].y & 63u) == SK_NONE) continue;
+    const uint32_t P = __ldg(part + ((r[u][NW / 2 - 1].y >> SK_BIN_SHIFT) & SK_BIN_MASK));
+    d[u] = fine ? P - p0 : P >> lg;
+  }
+  #pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (d[u] == ~0u) continue;
+    if (d[u] < SK_SPLIT_N) {
+      at[u] = atomicAdd(&s_cnt[d[u]], 1u);
+    } else {   /* past the second of the tile's groups: by itself */
+      const uint64_t o = atomicAdd(&cur[p0 + d[u]], 1u);
+      #pragma unroll
+      for (int q = 0; q < NW / 2; ++q) reinterpret_cast<ulonglong2 *>(out + o * NW)[q] = r[u][q];
+      d[u] = ~0u;
+    }
+  }
+  __syncthreads();
+  /* where each group's records start in the tile, and where they go */
+  constexpr int PER = SK_SPLIT_N / SK_SPLIT_TPB;
+  uint32_t c[PER], sum = 0;
+  #pragma unroll
+  for (int q = 0; q < PER; ++q) { c[q] = s_cnt[tid * PER + q]; sum += c[q]; }
+  uint32_t x = sum;
+  #pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(~0u, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_warp[tid >> 5] = x;
+  __syncthreads();
+  uint32_t run = x - sum, all = 0;
+  for (int q = 0; q < SK_SPLIT_TPB / 32; ++q) {
+    run += q < (tid >> 5) ? s_warp[q] : 0u;
+    all += s_warp[q];
+  }
+  #pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    s_cnt[tid * PER + q] = run;
+    if (c[q]) s_dst[tid * PER + q] = atomicAdd(&cur[p0 + tid * PER + q], c[q]) - run;   /* (modulo 2^32) */
+    run += c[q];
+  }
+  __syncthreads();
+  #pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (d[u] == ~0u) continue;
+    const uint32_t o = s_cnt[d[u]] + at[u];
+    #pragma unroll
+    for (int q = 0; q < NW / 2; ++q) reinterpret_cast<ulonglong2 *>(s_rec + (size_t)o * NW)[q] = r[u][q];
+    s_d[o] = (uint16_t)d[u];
+  }
+  __syncthreads();
+  for (uint32_t y = tid; y < all; y += SK_SPLIT_TPB) {
+    const uint32_t o = s_dst[s_d[y]] + y;
+    #pragma unroll
+    for (int q = 0; q < NW / 2; ++q)
+      reinterpret_cast<ulonglong2 *>(out + (uint64_t)o * NW)[q] = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)y * NW)[q];
+  }
+}
+/* cursors of the groups of 2^lg partitions */
+__global__ void k_sk_groups(const uint32_t *off, uint32_t nparts, int lg, uint32_t *cur) {
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((uint64_t)g << lg < nparts) cur[g] = off[g << lg];
+}
+
 /* ------------------------------------------------------------ counting
  * One CTA a partition.  Its records come in rounds; equal records (the same place read without
  * an error, from either strand: two thirds of them at 30x) are merged in a small hash of record

@@ -8,6 +8,7 @@ import pytest
 import bruno_gb300 as bg
 from helpers import assert_same, chain_set, sort_nodes, sort_ranked
 from oracle import oracle
+from test_gpu_batch import batch, plain, same_as_plain
 from test_gpu_parity import compare, compare_one_call, gpu_run, one_call_run
 
 pytestmark = pytest.mark.gpu
@@ -130,3 +131,36 @@ def test_edge_filter_from_the_entries(k, with_k1):
         thr = np.array([0, 65536, lo, hi, 0, 65536], dtype=np.uint64)
         ref = oracle.run(data, k=k, thresh=thr, min_update=True, keep_k2=True, keep_filtered=True, edge_filter=True)
         compare_one_call(one_call_run(data, k, True, thr, True, edge_filter=True), ref)
+
+
+@pytest.mark.parametrize("tiny", [0, 40])
+def test_records_to_partitions_in_two_passes(tiny):
+    """an input of more than 2^20 records (at most 17 k-mers each) in 2^12 partitions and more, alone and
+    in a batch behind samples whose partitions hold next to nothing: a tile of records then spans more
+    groups of partitions than it counts"""
+    rng = np.random.default_rng(5)
+    g = rng.integers(0, 4, 1_000_000)
+    at = rng.integers(0, len(g) - 100, 270_000)
+    codes = g[at[:, None] + np.arange(100)]
+    err = rng.random(codes.shape) < 0.01
+    codes = np.where(err, (codes + rng.integers(1, 4, codes.shape)) & 3, codes)
+    text = np.frombuffer(b"ACGT", dtype=np.uint8)[codes]
+    big = b"".join(b"@r\n" + row.tobytes() + b"\n+\n" + b"I" * 100 + b"\n" for row in text)
+    thr = bg.thresholds([2])
+    if not tiny:
+        ref = oracle.run(big, k=31, thresh=thr, min_update=True, threads=16)
+        with bg.Graph(k=31, thresh=thr, min_update=True) as gr:
+            gr.build_and_compact(big)
+            s = gr.sizes()
+            assert s["n_instances"] >= 17 << 20 and s["table_partitions"] >= 1 << 12
+            for n in ("n_instances", "n_k2", "n_nodes", "n_branch", "n_chain_nodes", "n_ranked", "n_chains"):
+                assert s[n] == ref[n], (n, s[n], ref[n])
+            assert_same(sort_nodes(*gr.nodes()), ref["nodes"], "graph nodes")
+            assert chain_set(*gr.chains()) == chain_set(*ref["chains"])
+        return
+    lines = big.split(b"\n")
+    small = [b"\n".join(lines[16 * i:16 * i + 16]) + b"\n" for i in range(tiny)]
+    samples = small[:tiny // 2] + [big] + small[tiny // 2:]
+    got, _ = batch(samples, k=31, thresholding=True, thresh=thr, min_update=True)
+    for i in (0, tiny // 2 - 1, tiny // 2, tiny // 2 + 1, tiny):
+        same_as_plain(got[i], plain(samples[i], k=31, thresholding=True, thresh=thr, min_update=True), f"sample {i}")
