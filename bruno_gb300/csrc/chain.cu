@@ -918,34 +918,63 @@ __global__ void __launch_bounds__(TPB) k_fast_place(const ChainState *cs, ChainS
  * counts, and the longest path in nodes.  cs2 starts as all ones, which no final state is. */
 constexpr uint32_t CS2_UNSET = 0xFFFFFFFFu;
 
-/* the final state of node v from its segment's: on from the segment's ends by its place in it, or to
- * the segment's own end where that is the path's (unset for nodes of cycles) */
-__device__ __forceinline__ ChainState expand_node(const ChainState *cs, uint64_t v, uint2 pl, const SegInfo *seg,
-                                                  const ChainState *rs2) {
+/* What a segment's nodes take their final states from, in the place of its own final state: per side
+ * the state at its path's end (the low 32 bits of P; SEG_END: the segment's own end) and the nodes
+ * from the segment's end to it (D); pad: its nodes, 0 on a cycle. */
+constexpr uint64_t SEG_END = 1ull << 32;
+__global__ void __launch_bounds__(TPB) k_seg_final(ChainState *rs2, const SegInfo *seg, const DevCounters *ctr) {
+  const uint64_t n = ctr->n_seg;
+  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
+    const ChainState g = rs2[x];
+    const SegInfo si = seg[x];
+    ChainState r;
+    r.pad = 0;
+    if (g.inD != CS2_UNSET) {
+      uint64_t P[2];
+      uint32_t D[2];
+      #pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const uint32_t Dg = side_dist(g, s);
+        if (side_terminal(Dg)) {
+          P[s] = SEG_END | (s ? si.R : si.L);
+          D[s] = 0;
+        } else {
+          const uint64_t Pg = side_ptr(g, s);
+          const SegInfo e = seg[(uint32_t)Pg];
+          P[s] = ((uint32_t)s ^ ((Pg & PF_FLIP) ? 1u : 0u)) ? e.R : e.L;
+          D[s] = Dg & DM;
+        }
+      }
+      r.inP = P[0]; r.outP = P[1]; r.inD = D[0]; r.outD = D[1]; r.pad = si.n;
+    } else {
+      r.inP = r.outP = 0; r.inD = r.outD = 0;
+    }
+    rs2[x] = r;
+  }
+}
+
+/* the final state of node v from its segment's (k_seg_final): on from the segment's ends by its place
+ * in it; a path's last node keeps its own terminal side (unset for nodes of cycles) */
+__device__ __forceinline__ ChainState expand_node(const ChainState *cs, uint64_t v, uint2 pl, const ChainState *fin) {
   ChainState st;
   st.inP = st.outP = st.pad = ~0ull;
   st.inD = st.outD = CS2_UNSET;
   if (pl.x == NONE32) return st;
-  const ChainState g = rs2[pl.x];
-  if (g.inD == CS2_UNSET) return st;
-  const SegInfo si = seg[pl.x];
-  const ChainState own = cs[v];
+  const ChainState g = fin[pl.x];
+  if (g.pad == 0) return st;
   const uint32_t rev = pl.y & 1u, off = pl.y >> SEG_OFF;
   uint64_t P[2];
   uint32_t D[2];
   #pragma unroll
   for (int s = 0; s < 2; ++s) {   /* the segment's side s, which the node's side s ^ rev leads to */
-    const uint32_t mine = (uint32_t)s ^ rev, steps = s ? si.n - 1u - off : off, Dg = side_dist(g, s);
-    if (side_terminal(Dg)) {
-      const uint32_t end = s ? si.R : si.L;
-      P[s] = steps ? (uint64_t)(end >> 1) | (((end & 1u) != mine) ? PF_FLIP : 0ull) : side_ptr(own, (int)mine);
-      D[s] = steps ? steps | TM : side_dist(own, (int)mine);
+    const uint32_t mine = (uint32_t)s ^ rev, steps = s ? (uint32_t)g.pad - 1u - off : off;
+    const uint64_t e = side_ptr(g, s);
+    if ((e & SEG_END) && steps == 0) {
+      P[s] = side_ptr(cs[v], (int)mine);
+      D[s] = side_dist(cs[v], (int)mine);
     } else {
-      const uint64_t Pg = side_ptr(g, s);
-      const SegInfo e = seg[(uint32_t)Pg];
-      const uint32_t end = ((uint32_t)s ^ ((Pg & PF_FLIP) ? 1u : 0u)) ? e.R : e.L;
-      P[s] = (uint64_t)(end >> 1) | (((end & 1u) != mine) ? PF_FLIP : 0ull);
-      D[s] = (steps + (Dg & DM)) | TM;
+      P[s] = (uint64_t)((uint32_t)e >> 1) | ((((uint32_t)e & 1u) != mine) ? PF_FLIP : 0ull);
+      D[s] = (steps + side_dist(g, s)) | TM;
     }
   }
   st.inP = rev ? P[1] : P[0]; st.inD = rev ? D[1] : D[0];
@@ -955,9 +984,8 @@ __device__ __forceinline__ ChainState expand_node(const ChainState *cs, uint64_t
 }
 
 /* place != NULL: the nodes' final states are made here from their segments' (written to cs2) */
-__global__ void __launch_bounds__(TPB) k_fast_mark(const ChainState *cs, ChainState *cs2, uint64_t M, const uint2 *place,
-                                                    const SegInfo *seg, const ChainState *rs2,
-                                                    uint8_t *removed, unsigned long long *nmax,
+__global__ void __launch_bounds__(TPB, 8) k_fast_mark(const ChainState *cs, ChainState *cs2, uint64_t M, const uint2 *place,
+                                                    const ChainState *fin, uint8_t *removed, unsigned long long *nmax,
                                                     const uint32_t *csample, unsigned long long *s_tally,
                                                     DevCounters *ctr) {
   unsigned long long ncy = 0, niso = 0, mx = 0, bad = 0;
@@ -968,7 +996,7 @@ __global__ void __launch_bounds__(TPB) k_fast_mark(const ChainState *cs, ChainSt
     if (v < M) {
       ChainState st;
       if (place) {
-        st = expand_node(cs, v, place[v], seg, rs2);
+        st = expand_node(cs, v, place[v], fin);
         cs2[v] = st;
       } else {
         st = cs2[v];
@@ -2955,9 +2983,13 @@ static bruno_status fast_list_rank(Ctx *c, bool &used) {
     k_fast_fill<<<gw, TPB, 0, c->stream>>>(rs, rs2, rnode, E0, E, c->dctr);
   }
   k_fast_rulers<<<blocks(Rb), TPB, 0, c->stream>>>(rs, rs2, rnode, E, c->dctr);
+  if (over_segs) {
+    k_seg_final<<<blocks(N), TPB, 0, c->stream>>>(rs2, seg, c->dctr);
+    c->launches += 1;
+  }
   cudaMemsetAsync(&c->dctr->n_cycle, 0, 16, c->stream);
   cudaMemsetAsync(&c->dctr->n_heads, 0, 8, c->stream);        /* longest path, in nodes */
-  k_fast_mark<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, M, in_seg, seg, rs2, (uint8_t *)c->removed.p, &c->dctr->n_heads,
+  k_fast_mark<<<sms * 8, TPB, 0, c->stream>>>(cs, cs2, M, in_seg, rs2, (uint8_t *)c->removed.p, &c->dctr->n_heads,
                                                c->S > 1 ? (const uint32_t *)c->csample.p : nullptr,
                                                c->S > 1 ? (unsigned long long *)c->s_tally.p : nullptr, c->dctr);
   c->launches += 3;
