@@ -2843,12 +2843,14 @@ bruno_status clean_typed(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t 
       const uint64_t q0 = ranges[b][0], q1 = ranges[b][1];
       cudaMemsetAsync(&c->dctr->cl_found, 0, 8, c->stream);
       const int gq = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (q1 - q0 + TPB - 1) / TPB));
-      if (q1 > q0) k_cl_find<KT><<<gq, TPB, 0, c->stream>>>(q, q0, q1, table, c->geom, k, min_freq, found, c->dctr);
+      if (q1 == q0) continue;
+      k_cl_find<KT><<<gq, TPB, 0, c->stream>>>(q, q0, q1, table, c->geom, k, min_freq, found, c->dctr);
       c->launches += 1;
       if ((st = sync_counters(c)) != BRUNO_OK) return st;
       const uint64_t nf = c->hctr->cl_found;
+      if (nf == 0) continue;   /* no edge left since the last look for edge-less nodes */
       const int gf = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (nf + TPB - 1) / TPB));
-      if (nf) k_cl_erase<KT><<<gf, TPB, 0, c->stream>>>(found, nf, table, c->geom, k);
+      k_cl_erase<KT><<<gf, TPB, 0, c->stream>>>(found, nf, table, c->geom, k);
       c->launches += 1;
       erased += nf;
       if ((st = isolated()) != BRUNO_OK) return st;
@@ -2872,7 +2874,7 @@ bruno_status clean_typed(Ctx *c, uint64_t *rounds, uint64_t *deadends, uint64_t 
     c->n_nodes = c->n_chain + c->n_branch;
     if ((st = extract_typed<KT>(c)) != BRUNO_OK) return st;
     if ((st = run_list_rank(c, c->cfg.min_update)) != BRUNO_OK) return st;
-    if ((st = cycles()) != BRUNO_OK) return st;
+    if (c->n_cycle && (st = cycles()) != BRUNO_OK) return st;   /* (edge-less nodes are out already) */
     (void)iter;
   }
   (void)KWD;
