@@ -568,10 +568,13 @@ __global__ void __launch_bounds__(TPB) k_lr_apply(ChainState *cs, const uint32_t
  * floor(log2(n_max - 1)) + 1 rounds for the longest path (1 if only cycles remain);
  * separate_cycles then removes exactly the cycle nodes.  list_rank and
  * list_rank_min_update reach the same state on such maps.  So the ranks are computed with
- * a ruling set: rulers (every path end plus a hashed 1/32 sample) walk to their
+ * a ruling set: rulers (every path end plus a hashed sample) walk to their
  * neighbouring rulers, the ruler lists are ranked by pointer jumping, and every node adds
  * its offset to its ruler's ranks. */
-constexpr uint32_t RULER_SAMPLE = 32;
+/* One node in 32 is a ruler; one segment in 8, of which there are an eighth as many: the longest walk,
+ * some 13 times the mean, is what a small graph's ranking waits for (1M nodes 0.30 -> 0.23 ms, 10M
+ * 0.93 -> 0.79, 49M 3.39 -> 3.20; one in 4: 0.22, 0.76, 3.25). */
+constexpr uint32_t RULER_SAMPLE = 32, RULER_SAMPLE_SEG = 8;
 /* A link of the ruler lists in one word, so that the lists can be jumped in place (a side reads a
  * neighbour's link while that one moves on: either is a valid link): ruler ordinal, flip, done,
  * distance (the caller checks that the chain nodes are fewer than 2^30). */
@@ -624,7 +627,7 @@ __global__ void __launch_bounds__(TPB) k_fast_check(ChainState *cs, uint64_t M, 
         if (side_terminal(D)) { term_side = true; continue; }
         if (D != 1 || (side_ptr(st, s) & (PF_EXT | PF_BLANK))) ++bad;
       }
-      ruler = term_side || (mix64(v * 0x9e3779b97f4a7c15ull + 0x632be59bd9b4e019ull) % RULER_SAMPLE) == 0;
+      ruler = term_side || (mix64(v * 0x9e3779b97f4a7c15ull + 0x632be59bd9b4e019ull) % (seg ? RULER_SAMPLE_SEG : RULER_SAMPLE)) == 0;
     }
     const unsigned long long o = block_append(ruler, &ctr->lr_remaining);
     if (v < M) cs[v].pad = (ruler ? o : (uint64_t)NONE32) | ((uint64_t)(seg ? seg[v].n : 1u) << 32);
@@ -2891,7 +2894,7 @@ bruno_status run_extract_chains(Ctx *c) { return c->W == 1 ? extract_typed<KW1>(
 
 /* The ruling-set ranking; returns false (and changes nothing) if the chain map is not
  * mutually consistent, in which case the round-synchronous path runs.  Over segments where the
- * chain indices follow the table's minimizer partitions (50M nodes, k = 31: 8.1 ms over the
+ * chain indices follow the table's minimizer partitions (49M nodes, k = 31: 3.2 ms, 8.1 over the
  * nodes); over the nodes themselves where they follow a hash, or with rank_fill = 1.  The host
  * waits once for the first rounds of pointer jumping (and before that for the number of segments
  * where it sizes gigabytes): what the kernels find inconsistent is looked at then, every
