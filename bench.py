@@ -487,47 +487,37 @@ def main():
     e2e_value = inst_step * args.steps * world / (ems / 1e3)
     d2h = nch + 8 * (nc + 1) + 8 * g.words * nc
 
-    # Roofline of the dominant kernel.  Each candidate's algorithmic bytes per launch (one
-    # launch per step each) and its CUDA-event time on the library's stream.  k <= 31:
-    #   k_extract      FASTQ bytes + 16 B read span per read read once, 8 B per record written
-    #   k_split        8 B per record read and written once
-    #   k_count_local  8 B per record read once + 32 B per table slot written once + 4 B per
-    #                  slot it lists for the filter
-    #   k_filter       32 B per slot it reads (the listed ones) + 32 B per graph node written once
+    # Roofline of the dominant kernel.  Each candidate's algorithmic bytes per step and its
+    # CUDA-event time on the library's stream.  k >= 19 is counted by super-k-mer records (16 bytes
+    # at k <= 31, 32 above), of which there is one a read and, on random sequence, one for every
+    # (w + 1) / 2 k-mers (w = k - 14, the 15-mers of a k-mer):
+    #   k_sk_extract  FASTQ bytes + 16 B read span per read read once, the records written
+    #   k_sk_split    the records read and written once (k_sk_scatter at k > 31)
+    #   k_sk_count    the records read once + a table slot (32 B, 64 B at k > 31) per slot written once
     mean = lambda key: statistics.mean(p[key] for p in kms)
     peak, peak_src = measured_peak()
     slots = sizes["table_slots"]
     listed = sizes["filter_slots_read"]
-    if w.k <= 31:
+    if w.k >= 19:
+        rec, slot = (16, 32) if w.k <= 31 else (32, 64)
+        recs = 2 * inst_step / (w.k - 13) + sizes["n_reads_used"]
+        kern = {
+            "k_sk_extract": (n + 16 * sizes["n_reads"] + rec * recs, mean("count_estimate")),
+            "k_sk_split" if w.k <= 31 else "k_sk_scatter": (2 * rec * recs, mean("count_split")),
+            "k_sk_count": (rec * recs + slot * slots, mean("count_insert") - mean("count_split")),
+        }
+    elif w.k <= 31:
+        # k < 19, by k-mer records:
+        #   k_extract      FASTQ bytes + 16 B read span per read read once, 8 B per record written
+        #   k_split        8 B per record read and written once
+        #   k_count_local  8 B per record read once + 32 B per table slot written once + 4 B per
+        #                  slot it lists for the filter
+        #   k_filter       32 B per slot it reads (the listed ones) + 32 B per graph node written once
         kern = {
             "k_extract": (n + 16 * sizes["n_reads"] + 8 * inst_step, mean("count_estimate")),
             "k_split": (16 * inst_step, mean("count_split")),
             "k_count_local": (8 * inst_step + 32 * slots + 4 * listed, mean("count_insert") - mean("count_split")),
             "k_filter": (32 * listed + 32 * sizes["n_nodes"], mean("filter_insert")),
-        }
-    elif sizes["table_partitions"] > 1:
-        # k > 31, partitioned (128-bit keys, 16-byte records, 64-byte slots):
-        #   k_extract      FASTQ bytes + 16 B read span per read read once, 16 B per record written
-        #   k_split_scatter 16 B per record read and written once (into its partition's region)
-        #   k_count_local2 16 B per record read once + 64 B per slot written once + 4 B per listed slot
-        #   k_filter       64 B per slot it reads + 64 B per graph node written once
-        kern = {
-            "k_extract": (n + 16 * sizes["n_reads"] + 16 * inst_step, mean("count_estimate")),
-            "k_split_scatter": (32 * inst_step, mean("count_split")),
-            "k_count_local2": (16 * inst_step + 64 * slots + 4 * listed, mean("count_insert") - mean("count_split")),
-            "k_filter": (64 * listed + 64 * sizes["n_nodes"], mean("filter_insert")),
-        }
-    else:
-        # k > 31 counted straight into the whole table (the fallback for skewed inputs):
-        #   k_hll          FASTQ bytes + 16 B read span per read read once (the distinct estimate)
-        #   k_table_init   64 B per slot written once
-        #   k_count        FASTQ bytes read once + one random 64-byte read-modify-write per instance
-        #   k_filter       64 B per slot it reads + 64 B per graph node written once
-        kern = {
-            "k_hll": (n + 16 * sizes["n_reads"], mean("count_estimate")),
-            "k_table_init": (64 * slots, mean("count_table_init")),
-            "k_count": (n + 64 * inst_step, mean("count_insert")),
-            "k_filter": (64 * listed + 64 * sizes["n_nodes"], mean("filter_insert")),
         }
     kernels = {k: {"alg_bytes_per_launch": b, "launch_ms": t, "achieved": b / (t / 1e3) / 1e9 if t > 0 else None,
                    "frac": b / (t / 1e3) / 1e9 / peak if t > 0 else None} for k, (b, t) in kern.items()}

@@ -3,8 +3,12 @@
  *
  *  k_tile_stats / k_index_lines   FASTQ record split (4-line records, trailing blank lines
  *                                 ignored), one pass over the bytes each.
+ *  superkmer.cuh                  the count from k = 19 on: super-k-mer records, minimizer
+ *                                 partitions, one CTA a partition.
+ *  k_extract_s, k_split,          the same by k-mer records and hash partitions: below, and where
+ *  k_count_local, ...             minimizers crowd.
  *  k_hll                          HyperLogLog estimate of distinct canonical k-mers, used to
- *                                 size the table.
+ *                                 size the table of the direct count.
  *  k_count                        debruijn_kmer_simple_biedge_parser + lex_less +
  *                                 compute_biedge_freqencies: one warp per read packs the
  *                                 read to 2-bit words with ballots, every lane then cuts its

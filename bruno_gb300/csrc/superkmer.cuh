@@ -12,9 +12,14 @@
  *                  bin tallied
  *   k_sk_estimate  a sample of the minimizers' k-mers -> HyperLogLog registers
  *   k_sk_plan_*    bins -> partitions of about equal k-mer counts (neighbouring bins share one)
- *   k_sk_scatter   records -> partition order
+ *   k_sk_scatter   records -> partition order; k_sk_split (many small records) in two passes
  *   k_sk_count     one CTA a partition: equal records merged into one with a weight, their
- *                  k-mers counted in shared memory, the k-mers to keep written to the table
+ *                  k-mers counted in shared memory, the k-mers to keep written to the table, or
+ *                  (one-call builds) the graph's nodes made of them
+ *
+ * 50 Mbp at 30x (1.2G k-mers, k = 31): extraction 4.9, split 2.8, count 12.1 ms, where k-mer records
+ * took 9.9 (extraction), 5.8 (split), 11.6 (count) and 3.3 (filter).  k = 63, 352M k-mers: 1.9, 0.8
+ * and 8.3 against 4.6, 5.3 and 11.1.
  *
  * Included by build.cu only, after its helpers (warp_sum, sm_cas128, CandArgs, ...).
  */
@@ -152,9 +157,10 @@ struct SkExtract {
  * prefix up to the end.  BL (16, 8 or 4) is the block, at most k - MZ_M, so that no window lies
  * inside one block.  Where the minimum changes a run starts; the tile's runs are listed, and each
  * lane builds the records of every 32nd run from the packed words.  Everything stays inside the
- * warp: with one tile a block of 256 threads the block's barriers cost half its time (6.4 ms at
- * 1.2G k-mers).  Output places come in chunks that a warp reserves (one counter cannot take an
- * atomic per tile); a chunk's unused end is marked SK_NONE. */
+ * warp: with one tile a block of 256 threads the block's barriers cost a quarter of its time (6.4 ms
+ * at 1.2G k-mers, now 4.9).  Bound by issue (0.64 of the SMs' peak, 133 instructions a k-mer); four
+ * blocks an SM instead of three spill (5.2 ms).  Output places come in chunks that a warp reserves (one counter
+ * cannot take an atomic per tile); a chunk's unused end is marked SK_NONE. */
 template <class KT, int BL>
 __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
   constexpr int NW = SkRec<KT>::NW, NB = 16 / BL, PAD = sk_pad<NW>;
@@ -529,7 +535,9 @@ __global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_apply(const unsigned lo
 
 /* Records -> partition order: one returning atomic on the partition's cursor and one store a
  * record.  A partition's open line stays in L2 until its records have filled it (2^18 open
- * 128-byte lines are 32 MB of the 129 MB), so the scattered stores leave as whole lines. */
+ * 128-byte lines are 32 MB of the 129 MB), so the scattered stores leave as whole lines.  Bound by the
+ * single stores and atomics (133M records of 16 bytes, 2^18 partitions: 3.55 ms, where reading and
+ * writing them takes 0.63; with places from bin counts and no atomics, to 2^21 open lines, 6.65). */
 constexpr int SK_SCATTER_U = 4;
 template <int NW>
 __global__ void __launch_bounds__(256) k_sk_scatter(const uint64_t *rec, uint64_t n, const uint32_t *part,
@@ -681,6 +689,10 @@ __global__ void k_sk_groups(const uint32_t *off, uint32_t nparts, int lg, uint32
  * keep_all: every k-mer is kept (the raw counts or other thresholds may still be asked for);
  * otherwise a k-mer that the filter's quick rule drops (its total below the (k+1)-mer lower bound;
  * filter_quick) is tallied and left out: at 30x and 0.5% errors three k-mers of four. */
+/* Bound by issue and by the block's phases (0.61 of the SMs' peak, 21 of 32 lanes at work: probe runs
+ * and entries of uneven length; a quarter of the stalls are barriers).  1.2G k-mers, k = 31: 12.1 ms
+ * with 384 threads (256: 12.6, 320: 12.2), items of 3 (4 and 5: 3% more) and two probes before a k-mer
+ * waits (three: 12.4, four: 12.6); making the nodes is 1.45 ms of it, and saves the filter's 3.3. */
 constexpr int SK_COUNT_TPB = 384;
 constexpr int SK_ITEM = 3;
 template <class KT> constexpr int SK_ITEMS = ((sizeof(KT) == 8 ? 17 : 49) + SK_ITEM - 1) / SK_ITEM;   /* items a record at most */

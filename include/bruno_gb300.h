@@ -60,10 +60,11 @@ typedef struct bruno_cfg {
   int32_t keep_filtered;    /* 1: record the filtered (k+2)-mer entries for copy-out */
   int32_t exact_ranking;    /* 1: always run the round-synchronous ranking; 0: use the O(M)
                                ruling-set ranking whenever the chain map is consistent */
-  int32_t direct_count;     /* counting path: 0 = automatic (hash-partitioned records counted
-                               partition by partition in one CTA's shared memory; a skewed input
-                               that overflows a partition falls back to L2-resident partitions at
-                               k <= 31 and to the whole-table count at k > 31), 1 = every
+  int32_t direct_count;     /* counting path: 0 = automatic (from k = 19 on super-k-mer records,
+                               below and for input that crowds few minimizers k-mer records, by
+                               partition in one CTA's shared memory; a skewed input that overflows
+                               a partition of k-mer records falls back to L2-resident partitions
+                               at k <= 31 and to the whole-table count at k > 31), 1 = every
                                instance straight into the whole table, 2 = the L2 partitions
                                always (k <= 31; k > 31 then counts into the whole table). */
   int32_t edge_filter;      /* with thresholding: 1 = the blocked driver's build_index_thresholded
@@ -104,7 +105,7 @@ typedef struct bruno_sizes {
   uint64_t n_ranked;        /* listranked chain nodes */
   uint64_t n_chains;        /* compacted chains */
   uint64_t n_chain_chars;   /* total bases over all compacted chains */
-  uint64_t table_slots;     /* k-mer table slots in use */
+  uint64_t table_slots;     /* k-mer table slots in use (super-k-mer counts leave out what the filter drops) */
   uint64_t collisions;      /* list-ranking sides that got >1 update in one round */
   uint64_t filter_flag_hist[16]; /* k_del[] histogram (debruijn_graph_map.hpp:1568) */
   uint64_t launches;        /* kernels launched by the last build */
@@ -113,7 +114,8 @@ typedef struct bruno_sizes {
                                k+2 bounds can trim an edge on one side only) and the compaction
                                grouped the nodes by representative */
   uint64_t filter_slots_read; /* table slots local_insert_by_freqencies read: every slot, or only those
-                                 the count listed (thresholded builds) */
+                                 the count listed; where the count makes the nodes itself (one-call
+                                 builds from k = 19 on) the k-mers it made them from */
 } bruno_sizes;
 
 typedef struct bruno_ctx bruno_ctx;
@@ -341,10 +343,11 @@ bruno_status bruno_host_free(void *p);
 /* Device times of the last build, milliseconds, from CUDA events on the context's stream:
  * ms[0..5] = phases parse, count_k2mers, filter_insert, chainmap, list_rank, compress;
  * ms[6..9] = counting sub-steps: distinct-count estimate (with the record extraction on
- * the partitioned path), whole-table initialisation (direct path only), the counting
+ * the partitioned paths), whole-table initialisation (direct path only), the counting
  * itself (split + per-partition counts, the L2 partition inserts, or k_count), and the
- * record split alone (shared-memory partition path only); ms[10] = the host-to-device
- * copies of FASTQ bytes given in host memory.  Writes min(n, 11) values. */
+ * record split alone (shared-memory partition paths only); ms[10] = the host-to-device
+ * copies of FASTQ bytes given in host memory.  Writes min(n, 11) values.  The times are
+ * worked out here, from events that the build left: the call waits for the build's last. */
 bruno_status bruno_phase_ms(bruno_ctx *ctx, double *ms, size_t n);
 
 /* ---------------------------------------------------------------------------------------
