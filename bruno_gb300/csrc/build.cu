@@ -3280,7 +3280,7 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
   for (uint32_t q = 0; q < S; ++q) {
     total += bytes[q];
     int b = 11, e = 0;
-    while (b < 21 && (bytes[q] >> 10 >> b)) ++b;
+    while (b < (bytes[q] >> 32 ? 22 : 21) && (bytes[q] >> 10 >> b)) ++b;
     while (e < 13 && (bytes[q] >> sample_bits >> (e + 1))) ++e;
     c->sk_bits[q] = b;
     c->sk_q[q] = e;
@@ -3451,6 +3451,7 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
  * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): a
  * bin too large for one CTA, more records than room, or partitions that overflow at every size
  * tried.  max_split: the partition plan's split bits. */
+constexpr double SK_MAX_KMERS = 3500.0;   /* k-mers of a partition, on average, that fit the largest block twice over */
 template <class KT>
 bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
   constexpr int NW = SkRec<KT>::NW, SU = Slot<KT>::U64;
@@ -3492,15 +3493,21 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
     uint32_t bin0 = 0;
     for (uint32_t q = 0; q < S; ++q) {
       const uint64_t slots = slots_for(c, distinct[q]), n_inst = S > 1 ? c->h_inst[q] : inst;
+      /* the fewest partitions of the configured slots, but four bins to a partition at least: a bin
+       * holds a few minimizers' k-mers, and partitions of one bin are so uneven that most are counted
+       * twice (k = 63, 3.5G k-mers, 2^21 partitions of 2^21 bins: 211 ms of counting; 2^20 of 2^22: 84).
+       * A batch, whose bins are shared out among its samples, keeps the plan (256 samples, 2.8G k-mers:
+       * 59 ms; with half the partitions 98) */
       const bruno_table_plan::Plan pl = bruno_table_plan::partitions(slots, part_slots(c) * 4 / SU, max_split);
-      if (!pl.fits) return BRUNO_OK;
-      const uint64_t n = 1ull << pl.pbits;
+      const int pbits = S > 1 ? pl.pbits : std::min(pl.pbits, std::max(8, c->sk_bits[q] - 2));
+      const uint64_t n = 1ull << pbits;
+      if (!(pl.fits || pbits < pl.pbits) || distinct[q] > SK_MAX_KMERS * (double)n) return BRUNO_OK;
       caps[q] = slots + 2 * n;   /* a partition's slots are rounded up by two */
-      sg[q].g = TableGeom{caps[q], 0, pl.pbits, base, nullptr, nullptr, bin0, 32 - c->sk_bits[q], c->cfg.k};
+      sg[q].g = TableGeom{caps[q], 0, pbits, base, nullptr, nullptr, bin0, 32 - c->sk_bits[q], c->cfg.k};
       sg[q].pbase = parts;
       sg[q].rec2_base = sg[q].cap2 = 0;
       plan[q] = SkPlan{before, std::max<uint64_t>(1, (n_inst + n - 1) / n), bin0, (uint32_t)parts, (uint32_t)n, 0u};
-      region[q] = pl.region;
+      region[q] = (slots + n - 1) >> pbits;
       before += n_inst;
       base += caps[q];
       parts += n;
