@@ -3213,7 +3213,7 @@ bool sk_takes(const Ctx *c) {
 }
 
 template <class KT, int BL>
-void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                unsigned long long *s_inst, unsigned long long *s_used) {
   constexpr size_t smem = sizeof(SkWarp<SkRec<KT>::NW>) * (SK_TPB / 32);
   static const int occ = [] {
@@ -3222,15 +3222,16 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sk_extract<KT, BL>, SK_TPB, smem) == cudaSuccess && o > 0
                ? o : 4;
   }();
-  const uint64_t most = items ? n_items : (nreads + 31) / 32;   /* a few reads a warp at least */
+  const uint64_t most = (r1 - r0 + 31) / 32;   /* a few reads a warp at least */
   const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * occ, most));
   SkExtract a{};
   a.rstart = (const uint64_t *)c->rstart.p;
   a.rend = (const uint64_t *)c->rend.p;
   a.r0 = r0;
   a.r1 = r1;
-  a.items = items;
-  a.n_items = n_items;
+  a.first = first;
+  a.s0 = s0;
+  a.n_first = n_first;
   a.k = c->cfg.k;
   a.skew_len = c->cfg.edge_filter ? (uint32_t)c->cfg.k + 1 : ~0u;
   a.chunk = c->sk_chunk;
@@ -3247,20 +3248,20 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_
   c->launches += 1;
 }
 template <class KT>
-void sk_launch_k(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+void sk_launch_k(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                  unsigned long long *s_inst, unsigned long long *s_used) {
   const int w1 = c->cfg.k - MZ_M;   /* the window blocks: the largest that no window fits inside */
-  if (w1 >= 16) sk_launch<KT, 16>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
-  else if (w1 >= 8) sk_launch<KT, 8>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
-  else sk_launch<KT, 4>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
+  if (w1 >= 16) sk_launch<KT, 16>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  else if (w1 >= 8) sk_launch<KT, 8>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  else sk_launch<KT, 4>(c, r0, r1, first, s0, n_first, s_inst, s_used);
 }
-void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const XItem *items, uint64_t n_items, uint64_t nreads,
+void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                 unsigned long long *s_inst, unsigned long long *s_used) {
-  if (nreads == 0) return;
-  if (c->W == 1) sk_launch_k<KW1>(c, r0, r1, items, n_items, nreads, s_inst, s_used);
-  else sk_launch<KW2, 16>(c, r0, r1, items, n_items, nreads, s_inst, s_used);   /* k > 31: windows of 18 and more */
+  if (r1 == r0) return;
+  if (c->W == 1) sk_launch_k<KW1>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  else sk_launch<KW2, 16>(c, r0, r1, first, s0, n_first, s_inst, s_used);   /* k > 31: windows of 18 and more */
 }
-void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, r1 - r0, nullptr, nullptr); }
+void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, 0, nullptr, nullptr); }
 
 /* Room for the records of samples of the given FASTQ bytes, their bins and their estimates.  A
  * read's quality line is as long as its sequence, so k-mer positions are at most half the bytes;
@@ -4066,22 +4067,13 @@ bruno_status extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector
 }
 }  // namespace
 
-/* the same by super-k-mers: items of one sample's reads, several a warp so that the warps even out */
+/* the same by super-k-mers: an even share of the reads a warp, which looks their samples up itself (a list
+ * of items would be a copy to the device that waits behind the groups' own: 23 groups of 256 MB then took
+ * 56 ms instead of 35, the copies alone 34) */
 namespace {
 bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f) {
-  bruno_status st;
-  const uint64_t nr = f.back() - f.front(), warps = (uint64_t)num_sms() * 32;
-  const uint64_t per = std::max<uint64_t>(32, std::min<uint64_t>(512, nr / (8 * warps)));
-  std::vector<XItem> items;
-  for (uint32_t q = q0; q < q1; ++q)
-    for (uint64_t a = f[q - q0]; a < f[q - q0 + 1]; a += per)
-      items.push_back(XItem{a, std::min<uint64_t>(f[q - q0 + 1], a + per), q, 0u});
-  if (items.empty()) return BRUNO_OK;
-  if ((st = ensure(c, c->xitems, items.size() * sizeof(XItem))) != BRUNO_OK) return st;
-  if ((st = cuda_check(c, cudaMemcpyAsync(c->xitems.p, items.data(), items.size() * sizeof(XItem), cudaMemcpyHostToDevice,
-                                          c->stream), "extraction items")) != BRUNO_OK)
-    return st;
-  sk_extract(c, 0, 0, (const XItem *)c->xitems.p, items.size(), nr, (unsigned long long *)c->s_inst.p,
+  const uint32_t n = q1 - q0;   /* their first reads are on the device already (first_reads) */
+  sk_extract(c, f.front(), f.back(), (const uint64_t *)c->fr_tmp.p + n, q0, n, (unsigned long long *)c->s_inst.p,
              (unsigned long long *)c->s_used.p);
   return cuda_check(c, cudaGetLastError(), "k_sk_extract");
 }

@@ -133,9 +133,9 @@ __global__ void __launch_bounds__(128) k_sk_estimate(const uint64_t *recs, const
 
 struct SkExtract {
   const uint64_t *rstart, *rend;
-  uint64_t r0, r1;                  /* reads, when there are no items */
-  const XItem *items;
-  uint64_t n_items;
+  uint64_t r0, r1;                  /* reads */
+  const uint64_t *first;            /* a batch: the first read (from r0 on) of samples s0, s0 + 1, ... */
+  uint32_t s0, n_first;
   int k;
   uint32_t skew_len;                /* a read of this length: the input is counted another way (~0: none) */
   uint32_t chunk;                   /* output records a warp reserves at once */
@@ -175,27 +175,24 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
   if (lane == 0) S.marks[SK_WORDS] = 0;
   if (lane < PAD) S.bases[lane] = 0;   /* (what a record cuts from there is masked off) */
   uint32_t cpos = 0, cend = 0;   /* the warp's chunk of the output (fewer than 2^32 records) */
-  /* items of one sample each, or (one sample) an even share of the reads */
-  uint32_t it, it1;
+  /* an even share of the reads, sample by sample */
+  uint64_t pos, end;
   {
-    const uint32_t warp = blockIdx.x * (SK_TPB / 32) + (threadIdx.x >> 5), warps = gridDim.x * (SK_TPB / 32);
-    const uint64_t n = a.items ? a.n_items : warps;
-    it = (uint32_t)(warp * n / warps);
-    it1 = (uint32_t)((warp + 1) * n / warps);
+    const uint64_t warp = blockIdx.x * (SK_TPB / 32) + (threadIdx.x >> 5), warps = gridDim.x * (SK_TPB / 32);
+    pos = (a.r1 - a.r0) * warp / warps;
+    end = (a.r1 - a.r0) * (warp + 1) / warps;
   }
-  for (; it < it1; ++it) {
-    uint64_t ra;
-    uint32_t n_reads;   /* reads of the item not yet taken */
+  while (pos < end) {
+    uint64_t ra = a.r0 + pos;
+    uint32_t n_reads = (uint32_t)(end - pos);   /* reads of the sample's share not yet taken */
     unsigned smp = 0;
-    if (a.items) {
-      ra = a.items[it].a;
-      n_reads = (uint32_t)(a.items[it].b - ra);
-      smp = a.items[it].s;
-    } else {
-      const uint32_t warps = gridDim.x * (SK_TPB / 32);
-      ra = a.r0 + (a.r1 - a.r0) * it / warps;
-      n_reads = (uint32_t)(a.r0 + (a.r1 - a.r0) * (it + 1) / warps - ra);
+    if (a.first) {
+      uint32_t lo = 0, hi = a.n_first;
+      while (hi - lo > 1) { const uint32_t m = (lo + hi) >> 1; if (__ldg(a.first + m) <= pos) lo = m; else hi = m; }
+      smp = a.s0 + lo;
+      if (lo + 1 < a.n_first) n_reads = (uint32_t)(min(end, __ldg(a.first + lo + 1)) - pos);
     }
+    pos += n_reads;
     unsigned inst = 0, used = 0;
     uint64_t sp = 0;           /* the read ra + lane */
     uint32_t len = 0;
