@@ -504,7 +504,8 @@ def main():
         kern = {
             "k_sk_extract": (n + 16 * sizes["n_reads"] + rec * recs, mean("count_estimate")),
             "k_sk_split" if w.k <= 31 else "k_sk_scatter": (2 * rec * recs, mean("count_split")),
-            "k_sk_count": (rec * recs + slot * slots, mean("count_insert") - mean("count_split")),
+            "k_sk_count<KW1>" if w.k <= 31 else "k_sk_count<KW2>": (rec * recs + slot * slots,
+                                                                     mean("count_insert") - mean("count_split")),
         }
     elif w.k <= 31:
         # k < 19, by k-mer records:
