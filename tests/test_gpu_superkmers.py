@@ -164,3 +164,21 @@ def test_records_to_partitions_in_two_passes(tiny):
     got, _ = batch(samples, k=31, thresholding=True, thresh=thr, min_update=True)
     for i in (0, tiny // 2 - 1, tiny // 2, tiny // 2 + 1, tiny):
         same_as_plain(got[i], plain(samples[i], k=31, thresholding=True, thresh=thr, min_update=True), f"sample {i}")
+
+
+@pytest.mark.parametrize("k", [31, 63])
+def test_partitions_of_four_bins_at_least(k):
+    """partitions so small (256 and 128 slots) that the plan asks for more of them than a quarter of the
+    bins: they get larger instead"""
+    rng = np.random.default_rng(k)
+    g = "".join("ACGT"[c] for c in rng.integers(0, 4, 200_000))
+    reads = []
+    for at in rng.integers(0, len(g) - 100, 30_000):
+        s = list(g[at:at + 100])
+        s[int(rng.integers(0, 100))] = "ACGT"[int(rng.integers(0, 4))]
+        reads.append("".join(s))
+    data = fastq(reads)
+    thr = bg.thresholds([2])
+    ref = oracle.run(data, k=k, thresh=thr, min_update=True, threads=16, keep_k2=True, keep_filtered=True)
+    compare_one_call(one_call_run(data, k, True, thr, True, part_slots=256), ref)
+    compare(gpu_run(data, k, True, thr, True, part_slots=256), ref)
