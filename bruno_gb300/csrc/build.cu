@@ -2653,7 +2653,7 @@ bruno_status extract_begin(Ctx *c, uint64_t upper, int max_blocks);
 void extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 int wx_blocks(uint64_t nr);
 bool sk_takes(const Ctx *c);
-bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes);
+bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t records = 0);
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f);
 }  // namespace
@@ -2679,8 +2679,9 @@ bruno_status run_index_reads(Ctx *c) {
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
   if (c->pre_extracted) {
-    /* every record holds its sequence and an equally long quality line, so the k-mer
-     * positions of all reads are at most half the bytes */
+    /* a record holds its sequence and, as a rule, an equally long quality line: k-mer positions are
+     * at most half the bytes (shorter quality lines are accepted too: the records may then need more
+     * room than this gives, which both extractions notice) */
     int blocks = 0;   /* one launch a segment, bounded as extract_reads bounds it (8 bytes a read at least) */
     for (auto &sg : c->segs) blocks += wx_blocks(sg.n / 8 + 1);
     if ((st = c->sk_on ? sk_begin(c, {total_bytes}) : extract_begin(c, total_bytes / 2 + 1, std::max(1, blocks))) != BRUNO_OK)
@@ -3264,12 +3265,12 @@ void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, 0, nullptr, nullptr); }
 
 /* Room for the records of samples of the given FASTQ bytes, their bins and their estimates.  A
- * read's quality line is as long as its sequence, so k-mer positions are at most half the bytes;
+ * read's quality line is mostly as long as its sequence, so k-mer positions are about half the bytes;
  * runs start at 2 / (w + 1) of them (w m-mers a window) and at every read, and get a quarter
- * more; input that needs more (it would have to be unlike any sequence) is counted by k-mer
- * records.  About 512 k-mers a bin: a partition, some thousands of k-mers, is then made up of
- * enough bins to even out. */
-bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
+ * more.  Input that needs more (short quality lines, repeats whose minimizers change often) is
+ * extracted once more, with room for the `records` places that the first time counted.  About 512
+ * k-mers a bin: a partition, some thousands of k-mers, is then made up of enough bins to even out. */
+bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t records) {
   bruno_status st;
   const uint32_t S = (uint32_t)bytes.size();
   const int k = c->cfg.k, w = k - MZ_M + 1;
@@ -3301,6 +3302,7 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes) {
   c->sk_chunk = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, (uint64_t)(recs / (8.0 * warps))));
   /* one extraction launch a segment, each with chunks of its own */
   c->sk_cap = (uint64_t)recs + total / (2 * k + 9) + 4096 + warps * c->sk_chunk * std::max<size_t>(1, c->segs.size());
+  if (records) c->sk_cap = records + warps * c->sk_chunk;
   const size_t rb = c->W == 1 ? 16 : 32;
   if ((st = ensure(c, c->sk_recs, c->sk_cap * rb)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->sk_hist, bins * 8)) != BRUNO_OK) return st;
@@ -3450,11 +3452,12 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
 
 /* The count by super-k-mers of the extracted records (one sample, or a batch's), kev[0] recorded
  * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): a
- * bin too large for one CTA, more records than room, or partitions that overflow at every size
- * tried.  max_split: the partition plan's split bits. */
+ * bin too large for one CTA, 2^32 records, or partitions that overflow at every size tried.
+ * max_split: the partition plan's split bits.  again(records): the extraction once more, with room
+ * for that many records (133M records: 5 ms, where the k-mer records take 48). */
 constexpr double SK_MAX_KMERS = 3500.0;   /* k-mers of a partition, on average, that fit the largest block twice over */
-template <class KT>
-bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
+template <class KT, class Again>
+bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bool second = false) {
   constexpr int NW = SkRec<KT>::NW, SU = Slot<KT>::U64;
   bruno_status st;
   used = false;
@@ -3477,6 +3480,10 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
   }
   if ((st = sync_counters(c)) != BRUNO_OK) return st;
   const uint64_t n_rec = c->hctr->n_sk, inst = c->hctr->n_instances;
+  if (n_rec > c->sk_cap && !second && !(n_rec >> 32) && !(c->hctr->err & DERR_SKEW)) {
+    if ((st = again(n_rec)) != BRUNO_OK) return st;
+    return count_superkmers<KT>(c, max_split, again, used, true);
+  }
   if (c->hctr->err || n_rec > c->sk_cap || inst >> 32 || n_rec >> 32) return BRUNO_OK;
   c->n_instances = inst;
   c->n_reads_used = c->hctr->n_reads_used;
@@ -3652,17 +3659,22 @@ bruno_status count_superkmers(Ctx *c, int max_split, bool &used) {
 /* one sample: extraction, unless the read index did it as the pieces landed, and the count */
 template <class KT>
 bruno_status count_one_superkmers(Ctx *c, bool &used) {
-  if (!c->pre_extracted) {
-    uint64_t bytes = 0;
-    for (auto &sg : c->segs) bytes += sg.n;
+  uint64_t bytes = 0;
+  for (auto &sg : c->segs) bytes += sg.n;
+  auto extract = [&](uint64_t records) -> bruno_status {
     cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
-    bruno_status st = sk_begin(c, {bytes});
+    bruno_status st = sk_begin(c, {bytes}, records);
     if (st != BRUNO_OK) return st;
-    cudaEventRecord(c->kev[0], c->stream);
+    if (!records) cudaEventRecord(c->kev[0], c->stream);
     sk_extract_reads(c, 0, c->n_reads);
+    return BRUNO_OK;
+  };
+  if (!c->pre_extracted) {
+    bruno_status st = extract(0);
+    if (st != BRUNO_OK) return st;
   }
   c->pre_extracted = false;   /* what was extracted serves this path alone */
-  return count_superkmers<KT>(c, MAX_SPLIT_BITS2, used);
+  return count_superkmers<KT>(c, MAX_SPLIT_BITS2, extract, used);
 }
 
 /* The partitioned count for k > 31: exact k-mer positions size 256 buckets of 16-byte records,
@@ -4115,10 +4127,18 @@ bruno_status run_count_samples(Ctx *c) {
       if ((st = sk_extract_samples(c, 0, S, c->samp_r0)) != BRUNO_OK) return st;
     }
     bool used = false;
-    if ((st = count_superkmers<KW1>(c, MAX_SPLIT_BITS, used)) != BRUNO_OK || used) return st;
-    cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
-    cudaMemsetAsync(c->s_inst.p, 0, (size_t)S * 8, c->stream);
-    cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
+    auto clear = [&] {
+      cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
+      cudaMemsetAsync(c->s_inst.p, 0, (size_t)S * 8, c->stream);
+      cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
+    };
+    auto again = [&](uint64_t records) -> bruno_status {
+      clear();
+      const bruno_status s2 = sk_begin(c, bytes, records);
+      return s2 != BRUNO_OK ? s2 : sk_extract_samples(c, 0, S, c->samp_r0);
+    };
+    if ((st = count_superkmers<KW1>(c, MAX_SPLIT_BITS, again, used)) != BRUNO_OK || used) return st;
+    clear();
   }
   c->sk_on = false;
   c->sk_gaps.clear();

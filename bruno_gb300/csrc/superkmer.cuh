@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(128) k_sk_estimate(const uint64_t *recs, const
                                                      const SkSample *samples, uint32_t S, unsigned int *hll,
                                                      const DevCounters *ctr) {
   constexpr int NW = SkRec<KT>::NW;
+  if (ctr->err) return;   /* records past their room: the caller makes room and comes again */
   const uint64_t n_list = min((unsigned long long)cap, ctr->n_sk_est);
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n_list; x += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t *rec = recs + (uint64_t)list[x] * NW;
@@ -409,7 +410,7 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
             atomicOr(&a.ctr->err, (unsigned long long)DERR_TABLE_FULL);
           }
           atomicAdd(&a.hist[bin], ((unsigned long long)n << 32) | 1ull);
-          if ((mix & X.smask) == 0) {
+          if ((mix & X.smask) == 0 && o < a.cap) {   /* (a record that was not stored is not read either) */
             const unsigned long long e = atomicAdd(&a.ctr->n_sk_est, 1ull);
             if (e < a.est_cap) a.est[e] = o;
           }

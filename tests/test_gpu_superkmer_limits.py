@@ -1,0 +1,77 @@
+"""Super-k-mer counting where an input outgrows what its plan foresaw, against the oracle and against
+the plain build: more records than their room."""
+import numpy as np
+import pytest
+
+import bruno_gb300 as bg
+from helpers import assert_same, chain_set, sort_nodes, sort_ranked
+from oracle import oracle
+from test_gpu_batch import batch, plain, same_as_plain
+
+pytestmark = pytest.mark.gpu
+
+ACGT = np.frombuffer(b"ACGT", dtype=np.uint8)
+SIZES = ("n_reads", "n_reads_used", "n_instances", "n_k2", "n_nodes", "n_branch", "n_chain_nodes", "iterations",
+         "n_cycle_nodes", "n_isolated", "n_ranked", "n_chains", "n_chain_chars")
+
+
+def rand_reads(rng, genome, n, length, err=0.0):
+    """n x length base codes of reads of either strand"""
+    at = rng.integers(0, len(genome) - length + 1, n)
+    c = genome[at[:, None] + np.arange(length)]
+    if err:
+        c = np.where(rng.random(c.shape) < err, (c + rng.integers(1, 4, c.shape)) & 3, c)
+    flip = rng.random(n) < 0.5
+    c[flip] = 3 - c[flip][:, ::-1]
+    return c
+
+
+def fastq(codes, qual=None):
+    """records of one read length, with `qual` quality characters (the read's length by default)"""
+    n, length = codes.shape
+    q = length if qual is None else qual
+    out = np.empty((n, 7 + length + q), dtype=np.uint8)
+    out[:, :3] = np.frombuffer(b"@r\n", dtype=np.uint8)
+    out[:, 3:3 + length] = ACGT[codes]
+    out[:, 3 + length:6 + length] = np.frombuffer(b"\n+\n", dtype=np.uint8)
+    out[:, 6 + length:6 + length + q] = ord("I")
+    out[:, 6 + length + q] = 10
+    return out.tobytes()
+
+
+def check(data, k, thr, thresholding=True, **cfg):
+    """a one-call build against the oracle; returns its sizes"""
+    ref = oracle.run(data, k=k, thresholding=thresholding, thresh=thr, min_update=True, threads=16,
+                     edge_filter=cfg.get("edge_filter", False))
+    with bg.Graph(k=k, thresholding=thresholding, thresh=thr, min_update=True, **cfg) as g:
+        g.build_and_compact(data)
+        s = g.sizes()
+        for n in SIZES:
+            if n in ref:
+                assert s[n] == ref[n], (n, s[n], ref[n])
+        assert_same(sort_nodes(*g.nodes()), ref["nodes"], "graph nodes")
+        assert_same(sort_ranked(*g.ranked()), ref["ranked"], "listranked chain nodes")
+        assert chain_set(*g.chains()) == chain_set(*ref["chains"])
+        return s
+
+
+# ------------------------------------------------------------------ more records than their room
+@pytest.mark.parametrize("k,chunk", [(21, 0), (21, 16 << 20), (33, 0)])
+def test_quality_lines_of_one_character(k, chunk):
+    """a quality line need not be as long as its sequence: nearly every byte is then a k-mer position,
+    and the records outgrow the room that half the bytes would need (24000 reads of 1 kb, k = 21: 5.8M
+    records, places for 4.7M; k = 33: 2.3M, places for 2.1M); at once and in pieces of a host copy"""
+    rng = np.random.default_rng(k)
+    data = fastq(rand_reads(rng, rng.integers(0, 4, 300_000), 24_000, 1000, 0.002), qual=1)
+    check(data, k, bg.thresholds([2]), h2d_chunk=chunk)
+
+
+@pytest.mark.parametrize("chunk", [0, 16 << 20])
+def test_quality_lines_of_one_character_in_a_batch(chunk):
+    rng = np.random.default_rng(chunk + 1)
+    samples = [fastq(rand_reads(rng, rng.integers(0, 4, 150_000), n, 1000, 0.002), qual=1)
+               for n in (9_000, 300, 9_000, 9_000)]
+    cfg = dict(k=21, thresholding=True, thresh=bg.thresholds([2]), min_update=True)
+    got, _ = batch(samples, h2d_chunk=chunk, **cfg)
+    for i, data in enumerate(samples):
+        same_as_plain(got[i], plain(data, **cfg), f"sample {i}")
