@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "seg_state.h"
 
 namespace bg {
 
@@ -653,7 +654,7 @@ __device__ __forceinline__ bool answers(const ChainState &t, int facing, uint32_
  * segment.
  *
  * Bound: 32 bytes read and 8 written a node, and about 6 rounds over 16 KB of shared memory. */
-constexpr int SEG_STOP = 12;   /* a state word: next state, steps to it from this bit on (0: it stops) */
+constexpr int SEG_STOP = bruno_seg::STOP;   /* a state word: next state, steps to it from this bit on (0: it stops) */
 __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_t M, uint2 *place, SegInfo *seg,
                                                    DevCounters *ctr) {
   __shared__ uint32_t nx[2 * SEG_N];
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_
   }
   if (tid == 0) s_n = 0;
   __syncthreads();
-  constexpr uint32_t IDX = (1u << SEG_STOP) - 1;
+  constexpr uint32_t IDX = bruno_seg::IDX;
   static_assert(2 * SEG_N == 1 << SEG_STOP, "a state fits its bits");
   for (int x = tid; x < 2 * n; x += TPB)   /* arriving at state y, the other side of its node points back */
     if (nx[x] >> SEG_STOP && nx[(nx[x] & IDX) ^ 1u] != ((uint32_t)(x ^ 1) | (1u << SEG_STOP))) ++bad;
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_
     for (int x = tid; x < 2 * n; x += TPB) {
       const uint32_t w = nx[x], t = nx[w & IDX];
       if ((w >> SEG_STOP) && (t >> SEG_STOP)) {
-        nx[x] = (t & IDX) | (((w >> SEG_STOP) + (t >> SEG_STOP)) << SEG_STOP);
+        nx[x] = bruno_seg::join(w, t);
         moved = true;
       }
     }

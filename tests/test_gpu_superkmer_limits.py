@@ -1,5 +1,5 @@
-"""Super-k-mer counting where an input outgrows what its plan foresaw, against the oracle and against
-the plain build: more records than their room."""
+"""Super-k-mer builds where an input outgrows what its plan foresaw, against the oracle and against the
+plain build: more records than their room, cycles within one block of chain nodes."""
 import numpy as np
 import pytest
 
@@ -75,3 +75,21 @@ def test_quality_lines_of_one_character_in_a_batch(chunk):
     got, _ = batch(samples, h2d_chunk=chunk, **cfg)
     for i, data in enumerate(samples):
         same_as_plain(got[i], plain(data, **cfg), f"sample {i}")
+
+
+# ------------------------------------------------------------------ segments of chain nodes
+@pytest.mark.parametrize("k", [31, 63])
+def test_circular_genomes_within_one_block(k):
+    """cycles whose nodes all lie in one block of the segment search (2048 nodes), around its edge, and
+    beside a linear genome"""
+    rng = np.random.default_rng(k)
+    for n in (k + 3, 150, 256, 777, 1024, 2047, 2048, 2049):
+        g = rng.integers(0, 4, n)
+        at = np.concatenate([np.arange(0, n, 3), rng.integers(0, n, 100)])
+        reads = g[(at[:, None] + np.arange(100)) % n]
+        reads[::2] = 3 - reads[::2][:, ::-1]
+        data = fastq(reads)
+        s = check(data, k, bg.thresholds([1]))
+        assert s["n_cycle_nodes"] == n and s["n_ranked"] == 0
+        line = rng.integers(0, 4, 1500)
+        check(data + fastq(rand_reads(rng, line, 300, 100)), k, bg.thresholds([1]))
