@@ -655,6 +655,7 @@ __device__ __forceinline__ bool answers(const ChainState &t, int facing, uint32_
  *
  * Bound: 32 bytes read and 8 written a node, and about 6 rounds over 16 KB of shared memory. */
 constexpr int SEG_STOP = bruno_seg::STOP;   /* a state word: next state, steps to it from this bit on (0: it stops) */
+constexpr uint16_t SEG_CLOSED = 0xFFFFu;    /* a state that opened no segment (2^11 segments a block at most) */
 __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_t M, uint2 *place, SegInfo *seg,
                                                    DevCounters *ctr) {
   __shared__ uint32_t nx[2 * SEG_N];
@@ -678,6 +679,7 @@ __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_
       nx[x] = w;
     }
   }
+  for (int x = tid; x < 2 * n; x += TPB) ord[x] = SEG_CLOSED;
   if (tid == 0) s_n = 0;
   __syncthreads();
   constexpr uint32_t IDX = bruno_seg::IDX;
@@ -709,7 +711,8 @@ __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_
     uint2 pl = make_uint2(NONE32, 0u);
     if (!(nx[e0] >> SEG_STOP) && !(nx[e1] >> SEG_STOP)) {
       const uint32_t l = min(e0, e1), rev = e0 > e1, off = (rev ? w1 : w0) >> SEG_STOP;
-      pl = make_uint2(s_base + ord[l], (off << SEG_OFF) | rev);
+      /* (pointers that disagree can lead to a stop whose node opened no segment there) */
+      if (ord[l] != SEG_CLOSED) pl = make_uint2(s_base + ord[l], (off << SEG_OFF) | rev);
       if ((l >> 1) == (uint32_t)i)
         seg[pl.x] = SegInfo{(uint32_t)(2 * base) + l, (uint32_t)(2 * base) + max(e0, e1),
                             (w0 >> SEG_STOP) + (w1 >> SEG_STOP) + 1u, 0u};

@@ -1,10 +1,10 @@
 """Super-k-mer builds where an input outgrows what its plan foresaw, against the oracle and against the
-plain build: more records than their room, cycles within one block of chain nodes."""
+plain build: more records than their room, cycles within one block of chain nodes, pointers that disagree."""
 import numpy as np
 import pytest
 
 import bruno_gb300 as bg
-from helpers import assert_same, chain_set, sort_nodes, sort_ranked
+from helpers import assert_same, chain_set, compress_ranked, sort_nodes, sort_ranked
 from oracle import oracle
 from test_gpu_batch import batch, plain, same_as_plain
 
@@ -93,3 +93,20 @@ def test_circular_genomes_within_one_block(k):
         assert s["n_cycle_nodes"] == n and s["n_ranked"] == 0
         line = rng.integers(0, 4, 1500)
         check(data + fastq(rand_reads(rng, line, 300, 100)), k, bg.thresholds([1]))
+
+
+@pytest.mark.parametrize("k", [21, 31, 45])
+def test_small_inconsistent_chain_maps(k):
+    """separate k and k+2 bounds on graphs of a few blocks: pointers that disagree inside a block and
+    between blocks; the compaction must be that of the listranked nodes, everything before it the oracle's"""
+    thr = [2, 65536, 2, 65536, 2, 65536]
+    for seed in range(12):
+        rng = np.random.default_rng(100 * k + seed)
+        genome = rng.integers(0, 4, int(rng.integers(200, 6000)))
+        data = fastq(rand_reads(rng, genome, 6 * len(genome) // 100, 100, 0.01))
+        ref = oracle.run(data, k=k, thresh=thr, min_update=True)
+        with bg.Graph(k=k, thresh=thr, min_update=True) as g:
+            g.build_and_compact(data)
+            assert g.sizes()["n_chain_nodes"] == ref["n_chain_nodes"]
+            assert_same(sort_nodes(*g.nodes()), ref["nodes"], "graph nodes")
+            assert chain_set(*g.chains()) == compress_ranked(*g.ranked(), k)
