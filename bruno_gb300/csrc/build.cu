@@ -5,8 +5,8 @@
  *                                 ignored), one pass over the bytes each.
  *  superkmer.cuh                  the count from k = 19 on: super-k-mer records, minimizer
  *                                 partitions, one CTA a partition.
- *  k_extract_s, k_split,          the same by k-mer records and hash partitions: below, and where
- *  k_count_local, ...             minimizers crowd.
+ *  k_extract_s, k_split,          the same by k-mer records and hash partitions: below k = 19, and
+ *  k_count_local, ...             what super-k-mers do not take (count_superkmers).
  *  k_hll                          HyperLogLog estimate of distinct canonical k-mers, used to
  *                                 size the table of the direct count.
  *  k_count                        debruijn_kmer_simple_biedge_parser + lex_less +
@@ -3341,7 +3341,7 @@ bruno_status sk_partition(Ctx *c, const std::vector<SkPlan> &plan, uint32_t part
                                           c->stream), "partition plan")) != BRUNO_OK)
     return st;
   const unsigned long long *hist = (const unsigned long long *)c->sk_hist.p;
-  k_sk_plan_sum<<<blocks, SK_PLAN_TPB, 0, c->stream>>>(hist, c->sk_bins, (ulonglong2 *)c->sk_sums.p, SK_MAX_BIN, c->dctr);
+  k_sk_plan_sum<<<blocks, SK_PLAN_TPB, 0, c->stream>>>(hist, c->sk_bins, (ulonglong2 *)c->sk_sums.p, c->dctr);
   k_sk_plan_apply<<<blocks, SK_PLAN_TPB, 0, c->stream>>>(hist, c->sk_bins, (const ulonglong2 *)c->sk_sums.p,
                                                          (const SkPlan *)c->sk_plan.p, (uint32_t)plan.size(), parts,
                                                          (uint32_t *)c->sk_part.p, (uint32_t *)c->sk_off.p,
@@ -3386,19 +3386,19 @@ struct SkShape {
     while ((bytes = sk_count_bytes<KT>(slots, round)) > MOST) slots -= 32;
   }
 };
-template <class KT>
+template <class KT, bool SUB = false>
 void sk_count_launch(const Ctx *c, const SkCount &a, uint32_t grid, size_t bytes) {
   static const bool attr = [] {
-    cudaFuncSetAttribute(k_sk_count<KT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
-    cudaFuncSetAttribute(k_sk_count<KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
+    cudaFuncSetAttribute(k_sk_count<KT, false, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
+    cudaFuncSetAttribute(k_sk_count<KT, true, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkShape<KT>::MOST);
     return true;
   }();
   (void)attr;
   /* threads: the block's 384 unless the partitions are small or the configured block is */
   int nt = std::min(SK_COUNT_TPB, count_threads(c));
   while (nt > 128 && (uint32_t)nt * 2 > a.slots) nt -= 128;
-  if (c->cfg.edge_filter) k_sk_count<KT, true><<<grid, nt, bytes, c->stream>>>(a);
-  else k_sk_count<KT, false><<<grid, nt, bytes, c->stream>>>(a);
+  if (c->cfg.edge_filter) k_sk_count<KT, true, SUB><<<grid, nt, bytes, c->stream>>>(a);
+  else k_sk_count<KT, false, SUB><<<grid, nt, bytes, c->stream>>>(a);
 }
 
 /* One launch's partitions (all, or a size class of a batch's) and its blocks' shape */
@@ -3410,20 +3410,116 @@ struct SkLaunch {
   uint32_t ncls;
 };
 
-/* The partitions counted (records in partition order), those that overflow their block's slots
- * once more with as many as fit; ok = false if that does not do either. */
+/* a block's shape in the launch's arguments */
 template <class KT>
-bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector<SkLaunch<KT>> &launches, bool &ok) {
+void sk_shaped(SkCount &a, const SkShape<KT> &s) {
+  a.slots = s.slots;
+  a.round = s.round;
+  a.hsize = sk_hash_size(s.round);
+  a.late = sk_late_at<KT>(s.slots, s.round);
+}
+
+/* Parts of the crowded partitions: at most SK_PART_KMERS k-mers each on average, half as many at least
+ * where they all differ.  Their entries of the partition table come after the partitions'. */
+constexpr uint64_t SK_PART_KMERS = 4096;
+uint64_t sk_parts_room(const Ctx *c, uint64_t n_rec) { return n_rec * (uint64_t)(c->cfg.k - MZ_M + 1) / (SK_PART_KMERS / 2); }
+
+/* The n partitions listed at `list` (superkmer.cuh, crowded partitions) by parts.  ok = false if
+ * their parts do not do either, or a count that must be exact could pass what an entry holds. */
+template <class KT>
+bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vector<SGeom> &sg, const uint32_t *list,
+                              uint32_t n, uint64_t room, bool &ok) {
+  constexpr int NW = SkRec<KT>::NW;
+  bruno_status st;
+  ok = false;
+  std::vector<uint32_t> part(n);
+  std::vector<uint2> rec(n);
+  if ((st = ensure(c, c->sk_items, (size_t)n * sizeof(uint2))) != BRUNO_OK) return st;
+  k_sk_crowd_records<<<(n + 255) / 256, 256, 0, c->stream>>>(list, n, a.off, (uint2 *)c->sk_items.p);
+  cudaMemcpyAsync(part.data(), list, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
+  cudaMemcpyAsync(rec.data(), c->sk_items.p, (size_t)n * sizeof(uint2), cudaMemcpyDeviceToHost, c->stream);
+  c->launches += 1;
+  if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "crowded partitions")) != BRUNO_OK) return st;
+  std::vector<SkCrowd> crowd(n);
+  std::vector<SkChunk> chunks;
+  uint64_t subs = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const uint64_t kmers = (uint64_t)rec[i].y * (uint64_t)(c->cfg.k - MZ_M + 1);   /* at most */
+    if (!a.nodes && kmers >> 25) return BRUNO_OK;
+    uint32_t lg = 1;
+    while (kmers >> lg > SK_PART_KMERS) ++lg;
+    uint32_t smp = 0;
+    while (smp + 1 < sg.size() && sg[smp + 1].pbase <= part[i]) ++smp;
+    crowd[i] = SkCrowd{part[i], (uint32_t)subs, lg, smp};
+    for (uint32_t r = 0; r < rec[i].y; r += SK_CHUNK<NW>)
+      chunks.push_back(SkChunk{rec[i].x + r, std::min(SK_CHUNK<NW>, rec[i].y - r), (uint32_t)subs, lg});
+    subs += 1ull << lg;
+    if (subs > room) return BRUNO_OK;
+  }
+  const size_t crowd_bytes = (size_t)n * sizeof(SkCrowd);   /* (16 bytes each, like the chunks) */
+  if ((st = ensure(c, c->sk_items, crowd_bytes + chunks.size() * sizeof(SkChunk))) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_sub_cnt, (subs + 1) * 8)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_sub_off, (subs + 1) * 4)) != BRUNO_OK) return st;
+  if ((st = ensure(c, c->sk_sub_smp, subs * 4)) != BRUNO_OK) return st;
+  if ((st = cuda_check(c, cudaMemcpyAsync(c->sk_items.p, crowd.data(), crowd_bytes, cudaMemcpyHostToDevice, c->stream),
+                       "crowded partitions")) != BRUNO_OK)
+    return st;
+  const SkChunk *ch = (const SkChunk *)((const char *)c->sk_items.p + crowd_bytes);
+  if ((st = cuda_check(c, cudaMemcpyAsync((void *)ch, chunks.data(), chunks.size() * sizeof(SkChunk), cudaMemcpyHostToDevice,
+                                          c->stream), "crowded partitions")) != BRUNO_OK)
+    return st;
+  k_sk_crowd_mark<<<n, 256, 0, c->stream>>>((const SkCrowd *)c->sk_items.p, parts, a.info, (uint32_t *)c->sk_sub_smp.p);
+  /* the parts' k-mers counted, then placed */
+  unsigned long long *cnt = (unsigned long long *)c->sk_sub_cnt.p;
+  cudaMemsetAsync(cnt, 0, (subs + 1) * 8, c->stream);
+  k_sk_expand<KT, false><<<(unsigned)chunks.size(), 256, 0, c->stream>>>(a.recs, ch, c->cfg.k, cnt, nullptr);
+  if ((st = scan_ctx(c, (const uint64_t *)cnt, (uint64_t *)cnt, subs + 1, &c->dctr->n_upper)) != BRUNO_OK) return st;
+  k_sk_crowd_off<<<(unsigned)std::min<uint64_t>(1024, (subs + 256) / 256), 256, 0, c->stream>>>(cnt, (uint32_t)subs + 1,
+                                                                                               (uint32_t *)c->sk_sub_off.p);
+  c->launches += 4;
+  if ((st = sync_counters(c)) != BRUNO_OK) return st;
+  const uint64_t kmers = c->hctr->n_upper;
+  if (kmers >> 32) return BRUNO_OK;
+  if ((st = ensure(c, c->sk_kmers, std::max<uint64_t>(1, kmers) * NW * 8)) != BRUNO_OK) return st;
+  k_sk_expand<KT, true><<<(unsigned)chunks.size(), 256, 0, c->stream>>>(a.recs, ch, c->cfg.k, cnt, (uint64_t *)c->sk_kmers.p);
+  a.recs = (const uint64_t *)c->sk_kmers.p;
+  a.off = (const uint32_t *)c->sk_sub_off.p;
+  a.sub0 = parts;
+  a.sub_smp = (const uint32_t *)c->sk_sub_smp.p;
+  a.cls = nullptr;
+  uint32_t left = (uint32_t)subs;
+  for (const double slots : {(double)SK_PART_KMERS / 2, 8000.0}) {   /* what overflows, with as many slots as fit */
+    const SkShape<KT> shape(slots, 0.0);
+    sk_shaped(a, shape);
+    cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
+    if ((st = ensure(c, c->sk_over, (size_t)subs * 8)) != BRUNO_OK) return st;
+    a.todo = left == subs ? nullptr : (const uint32_t *)c->sk_over.p;
+    a.over = (uint32_t *)c->sk_over.p + (left == subs ? 0 : subs);
+    sk_count_launch<KT, true>(c, a, left, shape.bytes);
+    c->launches += 1;
+    if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
+    cudaEventRecord(c->kev[3], c->stream);
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    left = (uint32_t)c->hctr->n_over;
+    if (left == 0 || c->hctr->err) break;
+  }
+  c->sk_subs = (uint32_t)subs;
+  ok = !c->hctr->err && left == 0;
+  return BRUNO_OK;
+}
+
+/* The partitions counted (records in partition order), those that overflow their block's slots
+ * once more with as many as fit, and those that these do not do for either, or that hold too many
+ * records for one block, by parts.  ok = false: the table or the parts are too small, or so many
+ * overflow that the estimate must have been too low (and `retry` is left). */
+template <class KT>
+bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector<SkLaunch<KT>> &launches,
+                            const std::vector<SGeom> &sg, uint64_t room, bool retry, bool &ok) {
   bruno_status st;
   uint32_t round = 128;
-  auto shaped = [&](const SkShape<KT> &s) {
-    a.slots = s.slots;
-    a.round = s.round;
-    a.hsize = sk_hash_size(s.round);
-    a.late = sk_late_at<KT>(s.slots, s.round);
-  };
+  c->sk_subs = 0;
   for (const SkLaunch<KT> &l : launches) {
-    shaped(l.shape);
+    sk_shaped(a, l.shape);
     a.cls = l.cls;
     a.ncls = l.ncls;
     round = std::max(round, l.shape.round);
@@ -3437,22 +3533,29 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
   if (n && !c->hctr->err) {
     const SkShape<KT> big(8000.0, round);
     cudaMemsetAsync(&c->dctr->n_over, 0, 8, c->stream);
-    a.todo = a.over;
-    a.over += parts;
-    shaped(big);
-    sk_count_launch<KT>(c, a, n, big.bytes);
+    SkCount b = a;
+    b.todo = a.over;
+    b.over = a.over + parts;
+    sk_shaped(b, big);
+    sk_count_launch<KT>(c, b, n, big.bytes);
     c->launches += 1;
     if ((st = cuda_check(c, cudaGetLastError(), "k_sk_count")) != BRUNO_OK) return st;
     cudaEventRecord(c->kev[3], c->stream);
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    const uint32_t crowded = (uint32_t)c->hctr->n_over;
+    if (crowded && !c->hctr->err) {
+      ok = false;
+      if (retry && crowded > parts / 2) return BRUNO_OK;
+      return sk_count_crowded<KT>(c, a, parts, sg, b.over, crowded, room, ok);
+    }
   }
   ok = !c->hctr->err && c->hctr->n_over == 0;
   return BRUNO_OK;
 }
 
 /* The count by super-k-mers of the extracted records (one sample, or a batch's), kev[0] recorded
- * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): a
- * bin too large for one CTA, 2^32 records, or partitions that overflow at every size tried.
+ * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): 2^32
+ * records, 2^26 in one bin, or partitions whose parts overflow too at every size tried.
  * max_split: the partition plan's split bits.  again(records): the extraction once more, with room
  * for that many records (133M records: 5 ms, where the k-mer records take 48). */
 constexpr double SK_MAX_KMERS = 3500.0;   /* k-mers of a partition, on average, that fit the largest block twice over */
@@ -3510,7 +3613,8 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
       const int pbits = S > 1 ? pl.pbits : std::min(pl.pbits, std::max(8, c->sk_bits[q] - 2));
       const uint64_t n = 1ull << pbits;
       if (!(pl.fits || pbits < pl.pbits) || distinct[q] > SK_MAX_KMERS * (double)n) return BRUNO_OK;
-      caps[q] = slots + 2 * n;   /* a partition's slots are rounded up by two */
+      /* a partition's slots are rounded up by two, and so are a crowded one's parts' */
+      caps[q] = slots + 2 * n + n_inst / 512;
       sg[q].g = TableGeom{caps[q], 0, pbits, base, nullptr, nullptr, bin0, 32 - c->sk_bits[q], c->cfg.k};
       sg[q].pbase = parts;
       sg[q].rec2_base = sg[q].cap2 = 0;
@@ -3537,7 +3641,8 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
     if ((st = ensure(c, c->sk_part, (size_t)c->sk_bins * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_off, (parts + 1) * 4)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_cur, (parts + SK_SPLIT_N) * 4)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->sk_info, parts * 8)) != BRUNO_OK) return st;
+    const uint64_t room = sk_parts_room(c, n_rec);
+    if ((st = ensure(c, c->sk_info, (parts + room) * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sk_over, parts * 8)) != BRUNO_OK) return st;
     if (S > 1 && (st = ensure(c, c->sk_bump, (size_t)S * 8)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->sgeom, S * sizeof(SGeom))) != BRUNO_OK) return st;
@@ -3607,7 +3712,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
       for (size_t l = 0; l < launches.size(); ++l) launches[l].cls = (const ClassRun *)c->grp_tmp.p + at[l];
     }
     bool ok = false;
-    if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, ok)) != BRUNO_OK) return st;
+    if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, sg, room, attempt < 2, ok)) != BRUNO_OK) return st;
     if (c->hctr->err & DERR_SKEW) return BRUNO_OK;
     if (ok) {
       std::vector<uint64_t> taken(S, c->hctr->sk_bump);

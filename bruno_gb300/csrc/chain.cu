@@ -251,7 +251,8 @@ __device__ __forceinline__ uint32_t ci_hash(KW2 x, uint32_t n) {
 }
 template <class KT>
 __global__ void __launch_bounds__(TPB, sizeof(KT) == 8 ? 6 : 4) k_chain_local(const uint64_t *table, TableGeom g0, const SGeom *sg,
-                                                      uint32_t nsamples, int k, uint64_t M, uint32_t cap, uint64_t *ckey,
+                                                      uint32_t nsamples, uint32_t parts, const uint32_t *sub_smp, int k,
+                                                      uint64_t M, uint32_t cap, uint64_t *ckey,
                                                       ChainState *cs, uint8_t *cedge, uint32_t *csample,
                                                       uint32_t max_probe, DevCounters *ctr) {
   constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW;
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(TPB, sizeof(KT) == 8 ? 6 : 4) k_chain_local(co
   uint16_t *s_edge = s_todo + 2 * cap;                  /* a node's slot, then its edge byte */
   __shared__ uint32_t s_n, s_left;
   const uint2 reg = g0.info[blockIdx.x];
+  if (reg.y & SK_SUBS) return;   /* a crowded partition: its parts have blocks of their own */
   const uint32_t R = reg.y, nt = blockDim.x, lane = threadIdx.x & 31, below = (1u << lane) - 1;
   bool bad = false;
   auto append = [&](bool want, uint32_t *n) -> uint32_t {   /* the warp's places in a list of the block */
@@ -280,7 +282,7 @@ __global__ void __launch_bounds__(TPB, sizeof(KT) == 8 ? 6 : 4) k_chain_local(co
   };
   /* 4 | the last base with a count, 0 if none has one */
   auto edge = [](uint64_t counts) { return counts ? 4u | (unsigned)(63 - __clzll(counts)) >> 4 : 0u; };
-  const uint32_t smp = nsamples > 1 ? sample_of_part(sg, nsamples, blockIdx.x) : 0u;
+  const uint32_t smp = nsamples <= 1 ? 0u : blockIdx.x < parts ? sample_of_part(sg, nsamples, blockIdx.x) : sub_smp[blockIdx.x - parts];
   bool local = true;
   for (uint32_t t0 = 0; t0 < R; ) {
     const uint32_t n = local ? R : min(cap, R - t0);
@@ -1539,8 +1541,9 @@ bruno_status extract_typed(Ctx *c) {
     const double mean = (double)(M + c->n_branch) / c->sk_parts;
     const uint32_t cap = (uint32_t)std::max(128.0, std::min((double)CI_NODES, 1.5 * mean + 64.0)) & ~31u;
     const int nt = KWD == 1 ? (mean > 500 ? TPB : mean > 120 ? TPB / 2 : TPB / 4) : mean > 300 ? TPB / 2 : TPB / 4;
-    k_chain_local<KT><<<c->sk_parts, nt, ci_bytes<KT>(cap), c->stream>>>(
-        (const uint64_t *)c->table.p, c->geom, (const SGeom *)c->sgeom.p, c->S, c->cfg.k, M, cap, (uint64_t *)c->ckey.p,
+    k_chain_local<KT><<<c->sk_parts + c->sk_subs, nt, ci_bytes<KT>(cap), c->stream>>>(
+        (const uint64_t *)c->table.p, c->geom, (const SGeom *)c->sgeom.p, c->S, c->sk_parts, (const uint32_t *)c->sk_sub_smp.p,
+        c->cfg.k, M, cap, (uint64_t *)c->ckey.p,
         (ChainState *)c->cstate.p, (uint8_t *)c->cedge.p, (uint32_t *)c->csample.p, 4096u, c->dctr);
   } else {
     k_chain_init<KT><<<sms * 8, TPB, 0, c->stream>>>((const uint64_t *)c->table.p, c->nslots, c->geom,

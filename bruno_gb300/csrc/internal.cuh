@@ -165,6 +165,7 @@ struct Ctx {
   /* counting by super-k-mers (superkmer.cuh): records as extracted and in partition order, the
    * minimizer bins' tallies and partitions, the partitions' first records and cursors */
   Buf sk_recs, sk_sorted, sk_hist, sk_part, sk_off, sk_cur, sk_samp, sk_plan, sk_sums, sk_info, sk_over, sk_bump, sk_est;
+  Buf sk_items, sk_sub_cnt, sk_sub_off, sk_sub_smp, sk_kmers;   /* crowded partitions: their k-mers, by part */
   bool sk_on = false;            /* this build extracts super-k-mers */
   /* one call builds the whole graph: the thresholds of the configuration are the ones the filter
    * will use and nobody asks for raw counts, so the count need not keep what the filter drops */
@@ -172,7 +173,8 @@ struct Ctx {
   bool nodes_made = false;       /* ... and the count made the nodes */
   bool nodes_erased = false;     /* nodes have left the graph since their lists were made */
   uint32_t sk_parts = 0;         /* minimizer partitions of the table, ... */
-  uint64_t sk_taken = 0;         /* ... and the slots in them */
+  uint32_t sk_subs = 0;          /* ... parts that crowded ones were cut into (sk_sub_smp: their samples), ... */
+  uint64_t sk_taken = 0;         /* ... and the slots in all of them */
   uint64_t sk_cap = 0, sk_est_cap = 0;
   std::vector<uint64_t> sk_gaps; /* a batch whose samples left table slots unwritten: their shares' sizes */
   uint32_t sk_bins = 0, sk_chunk = 32;

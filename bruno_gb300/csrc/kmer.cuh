@@ -217,6 +217,7 @@ struct TableGeom {
   uint64_t base;     /* first slot: a sample's table in a batch of samples starts here (0 otherwise) */
   /* tables filled by super-k-mers (superkmer.cuh): a k-mer's partition comes from its minimizer,
    * P = bins[bin0 + (mz_mix(minimizer) >> bin_shift)], and holds info[P].y slots from info[P].x on;
+   * a crowded partition (info[P].y: SK_SUBS | lg) is cut by the key into 2^lg, info[info[P].x] on;
    * bins == NULL: the partition is the top pbits bits of the key's mix, `region` slots each */
   const uint32_t *bins = nullptr;
   const uint2 *info = nullptr;
@@ -310,6 +311,10 @@ __device__ __forceinline__ void neighbour_minimizers(KT x, int k, unsigned cin, 
   mz[0] = min(in, mz_order((fl >> 2) | (cin << (2 * MZ_M - 2)), ((r_first << 2) | (3u - cin)) & MZ_MASK));
   mz[1] = min(out, mz_order(((f_last << 2) | cout) & MZ_MASK, (r_last >> 2) | ((3u - cout) << (2 * MZ_M - 2))));
 }
+constexpr uint32_t SK_SUBS = 1u << 31;
+/* which part of a crowded partition a key lies in, in the low bits (bin_home takes high ones) */
+__device__ __forceinline__ uint32_t key_sub(KW1 t) { return (uint32_t)t.v; }
+__device__ __forceinline__ uint32_t key_sub(KW2 t) { return (uint32_t)t.lo; }
 /* a key's place in such a partition: the mix's bits are all free there */
 __device__ __forceinline__ uint32_t bin_home(KW1 t, uint32_t region) { return __umulhi((uint32_t)(t.v >> 30), region); }
 __device__ __forceinline__ uint32_t bin_home(KW2 t, uint32_t region) { return __umulhi((uint32_t)(t.lo >> 32), region); }
@@ -339,7 +344,8 @@ struct Probe {
 /* the probe sequence of a table key with the given minimizer in a table filled by super-k-mers */
 template <class KT>
 __device__ __forceinline__ Probe bin_probe(const TableGeom &g, uint32_t minimizer, KT t) {
-  const uint2 r = __ldg(g.info + __ldg(g.bins + g.bin0 + (mz_mix(minimizer) >> g.bin_shift)));
+  uint2 r = __ldg(g.info + __ldg(g.bins + g.bin0 + (mz_mix(minimizer) >> g.bin_shift)));
+  if (r.y & SK_SUBS) r = __ldg(g.info + r.x + (key_sub(t) & ((1u << (r.y & 31u)) - 1u)));
   return Probe((uint64_t)r.x, r.y, bin_home(t, r.y));
 }
 /* the probe sequence of canonical k-mer x, whose table key is t */

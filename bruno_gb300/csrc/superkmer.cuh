@@ -16,6 +16,8 @@
  *   k_sk_count     one CTA a partition: equal records merged into one with a weight, their
  *                  k-mers counted in shared memory, the k-mers to keep written to the table, or
  *                  (one-call builds) the graph's nodes made of them
+ *   k_sk_expand    a crowded partition's records -> its k-mers with their weights, cut by their key
+ *                  into parts that k_sk_count then counts like partitions
  *
  * 50 Mbp at 30x (1.2G k-mers, k = 31): extraction 4.9, split 2.8, count 12.1 ms, where k-mer records
  * took 9.9 (extraction), 5.8 (split), 11.6 (count) and 3.3 (filter).  k = 63, 352M k-mers: 1.9, 0.8
@@ -439,13 +441,12 @@ struct SkPlan {   /* a sample */
   unsigned long long inst0, T;        /* k-mers of the samples before, k-mers a partition */
   unsigned int bin0, pbase, parts, pad;   /* first bin, first partition, partitions */
 };
-/* k-mers of one bin at most: one CTA counts it, and a count in shared memory must stay below 2^24 */
-constexpr unsigned long long SK_MAX_BIN = 1ull << 22;
+/* records of one bin at most: its k-mers, at most 49 a record, have 32 bits of its tally */
+constexpr unsigned long long SK_MAX_BIN = 1ull << 26;
 constexpr int SK_PLAN_TPB = 256, SK_PLAN_PER = 16, SK_PLAN_CHUNK = SK_PLAN_TPB * SK_PLAN_PER;
 
 __global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_sum(const unsigned long long *hist, uint32_t nbins,
-                                                             ulonglong2 *sums, unsigned long long max_bin,
-                                                             DevCounters *ctr) {
+                                                             ulonglong2 *sums, DevCounters *ctr) {
   unsigned long long inst = 0, rec = 0;
   bool big = false;
   for (uint32_t j = threadIdx.x; j < SK_PLAN_CHUNK; j += SK_PLAN_TPB) {
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_sum(const unsigned long
     if (b >= nbins) break;
     const unsigned long long v = hist[b];
     inst += v >> 32; rec += v & 0xFFFFFFFFull;
-    big |= (v >> 32) > max_bin;
+    big |= (v & 0xFFFFFFFFull) > SK_MAX_BIN;
   }
   inst = warp_sum(inst); rec = warp_sum(rec);
   __shared__ unsigned long long si[SK_PLAN_TPB / 32], sr[SK_PLAN_TPB / 32];
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(SK_PLAN_TPB) k_sk_plan_sum(const unsigned long
     for (int q = 1; q < SK_PLAN_TPB / 32; ++q) { inst += si[q]; rec += sr[q]; }
     sums[blockIdx.x] = make_ulonglong2(inst, rec);
   }
-  if (big) atomicOr(&ctr->err, (unsigned long long)DERR_SKEW);   /* a bin too large for one CTA */
+  if (big) atomicOr(&ctr->err, (unsigned long long)DERR_SKEW);
 }
 
 /* part[b] = partition of bin b (over all samples); off[P], cur[P] = first record of partition P
@@ -721,6 +722,8 @@ struct SkCount {
   const SGeom *sg;
   uint32_t nsamples;
   unsigned long long *bump;         /* per sample: table slots taken so far */
+  uint32_t sub0;                    /* parts of crowded partitions: the first one's place in info, */
+  const uint32_t *sub_smp;          /* their samples */
   DevCounters *ctr;
 };
 
@@ -824,20 +827,27 @@ constexpr uint32_t SK_MORE = E_BIG;
 __device__ __forceinline__ uint32_t sk_count_of(uint32_t w) { return w >> E_COUNT_SHIFT; }
 
 /* `fresh` is an entry word: a code and the occurrences to count.  One entry word of a slot tried for
- * it; `w` is what the word was seen to hold */
+ * it; `w` is what the word was seen to hold.  SAT: a count from 2^25 on stays where it is (a block's
+ * threads, with weights of 2^10 at most, cannot bring it to 2^26 before they see it) */
+template <bool SAT = false>
 __device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t fresh, unsigned &claims) {
   if (w == 0) {
     w = atomicCAS(e, 0u, fresh);
     if (w == 0) { ++claims; return true; }
   }
   if (entry_code(w) != entry_code(fresh)) return false;
-  atomicAdd(e, fresh & ~((1u << E_COUNT_SHIFT) - 1));
+  const uint32_t add = fresh & ~((1u << E_COUNT_SHIFT) - 1);
+  if (SAT) {
+    if (atomicAdd(e, add) >> 31) atomicSub(e, add);
+  } else {
+    atomicAdd(e, add);
+  }
   return true;
 }
 
 /* an entry word's occurrences into the shared-memory slots of a k-mer, continuation slots and all
  * (any lanes may call it); false if the slots are full */
-template <class KT>
+template <class KT, bool SAT>
 __device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, unsigned &claims) {
   SkSeq p(want, sl.n);
   for (uint32_t probe = 0; probe < SK_MAX_PROBE; ++probe, p.next(sl.n)) {
@@ -847,8 +857,8 @@ __device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, 
     if (claimed) { ++claims; return true; }
     if (KOps<KT>::eq(key, want)) {
       uint32_t *e = sl.entries(p.j);
-      if (sk_try_entry(e, *(volatile uint32_t *)e, fresh, claims)) return true;
-      if (sk_try_entry(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims)) return true;
+      if (sk_try_entry<SAT>(e, *(volatile uint32_t *)e, fresh, claims)) return true;
+      if (sk_try_entry<SAT>(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims)) return true;
       atomicOr(e + 1, SK_MORE);
       ((uint64_t *)&want)[KOps<KT>::WORDS - 1] |= KEY_CONT;
     }
@@ -996,7 +1006,119 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
   return din >= 2 || dout >= 2 || kpal || k1pal ? 2 : 1;
 }
 
-template <class KT, bool EF>
+/* Equal records merge into the first that claimed an entry of the record hash, which then has their
+ * number as its weight (a third of the entries stays free; every thread of the block calls it) */
+template <int NW>
+__device__ __forceinline__ void sk_merge(const uint64_t *s_rec, uint32_t *s_wt, uint32_t *s_hash, uint32_t hmask,
+                                         uint32_t nr, uint32_t tid, uint32_t nt) {
+  for (uint32_t i = tid; i < nr; i += nt) {
+    ulonglong2 rec[NW / 2];
+    uint64_t z = 0;
+    #pragma unroll
+    for (int q = 0; q < NW / 2; ++q) {
+      rec[q] = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)i * NW)[q];
+      z = (z ^ rec[q].x) * 0x9E3779B97F4A7C15ull ^ rec[q].y ^ (z >> 29);
+    }
+    z *= 0xD6E8FEB86659FD93ull;
+    uint32_t h = (uint32_t)(z >> 52) & hmask;
+    for (;;) {
+      const uint32_t o = atomicCAS(&s_hash[h], ~0u, i);
+      if (o == ~0u) { atomicAdd(&s_wt[i], 1u); break; }
+      bool same = true;
+      #pragma unroll
+      for (int q = 0; q < NW / 2; ++q) {
+        const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)o * NW)[q];
+        same &= v.x == rec[q].x && v.y == rec[q].y;
+      }
+      if (same) { atomicAdd(&s_wt[o], 1u); break; }
+      h = (h + 1) & hmask;
+    }
+  }
+}
+
+/* lex_less: the smaller strand's biedge, reverse-complemented on a flip */
+__device__ __forceinline__ unsigned sk_code(bool fwd, unsigned in5, unsigned out5) {
+  return fwd ? biedge_code(in5, out5) : biedge_code(out5 ? 5u - out5 : 0u, in5 ? 5u - in5 : 0u);
+}
+
+/* ------------------------------------------------------------ crowded partitions
+ * A minimizer that many places share (a tail of one base, an adapter, a satellite: k-mers that hold it
+ * and some of what lies around) can put more k-mers into a partition than a block's slots, or more
+ * records than one block should count.  Such a partition is cut by its k-mers' keys: its records go
+ * through blocks of SK_CHUNK, which merge the equal ones and write each k-mer with its weight to one of
+ * 2^lg parts, first counted, then placed; a part holds some thousand k-mers, is counted by a block and
+ * has a region of its own, which lookups find by the key.  160M k-mers, adapters in 2% of the reads:
+ * 5.9 ms a build (4.9 without the adapters); by k-mer records, where such an input used to go after the
+ * count had been tried at three sizes, 29.9, of which the k-mer records themselves take 17.1. */
+struct SkChunk { uint32_t r0, n, sub0, lg; };   /* records, first part, log2 of the parts */
+template <int NW> constexpr uint32_t SK_CHUNK = 2048 / NW;
+/* records of a partition at most that one block counts (a typical one: 500), and below 2^26 k-mers */
+constexpr uint32_t SK_MAX_RECORDS = 1u << 15;
+
+template <class KT, bool WRITE>
+__global__ void __launch_bounds__(256) k_sk_expand(const uint64_t *recs, const SkChunk *chunks, int k,
+                                                   unsigned long long *cur, uint64_t *out) {
+  constexpr int NW = SkRec<KT>::NW;
+  constexpr uint32_t N = SK_CHUNK<NW>, H = 2 * N;
+  __shared__ __align__(16) uint64_t s_rec[N * NW];
+  __shared__ uint32_t s_wt[N], s_hash[H];
+  const SkChunk ch = chunks[blockIdx.x];
+  const uint32_t tid = threadIdx.x, nt = blockDim.x;
+  for (uint32_t i = tid; i < ch.n * (NW / 2); i += nt)
+    reinterpret_cast<ulonglong2 *>(s_rec)[i] = reinterpret_cast<const ulonglong2 *>(recs + (uint64_t)ch.r0 * NW)[i];
+  for (uint32_t i = tid; i < N; i += nt) s_wt[i] = 0;
+  for (uint32_t i = tid; i < H; i += nt) s_hash[i] = ~0u;
+  __syncthreads();
+  sk_merge<NW>(s_rec, s_wt, s_hash, H - 1, ch.n, tid, nt);
+  __syncthreads();
+  for (uint32_t i = tid; i < ch.n; i += nt) {
+    const uint32_t weight = s_wt[i] << E_COUNT_SHIFT;
+    if (!weight) continue;
+    const uint64_t *w = s_rec + (size_t)i * NW;
+    const uint64_t last = w[NW - 1];
+    const int nk = (int)sk_n(last), n_out = nk - ((last & SK_RIGHT) ? 0 : 1);
+    KT f = KOps<KT>::extract(w, 1, k), r = KOps<KT>::rc(f, k);
+    unsigned in5 = (last & SK_LEFT) ? sk_base<NW>(w, 0) + 1u : 0u;
+    for (int d = 0; d < nk; ++d) {
+      const unsigned c = d < n_out ? sk_base<NW>(w, d + k + 1) : 0u;
+      const bool fwd = KOps<KT>::lt(f, r);
+      const KT key = fwd ? f : r;
+      const uint32_t fresh = (sk_code(fwd, in5, d < n_out ? c + 1u : 0u) << E_CODE_SHIFT) | weight;
+      in5 = KOps<KT>::first(f, k) + 1u;
+      f = KOps<KT>::append(f, c, k);
+      r = KOps<KT>::prepend(3u - c, r, k);
+      const unsigned long long o = atomicAdd(&cur[ch.sub0 + (key_sub(table_key(key)) & ((1u << ch.lg) - 1u))], 1ull);
+      if constexpr (WRITE) {
+        ulonglong2 *to = reinterpret_cast<ulonglong2 *>(out + o * NW);
+        if constexpr (NW == 2) {
+          to[0] = make_ulonglong2(((const uint64_t *)&key)[0], (uint64_t)fresh);
+        } else {
+          to[0] = make_ulonglong2(((const uint64_t *)&key)[0], ((const uint64_t *)&key)[KOps<KT>::WORDS - 1]);
+          to[1] = make_ulonglong2((uint64_t)fresh, 0ull);
+        }
+      }
+    }
+  }
+}
+
+struct SkCrowd { uint32_t part, sub0, lg, smp; };
+/* the records of the listed partitions */
+__global__ void k_sk_crowd_records(const uint32_t *list, uint32_t n, const uint32_t *off, uint2 *out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = make_uint2(off[list[i]], off[list[i] + 1] - off[list[i]]);
+}
+/* crowded partitions' entries of the partition table, and their parts' samples */
+__global__ void k_sk_crowd_mark(const SkCrowd *crowd, uint32_t parts, uint2 *info, uint32_t *sub_smp) {
+  const SkCrowd x = crowd[blockIdx.x];
+  if (threadIdx.x == 0) info[x.part] = make_uint2(parts + x.sub0, SK_SUBS | x.lg);
+  for (uint32_t i = threadIdx.x; i < 1u << x.lg; i += blockDim.x) sub_smp[x.sub0 + i] = x.smp;
+}
+__global__ void k_sk_crowd_off(const unsigned long long *base, uint32_t n, uint32_t *off) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) off[i] = (uint32_t)base[i];
+}
+
+/* SUB: the parts of crowded partitions, from their k-mers' records (off, todo and over are theirs) */
+template <class KT, bool EF, bool SUB>
 __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_count(SkCount a) {
   constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW, NE = Slot<KT>::ENTRIES, NW = SkRec<KT>::NW;
   extern __shared__ __align__(16) uint64_t sm[];
@@ -1006,7 +1128,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   __shared__ unsigned long long s_cand;
   if (a.ctr->err & DERR_SKEW) return;
   uint32_t part = a.todo ? a.todo[blockIdx.x] : blockIdx.x;
-  if (a.cls && !a.todo) {
+  if (!SUB && a.cls && !a.todo) {
     uint32_t lo = 0, hi = a.ncls;
     while (hi - lo > 1) { const uint32_t m = (lo + hi) >> 1; if (__ldg(&a.cls[m].run) <= blockIdx.x) lo = m; else hi = m; }
     part = a.cls[lo].pbase + (blockIdx.x - a.cls[lo].run);
@@ -1018,6 +1140,10 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   uint32_t *s_wt = reinterpret_cast<uint32_t *>(s_rec + (size_t)round * NW), *s_hash = s_wt + round;
   uint16_t *s_list = reinterpret_cast<uint16_t *>(s_hash);
   SkLate<KT> *s_late = reinterpret_cast<SkLate<KT> *>(sm + a.late);
+  if (!SUB && a.off[part + 1] - a.off[part] > SK_MAX_RECORDS) {
+    if (tid == 0) a.over[atomicAdd(&a.ctr->n_over, 1ull)] = part;
+    return;
+  }
   for (uint32_t i = tid; i < slots; i += nt) sl.clear(i);
   if (tid < 4) s_qh[tid] = 0;
   if (tid < 16) s_hist[tid] = 0;
@@ -1026,7 +1152,14 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
   const uint32_t hmask = a.hsize - 1;
   unsigned claims = 0;
   const uint32_t r1 = a.off[part + 1];
-  for (uint32_t r0 = a.off[part]; r0 < r1; r0 += round) {
+  if constexpr (SUB) {
+    __syncthreads();
+    for (uint32_t i = a.off[part] + tid; i < r1; i += nt) {
+      const uint64_t *w = a.recs + (uint64_t)i * NW;
+      if (!*(volatile uint32_t *)&s_full && !sk_insert<KT, true>(sl, KOps<KT>::load(w), (uint32_t)w[KWD], claims)) s_full = 1;
+    }
+  }
+  for (uint32_t r0 = a.off[part]; !SUB && r0 < r1; r0 += round) {
     const uint32_t nr = min(round, r1 - r0);
     for (uint32_t i = tid; i < nr * (NW / 2); i += nt)
       reinterpret_cast<ulonglong2 *>(s_rec)[i] = __ldcs(reinterpret_cast<const ulonglong2 *>(a.recs + (uint64_t)r0 * NW) + i);
@@ -1034,30 +1167,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     for (uint32_t i = tid; i <= hmask; i += nt) s_hash[i] = ~0u;
     if (tid == 0) { s_items = 0; s_late_n = 0; }
     __syncthreads();
-    /* equal records merge into the first that claimed a hash entry */
-    for (uint32_t i = tid; i < nr; i += nt) {
-      ulonglong2 rec[NW / 2];
-      uint64_t z = 0;
-      #pragma unroll
-      for (int q = 0; q < NW / 2; ++q) {
-        rec[q] = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)i * NW)[q];
-        z = (z ^ rec[q].x) * 0x9E3779B97F4A7C15ull ^ rec[q].y ^ (z >> 29);
-      }
-      z *= 0xD6E8FEB86659FD93ull;
-      uint32_t h = (uint32_t)(z >> 52) & hmask;
-      for (;;) {   /* a third of the entries stays free */
-        const uint32_t o = atomicCAS(&s_hash[h], ~0u, i);
-        if (o == ~0u) { atomicAdd(&s_wt[i], 1u); break; }
-        bool same = true;
-        #pragma unroll
-        for (int q = 0; q < NW / 2; ++q) {
-          const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(s_rec + (size_t)o * NW)[q];
-          same &= v.x == rec[q].x && v.y == rec[q].y;
-        }
-        if (same) { atomicAdd(&s_wt[o], 1u); break; }
-        h = (h + 1) & hmask;
-      }
-    }
+    sk_merge<NW>(s_rec, s_wt, s_hash, hmask, nr, tid, nt);
     __syncthreads();
     /* the distinct records' k-mers as items of SK_ITEM */
     for (uint32_t i0 = 0; i0 < nr; i0 += nt) {
@@ -1097,10 +1207,9 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         bool todo = d < n;
         const unsigned c = next >> 30, out5 = d < n_out ? c + 1u : 0u;
         next <<= 2;
-        /* lex_less: the smaller strand, with the biedge reverse-complemented on a flip */
         const bool fwd = KOps<KT>::lt(f, r);
         const KT key = fwd ? f : r;
-        const unsigned code = fwd ? biedge_code(in5, out5) : biedge_code(out5 ? 5u - out5 : 0u, in5 ? 5u - in5 : 0u);
+        const unsigned code = sk_code(fwd, in5, out5);
         const uint32_t fresh = (code << E_CODE_SHIFT) | weight;
         in5 = KOps<KT>::first(f, k) + 1u;
         f = KOps<KT>::append(f, c, k);
@@ -1128,7 +1237,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         if (todo) {   /* the rest, later */
           const uint32_t at = atomicAdd(&s_late_n, 1u);
           if (at < SK_LATE) s_late[at] = SkLate<KT>{key, fresh};
-          else if (!sk_insert<KT>(sl, key, fresh, claims)) s_full = 1;
+          else if (!*(volatile uint32_t *)&s_full && !sk_insert<KT, false>(sl, key, fresh, claims)) s_full = 1;
         }
         __syncwarp();
       }
@@ -1136,7 +1245,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     __syncthreads();
     const uint32_t late = min(s_late_n, SK_LATE);
     for (uint32_t y = tid; y < late; y += nt)
-      if (!sk_insert<KT>(sl, s_late[y].key, (uint32_t)s_late[y].fresh, claims)) s_full = 1;
+      if (!*(volatile uint32_t *)&s_full && !sk_insert<KT, false>(sl, s_late[y].key, (uint32_t)s_late[y].fresh, claims)) s_full = 1;
     __syncthreads();
     if (s_full) break;
   }
@@ -1259,10 +1368,11 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     make_node(tid);
     __syncthreads();
   }
-  if ((EF || a.nodes) && (tid == 32 || tid == 64)) reserve(tid / 32 - 1, sample_of_part(a.sg, a.nsamples, part));
+  if ((EF || a.nodes) && (tid == 32 || tid == 64))
+    reserve(tid / 32 - 1, SUB ? a.sub_smp[part] : sample_of_part(a.sg, a.nsamples, part));
   if (tid == 0) {
     const uint32_t R = want_R;
-    const uint32_t smp = sample_of_part(a.sg, a.nsamples, part);
+    const uint32_t smp = SUB ? a.sub_smp[part] : sample_of_part(a.sg, a.nsamples, part);
     const TableGeom &g = a.sg[smp].g;
     const unsigned long long lo = atomicAdd(&a.bump[smp], (unsigned long long)R);
     s_cand = a.cand ? atomicAdd(&a.ctr->n_cand, (unsigned long long)listed) : 0ull;
@@ -1271,7 +1381,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     s_slots = fits ? R : 0;
     s_smp = smp;
     s_base = (uint32_t)(g.base + lo);
-    a.info[part] = make_uint2((uint32_t)(g.base + lo), R);
+    a.info[SUB ? a.sub0 + part : part] = make_uint2((uint32_t)(g.base + lo), R);
     if (!a.cand) atomicAdd(&a.ctr->n_cand, (unsigned long long)listed);
     if (tslots) atomicAdd(&a.ctr->n_slots_claimed, (unsigned long long)tslots);
     if (!EF && s_claims) atomicAdd(&a.ctr->n_entries, (unsigned long long)s_claims);

@@ -61,8 +61,8 @@ typedef struct bruno_cfg {
   int32_t exact_ranking;    /* 1: always run the round-synchronous ranking; 0: use the O(M)
                                ruling-set ranking whenever the chain map is consistent */
   int32_t direct_count;     /* counting path: 0 = automatic (from k = 19 on super-k-mer records,
-                               below and for input that crowds few minimizers k-mer records, by
-                               partition in one CTA's shared memory; a skewed input that overflows
+                               below, and for the rare input that these do not take, k-mer records,
+                               by partition in one CTA's shared memory; a skewed input that overflows
                                a partition of k-mer records falls back to L2-resident partitions
                                at k <= 31 and to the whole-table count at k > 31), 1 = every
                                instance straight into the whole table, 2 = the L2 partitions

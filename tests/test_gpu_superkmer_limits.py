@@ -1,5 +1,6 @@
 """Super-k-mer builds where an input outgrows what its plan foresaw, against the oracle and against the
-plain build: more records than their room, cycles within one block of chain nodes, pointers that disagree."""
+plain build: more records than their room, cycles within one block of chain nodes, pointers that disagree,
+partitions with more k-mers or records than a block counts."""
 import numpy as np
 import pytest
 
@@ -7,6 +8,7 @@ import bruno_gb300 as bg
 from helpers import assert_same, chain_set, compress_ranked, sort_nodes, sort_ranked
 from oracle import oracle
 from test_gpu_batch import batch, plain, same_as_plain
+from test_gpu_parity import compare, gpu_run
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +112,96 @@ def test_small_inconsistent_chain_maps(k):
             assert g.sizes()["n_chain_nodes"] == ref["n_chain_nodes"]
             assert_same(sort_nodes(*g.nodes()), ref["nodes"], "graph nodes")
             assert chain_set(*g.chains()) == compress_ranked(*g.ranked(), k)
+
+
+# ------------------------------------------------------------------ crowded partitions
+ADAPTER = np.array(["ACGT".index(c) for c in "AGATCGGAAGAGCACACGTCTGAACTCCAGTCA"] + [0] * 200)
+
+
+def tailed(rng, codes, n, tail):
+    """n of the reads end in `tail`, from a place of their own on"""
+    c = codes.copy()
+    length = c.shape[1]
+    for i in rng.choice(len(c), n, replace=False):
+        p = int(rng.integers(8, length - 20))
+        c[i, p:] = tail[:length - p]
+    return c
+
+
+def crowded_reads(kind, seed, n=24_000, genome=120_000):
+    """reads of 100 bases whose k-mers crowd one minimizer or a few: the places where an adapter or a run
+    of one base begins (more k-mers than a block's slots), whole reads of one base (more records than a
+    block counts), a diverged satellite"""
+    rng = np.random.default_rng(seed)
+    g = rng.integers(0, 4, genome)
+    if kind == "satellite":
+        unit = rng.integers(0, 4, 171)
+        for p in range(0, genome - 2000, 4000):
+            t = np.resize(unit, 2000)
+            g[p:p + 2000] = np.where(rng.random(2000) < 0.1, (t + rng.integers(1, 4, 2000)) & 3, t)
+    c = rand_reads(rng, g, n, 100, 0.003)
+    if kind == "adapter":
+        c = tailed(rng, c, n // 3, ADAPTER)
+    elif kind == "poly-A":
+        c = tailed(rng, c, n // 3, np.zeros(200, dtype=int))
+    elif kind == "one base":
+        c[rng.random(n) < 0.4] = 3
+    return c
+
+
+@pytest.mark.parametrize("thr", [[2], []])
+@pytest.mark.parametrize("kind", ["adapter", "poly-A", "one base", "satellite"])
+@pytest.mark.parametrize("k", [21, 31, 45, 63])
+def test_crowded_partitions(k, kind, thr):
+    """one call, and the step calls with every count copied out"""
+    data = fastq(crowded_reads(kind, k))
+    check(data, k, bg.thresholds(thr), thresholding=bool(thr))
+    ref = oracle.run(data, k=k, thresholding=bool(thr), thresh=bg.thresholds(thr), min_update=True, keep_k2=True,
+                     keep_filtered=True, threads=16)
+    compare(gpu_run(data, k, bool(thr), bg.thresholds(thr), True), ref)
+
+
+@pytest.mark.parametrize("kind", ["adapter", "one base"])
+@pytest.mark.parametrize("k", [21, 30, 31, 63])
+def test_crowded_partitions_edge_filter(k, kind):
+    check(fastq(crowded_reads(kind, 7 * k)), k, bg.thresholds([3]), edge_filter=True)
+
+
+@pytest.mark.parametrize("chunk", [0, 1 << 20])
+def test_crowded_samples_of_a_batch(chunk):
+    """samples that crowd a partition among samples that do not, in one copy and in groups"""
+    rng = np.random.default_rng(11)
+    samples = [fastq(rand_reads(rng, rng.integers(0, 4, 20_000), 3_000, 100, 0.003)) for _ in range(6)]
+    for at, kind in ((1, "adapter"), (4, "one base"), (6, "poly-A")):
+        samples.insert(at, fastq(crowded_reads(kind, at)))
+    cfg = dict(k=31, thresholding=True, thresh=bg.thresholds([2]), min_update=True)
+    got, _ = batch(samples, h2d_chunk=chunk, **cfg)
+    for i, data in enumerate(samples):
+        same_as_plain(got[i], plain(data, **cfg), f"sample {i}")
+
+
+def test_crowded_partitions_cleaned():
+    """cleaning looks nodes up, erases them and lists them again: in a table with crowded partitions too"""
+    data = fastq(crowded_reads("adapter", 3))
+    thr = bg.thresholds([1])
+    ref = oracle.run(data, k=31, thresh=thr, min_update=True, threads=16, clean=True)
+    with bg.Graph(k=31, thresh=thr, min_update=True) as g:
+        g.build_and_compact(data)
+        stats = g.clean_deadend_and_bubbles_naive()
+        for n in ("rounds", "deadends", "bubbles", "edges"):
+            assert stats[n] == ref["clean_stats"][n], n
+        assert_same(sort_nodes(*g.nodes()), ref["clean"]["nodes"], "cleaned nodes")
+        assert chain_set(*g.chains()) == chain_set(*ref["clean"]["chains"])
+
+
+@pytest.mark.parametrize("k", [31, 45])
+def test_a_count_past_what_a_block_may_hold(k):
+    """one biedge of one k-mer counted more than 2^25 times (300 bases a read, all alike, beside a
+    genome's reads): capped where only the filter reads it, exact where the counts are copied out"""
+    n = (1 << 25) // (300 - k - 1) + 2000
+    rng = np.random.default_rng(k)
+    data = fastq(np.zeros((n, 300), dtype=np.int8)) + fastq(rand_reads(rng, rng.integers(0, 4, 30_000), 6_000, 100, 0.003))
+    check(data, k, bg.thresholds([2]))
+    ref = oracle.run(data, k=k, thresh=bg.thresholds([2]), min_update=True, keep_k2=True, keep_filtered=True, threads=16)
+    assert int(ref["k2"][2].max()) > 1 << 25
+    compare(gpu_run(data, k, True, bg.thresholds([2]), True), ref)
