@@ -3410,6 +3410,10 @@ struct SkLaunch {
   uint32_t ncls;
 };
 
+/* what came of counting the partitions: done; the table is too small or the estimate was too low, to be
+ * tried again with twice as many slots; not by super-k-mers, whatever the slots */
+enum class SkCounted { DONE, AGAIN, NO };
+
 /* a block's shape in the launch's arguments */
 template <class KT>
 void sk_shaped(SkCount &a, const SkShape<KT> &s) {
@@ -3424,14 +3428,14 @@ void sk_shaped(SkCount &a, const SkShape<KT> &s) {
 constexpr uint64_t SK_PART_KMERS = 4096;
 uint64_t sk_parts_room(const Ctx *c, uint64_t n_rec) { return n_rec * (uint64_t)(c->cfg.k - MZ_M + 1) / (SK_PART_KMERS / 2); }
 
-/* The n partitions listed at `list` (superkmer.cuh, crowded partitions) by parts.  ok = false if
- * their parts do not do either, or a count that must be exact could pass what an entry holds. */
+/* The n partitions listed at `list` (superkmer.cuh, crowded partitions) by parts; NO if their parts do
+ * not do either, or a count that must be exact could pass what an entry holds. */
 template <class KT>
 bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vector<SGeom> &sg, const uint32_t *list,
-                              uint32_t n, uint64_t room, bool &ok) {
+                              uint32_t n, uint64_t room, SkCounted &out) {
   constexpr int NW = SkRec<KT>::NW;
   bruno_status st;
-  ok = false;
+  out = SkCounted::NO;
   std::vector<uint32_t> part(n);
   std::vector<uint2> rec(n);
   if ((st = ensure(c, c->sk_items, (size_t)n * sizeof(uint2))) != BRUNO_OK) return st;
@@ -3504,17 +3508,17 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
     if (left == 0 || c->hctr->err) break;
   }
   c->sk_subs = (uint32_t)subs;
-  ok = !c->hctr->err && left == 0;
+  out = c->hctr->err ? SkCounted::AGAIN : left == 0 ? SkCounted::DONE : SkCounted::NO;
   return BRUNO_OK;
 }
 
 /* The partitions counted (records in partition order), those that overflow their block's slots
  * once more with as many as fit, and those that these do not do for either, or that hold too many
- * records for one block, by parts.  ok = false: the table or the parts are too small, or so many
- * overflow that the estimate must have been too low (and `retry` is left). */
+ * records for one block, by parts.  AGAIN: the table is too small, or so many overflow that the
+ * estimate must have been too low (and `retry` is left). */
 template <class KT>
 bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector<SkLaunch<KT>> &launches,
-                            const std::vector<SGeom> &sg, uint64_t room, bool retry, bool &ok) {
+                            const std::vector<SGeom> &sg, uint64_t room, bool retry, SkCounted &out) {
   bruno_status st;
   uint32_t round = 128;
   c->sk_subs = 0;
@@ -3544,12 +3548,12 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     const uint32_t crowded = (uint32_t)c->hctr->n_over;
     if (crowded && !c->hctr->err) {
-      ok = false;
+      out = SkCounted::AGAIN;
       if (retry && crowded > parts / 2) return BRUNO_OK;
-      return sk_count_crowded<KT>(c, a, parts, sg, b.over, crowded, room, ok);
+      return sk_count_crowded<KT>(c, a, parts, sg, b.over, crowded, room, out);
     }
   }
-  ok = !c->hctr->err && c->hctr->n_over == 0;
+  out = c->hctr->err ? SkCounted::AGAIN : SkCounted::DONE;
   return BRUNO_OK;
 }
 
@@ -3711,10 +3715,10 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
         return st;
       for (size_t l = 0; l < launches.size(); ++l) launches[l].cls = (const ClassRun *)c->grp_tmp.p + at[l];
     }
-    bool ok = false;
-    if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, sg, room, attempt < 2, ok)) != BRUNO_OK) return st;
-    if (c->hctr->err & DERR_SKEW) return BRUNO_OK;
-    if (ok) {
+    SkCounted counted;
+    if ((st = sk_count_parts<KT>(c, a, (uint32_t)parts, launches, sg, room, attempt < 2, counted)) != BRUNO_OK) return st;
+    if ((c->hctr->err & DERR_SKEW) || counted == SkCounted::NO) return BRUNO_OK;
+    if (counted == SkCounted::DONE) {
       std::vector<uint64_t> taken(S, c->hctr->sk_bump);
       if (S > 1) {
         cudaMemcpyAsync(taken.data(), c->sk_bump.p, (size_t)S * 8, cudaMemcpyDeviceToHost, c->stream);
