@@ -3559,7 +3559,8 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
 
 /* The count by super-k-mers of the extracted records (one sample, or a batch's), kev[0] recorded
  * before the extraction.  used = false (nothing counted, the caller takes the k-mer records): 2^32
- * records, 2^26 in one bin, or partitions whose parts overflow too at every size tried.
+ * records, 2^26 in one bin, a table of 2^32 slots or more than fits the device (the k-mer records' own
+ * estimate may be lower), or partitions whose parts overflow too at every size tried.
  * max_split: the partition plan's split bits.  again(records): the extraction once more, with room
  * for that many records (133M records: 5 ms, where the k-mer records take 48). */
 constexpr double SK_MAX_KMERS = 3500.0;   /* k-mers of a partition, on average, that fit the largest block twice over */
@@ -3598,6 +3599,9 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
   for (uint32_t q = 0; q < S; ++q)
     distinct[q] = S > 1 ? hll_estimate(hs[q], zeros_word(zeros + 4 * q), c->sk_q[q])
                         : hll_estimate(c->hctr->hll_sum, c->hctr->hll_zeros, c->sk_q[0]);
+  /* the estimate samples minimizers: one that many places share counts for all like it, so that it can
+   * be far too high where such a one is in the sample (there are no more k-mers than occurrences) */
+  for (uint32_t q = 0; q < S; ++q) distinct[q] = std::min(distinct[q], (double)(S > 1 ? c->h_inst[q] : inst));
   const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
   const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
   for (int attempt = 0; attempt < 3; ++attempt) {
@@ -3629,9 +3633,8 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
       parts += n;
       bin0 += 1u << c->sk_bits[q];
     }
-    if (parts >> 31) return BRUNO_OK;
-    if ((st = table_room(c, base)) != BRUNO_OK) return st;
-    if ((st = ensure(c, c->table, base * SU * 8)) != BRUNO_OK) return st;
+    if (parts >> 31 || base >> 32) return BRUNO_OK;
+    if ((st = ensure(c, c->table, base * SU * 8)) != BRUNO_OK) return st == BRUNO_ERR_OOM ? BRUNO_OK : st;
     /* one call: the count makes the nodes, and lists them; a kept k-mer takes inv_load slots */
     const bool nodes = sk_makes_nodes(c);
     const uint64_t list_cap = (uint64_t)((double)base / inv_load) + 1;
@@ -3977,6 +3980,14 @@ bruno_status build_k1w_table(Ctx *c) {
   return set_err(c, BRUNO_ERR_TABLE_FULL, "(k+1)-mer table full after regrowth");
 }
 
+/* the k-mer records take over: their buffers may need the room */
+void sk_release(Ctx *c) {
+  for (Buf *b : {&c->sk_recs, &c->sk_sorted, &c->sk_kmers}) {
+    if (b->p) cudaFreeAsync(b->p, c->stream);
+    *b = Buf{};
+  }
+}
+
 template <class KT>
 bruno_status count_paths(Ctx *c) {
   if (c->sk_on) {
@@ -3984,6 +3995,7 @@ bruno_status count_paths(Ctx *c) {
     bruno_status st = count_one_superkmers<KT>(c, used);
     if (st != BRUNO_OK || used) return st;
     c->have_cand = false;
+    sk_release(c);
   }
   if (c->cfg.edge_filter && sizeof(KT) == 16) {   /* k > 31: the 128-bit (k+1)-mer table, partitioned count */
     bruno_status st = build_k1w_table(c);
@@ -4248,6 +4260,7 @@ bruno_status run_count_samples(Ctx *c) {
     };
     if ((st = count_superkmers<KW1>(c, MAX_SPLIT_BITS, again, used)) != BRUNO_OK || used) return st;
     clear();
+    sk_release(c);
   }
   c->sk_on = false;
   c->sk_gaps.clear();

@@ -1,6 +1,9 @@
 """Super-k-mer builds where an input outgrows what its plan foresaw, against the oracle and against the
 plain build: more records than their room, cycles within one block of chain nodes, pointers that disagree,
 partitions with more k-mers or records than a block counts."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -9,6 +12,7 @@ from helpers import assert_same, chain_set, compress_ranked, sort_nodes, sort_ra
 from oracle import oracle
 from test_gpu_batch import batch, plain, same_as_plain
 from test_gpu_parity import compare, gpu_run
+from test_gpu_superkmers import low_mmer
 
 pytestmark = pytest.mark.gpu
 
@@ -205,3 +209,39 @@ def test_a_count_past_what_a_block_may_hold(k):
     ref = oracle.run(data, k=k, thresh=bg.thresholds([2]), min_update=True, keep_k2=True, keep_filtered=True, threads=16)
     assert int(ref["k2"][2].max()) > 1 << 25
     compare(gpu_run(data, k, True, bg.thresholds([2]), True), ref)
+
+
+ESTIMATE = r"""
+import numpy as np, torch
+import bruno_gb300 as bg
+c = np.load("{reads}")
+name = b"@" + b"r" * 10000
+data = b"".join(name + b"\n" + r.tobytes() + b"\n+\n" + b"I" * len(r) + b"\n" for r in c)
+torch.zeros(1, device="cuda")
+before = torch.cuda.mem_get_info()[0]
+with bg.Graph(k=31, thresh=bg.thresholds([2]), min_update=True) as g:
+    g.build_and_compact(data)
+    print(g.sizes()["n_instances"], (before - torch.cuda.mem_get_info()[0]) >> 20)
+"""
+
+
+def test_estimate_with_a_crowded_minimizer_in_its_sample(tmp_path):
+    """the distinct estimate samples one minimizer in 32 of a 61 MB input; with 6000 places on one that is
+    in the sample it comes to 3.8M, but the table is planned for no more than the 0.63M k-mers there are
+    (the build then holds some 200 MB, 210 MB less than with slots for the estimate)"""
+    rng = np.random.default_rng(2)
+    pack = lambda v: int("".join(f"{int(x):02b}" for x in v), 2)
+    while True:   # an M-mer of a small order whose bin bits end in five zeros (kmer.cuh mz_order, mz_mix)
+        fwd = np.array(["ACGT".index(c) for c in low_mmer(int(rng.integers(1 << 30)))])
+        h = ((min(pack(fwd), pack(3 - fwd[::-1])) ^ 0x2C9277B5) * 0x9E3779B1 & 0xFFFFFFFE) >> 1
+        h = h * 0xC2B2AE35 & 0xFFFFFFFF
+        h = (h ^ (h >> 15)) * 0x27D4EB2F & 0xFFFFFFFF
+        if (h ^ (h >> 16)) & 31 == 0:
+            break
+    c = rng.integers(0, 4, (6000, 135))
+    c[:, 60:75] = fwd
+    np.save(tmp_path / "reads.npy", ACGT[c])
+    r = subprocess.run([sys.executable, "-c", ESTIMATE.format(reads=tmp_path / "reads.npy")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    instances, held = (int(x) for x in r.stdout.split())
+    assert instances == 6000 * 105 and held < 300, held
