@@ -26,6 +26,7 @@
 #include <cstddef>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "table_plan.h"
 #include "internal.cuh"
@@ -3206,21 +3207,20 @@ bool sk_makes_nodes(const Ctx *c) { return c->one_call && !c->cfg.keep_k2 && !c-
  * record; a forced counting path or table size keeps the k-mer records.  The (k+1)-mer filter drops
  * edges before anything is counted, so only a count that makes the nodes can do without them in the
  * table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33 by
- * a table of (k+1)-mers); a read of exactly k + 1 bases has a (k+1)-mer and no k-mer, and such an
- * input goes by the table. */
+ * a table of (k+1)-mers). */
 bool sk_takes(const Ctx *c) {
   return c->cfg.k >= MZ_M + 4 && (!c->cfg.edge_filter || sk_makes_nodes(c)) && c->force_direct_count == 0 &&
          c->cfg.table_slots == 0;
 }
 
-template <class KT, int BL>
+template <class KT, int BL, bool EDGES>
 void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                unsigned long long *s_inst, unsigned long long *s_used) {
   constexpr size_t smem = sizeof(SkWarp<SkRec<KT>::NW>) * (SK_TPB / 32);
   static const int occ = [] {
-    cudaFuncSetAttribute(k_sk_extract<KT, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_sk_extract<KT, BL, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int o = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sk_extract<KT, BL>, SK_TPB, smem) == cudaSuccess && o > 0
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sk_extract<KT, BL, EDGES>, SK_TPB, smem) == cudaSuccess && o > 0
                ? o : 4;
   }();
   const uint64_t most = (r1 - r0 + 31) / 32;   /* a few reads a warp at least */
@@ -3234,7 +3234,6 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t
   a.s0 = s0;
   a.n_first = n_first;
   a.k = c->cfg.k;
-  a.skew_len = c->cfg.edge_filter ? (uint32_t)c->cfg.k + 1 : ~0u;
   a.chunk = c->sk_chunk;
   a.samples = (const SkSample *)c->sk_samp.p;
   a.out = (uint64_t *)c->sk_recs.p;
@@ -3245,22 +3244,27 @@ void sk_launch(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t
   a.s_inst = s_inst;
   a.s_used = s_used;
   a.ctr = c->dctr;
-  k_sk_extract<KT, BL><<<(unsigned)grid, SK_TPB, smem, c->stream>>>(a);
+  k_sk_extract<KT, BL, EDGES><<<(unsigned)grid, SK_TPB, smem, c->stream>>>(a);
   c->launches += 1;
 }
-template <class KT>
-void sk_launch_k(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
+template <bool EDGES>
+void sk_launch_w1(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                  unsigned long long *s_inst, unsigned long long *s_used) {
   const int w1 = c->cfg.k - MZ_M;   /* the window blocks: the largest that no window fits inside */
-  if (w1 >= 16) sk_launch<KT, 16>(c, r0, r1, first, s0, n_first, s_inst, s_used);
-  else if (w1 >= 8) sk_launch<KT, 8>(c, r0, r1, first, s0, n_first, s_inst, s_used);
-  else sk_launch<KT, 4>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  if (w1 >= 16) sk_launch<KW1, 16, EDGES>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  else if (w1 >= 8) sk_launch<KW1, 8, EDGES>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+  else sk_launch<KW1, 4, EDGES>(c, r0, r1, first, s0, n_first, s_inst, s_used);
 }
 void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_t s0, uint32_t n_first,
                 unsigned long long *s_inst, unsigned long long *s_used) {
   if (r1 == r0) return;
-  if (c->W == 1) sk_launch_k<KW1>(c, r0, r1, first, s0, n_first, s_inst, s_used);
-  else sk_launch<KW2, 16>(c, r0, r1, first, s0, n_first, s_inst, s_used);   /* k > 31: windows of 18 and more */
+  auto by_edges = [&](auto edges) {
+    constexpr bool EDGES = decltype(edges)::value;
+    if (c->W == 1) sk_launch_w1<EDGES>(c, r0, r1, first, s0, n_first, s_inst, s_used);
+    else sk_launch<KW2, 16, EDGES>(c, r0, r1, first, s0, n_first, s_inst, s_used);   /* k > 31: windows of 18 and more */
+  };
+  if (c->cfg.edge_filter) by_edges(std::true_type{});
+  else by_edges(std::false_type{});
 }
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, 0, nullptr, nullptr); }
 
@@ -3601,7 +3605,8 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
                         : hll_estimate(c->hctr->hll_sum, c->hctr->hll_zeros, c->sk_q[0]);
   /* the estimate samples minimizers: one that many places share counts for all like it, so that it can
    * be far too high where such a one is in the sample (there are no more k-mers than occurrences) */
-  for (uint32_t q = 0; q < S; ++q) distinct[q] = std::min(distinct[q], (double)(S > 1 ? c->h_inst[q] : inst));
+  const uint64_t placed = inst + c->hctr->n_sk_edges;   /* k-mer occurrences in the records (one sample) */
+  for (uint32_t q = 0; q < S; ++q) distinct[q] = std::min(distinct[q], (double)(S > 1 ? c->h_inst[q] : placed));
   const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
   const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
   for (int attempt = 0; attempt < 3; ++attempt) {
@@ -3611,7 +3616,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
     uint64_t base = 0, parts = 0, before = 0;
     uint32_t bin0 = 0;
     for (uint32_t q = 0; q < S; ++q) {
-      const uint64_t slots = slots_for(c, distinct[q]), n_inst = S > 1 ? c->h_inst[q] : inst;
+      const uint64_t slots = slots_for(c, distinct[q]), n_inst = S > 1 ? c->h_inst[q] : placed;
       /* the fewest partitions of the configured slots, but four bins to a partition at least: a bin
        * holds a few minimizers' k-mers, and partitions of one bin are so uneven that most are counted
        * twice (k = 63, 3.5G k-mers, 2^21 partitions of 2^21 bins: 211 ms of counting; 2^20 of 2^22: 84).

@@ -29,6 +29,7 @@ struct DevCounters {
   unsigned long long bad_line;         /* first malformed line, ~0 if none */
   unsigned long long n_records;
   unsigned long long n_sk, n_sk_est;   /* super-k-mer record places taken, records listed for the estimate */
+  unsigned long long n_sk_edges;       /* k-mers of reads of k + 1 bases, under the (k+1)-mer filter */
   unsigned long long n_instances, n_reads_used;
   double hll_sum;                      /* one sample's HyperLogLog registers: sum of 2^-register, ... */
   unsigned int hll_zeros, hll_pad;     /* ... registers at zero */

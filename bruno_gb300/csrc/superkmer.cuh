@@ -39,7 +39,29 @@ template <> struct SkRec<KW2> { static constexpr int NW = 4; };
 constexpr uint64_t SK_LEFT = 1ull << 6, SK_RIGHT = 1ull << 7;
 constexpr int SK_BIN_SHIFT = 8, SK_BIN_BITS = 22;
 constexpr uint64_t SK_BIN_MASK = (1ull << SK_BIN_BITS) - 1;
-__device__ __forceinline__ unsigned sk_n(uint64_t last) { return (unsigned)(last & 63u) + 1u; }
+/* A read of k + 1 bases has a (k+1)-mer and no (k+2)-mer: under the (k+1)-mer filter its two k-mers
+ * are one or two records of n = 2 or 1 whose low bits are SK_EDGE + n: their occurrences count for the
+ * edge between them, and for no biedge (EDGES: there can be such records) */
+constexpr unsigned SK_EDGE = 60;
+template <bool EDGES = true>
+__device__ __forceinline__ unsigned sk_n(uint64_t last) {
+  const unsigned x = (unsigned)(last & 63u);
+  return EDGES && x > SK_EDGE ? x - SK_EDGE : x + 1u;
+}
+template <bool EDGES = true>
+__device__ __forceinline__ bool sk_edge(uint64_t last) { return EDGES && (last & 63u) > SK_EDGE; }
+/* the entry codes of such an edge, the ones that no (k+2)-mer has: 1 (neither base), 0 and 26..31 */
+__device__ __forceinline__ unsigned sk_edge_code(unsigned in5, unsigned out5) {
+  const unsigned x = in5 ? in5 - 1u : out5 + 3u;
+  return x < 2u ? x : x + 24u;
+}
+__device__ __forceinline__ bool sk_edge_bases(unsigned code, unsigned &in5, unsigned &out5) {
+  if (code >= 2u && code < 26u) return false;
+  const unsigned x = code < 2u ? code : code - 24u;
+  in5 = x < 4u ? x + 1u : 0u;
+  out5 = x < 4u ? 0u : x - 3u;
+  return true;
+}
 
 /* a sample's minimizer bins: bin0 + (mz_mix >> shift); the k-mers of records whose mix has no
  * bit of smask feed the estimate */
@@ -99,7 +121,7 @@ __device__ __forceinline__ uint32_t rev_pairs32(uint32_t x) {
   return ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
 }
 
-/* no record: the unused end of a chunk that a warp reserved (n - 1 is at most 48) */
+/* no record: the unused end of a chunk that a warp reserved (n - 1 is at most 48, SK_EDGE + n at most 62) */
 constexpr uint64_t SK_NONE = 63;
 
 /* HyperLogLog registers fed with the k-mers of the records listed; registers are read before they
@@ -140,7 +162,6 @@ struct SkExtract {
   const uint64_t *first;            /* a batch: the first read (from r0 on) of samples s0, s0 + 1, ... */
   uint32_t s0, n_first;
   int k;
-  uint32_t skew_len;                /* a read of this length: the input is counted another way (~0: none) */
   uint32_t chunk;                   /* output records a warp reserves at once */
   const SkSample *samples;
   uint64_t *out;
@@ -163,8 +184,9 @@ struct SkExtract {
  * warp: with one tile a block of 256 threads the block's barriers cost a quarter of its time (6.4 ms
  * at 1.2G k-mers, now 4.9).  Bound by issue (0.64 of the SMs' peak, 133 instructions a k-mer); four
  * blocks an SM instead of three spill (5.2 ms).  Output places come in chunks that a warp reserves (one counter
- * cannot take an atomic per tile); a chunk's unused end is marked SK_NONE. */
-template <class KT, int BL>
+ * cannot take an atomic per tile); a chunk's unused end is marked SK_NONE.  EDGES: the (k+1)-mer
+ * filter's, with reads of k + 1 bases (as a switch it cost the others 2%). */
+template <class KT, int BL, bool EDGES>
 __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
   constexpr int NW = SkRec<KT>::NW, NB = 16 / BL, PAD = sk_pad<NW>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -196,7 +218,7 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
       if (lo + 1 < a.n_first) n_reads = (uint32_t)(min(end, __ldg(a.first + lo + 1)) - pos);
     }
     pos += n_reads;
-    unsigned inst = 0, used = 0;
+    unsigned inst = 0, used = 0, edges = 0;   /* edges: k-mers of reads of k + 1 bases */
     uint64_t sp = 0;           /* the read ra + lane */
     uint32_t len = 0;
     if (lane < n_reads) { sp = a.rstart[ra + lane]; len = (uint32_t)(a.rend[ra + lane] - sp); }
@@ -231,7 +253,7 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
         q0 += n;
         if (!long_ok || q0 >= nk) q0 = 0; else reads = 0;
       } else {
-        const uint32_t L = len >= (uint32_t)k + 2 ? min(len, 16u * SK_WORDS + 1) : 0u;
+        const uint32_t L = len >= (uint32_t)k + (EDGES ? 1 : 2) ? min(len, 16u * SK_WORDS + 1) : 0u;
         const uint32_t nw = (L + 15) >> 4;
         uint32_t x = nw;
         #pragma unroll
@@ -242,7 +264,6 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
         /* x never falls, so the reads that fit come first */
         const bool fits = lane < n_reads && x <= SK_WORDS, kept = fits && nw;
         const unsigned mf = __ballot_sync(~0u, fits), mk = __ballot_sync(~0u, kept);
-        if (fits && len == a.skew_len) atomicOr(&a.ctr->err, (unsigned long long)DERR_SKEW);
         reads = __popc(mf);
         n_words = mf ? __shfl_sync(~0u, x, 31 - __clz(mf)) : 0u;
         if (kept) {
@@ -324,11 +345,12 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
           st |= h[i] != prev ? 1u << i : 0u;
           prev = h[i];
         }
-        if (p0 == 0) { st |= 1u; used += !pre; }
+        const bool edge = EDGES && L == k + 1 && !pre && !post;   /* (not a piece of a longer read) */
+        if (p0 == 0) { st |= 1u; used += !pre && !edge; }
         st &= nk >= 16 ? 0xFFFFu : nk > 0 ? (1u << nk) - 1 : 0u;
         marks = st;
         if (nk >= 0 && nk < 16) marks |= 1u << nk;
-        inst += (unsigned)max(0, min(16, nk));
+        (edge ? edges : inst) += (unsigned)max(0, min(16, nk));
       }
       S.marks[lane] = marks;
       const uint32_t cnt = __popc(st);
@@ -401,7 +423,9 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
           #pragma unroll
           for (int u = 0; u < 2 * NW; ++u) v[u] &= __funnelshift_lc(0u, ~0u, (unsigned)max(0, 32 * (u + 1) - bits));
           if (!hl) v[0] &= ~0u >> 2;
-          v[2 * NW - 1] |= (bin << SK_BIN_SHIFT) | (hr ? (uint32_t)SK_RIGHT : 0u) | (hl ? (uint32_t)SK_LEFT : 0u) | (uint32_t)(n - 1);
+          const bool edge = EDGES && S.len[r] == k + 1 && !pre && !post;
+          v[2 * NW - 1] |= (bin << SK_BIN_SHIFT) | (hr ? (uint32_t)SK_RIGHT : 0u) | (hl ? (uint32_t)SK_LEFT : 0u) |
+                           (edge ? SK_EDGE + n : (uint32_t)(n - 1));
           if (o < a.cap) {
             ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(a.out + (uint64_t)o * NW);
             #pragma unroll
@@ -422,6 +446,10 @@ __global__ void __launch_bounds__(SK_TPB, 3) k_sk_extract(SkExtract a) {
       }
     }
     const unsigned long long iw = warp_sum(inst), uw = warp_sum(used);
+    if (EDGES) {
+      const unsigned long long ew = warp_sum(edges);
+      if (lane == 0 && ew) atomicAdd(&a.ctr->n_sk_edges, ew);
+    }
     if (lane == 0) {
       if (iw) atomicAdd(&a.ctr->n_instances, iw);
       if (uw) atomicAdd(&a.ctr->n_reads_used, uw);
@@ -904,7 +932,8 @@ __device__ __forceinline__ uint32_t sk_top20(KW2 x, int k) { return (uint32_t)KO
  * those of its (k+1)-mer: no table of (k+1)-mers.  Twice those where the (k+1)-mer is its own reverse
  * complement (both its k-mers are this one); and where the k-mer is, its out edge in b is its in edge
  * in the complement of b, seen from the other strand.  Edges outside the bounds leave the entries;
- * entries then alike are one, entries without edges none (flag 0 tallies what is left). */
+ * entries then alike are one, entries without edges none (flag 0 tallies what is left).  Edges of reads of
+ * k + 1 bases (sk_edge_bases) count for the (k+1)-mers alone. */
 template <class KT, bool EF>
 __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key, const SkCount &a, uint64_t *pw,
                                        uint32_t &few, unsigned int *hist) {
@@ -929,7 +958,9 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
         const uint32_t w = (uint32_t)(x >> (32 * z));
         if (w == 0) continue;
         const uint32_t c = sk_count_of(w), half = (c + 1) >> 1;
-        const unsigned code = entry_code(w), in5 = code_in5(code), out5 = code_out5(code);
+        const unsigned code = entry_code(w);
+        unsigned in5 = code_in5(code), out5 = code_out5(code);
+        if (EF) sk_edge_bases(code, in5, out5);
         kf += c;
         const uint32_t vi = !EF && oddk && high && !kpal && last == 4u - in5 ? half : c;
         const uint32_t vo = !EF && oddk && low && !kpal && first == 4u - out5 ? half : c;
@@ -962,6 +993,7 @@ __device__ __forceinline__ int sk_node(const SkSlots<KT> &sl, uint32_t q, KT key
       const unsigned code = entry_code(w);
       unsigned in5 = code_in5(code), out5 = code_out5(code), f = 0;
       if (EF) {
+        if (sk_edge_bases(code, in5, out5)) continue;
         if (!((ok << 1) >> in5 & 1u)) in5 = 0;
         if (!((ok >> 3) >> out5 & 1u)) out5 = 0;
         if (in5 == 0 && out5 == 0) continue;
@@ -1037,8 +1069,9 @@ __device__ __forceinline__ void sk_merge(const uint64_t *s_rec, uint32_t *s_wt, 
 }
 
 /* lex_less: the smaller strand's biedge, reverse-complemented on a flip */
-__device__ __forceinline__ unsigned sk_code(bool fwd, unsigned in5, unsigned out5) {
-  return fwd ? biedge_code(in5, out5) : biedge_code(out5 ? 5u - out5 : 0u, in5 ? 5u - in5 : 0u);
+__device__ __forceinline__ unsigned sk_code(bool fwd, unsigned in5, unsigned out5, bool edge) {
+  const unsigned in = fwd ? in5 : out5 ? 5u - out5 : 0u, out = fwd ? out5 : in5 ? 5u - in5 : 0u;
+  return edge ? sk_edge_code(in, out) : biedge_code(in, out);
 }
 
 /* ------------------------------------------------------------ crowded partitions
@@ -1083,7 +1116,7 @@ __global__ void __launch_bounds__(256) k_sk_expand(const uint64_t *recs, const S
       const unsigned c = d < n_out ? sk_base<NW>(w, d + k + 1) : 0u;
       const bool fwd = KOps<KT>::lt(f, r);
       const KT key = fwd ? f : r;
-      const uint32_t fresh = (sk_code(fwd, in5, d < n_out ? c + 1u : 0u) << E_CODE_SHIFT) | weight;
+      const uint32_t fresh = (sk_code(fwd, in5, d < n_out ? c + 1u : 0u, sk_edge(last)) << E_CODE_SHIFT) | weight;
       in5 = KOps<KT>::first(f, k) + 1u;
       f = KOps<KT>::append(f, c, k);
       r = KOps<KT>::prepend(3u - c, r, k);
@@ -1172,7 +1205,7 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     /* the distinct records' k-mers as items of SK_ITEM */
     for (uint32_t i0 = 0; i0 < nr; i0 += nt) {
       const uint32_t i = i0 + tid;
-      const unsigned n = i < nr && s_wt[i] ? sk_n(s_rec[(size_t)i * NW + NW - 1]) : 0u;
+      const unsigned n = i < nr && s_wt[i] ? sk_n<EF>(s_rec[(size_t)i * NW + NW - 1]) : 0u;
       const uint32_t ni = (n + SK_ITEM - 1) / SK_ITEM;
       uint32_t x = ni;
       #pragma unroll
@@ -1194,8 +1227,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
       const int o0 = SK_ITEM * (int)(it >> 10);
       const uint64_t *w = s_rec + (size_t)id * NW;
       const uint64_t last = w[NW - 1];
-      const int nk = (int)sk_n(last), n = has ? min(nk - o0, SK_ITEM) : 0;
-      const uint32_t weight = s_wt[id] << E_COUNT_SHIFT;
+      const int nk = (int)sk_n<EF>(last), n = has ? min(nk - o0, SK_ITEM) : 0;
+      const uint32_t weight = (s_wt[id] << E_COUNT_SHIFT) | (sk_edge<EF>(last) ? 1u : 0u);   /* (lowest bit: an edge) */
       KT f = KOps<KT>::extract(w, o0 + 1, k), r = KOps<KT>::rc(f, k);
       /* in5, out5 of the k-mers: the base before (0: none), then the bases after from the top of `next` */
       unsigned in5 = o0 > 0 || (last & SK_LEFT) ? sk_base<NW>(w, o0) + 1u : 0u;
@@ -1209,8 +1242,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
         next <<= 2;
         const bool fwd = KOps<KT>::lt(f, r);
         const KT key = fwd ? f : r;
-        const unsigned code = sk_code(fwd, in5, out5);
-        const uint32_t fresh = (code << E_CODE_SHIFT) | weight;
+        const unsigned code = sk_code(fwd, in5, out5, EF && (weight & 1u));
+        const uint32_t fresh = (code << E_CODE_SHIFT) | (weight & ~1u);
         in5 = KOps<KT>::first(f, k) + 1u;
         f = KOps<KT>::append(f, c, k);
         r = KOps<KT>::prepend(3u - c, r, k);

@@ -1,6 +1,6 @@
 """Super-k-mer builds where an input outgrows what its plan foresaw, against the oracle and against the
 plain build: more records than their room, cycles within one block of chain nodes, pointers that disagree,
-partitions with more k-mers or records than a block counts."""
+partitions with more k-mers or records than a block counts, reads of k + 1 bases under the (k+1)-mer filter."""
 import subprocess
 import sys
 
@@ -245,3 +245,32 @@ def test_estimate_with_a_crowded_minimizer_in_its_sample(tmp_path):
     assert r.returncode == 0, r.stderr
     instances, held = (int(x) for x in r.stdout.split())
     assert instances == 6000 * 105 and held < 300, held
+
+
+# ------------------------------------------------------------------ reads of k + 1 bases under the (k+1)-mer filter
+def trimmed(codes, lens):
+    return b"".join(b"@r\n" + ACGT[c[:n]].tobytes() + b"\n+\n" + b"I" * int(n) + b"\n" for c, n in zip(codes, lens))
+
+
+@pytest.mark.parametrize("share", [0.002, 0.3, 1.0])
+@pytest.mark.parametrize("k", [19, 22, 31, 32, 45, 63])
+def test_edge_filter_with_reads_of_k_plus_1_bases(k, share):
+    """reads cut to k + 1 bases beside longer ones, few, many or all: their (k+1)-mers decide which edges
+    the others keep; homopolymers and palindromes among them"""
+    rng = np.random.default_rng(k)
+    genome = rng.integers(0, 4, 3000)
+    half = rng.integers(0, 4, (k + 1) // 2)
+    genome[500:500 + 2 * len(half)] = np.concatenate([half, 3 - half[::-1]])
+    genome[900:960] = 0
+    c = rand_reads(rng, genome, 4000, 100, 0.01)
+    lens = np.where(rng.random(4000) < share, k + 1, rng.integers(k, 101, 4000))
+    data = trimmed(c, lens)
+    for lo, hi in ((2, 65536), (4, 65536), (2, 12)):
+        check(data, k, np.array([0, 65536, lo, hi, 0, 65536], dtype=np.uint64), edge_filter=True)
+
+
+def test_edge_filter_with_crowded_reads_of_k_plus_1_bases():
+    rng = np.random.default_rng(4)
+    c = crowded_reads("adapter", 5)
+    data = trimmed(c, np.where(rng.random(len(c)) < 0.2, 32, 100)) + trimmed(np.zeros((40_000, 32), dtype=int), [32] * 40_000)
+    check(data, 31, bg.thresholds([3]), edge_filter=True)
