@@ -3208,9 +3208,15 @@ bool sk_makes_nodes(const Ctx *c) { return c->one_call && !c->cfg.keep_k2 && !c-
  * edges before anything is counted, so only a count that makes the nodes can do without them in the
  * table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33 by
  * a table of (k+1)-mers). */
+uint64_t sk_room(const Ctx *c, uint64_t total, uint32_t &chunk);
 bool sk_takes(const Ctx *c) {
-  return c->cfg.k >= MZ_M + 4 && (!c->cfg.edge_filter || sk_makes_nodes(c)) && c->force_direct_count == 0 &&
-         c->cfg.table_slots == 0;
+  if (c->cfg.k < MZ_M + 4 || (c->cfg.edge_filter && !sk_makes_nodes(c)) || c->force_direct_count != 0 ||
+      c->cfg.table_slots != 0)
+    return false;
+  uint64_t bytes = 0;   /* record places have 32 bits: known from the bytes, before anything is extracted */
+  for (auto &sg : c->segs) bytes += sg.n;
+  uint32_t chunk;
+  return sk_room(c, bytes, chunk) >> 32 == 0;
 }
 
 template <class KT, int BL, bool EDGES>
@@ -3268,16 +3274,28 @@ void sk_extract(Ctx *c, uint64_t r0, uint64_t r1, const uint64_t *first, uint32_
 }
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1) { sk_extract(c, r0, r1, nullptr, 0, 0, nullptr, nullptr); }
 
-/* Room for the records of samples of the given FASTQ bytes, their bins and their estimates.  A
- * read's quality line is mostly as long as its sequence, so k-mer positions are about half the bytes;
- * runs start at 2 / (w + 1) of them (w m-mers a window) and at every read, and get a quarter
- * more.  Input that needs more (short quality lines, repeats whose minimizers change often) is
- * extracted once more, with room for the `records` places that the first time counted.  About 512
- * k-mers a bin: a partition, some thousands of k-mers, is then made up of enough bins to even out. */
+/* Room for the records of `total` FASTQ bytes.  A read's quality line is mostly as long as its
+ * sequence, so k-mer positions are about half the bytes; runs start at 2 / (w + 1) of them (w m-mers a
+ * window) and at every read, and get a quarter more.  Input that needs more (short quality lines,
+ * repeats whose minimizers change often) is extracted once more, with room for what the first time
+ * counted. */
+uint64_t sk_room(const Ctx *c, uint64_t total, uint32_t &chunk) {
+  const int k = c->cfg.k, w = k - MZ_M + 1;
+  /* a warp reserves output places by the chunk: an eighth of its share of the records, so that the
+   * last chunks' unused places stay few */
+  const double recs = (double)total * 0.5 * 2.5 / (w + 1);
+  const uint64_t warps = (uint64_t)num_sms() * 64;
+  chunk = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, (uint64_t)(recs / (8.0 * warps))));
+  /* one extraction launch a segment, each with chunks of its own */
+  return (uint64_t)recs + total / (2 * k + 9) + 4096 + warps * chunk * std::max<size_t>(1, c->segs.size());
+}
+
+/* Buffers for samples of the given FASTQ bytes (or for `records` records), their bins and their
+ * estimates.  About 512 k-mers a bin: a partition, some thousands of k-mers, is then made up of enough
+ * bins to even out. */
 bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t records) {
   bruno_status st;
   const uint32_t S = (uint32_t)bytes.size();
-  const int k = c->cfg.k, w = k - MZ_M + 1;
   uint64_t total = 0;
   /* the estimate is made from about 2^20 k-mers, in a batch 2^17 each */
   const int sample_bits = S == 1 ? 21 : 18;
@@ -3299,14 +3317,8 @@ bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t recor
     for (int &b : c->sk_bits) b = std::max(4, b - 1);   /* 2^14 samples of 2^4 bins still fit */
   }
   c->sk_bins = (uint32_t)bins;
-  /* a warp reserves output places by the chunk: an eighth of its share of the records, so that the
-   * last chunks' unused places stay few */
-  const double recs = (double)total * 0.5 * 2.5 / (w + 1);
-  const uint64_t warps = (uint64_t)num_sms() * 64;
-  c->sk_chunk = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, (uint64_t)(recs / (8.0 * warps))));
-  /* one extraction launch a segment, each with chunks of its own */
-  c->sk_cap = (uint64_t)recs + total / (2 * k + 9) + 4096 + warps * c->sk_chunk * std::max<size_t>(1, c->segs.size());
-  if (records) c->sk_cap = records + warps * c->sk_chunk;
+  c->sk_cap = sk_room(c, total, c->sk_chunk);
+  if (records) c->sk_cap = records + (uint64_t)num_sms() * 64 * c->sk_chunk;
   const size_t rb = c->W == 1 ? 16 : 32;
   if ((st = ensure(c, c->sk_recs, c->sk_cap * rb)) != BRUNO_OK) return st;
   if ((st = ensure(c, c->sk_hist, bins * 8)) != BRUNO_OK) return st;
@@ -3596,7 +3608,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
     if ((st = again(n_rec)) != BRUNO_OK) return st;
     return count_superkmers<KT>(c, max_split, again, used, true);
   }
-  if (c->hctr->err || n_rec > c->sk_cap || inst >> 32 || n_rec >> 32) return BRUNO_OK;
+  if (c->hctr->err || n_rec > c->sk_cap || n_rec >> 32) return BRUNO_OK;
   c->n_instances = inst;
   c->n_reads_used = c->hctr->n_reads_used;
   const unsigned char *zeros = (const unsigned char *)(hs.data() + S);   /* S 32-bit words after the sums */
