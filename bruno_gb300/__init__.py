@@ -89,7 +89,7 @@ EXPORTS = (
     "bruno_load_fastq", "bruno_compute_biedge_freqencies", "bruno_local_insert_by_freqencies",
     "bruno_extract_chains", "bruno_list_rank", "bruno_to_compressed_chains", "bruno_build_and_compact",
     "bruno_get_sizes", "bruno_copy_k2", "bruno_copy_filtered", "bruno_copy_nodes", "bruno_copy_ranked",
-    "bruno_copy_chains", "bruno_copy_chain_edges", "bruno_copy_chain_summaries", "bruno_host_alloc", "bruno_host_free", "bruno_phase_ms",
+    "bruno_copy_chains", "bruno_copy_chain_edges", "bruno_copy_chain_summaries", "bruno_host_alloc", "bruno_host_free", "bruno_phase_ms", "bruno_counting_path",
     "bruno_count_biedges_noalloc", "bruno_pool_create", "bruno_pool_submit", "bruno_pool_wait",
     "bruno_pool_result_free", "bruno_pool_destroy", "bruno_clean_deadend_and_bubbles_naive",
     "bruno_device_results", "bruno_graph_find_if", "bruno_graph_erase_if", "bruno_graph_erase_nodes",
@@ -131,6 +131,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
         "bruno_copy_chain_summaries": [P, P, P, P, SZ, PSZ],
         "bruno_host_alloc": [SZ, ctypes.POINTER(P)], "bruno_host_free": [P],
         "bruno_phase_ms": [P, ctypes.POINTER(ctypes.c_double), SZ],
+        "bruno_counting_path": [P, ctypes.POINTER(I32), ctypes.POINTER(U64)],
         "bruno_count_biedges_noalloc": [I32, I32, P, P, SZ, P, P, P, SZ, PSZ, P],
         "bruno_pool_create": [ctypes.POINTER(_Cfg), I32, U64, ctypes.POINTER(P)],
         "bruno_pool_submit": [P, P, SZ, ctypes.POINTER(U64)],
@@ -464,6 +465,14 @@ class Graph:
         a = (ctypes.c_double * len(self.PHASES))()
         self._check(self.lib.bruno_phase_ms(self.ctx, a, len(self.PHASES)), "phase_ms")
         return dict(zip(self.PHASES, list(a)))
+
+    COUNTING_PATHS = ("none", "super_kmers", "kmer_records", "l2_partitions", "whole_table")
+
+    def counting_path(self) -> tuple[str, int]:
+        """how the last build counted (one of COUNTING_PATHS), and the records it counted"""
+        path, records = ctypes.c_int32(), ctypes.c_uint64()
+        self._check(self.lib.bruno_counting_path(self.ctx, ctypes.byref(path), ctypes.byref(records)), "counting_path")
+        return self.COUNTING_PATHS[path.value], int(records.value)
 
     def _ptr(self, a: np.ndarray):
         return a.ctypes.data_as(ctypes.c_void_p)

@@ -2778,6 +2778,11 @@ uint64_t slots_for(const Ctx *c, double distinct) {
   return (uint64_t)(distinct * 1.04 / load) + 1024;
 }
 
+void counted_by(Ctx *c, int32_t path, uint64_t records) {
+  c->count_path = path;
+  c->count_records = records;
+}
+
 /* the direct count: every instance probes the whole table (k > 31, or a degenerate input
  * whose instances crowd one hash bucket) */
 template <class KT>
@@ -2826,6 +2831,7 @@ bruno_status count_direct(Ctx *c) {
       c->n_reads_used = c->hctr->n_reads_used;
       c->n_entries = c->hctr->n_entries;
       c->n_slots_claimed = c->hctr->n_slots_claimed;
+      counted_by(c, BRUNO_COUNT_WHOLE_TABLE, 0);
       return BRUNO_OK;
     }
     slots *= 2;  /* the estimate was too low: grow and count again */
@@ -3190,6 +3196,7 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
       c->n_slots_claimed = c->hctr->n_slots_claimed;
       if (counted_local) take_candidates(c);
       else c->have_cand = false;
+      counted_by(c, counted_local ? BRUNO_COUNT_KMER_RECORDS : BRUNO_COUNT_L2_PARTITIONS, c->n_instances);
       used = true;
       return BRUNO_OK;
     }
@@ -3747,6 +3754,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
       for (uint32_t q = 0; q < S; ++q) sg[q].g.nslots = taken[q];
       c->geom = sg[0].g;
       c->nslots = S == 1 ? taken[0] : base;
+      counted_by(c, BRUNO_COUNT_SUPER_KMERS, n_rec);
       c->sk_parts = (uint32_t)parts;
       c->sk_taken = 0;
       for (uint64_t t : taken) c->sk_taken += t;
@@ -3917,6 +3925,7 @@ bruno_status count_partitioned_w2(Ctx *c, bool &used) {
       c->n_slots_claimed = c->hctr->n_slots_claimed;
       c->have_cand = ca.cand != nullptr;
       take_candidates(c);
+      counted_by(c, BRUNO_COUNT_KMER_RECORDS, c->n_instances);
       used = true;
       return BRUNO_OK;
     }
@@ -4365,6 +4374,7 @@ bruno_status run_count_samples(Ctx *c) {
     cudaEventRecord(c->kev[3], c->stream);
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     if (!(c->hctr->err & DERR_TABLE_FULL)) {
+      counted_by(c, BRUNO_COUNT_KMER_RECORDS, c->n_instances);
       c->h_sgeom = sg;
       c->n_entries = c->hctr->n_entries;
       c->n_slots_claimed = c->hctr->n_slots_claimed;

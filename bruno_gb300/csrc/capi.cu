@@ -211,6 +211,8 @@ bruno_status bruno_reset(bruno_ctx *c) {
   c->n_reads = c->n_reads_used = c->n_instances = c->n_entries = 0;
   c->n_k2 = c->n_filtered = 0;
   c->k2_dumped = false;
+  c->count_path = BRUNO_COUNT_NONE;
+  c->count_records = 0;
   c->h2d_pending = false;
   c->h2d_piped = false;
   c->host_loads = 0;
@@ -864,6 +866,13 @@ bruno_status bruno_host_alloc(size_t bytes, void **out) {
 
 bruno_status bruno_host_free(void *p) {
   if (p && cudaFreeHost(p) != cudaSuccess) { cudaGetLastError(); return BRUNO_ERR_CUDA; }
+  return BRUNO_OK;
+}
+
+bruno_status bruno_counting_path(bruno_ctx *c, int32_t *path, uint64_t *records) {
+  if (!c || !path || !records) return BRUNO_ERR_ARG;
+  *path = c->count_path;
+  *records = c->count_records;
   return BRUNO_OK;
 }
 

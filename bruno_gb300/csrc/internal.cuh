@@ -141,6 +141,8 @@ struct Ctx {
   uint64_t n_reads = 0, n_reads_used = 0, n_instances = 0;
 
   /* k-mer table */
+  int32_t count_path = 0;        /* BRUNO_COUNT_*, and the records that were counted */
+  uint64_t count_records = 0;
   Buf table;
   TableGeom geom{0, 0, 0, 0};
   uint64_t nslots = 0, n_entries = 0, n_slots_claimed = 0;

@@ -350,6 +350,14 @@ bruno_status bruno_host_free(void *p);
  * worked out here, from events that the build left: the call waits for the build's last. */
 bruno_status bruno_phase_ms(bruno_ctx *ctx, double *ms, size_t n);
 
+/* How the last build counted (bruno_cfg.direct_count says when which), and the records it counted:
+ * super-k-mer record places or k-mer records (0: none are made). */
+enum {
+  BRUNO_COUNT_NONE = 0, BRUNO_COUNT_SUPER_KMERS = 1, BRUNO_COUNT_KMER_RECORDS = 2, BRUNO_COUNT_L2_PARTITIONS = 3,
+  BRUNO_COUNT_WHOLE_TABLE = 4
+};
+bruno_status bruno_counting_path(bruno_ctx *ctx, int32_t *path, uint64_t *records);
+
 /* ---------------------------------------------------------------------------------------
  * Batched form: many samples built in one pass.  No counterpart in the reference (one graph per
  * MPI job there).  The n_samples FASTQ buffers (host memory, or device memory with is_device)

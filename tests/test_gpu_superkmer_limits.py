@@ -51,6 +51,7 @@ def check(data, k, thr, thresholding=True, **cfg):
                      edge_filter=cfg.get("edge_filter", False))
     with bg.Graph(k=k, thresholding=thresholding, thresh=thr, min_update=True, **cfg) as g:
         g.build_and_compact(data)
+        assert g.counting_path()[0] == "super_kmers"
         s = g.sizes()
         for n in SIZES:
             if n in ref:
@@ -279,7 +280,7 @@ def test_edge_filter_with_crowded_reads_of_k_plus_1_bases():
 # ------------------------------------------------------------------ more than 2^32 k-mers
 def test_more_than_2_32_kmers():
     """a 30x build of 5 Mbp whose input comes 29 times over: 4.35G k-mers, the graph of the input once with 29
-    times the counts, and no other counting path (its partitions are the plan's, not the 256 of the L2 count)"""
+    times the counts, by super-k-mers"""
     import torch
     rng = np.random.default_rng(8)
     one = fastq(rand_reads(rng, rng.integers(0, 4, 5_000_000), 1_250_000, 150, 0.005))
@@ -288,6 +289,7 @@ def test_more_than_2_32_kmers():
     def build(data, size, lower):
         with bg.Graph(k=31, thresh=bg.thresholds([lower]), min_update=True) as g:
             g.build_and_compact(data.data_ptr(), size, is_device=True)
+            assert g.counting_path()[0] == "super_kmers"
             return g.sizes(), sort_nodes(*g.nodes()), chain_set(*g.chains())
 
     a = torch.from_numpy(np.frombuffer(one, dtype=np.uint8).copy()).cuda()
@@ -300,7 +302,6 @@ def test_more_than_2_32_kmers():
     assert s["n_instances"] == n * s1["n_instances"] > 1 << 32
     for key in ("n_k2", "n_nodes", "n_branch", "n_chain_nodes", "n_chains"):
         assert s[key] == s1[key], key
-    assert s["table_partitions"] > 256
     assert_same((nodes[0], nodes[2]), (nodes1[0], nodes1[2]), "nodes")
     assert np.array_equal(nodes[1], np.minimum(65535, n * nodes1[1].astype(np.int64)).astype(nodes[1].dtype))
     assert chains == chains1
