@@ -2675,7 +2675,7 @@ bruno_status run_index_reads(Ctx *c) {
   if ((st = ensure(c, c->tile_base, std::max<uint64_t>(1, total_tiles) * 8)) != BRUNO_OK) return st;
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
-  c->sk_on = sk_takes(c) && (c->S == 1 || !c->samp_off.empty());
+  c->sk_on = sk_takes(c);
   c->pre_extracted = piped && c->S == 1 && (!c->cfg.edge_filter || c->sk_on) && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
@@ -4165,8 +4165,8 @@ __global__ void k_sample_first_read(const uint64_t *rstart, uint64_t nreads, con
 }  // namespace
 
 /* The batched form's count: S samples, concatenated in one device copy, each counted into
- * partitions of its own in one pass of every counting kernel (the plain path's kernels; the
- * plain build is a batch of one).  Needs k <= 31 and the shared-memory partitions. */
+ * partitions of its own in one pass of every counting kernel (the plain path's kernels; a batch
+ * of one sample is the plain build).  Needs k <= 31 and the shared-memory partitions. */
 namespace {
 /* The first read of each sample q in [q0, q1), among reads [r0, r1) (every read before r0 lies
  * before sample q0, every read of these samples before r1); out gets q1 - q0 + 1 values, the
@@ -4248,8 +4248,8 @@ bruno_status batch_segment(Ctx *c, size_t si, uint64_t r0, uint64_t r1) {
 }
 
 /* The batched form's count: S samples, concatenated in one device copy, each counted into
- * partitions of its own in one pass of every counting kernel (the plain path's kernels; the
- * plain build is a batch of one).  Needs k <= 31 and the shared-memory partitions. */
+ * partitions of its own in one pass of every counting kernel (the plain path's kernels; a batch
+ * of one sample is the plain build).  Needs k <= 31 and the shared-memory partitions. */
 bruno_status run_count_samples(Ctx *c) {
   bruno_status st;
   c->have_cand = c->nodes_made = false;
@@ -4261,7 +4261,7 @@ bruno_status run_count_samples(Ctx *c) {
   cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
   cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
   bool indexed = false;
-  if (S > 1 && sk_takes(c)) {   /* by super-k-mers, if the samples' minimizers allow it */
+  if (sk_takes(c)) {   /* by super-k-mers */
     std::vector<uint64_t> bytes(S);
     for (uint32_t q = 0; q < S; ++q) bytes[q] = c->samp_off[q + 1] - c->samp_off[q];
     if ((st = sk_begin(c, bytes)) != BRUNO_OK) return st;

@@ -203,6 +203,8 @@ bruno_status bruno_reset(bruno_ctx *c) {
   c->segs.clear();
   c->stage = 0;
   c->S = 1;   /* the plain build; bruno_build_samples sets a batch */
+  c->batch = false;
+  c->h_tally.clear();
   c->samp_off.clear();
   c->samp_r0.clear();
   c->batch_piped = false;
@@ -374,7 +376,7 @@ bruno_status bruno_to_compressed_chains(bruno_ctx *c) {
 
 bruno_status bruno_clean_deadend_and_bubbles_naive(bruno_ctx *c, bruno_clean_stats *stats) {
   if (!c) return BRUNO_ERR_ARG;
-  if (c->S > 1) return set_err(c, BRUNO_ERR_ARG, "graph cleaning works on one graph; build it with bruno_build_and_compact");
+  if (c->batch) return set_err(c, BRUNO_ERR_ARG, "graph cleaning works on one graph; build it with bruno_build_and_compact");
   if (c->stage < 5) return set_err(c, BRUNO_ERR_ARG, "cleaning needs ranked chains");
   if (c->cleaned) return set_err(c, BRUNO_ERR_ARG, "the graph is cleaned already; call bruno_reset first");
   bruno_clean_stats s{};
@@ -610,6 +612,31 @@ __global__ void k_gather_u64(const uint64_t *src, const uint64_t *idx, uint32_t 
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[idx[i]];
 }
 
+/* a batch of one sample is the plain build: its tallies and ranges from that build's sizes */
+static bruno_status build_one_sample(bruno_ctx *c, const char *buf, size_t nbytes, int32_t is_device) {
+  const bruno_status st = bruno_build_and_compact(c, buf, nbytes, is_device);
+  if (st != BRUNO_OK) return st;
+  c->batch = true;
+  c->samp_r0 = {0, c->n_reads};
+  c->h_inst = {c->n_instances};
+  c->h_used = {c->n_reads_used};
+  c->h_iter = {c->iterations};
+  c->h_rank0 = {0, c->n_ranked};
+  c->h_head0 = {0, c->n_heads};
+  c->h_sgeom = {SGeom{c->geom, 0, 0, 0}};
+  c->h_sgeom[0].g.nslots = c->nslots;
+  c->h_tally.assign(T_NUM, 0);
+  c->h_tally[T_ENTRIES] = c->n_entries;
+  c->h_tally[T_CHAIN] = c->n_chain;
+  c->h_tally[T_BRANCH] = c->n_branch;
+  c->h_tally[T_CYCLE] = c->n_cycle;
+  c->h_tally[T_ISOLATED] = c->n_isolated;
+  c->h_tally[T_RANKED] = c->n_ranked;
+  c->h_tally[T_HEADS] = c->n_heads;
+  c->h_tally[T_CHARS] = c->n_chain_chars;
+  return BRUNO_OK;
+}
+
 bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const size_t *nbytes, size_t n_samples,
                                  int32_t is_device) {
   if (!c || !bufs || !nbytes || n_samples == 0) return BRUNO_ERR_ARG;
@@ -622,6 +649,7 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
   if (c->cfg.thresholding && (c->cfg.thresh[0] != 0 || c->cfg.thresh[1] < 65536 || c->cfg.thresh[4] != 0 ||
                               c->cfg.thresh[5] < 65536))
     return set_err(c, BRUNO_ERR_ARG, "batch: only the (k+1)-mer bounds may be set (one -L / -U value)");
+  if (n_samples == 1) return build_one_sample(c, bufs[0], nbytes[0], is_device);
   bruno_status st = bruno_reset(c);
   if (st != BRUNO_OK) return st;
   /* one device copy of all samples, one after another; a sample whose last byte is not a newline
@@ -705,6 +733,7 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
     if (st != BRUNO_OK) return st;
   }
   c->S = (uint32_t)n_samples;
+  c->batch = true;
   c->stage = 1;
   phase_begin(c, 1);
   c->one_call = true;
@@ -756,7 +785,7 @@ bruno_status bruno_build_samples(bruno_ctx *c, const char *const *bufs, const si
 
 static bruno_status batch_sample(bruno_ctx *c, size_t sample) {
   if (!c) return BRUNO_ERR_ARG;
-  if (c->S <= 1 || c->stage < 6 || c->h_tally.empty()) return set_err(c, BRUNO_ERR_ARG, "no batch built");
+  if (!c->batch || c->stage < 6 || c->h_tally.empty()) return set_err(c, BRUNO_ERR_ARG, "no batch built");
   if (sample >= c->S) return set_err(c, BRUNO_ERR_ARG, "sample index out of range");
   return BRUNO_OK;
 }
@@ -769,7 +798,7 @@ bruno_status bruno_sample_count(bruno_ctx *c, size_t *n_samples) {
 
 bruno_status bruno_sample_ranges(bruno_ctx *c, uint64_t *ranked0, uint64_t *chains0, uint64_t *chars0) {
   if (!c) return BRUNO_ERR_ARG;
-  if (c->S <= 1 || c->stage < 6 || c->h_tally.empty()) return set_err(c, BRUNO_ERR_ARG, "no batch built");
+  if (!c->batch || c->stage < 6 || c->h_tally.empty()) return set_err(c, BRUNO_ERR_ARG, "no batch built");
   uint64_t chars = 0;
   for (uint32_t q = 0; q <= c->S; ++q) {
     if (ranked0) ranked0[q] = c->h_rank0[q];

@@ -151,6 +151,7 @@ struct Ctx {
   /* batched form: S samples, one after another in the FASTQ; per sample its byte offset in the
    * device copy (S + 1 values), first read (S + 1), table geometry and tallies */
   uint32_t S = 1;
+  bool batch = false;                      /* built by bruno_build_samples (of one sample: the plain build) */
   std::vector<uint64_t> samp_off, samp_r0;
   /* a batch copied from the host in groups of whole samples: segment i holds samples
    * [seg_samp[i], seg_samp[i + 1]), and the read index extracts each group as it lands */
