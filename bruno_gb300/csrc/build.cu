@@ -3627,6 +3627,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
   const uint64_t placed = inst + c->hctr->n_sk_edges;   /* k-mer occurrences in the records (one sample) */
   for (uint32_t q = 0; q < S; ++q) distinct[q] = std::min(distinct[q], (double)(S > 1 ? c->h_inst[q] : placed));
   const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
+  const bool all = !c->one_call || !c->cfg.thresholding || c->cfg.keep_k2;   /* every k-mer is kept */
   const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
   for (int attempt = 0; attempt < 3; ++attempt) {
     std::vector<SGeom> sg(S);
@@ -3645,8 +3646,10 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
       const int pbits = S > 1 ? pl.pbits : std::min(pl.pbits, std::max(8, c->sk_bits[q] - 2));
       const uint64_t n = 1ull << pbits;
       if (!(pl.fits || pbits < pl.pbits) || distinct[q] > SK_MAX_KMERS * (double)n) return BRUNO_OK;
-      /* a partition's slots are rounded up by two, and so are a crowded one's parts' */
-      caps[q] = slots + 2 * n + n_inst / 512;
+      /* a partition's slots are rounded up by two, and so are a crowded one's parts'; where every k-mer is
+       * kept the estimate's error comes on top (2 to 3%: a sample of minimizers, each with the k-mers of
+       * its place) */
+      caps[q] = slots + (all ? slots / 7 : 0) + 2 * n + n_inst / 512;
       sg[q].g = TableGeom{caps[q], 0, pbits, base, nullptr, nullptr, bin0, 32 - c->sk_bits[q], c->cfg.k};
       sg[q].pbase = parts;
       sg[q].rec2_base = sg[q].cap2 = 0;
@@ -3696,7 +3699,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
     a.recs = sorted;
     a.off = (const uint32_t *)c->sk_off.p;
     a.k = c->cfg.k;
-    a.keep_all = !nodes && !(c->one_call && c->cfg.thresholding && !c->cfg.keep_k2);
+    a.keep_all = !nodes && all;
     a.thresholding = c->cfg.thresholding;
     for (int i = 0; i < 6; ++i) a.t[i] = (uint32_t)std::min<uint64_t>(65536, c->cfg.thresh[i]);
     a.inv_load = inv_load;
