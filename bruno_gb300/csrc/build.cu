@@ -3210,19 +3210,28 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
 /* One call: the count makes the nodes and nobody asks for what was counted */
 bool sk_makes_nodes(const Ctx *c) { return c->one_call && !c->cfg.keep_k2 && !c->cfg.keep_filtered; }
 
+/* every k-mer is kept: the raw counts or other thresholds may still be asked for, or there are none */
+bool sk_keeps_all(const Ctx *c) { return !c->one_call || !c->cfg.thresholding || c->cfg.keep_k2; }
+
 /* k from 19: below, windows hold fewer than 5 m-mers and a run is hardly longer than a k-mer's own
- * record; a forced counting path or table size keeps the k-mer records.  The (k+1)-mer filter drops
- * edges before anything is counted, so only a count that makes the nodes can do without them in the
- * table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33 by
- * a table of (k+1)-mers). */
+ * record.  Where every k-mer is kept the count has nothing to leave out, and below k = 24 the k-mer
+ * records' shorter runs in the table win (200 kbp at 60x, steps: k = 19 1.04 ms against 1.13 by
+ * super-k-mers, 21 1.05 and 1.15, 23 1.08 and 1.12, 24 1.14 and 1.09; from 27 on with a target load of 0.7, unthresholded:
+ * 25 1.39 and 1.48, 27 1.44 and 1.40), except in small builds, which are a chain of launches (0.8 MB:
+ * 0.7 ms against 0.5).  A forced counting path or table size keeps the k-mer records.  The (k+1)-mer
+ * filter drops edges before anything is counted, so only a count that makes the nodes can do without them
+ * in the table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33
+ * by a table of (k+1)-mers). */
+constexpr uint64_t SK_SMALL = 2ull << 20;   /* bytes a sample */
 uint64_t sk_room(const Ctx *c, uint64_t total, uint32_t &chunk);
 bool sk_takes(const Ctx *c) {
-  if (c->cfg.k < MZ_M + 4 || (c->cfg.edge_filter && !sk_makes_nodes(c)) || c->force_direct_count != 0 ||
+  uint64_t bytes = 0;
+  for (auto &sg : c->segs) bytes += sg.n;
+  const int least = !sk_keeps_all(c) || bytes / c->S < SK_SMALL ? MZ_M + 4 : c->cfg.max_load > 0.6 ? 27 : 24;
+  if (c->cfg.k < least || (c->cfg.edge_filter && !sk_makes_nodes(c)) || c->force_direct_count != 0 ||
       c->cfg.table_slots != 0)
     return false;
-  uint64_t bytes = 0;   /* record places have 32 bits: known from the bytes, before anything is extracted */
-  for (auto &sg : c->segs) bytes += sg.n;
-  uint32_t chunk;
+  uint32_t chunk;   /* record places have 32 bits: known from the bytes, before anything is extracted */
   return sk_room(c, bytes, chunk) >> 32 == 0;
 }
 
@@ -3627,7 +3636,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
   const uint64_t placed = inst + c->hctr->n_sk_edges;   /* k-mer occurrences in the records (one sample) */
   for (uint32_t q = 0; q < S; ++q) distinct[q] = std::min(distinct[q], (double)(S > 1 ? c->h_inst[q] : placed));
   const double recs_per_kmer = inst ? (double)n_rec / (double)inst : 0.0;
-  const bool all = !c->one_call || !c->cfg.thresholding || c->cfg.keep_k2;   /* every k-mer is kept */
+  const bool all = sk_keeps_all(c);
   const double inv_load = std::max(1.05, std::min(SK_MAX_INV_LOAD, 1.0 / (c->cfg.max_load > 0 ? c->cfg.max_load : 0.5)));
   for (int attempt = 0; attempt < 3; ++attempt) {
     std::vector<SGeom> sg(S);

@@ -42,6 +42,24 @@ def test_path(k, cfg, want):
         assert records == 0
 
 
+@pytest.mark.parametrize("k,least", [(22, False), (23, False), (24, True), (26, True), (27, True)])
+def test_path_where_every_kmer_is_kept(k, least):
+    """steps, raw counts and unthresholded builds of more than 2 MB by k-mer records below k = 24 (27 with a
+    target load above 0.6), thresholded builds in one call and small ones by super-k-mers; the same graph"""
+    rng = np.random.default_rng(k)
+    data = fastq(rand_reads(rng, rng.integers(0, 4, 60_000), 12_000, 100, 0.005))
+    assert len(data) > 2 << 20
+    want = "super_kmers" if least else "kmer_records"
+    assert path_of(data, k)[0] == "super_kmers"
+    assert path_of(data, k, keep_k2=True)[0] == want
+    assert path_of(data, k, thresholding=False)[0] == want
+    assert path_of(data, k, thresholding=False, max_load=0.7)[0] == ("super_kmers" if k >= 27 else "kmer_records")
+    assert path_of(data[:207 * 9_000], k, thresholding=False)[0] == "super_kmers"   # (207 bytes a record)
+    thr = bg.thresholds([2])
+    ref = oracle.run(data, k=k, thresh=thr, min_update=True, threads=16, keep_k2=True, keep_filtered=True)
+    compare(gpu_run(data, k, True, thr, True), ref)
+
+
 def test_path_is_forgotten():
     with bg.Graph(k=31, thresh=bg.thresholds([2]), min_update=True) as g:
         assert g.counting_path() == ("none", 0)
