@@ -614,9 +614,14 @@ __device__ __forceinline__ uint32_t side_dist(const ChainState &s, int side) { r
  * read that gives it the next pointer.  The other half -- every chain pointer is answered by
  * the facing side of its target -- is checked by the first walk for every node it passes and
  * by the marking pass for the nodes no walk reaches. */
+/* pointers have been found inconsistent: the round-synchronous ranking will run, and what is queued up to
+ * the host's next look at the counters has nothing to do (the same for every thread of the block) */
+__device__ __forceinline__ bool fast_declined(const DevCounters *ctr) { return __syncthreads_or(ctr->lr_multi != 0); }
+
 /* n_dev: the number of nodes in device memory (segments), or NULL */
 __global__ void __launch_bounds__(TPB) k_fast_check(ChainState *cs, uint64_t M, const unsigned long long *n_dev,
                                                     const SegInfo *seg, uint32_t *rnode, DevCounters *ctr) {
+  if (fast_declined(ctr)) return;
   if (n_dev) M = *n_dev;
   unsigned long long bad = 0;
   for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < M; i0 += (uint64_t)gridDim.x * blockDim.x) {
@@ -729,6 +734,7 @@ __global__ void __launch_bounds__(TPB) k_seg_local(const ChainState *cs, uint64_
  * terminal side */
 __global__ void __launch_bounds__(TPB) k_seg_link(const ChainState *cs, const uint2 *place, const SegInfo *seg,
                                                   ChainState *rs, DevCounters *ctr) {
+  if (fast_declined(ctr)) return;
   const uint64_t n = ctr->n_seg;
   unsigned long long bad = 0;
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
@@ -765,6 +771,7 @@ __global__ void __launch_bounds__(TPB) k_seg_link(const ChainState *cs, const ui
 __global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const uint32_t *rnode, uint64_t M,
                                                     const unsigned long long *n_dev, Jump *E0, uint64_t *place,
                                                     DevCounters *ctr) {
+  if (fast_declined(ctr)) return;
   unsigned long long bad = 0;
   const uint64_t R = ctr->lr_remaining;
   if (n_dev) M = *n_dev;
@@ -803,7 +810,7 @@ __global__ void __launch_bounds__(TPB) k_fast_walk(const ChainState *cs, const u
 __global__ void __launch_bounds__(TPB) k_fast_jump(const Jump *E, Jump *F, DevCounters *ctr, int round) {
   unsigned long long undone = 0;
   const uint64_t R = ctr->lr_remaining;
-  if (round > 0 && ctr->lr_round[round - 1] == 0) return;
+  if (ctr->lr_multi || (round > 0 && ctr->lr_round[round - 1] == 0)) return;
   for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * R; q += (uint64_t)gridDim.x * blockDim.x) {
     Jump e;
     e.w = *(volatile const uint64_t *)&E[q].w;
@@ -2920,6 +2927,10 @@ static bruno_status fast_list_rank(Ctx *c, bool &used) {
   cudaMemsetAsync(&c->dctr->n_seg, 0, 8 + sizeof(c->dctr->lr_round), c->stream);
   const bool over_segs = c->geom.bins && c->cfg.rank_fill != 1 && M > 0;
   constexpr uint64_t WAIT = 4ull << 20;   /* from here on sizes are worth waiting for */
+  /* bounds on k-mers or (k+2)-mers can trim an edge on one side only: mostly found by the first check,
+   * which is then waited for (2M nodes: nine kernels with nothing to do take 0.1 ms of 3.4) */
+  const uint64_t *t = c->thr_used;
+  const bool doubtful = c->cfg.thresholding && (t[0] > 0 || t[1] <= 0xFFFF || t[4] > 0 || t[5] <= 0xFFFF);
   auto blocks = [&](uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (n + TPB - 1) / TPB)); };
   uint64_t N = M;                          /* nodes or segments ranked (segments: at most) */
   ChainState *rs = cs, *rs2 = nullptr;
@@ -2948,7 +2959,7 @@ static bruno_status fast_list_rank(Ctx *c, bool &used) {
   k_fast_check<<<blocks(N), TPB, 0, c->stream>>>(rs, N, n_dev, seg, rnode, c->dctr);
   c->launches += 1;
   uint64_t Rb = std::max<uint64_t>(1, N);   /* rulers at most */
-  if (N > WAIT) {
+  if (N > WAIT || doubtful) {
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     if (c->hctr->lr_multi != 0) return BRUNO_OK;
     Rb = std::max<uint64_t>(1, c->hctr->lr_remaining);
