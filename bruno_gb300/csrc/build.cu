@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
   const long long E = ctr->last_nonws + 1;  /* effective end (exclusive) */
   uint64_t base = tile_base[blockIdx.x];
   unsigned long long nl_eff = 0;  /* newlines ending lines before E, max over this thread */
+  unsigned long long seq = 0;     /* sequence ends less sequence starts: over all reads, their bases */
   if (blockIdx.x == 0 && threadIdx.x == 0 && E > 0 && buf[0] != '@') atomicMin(&ctr->bad_line, 0ull);
   /* stripes of TPB*64 bytes, 64 consecutive bytes per thread (four 16-byte loads in flight),
    * in byte order: one block scan per stripe */
@@ -196,11 +197,12 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
         nl_eff = ln + 1;
         const uint64_t r = ln >> 2;
         const unsigned role = (unsigned)(ln & 3);
-        if (role == 0 && rbase + r < rcap) rstart[rbase + r] = (uint64_t)(buf + p + 1);
+        if (role == 0 && rbase + r < rcap) { rstart[rbase + r] = (uint64_t)(buf + p + 1); seq -= p + 1; }
         if (role == 1 && rbase + r < rcap) {
           uint64_t e = p;
           if (e > 0 && buf[e - 1] == '\r') --e;
           rend[rbase + r] = (uint64_t)(buf + e);
+          seq += e;
         }
         /* the first byte of line ln+1 */
         const unsigned nrole = (unsigned)((ln + 1) & 3);
@@ -214,8 +216,14 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
     base += total;
   }
   __shared__ unsigned long long snl[TPB / 32];
-  for (int o = 16; o > 0; o >>= 1) nl_eff = max(nl_eff, __shfl_down_sync(~0u, nl_eff, o));
-  if ((threadIdx.x & 31) == 0) snl[threadIdx.x >> 5] = nl_eff;
+  for (int o = 16; o > 0; o >>= 1) {
+    nl_eff = max(nl_eff, __shfl_down_sync(~0u, nl_eff, o));
+    seq += __shfl_down_sync(~0u, seq, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    snl[threadIdx.x >> 5] = nl_eff;
+    if (seq) atomicAdd(&ctr->n_seq, seq);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long m = 0;
@@ -2654,6 +2662,8 @@ bruno_status extract_begin(Ctx *c, uint64_t upper, int max_blocks);
 void extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 int wx_blocks(uint64_t nr);
 bool sk_takes(const Ctx *c);
+bool sk_pays(const Ctx *c, double length);
+constexpr double BATCH_READS = 100.0;   /* a batch's choice of records comes before its reads are known */
 bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t records = 0);
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f);
@@ -2675,20 +2685,11 @@ bruno_status run_index_reads(Ctx *c) {
   if ((st = ensure(c, c->tile_base, std::max<uint64_t>(1, total_tiles) * 8)) != BRUNO_OK) return st;
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
-  c->sk_on = sk_takes(c);
-  c->pre_extracted = piped && c->S == 1 && (!c->cfg.edge_filter || c->sk_on) && c->force_direct_count != 1 && (c->W == 1 || c->sk_on);
+  c->sk_on = sk_takes(c) && (c->S == 1 || sk_pays(c, BATCH_READS));
+  c->pre_extracted = false;
+  const bool pieces = piped && c->S == 1 && c->force_direct_count != 1;
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
   cudaMemsetAsync(c->dctr, 0, offsetof(DevCounters, hll), c->stream);
-  if (c->pre_extracted) {
-    /* a record holds its sequence and, as a rule, an equally long quality line: k-mer positions are
-     * at most half the bytes (shorter quality lines are accepted too: the records may then need more
-     * room than this gives, which both extractions notice) */
-    int blocks = 0;   /* one launch a segment, bounded as extract_reads bounds it (8 bytes a read at least) */
-    for (auto &sg : c->segs) blocks += wx_blocks(sg.n / 8 + 1);
-    if ((st = c->sk_on ? sk_begin(c, {total_bytes}) : extract_begin(c, total_bytes / 2 + 1, std::max(1, blocks))) != BRUNO_OK)
-      return st;
-    cudaEventRecord(c->kev[0], c->stream);
-  }
   /* the read arrays need the record count first; newline counts give an upper bound */
   uint64_t rcap = 0;
   for (size_t si = 0; si < c->segs.size(); ++si) {
@@ -2714,7 +2715,7 @@ bruno_status run_index_reads(Ctx *c) {
     }
     /* grow keeping the spans of earlier files; pieces of one input grow once, for all pieces
      * at the first piece's records per byte */
-    if ((c->pre_extracted || batch_hook) && si == 0 && sg.n > 0)
+    if ((pieces || batch_hook) && si == 0)
       upper = std::max<uint64_t>(upper, (uint64_t)((double)upper * (double)total_bytes / (double)sg.n * 1.05) + 1);
     if ((st = ensure(c, c->rstart, (rcap + upper) * 8, true)) != BRUNO_OK) return st;
     if ((st = ensure(c, c->rend, (rcap + upper) * 8, true)) != BRUNO_OK) return st;
@@ -2729,12 +2730,27 @@ bruno_status run_index_reads(Ctx *c) {
     if (h.bad_line != ~0ull || (lines & 3) != 0)
       return set_err(c, BRUNO_ERR_BAD_INPUT, "malformed FASTQ in file " + std::to_string(si) + " near line " +
                                                  std::to_string(h.bad_line != ~0ull ? h.bad_line : lines));
+    if (pieces && rcap == 0) {   /* the first reads say which records these are going to be */
+      c->sk_on = c->sk_on && sk_pays(c, (double)h.n_seq / (double)(lines / 4));
+      c->pre_extracted = c->sk_on || (c->W == 1 && !c->cfg.edge_filter);
+    }
+    if (c->pre_extracted && rcap == 0) {
+      /* a record holds its sequence and, as a rule, an equally long quality line: k-mer positions are
+       * at most half the bytes (shorter quality lines are accepted too: the records may then need more
+       * room than this gives, which both extractions notice) */
+      int blocks = 0;   /* one launch a segment, bounded as extract_reads bounds it (8 bytes a read at least) */
+      for (auto &x : c->segs) blocks += wx_blocks(x.n / 8 + 1);
+      if ((st = c->sk_on ? sk_begin(c, {total_bytes}) : extract_begin(c, total_bytes / 2 + 1, std::max(1, blocks))) != BRUNO_OK)
+        return st;
+      cudaEventRecord(c->kev[0], c->stream);
+    }
     if (c->pre_extracted && c->sk_on) sk_extract_reads(c, rcap, rcap + lines / 4);
     else if (c->pre_extracted) extract_reads(c, rcap, rcap + lines / 4);
     if (batch_hook && (st = batch_segment(c, si, rcap, rcap + lines / 4)) != BRUNO_OK) return st;
     rcap += lines / 4;
   }
   c->n_reads = rcap;
+  if (c->S == 1 && !c->pre_extracted && rcap) c->sk_on = c->sk_on && sk_pays(c, (double)c->hctr->n_seq / (double)rcap);
   return BRUNO_OK;
 }
 
@@ -3210,29 +3226,42 @@ bruno_status count_partitioned(Ctx *c, bool &used) {
 /* One call: the count makes the nodes and nobody asks for what was counted */
 bool sk_makes_nodes(const Ctx *c) { return c->one_call && !c->cfg.keep_k2 && !c->cfg.keep_filtered; }
 
-/* every k-mer is kept: the raw counts or other thresholds may still be asked for, or there are none */
-bool sk_keeps_all(const Ctx *c) { return !c->one_call || !c->cfg.thresholding || c->cfg.keep_k2; }
+/* every k-mer is written to the table: the raw counts or other thresholds may still be asked for */
+bool sk_writes_all(const Ctx *c) { return !c->one_call || !c->cfg.thresholding || c->cfg.keep_k2; }
+/* ... or all of them become nodes, or may: the quick rule leaves nothing out */
+bool sk_keeps_all(const Ctx *c) { return sk_writes_all(c) || c->cfg.thresh[2] <= 1; }
 
 /* k from 19: below, windows hold fewer than 5 m-mers and a run is hardly longer than a k-mer's own
- * record.  Where every k-mer is kept the count has nothing to leave out, and below k = 24 the k-mer
- * records' shorter runs in the table win (200 kbp at 60x, steps: k = 19 1.04 ms against 1.13 by
- * super-k-mers, 21 1.05 and 1.15, 23 1.08 and 1.12, 24 1.14 and 1.09; from 27 on with a target load of 0.7, unthresholded:
- * 25 1.39 and 1.48, 27 1.44 and 1.40), except in small builds, which are a chain of launches (0.8 MB:
- * 0.7 ms against 0.5).  A forced counting path or table size keeps the k-mer records.  The (k+1)-mer
- * filter drops edges before anything is counted, so only a count that makes the nodes can do without them
- * in the table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33
- * by a table of (k+1)-mers). */
-constexpr uint64_t SK_SMALL = 2ull << 20;   /* bytes a sample */
+ * record.  A forced counting path or table size keeps the k-mer records.  The (k+1)-mer filter drops
+ * edges before anything is counted, so only a count that makes the nodes can do without them in the
+ * table: there it is a step of making them (2 Mbp at 20x, k = 31: 0.81 ms of counting against 3.33 by a
+ * table of (k+1)-mers). */
 uint64_t sk_room(const Ctx *c, uint64_t total, uint32_t &chunk);
-bool sk_takes(const Ctx *c) {
+uint64_t fastq_bytes(const Ctx *c) {
   uint64_t bytes = 0;
   for (auto &sg : c->segs) bytes += sg.n;
-  const int least = !sk_keeps_all(c) || bytes / c->S < SK_SMALL ? MZ_M + 4 : c->cfg.max_load > 0.6 ? 27 : 24;
-  if (c->cfg.k < least || (c->cfg.edge_filter && !sk_makes_nodes(c)) || c->force_direct_count != 0 ||
+  return bytes;
+}
+bool sk_takes(const Ctx *c) {
+  if (c->cfg.k < MZ_M + 4 || (c->cfg.edge_filter && !sk_makes_nodes(c)) || c->force_direct_count != 0 ||
       c->cfg.table_slots != 0)
     return false;
   uint32_t chunk;   /* record places have 32 bits: known from the bytes, before anything is extracted */
-  return sk_room(c, bytes, chunk) >> 32 == 0;
+  return sk_room(c, fastq_bytes(c), chunk) >> 32 == 0;
+}
+/* Where every k-mer is kept the count has nothing to leave out, and the k-mer records' shorter runs in
+ * the table win unless a super-k-mer record stands for several k-mers: from 5 on for reads of the given
+ * mean length, which k = 24 has with 100 bases and k = 31 with 45 (200 kbp at 60x, 100 bases, steps: k =
+ * 19, 3.9 a record, 1.04 ms against 1.13 by super-k-mers; 21, 4.4, 1.05 and 1.15; 23, 4.8, 1.08 and 1.12;
+ * 24, 5.2, 1.14 and 1.09; k = 31 with 36 bases, 3.9: 3.4 and 3.8); from 6.2 with a target load above 0.6
+ * (unthresholded, load 0.7: k = 25, 5.6, 1.39 and 1.48; 27, 6.5, 1.44 and 1.40).  Small builds are a
+ * chain of launches, fewer of them here (0.8 MB: 0.7 ms and 0.5). */
+constexpr uint64_t SK_SMALL = 2ull << 20;   /* bytes a sample */
+bool sk_pays(const Ctx *c, double length) {
+  if (!sk_keeps_all(c) || c->cfg.edge_filter || fastq_bytes(c) / c->S < SK_SMALL) return true;
+  const double kmers = std::max(1.0, length - c->cfg.k + 1.0), w = c->cfg.k - MZ_M + 1;
+  const double records = 1.0 + (kmers - 1.0) * 2.0 / (w + 1.0);
+  return kmers / records >= (c->cfg.max_load > 0.6 ? 6.2 : 5.0);
 }
 
 template <class KT, int BL, bool EDGES>
@@ -3708,7 +3737,7 @@ bruno_status count_superkmers(Ctx *c, int max_split, Again again, bool &used, bo
     a.recs = sorted;
     a.off = (const uint32_t *)c->sk_off.p;
     a.k = c->cfg.k;
-    a.keep_all = !nodes && all;
+    a.keep_all = !nodes && sk_writes_all(c);
     a.thresholding = c->cfg.thresholding;
     for (int i = 0; i < 6; ++i) a.t[i] = (uint32_t)std::min<uint64_t>(65536, c->cfg.thresh[i]);
     a.inv_load = inv_load;
@@ -4273,7 +4302,7 @@ bruno_status run_count_samples(Ctx *c) {
   cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
   cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
   bool indexed = false;
-  if (sk_takes(c)) {   /* by super-k-mers */
+  if (sk_takes(c) && sk_pays(c, BATCH_READS)) {   /* by super-k-mers */
     std::vector<uint64_t> bytes(S);
     for (uint32_t q = 0; q < S; ++q) bytes[q] = c->samp_off[q + 1] - c->samp_off[q];
     if ((st = sk_begin(c, bytes)) != BRUNO_OK) return st;

@@ -61,11 +61,13 @@ typedef struct bruno_cfg {
   int32_t exact_ranking;    /* 1: always run the round-synchronous ranking; 0: use the O(M)
                                ruling-set ranking whenever the chain map is consistent */
   int32_t direct_count;     /* counting path: 0 = automatic (from k = 19 on super-k-mer records --
-                               where every k-mer is kept and the input is not small, from 24 or 27
-                               on --, below, and for the rare input that these do not take, k-mer
-                               records, by partition in one CTA's shared memory; a skewed input that
-                               overflows a partition of k-mer records falls back to L2-resident
-                               partitions at k <= 31 and to the whole-table count at k > 31), 1 = every
+                               where every k-mer is kept and the input is not small, only if the
+                               reads are long enough for a record to stand for several k-mers, at 100
+                               bases from k = 24 on --, otherwise, and for the rare input that these
+                               do not take, k-mer records, by partition in one CTA's shared memory; a
+                               skewed input that overflows a partition of k-mer records falls back to
+                               L2-resident partitions at k <= 31 and to the whole-table count at
+                               k > 31), 1 = every
                                instance straight into the whole table, 2 = the L2 partitions
                                always (k <= 31; k > 31 then counts into the whole table). */
   int32_t edge_filter;      /* with thresholding: 1 = the blocked driver's build_index_thresholded

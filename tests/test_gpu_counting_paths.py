@@ -55,9 +55,26 @@ def test_path_where_every_kmer_is_kept(k, least):
     assert path_of(data, k, thresholding=False)[0] == want
     assert path_of(data, k, thresholding=False, max_load=0.7)[0] == ("super_kmers" if k >= 27 else "kmer_records")
     assert path_of(data[:207 * 9_000], k, thresholding=False)[0] == "super_kmers"   # (207 bytes a record)
+    with bg.Graph(k=k, thresh=bg.thresholds([1]), min_update=True) as g:   # (bounds that drop nothing)
+        g.build_and_compact(data)
+        assert g.counting_path()[0] == want
     thr = bg.thresholds([2])
     ref = oracle.run(data, k=k, thresh=thr, min_update=True, threads=16, keep_k2=True, keep_filtered=True)
     compare(gpu_run(data, k, True, thr, True), ref)
+
+
+@pytest.mark.parametrize("chunk", [0, 1 << 20])
+@pytest.mark.parametrize("length,want", [(36, "kmer_records"), (50, "super_kmers"), (300, "super_kmers")])
+def test_path_by_the_reads_lengths(length, want, chunk):
+    """an unthresholded build at k = 31: reads of six k-mers go by k-mer records, at once and in pieces of a
+    host copy, whose first piece says; with thresholds they do not"""
+    rng = np.random.default_rng(length)
+    data = fastq(rand_reads(rng, rng.integers(0, 4, 60_000), 4_000_000 // length, length, 0.005))
+    assert path_of(data, 31, thresholding=False, h2d_chunk=chunk)[0] == want
+    assert path_of(data, 31, h2d_chunk=chunk)[0] == "super_kmers"
+    ref = oracle.run(data, k=31, thresholding=False, thresh=bg.thresholds(), min_update=True, threads=16, keep_k2=True,
+                     keep_filtered=True)
+    compare(gpu_run(data, 31, False, bg.thresholds(), True, h2d_chunk=chunk), ref)
 
 
 def test_path_is_forgotten():

@@ -45,13 +45,13 @@ def fastq(codes, qual=None):
     return out.tobytes()
 
 
-def check(data, k, thr, thresholding=True, **cfg):
-    """a one-call build against the oracle; returns its sizes"""
+def check(data, k, thr, thresholding=True, superkmers=True, **cfg):
+    """a one-call build (by super-k-mers, unless said) against the oracle; returns its sizes"""
     ref = oracle.run(data, k=k, thresholding=thresholding, thresh=thr, min_update=True, threads=16,
                      edge_filter=cfg.get("edge_filter", False))
     with bg.Graph(k=k, thresholding=thresholding, thresh=thr, min_update=True, **cfg) as g:
         g.build_and_compact(data)
-        assert g.counting_path()[0] == "super_kmers"
+        assert (g.counting_path()[0] == "super_kmers") == superkmers
         s = g.sizes()
         for n in SIZES:
             if n in ref:
@@ -158,9 +158,9 @@ def crowded_reads(kind, seed, n=24_000, genome=120_000):
 @pytest.mark.parametrize("kind", ["adapter", "poly-A", "one base", "satellite"])
 @pytest.mark.parametrize("k", [21, 31, 45, 63])
 def test_crowded_partitions(k, kind, thr):
-    """one call, and the step calls with every count copied out"""
+    """one call, and the step calls with every count copied out (k = 21 keeps every k-mer by k-mer records)"""
     data = fastq(crowded_reads(kind, k))
-    check(data, k, bg.thresholds(thr), thresholding=bool(thr))
+    check(data, k, bg.thresholds(thr), thresholding=bool(thr), superkmers=bool(thr) or k > 21)
     ref = oracle.run(data, k=k, thresholding=bool(thr), thresh=bg.thresholds(thr), min_update=True, keep_k2=True,
                      keep_filtered=True, threads=16)
     compare(gpu_run(data, k, bool(thr), bg.thresholds(thr), True), ref)
