@@ -106,13 +106,11 @@ __device__ __forceinline__ uint32_t slot_aux(const uint64_t *s) {
   return (uint32_t)(s[Slot<KT>::KEYW + 2] >> 32);
 }
 
-/* slot index of a live node with canonical key x, -1 if absent */
+/* slot index of the live node with table key `bare` along its probe sequence, -1 if absent */
 template <class KT>
-__device__ __forceinline__ long long table_find(const uint64_t *table, const TableGeom &g, uint32_t max_probe,
-                                                KT kmer) {
+__device__ __forceinline__ long long table_find_from(const uint64_t *table, Probe pr, uint32_t max_probe, KT bare) {
   constexpr int SU = Slot<KT>::U64;
-  const KT bare = table_key(kmer), x = as_node(bare);
-  Probe pr = table_probe(g, kmer, bare);
+  const KT x = as_node(bare);
   for (uint32_t p = 0; p < max_probe; ++p, pr.next()) {
     const uint64_t *s = table + pr.i * SU;
     KT key = KOps<KT>::load(s);
@@ -121,6 +119,14 @@ __device__ __forceinline__ long long table_find(const uint64_t *table, const Tab
       return -1;
   }
   return -1;
+}
+
+/* slot index of a live node with canonical key x, -1 if absent */
+template <class KT>
+__device__ __forceinline__ long long table_find(const uint64_t *table, const TableGeom &g, uint32_t max_probe,
+                                                KT kmer) {
+  const KT bare = table_key(kmer);
+  return table_find_from<KT>(table, table_probe(g, kmer, bare), max_probe, bare);
 }
 
 /* Two lookups in lockstep: both first probes are in flight together, and each probe reads
@@ -205,7 +211,11 @@ __global__ void __launch_bounds__(TPB) k_chain_init(const uint64_t *table, uint6
       want[q] = flip[q] ? y : n;
     }
     uint32_t mz[2] = {0, 0};
-    if (g.bins) neighbour_minimizers<KT>(K, k, (unsigned)max(inc, 0), (unsigned)max(outc, 0), mz);
+    if (g.bins) {
+      const NeighbourMinimizers<KT> nm(K, k);
+      mz[0] = nm.before((unsigned)max(inc, 0));
+      mz[1] = nm.after((unsigned)max(outc, 0));
+    }
     long long found[2];
     uint64_t raw[2][SU];
     table_find2<KT>(table, g, max_probe, want, mz, has, found, raw);
@@ -2590,23 +2600,27 @@ __global__ void __launch_bounds__(TPB) k_check_refs(const uint64_t *table, uint6
     const uint64_t *s = table + i * SU;
     if (!key_is_node(KOps<KT>::load(s))) continue;
     const KT K = key_kmer(node_key(KOps<KT>::load(s)));
-    const uint64_t ow = s[KWD], iw = s[KWD + 1];
-    unsigned din = 0, dout = 0;
-    for (unsigned c = 0; c < 4; ++c) {
-      for (int side = 0; side < 2; ++side) {
-        if (!count_at(side ? iw : ow, c)) continue;
-        ++q;
-        side ? ++din : ++dout;
-        /* the neighbour and the edge it should have back: K.c has an in edge from first(K);
-         * c.K has an out edge to last(K) */
-        KT y = side ? KOps<KT>::prepend(c, K, k) : KOps<KT>::append(K, c, k);
-        unsigned e = side ? (1u << KOps<KT>::last(K)) : ((1u << KOps<KT>::first(K, k)) << 4);
-        canon_edge(y, e, k);
-        const long long sl = table_find<KT>(table, g, 4096u, y);
-        if (sl < 0) { ++absent; continue; }
-        atomicOr(&ref[(uint64_t)sl >> 5], 1u << ((uint64_t)sl & 31));
-        if (!has_edge<KT>(table, sl, e)) ++unanswered;
-      }
+    /* the node's edges, out over base c as bit c, in as bit 4 + c: each lane goes through its own */
+    unsigned edges = 0;
+    for (unsigned c = 0; c < 4; ++c)
+      edges |= (count_at(s[KWD], c) ? 1u << c : 0u) | (count_at(s[KWD + 1], c) ? 16u << c : 0u);
+    const unsigned din = __popc(edges >> 4), dout = __popc(edges & 15u);
+    q += din + dout;
+    NeighbourMinimizers<KT> nm(K, g.bins ? k : MZ_M);
+    for (; edges; edges &= edges - 1) {
+      const unsigned b = __ffs(edges) - 1, c = b & 3u;
+      const bool side = b & 4u;
+      /* the neighbour and the edge it should have back: K.c has an in edge from first(K);
+       * c.K has an out edge to last(K) */
+      KT y = side ? KOps<KT>::prepend(c, K, k) : KOps<KT>::append(K, c, k);
+      unsigned e = side ? (1u << KOps<KT>::last(K)) : ((1u << KOps<KT>::first(K, k)) << 4);
+      canon_edge(y, e, k);
+      const KT bare = table_key(y);
+      const Probe pr = g.bins ? bin_probe(g, side ? nm.before(c) : nm.after(c), bare) : Probe(g, table_home(g, bare));
+      const long long sl = table_find_from<KT>(table, pr, 4096u, bare);
+      if (sl < 0) { ++absent; continue; }
+      atomicOr(&ref[(uint64_t)sl >> 5], 1u << ((uint64_t)sl & 31));
+      if (!has_edge<KT>(table, sl, e)) ++unanswered;
     }
     atomicAdd(&s_hist[din * 5 + dout], 1ull);
   }

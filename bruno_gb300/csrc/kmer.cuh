@@ -277,40 +277,49 @@ __device__ __forceinline__ uint32_t kmer_minimizer(KW2 x, int k) {
   }
   return best;
 }
-/* The minimizers of a k-mer's in neighbour (base cin before it) and out neighbour (cout after it):
- * each shares all its MZ_M-mers but one with the k-mer, so both come from one pass over them. */
+/* The minimizers of a k-mer's neighbours: each shares all its MZ_M-mers but one with the k-mer, so they
+ * come from one pass over them (in, out: the smallest that in, out neighbours share with it). */
 template <class KT>
-__device__ __forceinline__ void neighbour_minimizers(KT x, int k, unsigned cin, unsigned cout, uint32_t *mz) {
-  constexpr int W = KOps<KT>::WORDS;
-  KT f = x, r = KOps<KT>::rc(x, k);
-  const uint32_t r_first = (uint32_t)((const uint64_t *)&r)[0] & MZ_MASK;   /* the first m-mer's complement ends r */
-  uint64_t rt[W];   /* r, its first base in the top bits, high word first */
-  if constexpr (W == 1) {
-    rt[0] = r.v << (64 - 2 * k);
-  } else {
-    const int s = 128 - 2 * k;
-    rt[0] = s >= 64 ? r.lo << (s - 64) : (r.hi << s) | (s ? r.lo >> (64 - s) : 0);
-    rt[1] = s >= 64 ? 0 : r.lo << s;
-  }
-  uint32_t o = 0, in = ~0u, out = ~0u, f_last = 0, r_last = 0, fl = 0;
-  const int w1 = k - MZ_M;
-  for (int i = 0; i <= w1; ++i) {   /* from the last m-mer to the first */
-    fl = (uint32_t)((const uint64_t *)&f)[0] & MZ_MASK;
-    const uint32_t rl = (uint32_t)(rt[0] >> (64 - 2 * MZ_M));
-    o = mz_order(fl, rl);
-    if (i == 0) { f_last = fl; r_last = rl; }
-    else in = min(in, o);
-    if (i < w1) out = min(out, o);
-    if constexpr (W == 1) { f.v >>= 2; rt[0] <<= 2; }
-    else {
-      f = {(f.lo >> 2) | (f.hi << 62), f.hi >> 2};
-      rt[0] = (rt[0] << 2) | (rt[1] >> 62);
-      rt[1] <<= 2;
+struct NeighbourMinimizers {
+  uint32_t in, out, f_first, r_first, f_last, r_last;   /* and the first and last MZ_M-mer, on both strands */
+  __device__ __forceinline__ NeighbourMinimizers(KT x, int k) : in(~0u), out(~0u), f_last(0), r_last(0) {
+    constexpr int W = KOps<KT>::WORDS;
+    KT f = x, r = KOps<KT>::rc(x, k);
+    r_first = (uint32_t)((const uint64_t *)&r)[0] & MZ_MASK;   /* the first m-mer's complement ends r */
+    uint64_t rt[W];   /* r, its first base in the top bits, high word first */
+    if constexpr (W == 1) {
+      rt[0] = r.v << (64 - 2 * k);
+    } else {
+      const int s = 128 - 2 * k;
+      rt[0] = s >= 64 ? r.lo << (s - 64) : (r.hi << s) | (s ? r.lo >> (64 - s) : 0);
+      rt[1] = s >= 64 ? 0 : r.lo << s;
     }
+    const int w1 = k - MZ_M;
+    uint32_t fl = 0;
+    for (int i = 0; i <= w1; ++i) {   /* from the last m-mer to the first */
+      fl = (uint32_t)((const uint64_t *)&f)[0] & MZ_MASK;
+      const uint32_t rl = (uint32_t)(rt[0] >> (64 - 2 * MZ_M));
+      const uint32_t o = mz_order(fl, rl);
+      if (i == 0) { f_last = fl; r_last = rl; }
+      else in = min(in, o);
+      if (i < w1) out = min(out, o);
+      if constexpr (W == 1) { f.v >>= 2; rt[0] <<= 2; }
+      else {
+        f = {(f.lo >> 2) | (f.hi << 62), f.hi >> 2};
+        rt[0] = (rt[0] << 2) | (rt[1] >> 62);
+        rt[1] <<= 2;
+      }
+    }
+    f_first = fl;
   }
-  mz[0] = min(in, mz_order((fl >> 2) | (cin << (2 * MZ_M - 2)), ((r_first << 2) | (3u - cin)) & MZ_MASK));
-  mz[1] = min(out, mz_order(((f_last << 2) | cout) & MZ_MASK, (r_last >> 2) | ((3u - cout) << (2 * MZ_M - 2))));
-}
+  /* of the in neighbour with base c before the k-mer, of the out neighbour with base c after it */
+  __device__ __forceinline__ uint32_t before(unsigned c) const {
+    return min(in, mz_order((f_first >> 2) | (c << (2 * MZ_M - 2)), ((r_first << 2) | (3u - c)) & MZ_MASK));
+  }
+  __device__ __forceinline__ uint32_t after(unsigned c) const {
+    return min(out, mz_order(((f_last << 2) | c) & MZ_MASK, (r_last >> 2) | ((3u - c) << (2 * MZ_M - 2))));
+  }
+};
 constexpr uint32_t SK_SUBS = 1u << 31;
 /* which part of a crowded partition a key lies in, in the low bits (bin_home takes high ones) */
 __device__ __forceinline__ uint32_t key_sub(KW1 t) { return (uint32_t)t.v; }
