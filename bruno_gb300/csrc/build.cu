@@ -1864,15 +1864,14 @@ __device__ __forceinline__ uint64_t sm_cas128(uint32_t a, uint64_t cmp_lo, uint6
 
 /* one step of count_in_entries on entry word e (snapshot w): claim it if empty, count if it
  * holds the code; true when the record is counted */
-__device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned code, uint32_t weight,
-                                              unsigned long long &claims) {
+__device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned code, unsigned long long &claims) {
   if (w == 0) {
-    const uint32_t old = atomicCAS(e, 0u, (code << E_CODE_SHIFT) | (weight << E_COUNT_SHIFT));
+    const uint32_t old = atomicCAS(e, 0u, (code << E_CODE_SHIFT) | (1u << E_COUNT_SHIFT));
     if (old == 0) { ++claims; return true; }
     w = old;
   }
   if (entry_code(w) == code) {
-    atomicAdd(e, weight << E_COUNT_SHIFT);   /* a partition counted here holds fewer than 2^24 records */
+    atomicAdd(e, 1u << E_COUNT_SHIFT);   /* a partition counted here holds fewer than 2^24 records */
     return true;
   }
   return false;
@@ -1883,10 +1882,10 @@ __device__ __forceinline__ bool sm_entry_step(uint32_t *e, uint32_t w, unsigned 
  * (most k-mers hold one or two edges); `first` are the words already read */
 template <int NE, int FIRST>
 __device__ __forceinline__ bool sm_count_entries_lazy(uint32_t *e, uint32_t e_addr, const uint32_t *first,
-                                                      unsigned code, uint32_t weight, unsigned long long &claims) {
+                                                      unsigned code, unsigned long long &claims) {
   #pragma unroll
   for (int i = 0; i < FIRST; ++i)
-    if (sm_entry_step(e + i, first[i], code, weight, claims)) return true;
+    if (sm_entry_step(e + i, first[i], code, claims)) return true;
   #pragma unroll
   for (int g = FIRST; g < NE; g += 4) {
     uint64_t w0, w1;
@@ -1894,14 +1893,14 @@ __device__ __forceinline__ bool sm_count_entries_lazy(uint32_t *e, uint32_t e_ad
     const uint32_t s[4] = {(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32)};
     #pragma unroll
     for (int i = 0; i < 4; ++i)
-      if (g + i < NE && sm_entry_step(e + g + i, s[i], code, weight, claims)) return true;
+      if (g + i < NE && sm_entry_step(e + g + i, s[i], code, claims)) return true;
   }
   return false;
 }
 
 /* one record into the partition held in shared memory; false if the region is full */
 __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_t region, uint64_t h, unsigned code,
-                                         uint32_t home, uint32_t weight, unsigned long long &slot_claims,
+                                         uint32_t home, unsigned long long &slot_claims,
                                          unsigned long long &entry_claims) {
   bool seen_primary = false;
   uint32_t j = home;
@@ -1911,7 +1910,7 @@ __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_
     asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(key), "=l"(w01) : "r"(a) : "memory");
     const uint64_t want = h | (seen_primary ? KEY_CONT : 0);
     if (key == KEY_EMPTY) {
-      const uint64_t ne0 = (uint64_t)((code << E_CODE_SHIFT) | (weight << E_COUNT_SHIFT));
+      const uint64_t ne0 = (uint64_t)((code << E_CODE_SHIFT) | (1u << E_COUNT_SHIFT));
       uint64_t ohi;
       const uint64_t olo = sm_cas128(a, KEY_EMPTY, 0ull, want, ne0, ohi);
       if (olo == KEY_EMPTY && ohi == 0) { ++slot_claims; ++entry_claims; return true; }
@@ -1921,7 +1920,7 @@ __device__ __forceinline__ bool sm_count(uint64_t *sm, uint32_t sm_base, uint32_
     if (key == want) {
       seen_primary = true;
       const uint32_t first[2] = {(uint32_t)w01, (uint32_t)(w01 >> 32)};
-      if (sm_count_entries_lazy<6, 2>((uint32_t *)(sm + (uint64_t)j * 4 + 1), a + 8u, first, code, weight, entry_claims))
+      if (sm_count_entries_lazy<6, 2>((uint32_t *)(sm + (uint64_t)j * 4 + 1), a + 8u, first, code, entry_claims))
         return true;
     }
     j = (j + 1 == region) ? 0u : j + 1;
@@ -2044,7 +2043,7 @@ __global__ void __launch_bounds__(1024) k_count_local(const uint64_t *recs, cons
     if (rec == 0ull) continue;   /* an unused chunk tail, when the buckets are the partitions */
     const uint64_t h = bucket_hi | (rec >> 5);
     const uint32_t home = (uint32_t)__umul64hi(h << (2 + G.g.pbits), G.g.region);
-    if (!sm_count(sm, sm_base, region, h, (unsigned)(rec & 31), home, 1u, slots, entries)) full = true;
+    if (!sm_count(sm, sm_base, region, h, (unsigned)(rec & 31), home, slots, entries)) full = true;
   }
   __syncthreads();
   ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(table + (G.g.base + j * G.g.region) * 4);
@@ -2206,8 +2205,8 @@ void launch_scatter(const typename ScatterRec<KT>::T *records, const unsigned lo
 /* one record into a 64-byte slot region in shared memory (key 2 words, 12 entry words);
  * false if the region is full */
 __device__ __forceinline__ bool sm_count2(uint64_t *sm, uint32_t sm_base, uint32_t region, uint64_t lo, uint64_t hi,
-                                          unsigned code, uint32_t home, uint32_t weight,
-                                          unsigned long long &slot_claims, unsigned long long &entry_claims) {
+                                          unsigned code, uint32_t home, unsigned long long &slot_claims,
+                                          unsigned long long &entry_claims) {
   bool seen_primary = false;
   uint32_t j = home;
   for (uint32_t probe = 0; probe < region; ++probe) {
@@ -2223,7 +2222,7 @@ __device__ __forceinline__ bool sm_count2(uint64_t *sm, uint32_t sm_base, uint32
     }
     if (k0 == lo && k1 == whi) {   /* the entries, four at a time as far as they are needed */
       seen_primary = true;
-      if (sm_count_entries_lazy<12, 0>((uint32_t *)(sm + (uint64_t)j * 8 + 2), a + 16u, nullptr, code, weight, entry_claims))
+      if (sm_count_entries_lazy<12, 0>((uint32_t *)(sm + (uint64_t)j * 8 + 2), a + 16u, nullptr, code, entry_claims))
         return true;
     }
     j = (j + 1 == region) ? 0u : j + 1;
@@ -2259,7 +2258,7 @@ __global__ void __launch_bounds__(PTPB2, 3) k_count_local2(const unsigned long l
     nxt = i + nt < n ? __ldcs(rp + i + nt) : make_ulonglong2(0ull, 0ull);
     const uint64_t h = bucket_hi | (r.x >> 8);   /* the table key is (h, high word) */
     const uint32_t home = (uint32_t)__umul64hi(h << g.pbits, g.region);
-    if (!sm_count2(sm, sm_base, region, h, r.y, (unsigned)(r.x & 31u), home, 1u, slots, entries)) full = true;
+    if (!sm_count2(sm, sm_base, region, h, r.y, (unsigned)(r.x & 31u), home, slots, entries)) full = true;
   }
   __syncthreads();   /* every record is read: the region's memory is free for the slots */
   ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(reg);
