@@ -368,6 +368,29 @@ def run_served(args):
         b.free()
 
 
+def counting_kernels(k: int, path: str, records: int, fastq: int, sizes: dict, mean) -> dict:
+    """(bytes, ms) of a step's counting kernels by the path that ran.  Bytes: what a kernel reads and
+    writes if it does each once: FASTQ and 16 B of span a read, the records (super-k-mers of 16 bytes at k <= 31,
+    32 above; k-mer records of 8, 16), the table slots (32, 64) written once, 4 B per slot listed for the
+    filter.  By L2 partitions or the whole table: a 64-byte update (two slots' sectors at k > 31) per k-mer."""
+    wide, inst, slots, listed = k > 31, sizes["n_instances"], sizes["table_slots"], sizes["filter_slots_read"]
+    reads, slot = fastq + 16 * sizes["n_reads"], 64 if wide else 32
+    count = mean("count_insert") - mean("count_split")
+    filt = {"k_filter": (slot * listed + slot * sizes["n_nodes"], mean("filter_insert"))}
+    if path == "super_kmers":
+        rec = 32 if wide else 16
+        split = "k_sk_scatter" if wide or records < 1 << 20 or sizes["table_partitions"] < 1 << 12 else "k_sk_split"
+        return {"k_sk_extract": (reads + rec * records, mean("count_estimate")),
+                split: (2 * rec * records, mean("count_split")),
+                f"k_sk_count<KW{2 if wide else 1}>": (rec * records + slot * slots, count)}
+    if path == "kmer_records":
+        rec, own = (16, "2") if wide else (8, "")
+        return {"k_extract_s": (reads + rec * records, mean("count_estimate")),
+                "k_split_scatter" if wide else "k_split": (2 * rec * records, mean("count_split")),
+                "k_count_local" + own: (rec * records + slot * slots + 4 * listed, count), **filt}
+    return {"k_insert" if path == "l2_partitions" else "k_count": (64 * (2 if wide else 1) * inst, mean("count_insert")), **filt}
+
+
 def main():
     args = parse_args()
     from bruno_gb300 import synth
@@ -487,39 +510,12 @@ def main():
     e2e_value = inst_step * args.steps * world / (ems / 1e3)
     d2h = nch + 8 * (nc + 1) + 8 * g.words * nc
 
-    # Roofline of the dominant kernel.  Each candidate's algorithmic bytes per step and its
-    # CUDA-event time on the library's stream.  k >= 19 is counted by super-k-mer records (16 bytes
-    # at k <= 31, 32 above), of which there is one a read and, on random sequence, one for every
-    # (w + 1) / 2 k-mers (w = k - 14, the 15-mers of a k-mer):
-    #   k_sk_extract  FASTQ bytes + 16 B read span per read read once, the records written
-    #   k_sk_split    the records read and written once (k_sk_scatter at k > 31)
-    #   k_sk_count    the records read once + a table slot (32 B, 64 B at k > 31) per slot written once
+    # Roofline of the dominant kernel: each counting kernel's bytes per step (below) against its
+    # CUDA-event time on the library's stream, for the path that the library says it took
     mean = lambda key: statistics.mean(p[key] for p in kms)
     peak, peak_src = measured_peak()
-    slots = sizes["table_slots"]
-    listed = sizes["filter_slots_read"]
-    if w.k >= 19:
-        rec, slot = (16, 32) if w.k <= 31 else (32, 64)
-        recs = 2 * inst_step / (w.k - 13) + sizes["n_reads_used"]
-        kern = {
-            "k_sk_extract": (n + 16 * sizes["n_reads"] + rec * recs, mean("count_estimate")),
-            "k_sk_split" if w.k <= 31 else "k_sk_scatter": (2 * rec * recs, mean("count_split")),
-            "k_sk_count<KW1>" if w.k <= 31 else "k_sk_count<KW2>": (rec * recs + slot * slots,
-                                                                     mean("count_insert") - mean("count_split")),
-        }
-    elif w.k <= 31:
-        # k < 19, by k-mer records:
-        #   k_extract      FASTQ bytes + 16 B read span per read read once, 8 B per record written
-        #   k_split        8 B per record read and written once
-        #   k_count_local  8 B per record read once + 32 B per table slot written once + 4 B per
-        #                  slot it lists for the filter
-        #   k_filter       32 B per slot it reads (the listed ones) + 32 B per graph node written once
-        kern = {
-            "k_extract": (n + 16 * sizes["n_reads"] + 8 * inst_step, mean("count_estimate")),
-            "k_split": (16 * inst_step, mean("count_split")),
-            "k_count_local": (8 * inst_step + 32 * slots + 4 * listed, mean("count_insert") - mean("count_split")),
-            "k_filter": (32 * listed + 32 * sizes["n_nodes"], mean("filter_insert")),
-        }
+    path, records = g.counting_path()
+    kern = counting_kernels(w.k, path, records, n, sizes, mean)
     kernels = {k: {"alg_bytes_per_launch": b, "launch_ms": t, "achieved": b / (t / 1e3) / 1e9 if t > 0 else None,
                    "frac": b / (t / 1e3) / 1e9 / peak if t > 0 else None} for k, (b, t) in kern.items()}
     top = max(kernels, key=lambda k: kernels[k]["launch_ms"])
@@ -560,11 +556,13 @@ def main():
                                                                         "chainmap", "list_rank", "compress"))
                                                      for p in e2e_phases) if e2e_phases else None,
                         "contexts": max(1, args.e2e_workers)},
-                "roofline": {"bound": "hbm", "kernel": top, "achieved": kernels[top]["achieved"], "peak": peak,
+                "roofline": {"bound": "issue" if top.startswith("k_sk_") else "hbm", "counting_path": path, "kernel": top, "achieved": kernels[top]["achieved"], "peak": peak,
                              "unit": "GB/s", "frac": kernels[top]["frac"], "peak_source": peak_src,
                              "traffic": traffic, "alg_bytes_per_launch": kernels[top]["alg_bytes_per_launch"],
                              "launch_ms": kernels[top]["launch_ms"], "kernels": kernels},
-                "path_roofline": {"bound": "hbm", "alg_bytes_per_step": path_bytes, "achieved": path_achieved,
+                "path_roofline": {"bound": "hbm", "model": "a 64-byte table update per k-mer occurrence; the kernels that "
+                                                          "ran move less (roofline.kernels)",
+                                  "alg_bytes_per_step": path_bytes, "achieved": path_achieved,
                                   "peak": peak, "unit": "GB/s", "frac": path_achieved / peak},
                 "gpu_launches": launches, "clocks": clk.summary(), "phase_ms": phases,
                 "sizes": {k: sizes[k] for k in ("n_reads", "n_instances", "n_k2", "n_nodes", "n_branch",
