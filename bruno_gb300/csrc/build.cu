@@ -394,15 +394,15 @@ struct CountArgs {
 
 
 
-/* One more occurrence of the entry whose word lives at `key` (its address), in the exact
+/* n more occurrences of the entry whose word lives at `key` (its address), in the exact
  * side table of counts past 2^24.  Every such entry needs 2^24 occurrences, so at most
  * n_instances / 2^24 of them exist: the table cannot fill below 2^34 instances. */
-__device__ __forceinline__ void big_add(DevCounters *ctr, unsigned long long key) {
+__device__ __forceinline__ void big_add(DevCounters *ctr, unsigned long long key, unsigned long long n = 1) {
   unsigned h = (unsigned)mix64(key) & (BIG_SLOTS - 1);
   for (int p = 0; p < BIG_SLOTS; ++p, h = (h + 1) & (BIG_SLOTS - 1)) {
     const unsigned long long prev = atomicCAS(&ctr->big_key[h], 0ull, key);
     if (prev == 0ull) atomicAdd(&ctr->n_big, 1ull);
-    if (prev == 0ull || prev == key) { atomicAdd(&ctr->big_cnt[h], 1ull); return; }
+    if (prev == 0ull || prev == key) { atomicAdd(&ctr->big_cnt[h], n); return; }
   }
   atomicOr(&ctr->err, (unsigned long long)DERR_INVARIANT);
 }
@@ -3489,7 +3489,7 @@ constexpr uint64_t SK_PART_KMERS = 4096;
 uint64_t sk_parts_room(const Ctx *c, uint64_t n_rec) { return n_rec * (uint64_t)(c->cfg.k - MZ_M + 1) / (SK_PART_KMERS / 2); }
 
 /* The n partitions listed at `list` (superkmer.cuh, crowded partitions) by parts; NO if their parts do
- * not do either, or a count that must be exact could pass what an entry holds. */
+ * not do either. */
 template <class KT>
 bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vector<SGeom> &sg, const uint32_t *list,
                               uint32_t n, uint64_t room, SkCounted &out) {
@@ -3506,10 +3506,10 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
   if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "crowded partitions")) != BRUNO_OK) return st;
   std::vector<SkCrowd> crowd(n);
   std::vector<SkChunk> chunks;
-  uint64_t subs = 0;
+  uint64_t subs = 0, most = 0;
   for (uint32_t i = 0; i < n; ++i) {
     const uint64_t kmers = (uint64_t)rec[i].y * (uint64_t)(c->cfg.k - MZ_M + 1);   /* at most */
-    if (!a.nodes && kmers >> 25) return BRUNO_OK;
+    most = std::max(most, kmers);
     uint32_t lg = 1;
     while (kmers >> lg > SK_PART_KMERS) ++lg;
     uint32_t smp = 0;
@@ -3551,6 +3551,13 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
   a.sub0 = parts;
   a.sub_smp = (const uint32_t *)c->sk_sub_smp.p;
   a.cls = nullptr;
+  /* counts that must be exact where a partition holds more than an entry counts to: the records past
+   * that are kept for the side table */
+  if (!a.nodes && most >> 25) {
+    a.past_cap = kmers;
+    if ((st = ensure(c, c->sk_past, kmers * NW * 8)) != BRUNO_OK) return st;
+    a.past = (uint64_t *)c->sk_past.p;
+  }
   uint32_t left = (uint32_t)subs;
   for (const double slots : {(double)SK_PART_KMERS / 2, 8000.0}) {   /* what overflows, with as many slots as fit */
     const SkShape<KT> shape(slots, 0.0);
@@ -3565,7 +3572,15 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
     cudaEventRecord(c->kev[3], c->stream);
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     left = (uint32_t)c->hctr->n_over;
-    if (left == 0 || c->hctr->err) break;
+    if (left == 0 || c->hctr->err || c->hctr->n_sk_past) break;   /* (a part counted again would keep its again) */
+  }
+  if (c->hctr->n_sk_past && left == 0 && !c->hctr->err) {
+    cudaMemsetAsync(c->dctr->big_key, 0, sizeof(c->dctr->big_key) + sizeof(c->dctr->big_cnt), c->stream);
+    k_sk_past<KT><<<num_sms() * 4, 256, 0, c->stream>>>((const uint64_t *)c->sk_past.p, c->hctr->n_sk_past,
+                                                        (uint64_t *)c->table.p, a.sg, c->dctr);
+    c->launches += 1;
+    if ((st = sync_counters(c)) != BRUNO_OK) return st;
+    if (c->hctr->err & DERR_INVARIANT) return set_err(c, BRUNO_ERR_INVARIANT, "a counted k-mer is not in the table");
   }
   c->sk_subs = (uint32_t)subs;
   out = c->hctr->err ? SkCounted::AGAIN : left == 0 ? SkCounted::DONE : SkCounted::NO;

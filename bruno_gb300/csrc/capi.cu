@@ -159,7 +159,7 @@ bruno_status bruno_ctx_destroy(bruno_ctx *c) {
                  &c->cl_trec, &c->cl_tslot, &c->cl_sums, &c->cl_norm, &c->cl_htab, &c->cl_q, &c->cl_found,
                  &c->records, &c->bucket_cnt, &c->records2, &c->sub_cnt, &c->bigres, &c->cand, &c->scan_tmp, &c->fr_tmp,
                  &c->xsamp, &c->hllreg, &c->hsum, &c->sgeom, &c->s_tally, &c->s_inst, &c->s_used, &c->xitems,
-                 &c->sk_recs, &c->sk_sorted, &c->sk_hist, &c->sk_part, &c->sk_off, &c->sk_cur, &c->sk_samp, &c->sk_plan, &c->sk_sums, &c->sk_info, &c->sk_over, &c->sk_bump, &c->sk_est, &c->sk_items, &c->sk_sub_cnt, &c->sk_sub_off, &c->sk_sub_smp, &c->sk_kmers,
+                 &c->sk_recs, &c->sk_sorted, &c->sk_hist, &c->sk_part, &c->sk_off, &c->sk_cur, &c->sk_samp, &c->sk_plan, &c->sk_sums, &c->sk_info, &c->sk_over, &c->sk_bump, &c->sk_est, &c->sk_items, &c->sk_sub_cnt, &c->sk_sub_off, &c->sk_sub_smp, &c->sk_kmers, &c->sk_past,
                  &c->split_items, &c->csample, &c->r_samp, &c->h_samp, &c->grp_tmp};
   for (Buf *b : bufs) release(*b);
   for (Buf &b : c->seg_bufs) release(b);

@@ -52,6 +52,7 @@ struct DevCounters {
   unsigned long long n_big, n_big_res; /* entries counted past 2^24 (keys in big_key), resolved */
   unsigned long long sk_bump;          /* table slots taken by the one sample's regions */
   unsigned long long n_over;           /* partitions whose k-mers overflowed their CTA's slots */
+  unsigned long long n_sk_past;        /* k-mer records past what an entry in shared memory counts to */
   unsigned long long n_cand;           /* slots the count listed for the filter */
   unsigned long long quick_hist[16];   /* the filter flags of the entries the count dropped */
   unsigned int hll[1 << 12];           /* HyperLogLog registers, p = 12 */
@@ -170,7 +171,7 @@ struct Ctx {
   /* counting by super-k-mers (superkmer.cuh): records as extracted and in partition order, the
    * minimizer bins' tallies and partitions, the partitions' first records and cursors */
   Buf sk_recs, sk_sorted, sk_hist, sk_part, sk_off, sk_cur, sk_samp, sk_plan, sk_sums, sk_info, sk_over, sk_bump, sk_est;
-  Buf sk_items, sk_sub_cnt, sk_sub_off, sk_sub_smp, sk_kmers;   /* crowded partitions: their k-mers, by part */
+  Buf sk_items, sk_sub_cnt, sk_sub_off, sk_sub_smp, sk_kmers, sk_past;   /* crowded partitions: their k-mers, by part */
   bool sk_on = false;            /* this build extracts super-k-mers */
   /* one call builds the whole graph: the thresholds of the configuration are the ones the filter
    * will use and nobody asks for raw counts, so the count need not keep what the filter drops */

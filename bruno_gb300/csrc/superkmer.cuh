@@ -752,6 +752,8 @@ struct SkCount {
   unsigned long long *bump;         /* per sample: table slots taken so far */
   uint32_t sub0;                    /* parts of crowded partitions: the first one's place in info, */
   const uint32_t *sub_smp;          /* their samples */
+  uint64_t *past;                   /* their k-mer records that an entry no longer takes (SkPast) */
+  uint64_t past_cap;
   DevCounters *ctr;
 };
 
@@ -856,9 +858,9 @@ __device__ __forceinline__ uint32_t sk_count_of(uint32_t w) { return w >> E_COUN
 
 /* `fresh` is an entry word: a code and the occurrences to count.  One entry word of a slot tried for
  * it; `w` is what the word was seen to hold.  SAT: a count from 2^25 on stays where it is (a block's
- * threads, with weights of 2^10 at most, cannot bring it to 2^26 before they see it) */
+ * threads, with weights of 2^10 at most, cannot bring it to 2^26 before they see it), and `past` says so */
 template <bool SAT = false>
-__device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t fresh, unsigned &claims) {
+__device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t fresh, unsigned &claims, bool &past) {
   if (w == 0) {
     w = atomicCAS(e, 0u, fresh);
     if (w == 0) { ++claims; return true; }
@@ -866,17 +868,34 @@ __device__ __forceinline__ bool sk_try_entry(uint32_t *e, uint32_t w, uint32_t f
   if (entry_code(w) != entry_code(fresh)) return false;
   const uint32_t add = fresh & ~((1u << E_COUNT_SHIFT) - 1);
   if (SAT) {
-    if (atomicAdd(e, add) >> 31) atomicSub(e, add);
+    past = atomicAdd(e, add) >> 31;
+    if (past) atomicSub(e, add);
   } else {
     atomicAdd(e, add);
   }
   return true;
 }
 
+/* k-mer records whose occurrences an entry no longer takes, for counts that must be exact (rec: NULL
+ * where only the filter reads them) */
+struct SkPast { uint64_t *rec; uint64_t cap; DevCounters *ctr; };
+
 /* an entry word's occurrences into the shared-memory slots of a k-mer, continuation slots and all
  * (any lanes may call it); false if the slots are full */
 template <class KT, bool SAT>
-__device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, unsigned &claims) {
+__device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, unsigned &claims, SkPast over = SkPast{}) {
+  constexpr int NW = SkRec<KT>::NW, KWD = Slot<KT>::KEYW;
+  const KT kmer = want;
+  auto done = [&](bool past) {
+    if (!SAT || !past || !over.rec) return true;
+    const unsigned long long o = atomicAdd(&over.ctr->n_sk_past, 1ull);
+    if (o < over.cap) {
+      KOps<KT>::store(over.rec + o * NW, kmer);
+      over.rec[o * NW + KWD] = fresh;
+    }
+    return true;
+  };
+  bool past = false;
   SkSeq p(want, sl.n);
   for (uint32_t probe = 0; probe < SK_MAX_PROBE; ++probe, p.next(sl.n)) {
     uint64_t seen;
@@ -885,8 +904,8 @@ __device__ __noinline__ bool sk_insert(SkSlots<KT> sl, KT want, uint32_t fresh, 
     if (claimed) { ++claims; return true; }
     if (KOps<KT>::eq(key, want)) {
       uint32_t *e = sl.entries(p.j);
-      if (sk_try_entry<SAT>(e, *(volatile uint32_t *)e, fresh, claims)) return true;
-      if (sk_try_entry<SAT>(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims)) return true;
+      if (sk_try_entry<SAT>(e, *(volatile uint32_t *)e, fresh, claims, past)) return done(past);
+      if (sk_try_entry<SAT>(e + 1, *(volatile uint32_t *)(e + 1), fresh, claims, past)) return done(past);
       atomicOr(e + 1, SK_MORE);
       ((uint64_t *)&want)[KOps<KT>::WORDS - 1] |= KEY_CONT;
     }
@@ -1150,6 +1169,31 @@ __global__ void k_sk_crowd_off(const unsigned long long *base, uint32_t n, uint3
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) off[i] = (uint32_t)base[i];
 }
 
+/* Those records, once the table is written: their occurrences go to the side table of counts past an
+ * entry word's own, under the word's address (one sample's table) */
+template <class KT>
+__global__ void __launch_bounds__(256) k_sk_past(const uint64_t *rec, uint64_t n, uint64_t *table, const SGeom *sg,
+                                                 DevCounters *ctr) {
+  constexpr int SU = Slot<KT>::U64, KWD = Slot<KT>::KEYW, NE = Slot<KT>::ENTRIES, NW = SkRec<KT>::NW;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const KT x = KOps<KT>::load(rec + i * NW), t = table_key(x);
+    const uint32_t fresh = (uint32_t)rec[i * NW + KWD];
+    uint32_t *at = nullptr;
+    Probe pr = table_probe(sg[0].g, x, t);
+    for (uint64_t p = pr.lo; p < pr.hi && !at; ++p, pr.next()) {
+      const KT key = KOps<KT>::load(table + pr.i * SU);
+      if (key_is_empty(key)) break;
+      if (!key_matches(key, t, false) && !key_matches(key, t, true)) continue;
+      uint32_t *e = reinterpret_cast<uint32_t *>(table + pr.i * SU + KWD);
+      for (int q = 0; q < NE && !at; ++q)
+        if (e[q] && entry_code(e[q]) == entry_code(fresh)) at = e + q;
+    }
+    if (!at) { atomicOr(&ctr->err, (unsigned long long)DERR_INVARIANT); continue; }
+    atomicOr(at, E_BIG);
+    big_add(ctr, (unsigned long long)(uintptr_t)at, fresh >> E_COUNT_SHIFT);
+  }
+}
+
 /* SUB: the parts of crowded partitions, from their k-mers' records (off, todo and over are theirs) */
 template <class KT, bool EF, bool SUB>
 __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_count(SkCount a) {
@@ -1189,7 +1233,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
     __syncthreads();
     for (uint32_t i = a.off[part] + tid; i < r1; i += nt) {
       const uint64_t *w = a.recs + (uint64_t)i * NW;
-      if (!*(volatile uint32_t *)&s_full && !sk_insert<KT, true>(sl, KOps<KT>::load(w), (uint32_t)w[KWD], claims)) s_full = 1;
+      if (!*(volatile uint32_t *)&s_full && !sk_insert<KT, true>(sl, KOps<KT>::load(w), (uint32_t)w[KWD], claims, SkPast{a.past, a.past_cap, a.ctr}))
+        s_full = 1;
     }
   }
   for (uint32_t r0 = a.off[part]; !SUB && r0 < r1; r0 += round) {
@@ -1265,7 +1310,8 @@ __global__ void __launch_bounds__(SK_COUNT_TPB, sizeof(KT) == 8 ? 4 : 3) k_sk_co
           uint32_t *e = sl.entries(p.j);
           uint32_t cur = (uint32_t)seen;
           if (cur != 0 && entry_code(cur) != code) { cur = (uint32_t)(seen >> 32); ++e; }
-          todo = !sk_try_entry(e, cur, fresh, claims);
+          bool past;
+          todo = !sk_try_entry(e, cur, fresh, claims, past);
         }
         if (todo) {   /* the rest, later */
           const uint32_t at = atomicAdd(&s_late_n, 1u);

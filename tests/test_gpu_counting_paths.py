@@ -1,6 +1,5 @@
 """Which counting path runs, and the one by k-mer records at the lengths where super-k-mers run by
-default: an explicit table size keeps it (a batch takes no notice of the size itself), and some counts
-that must be exact come to it by themselves."""
+default: an explicit table size keeps it (a batch takes no notice of the size itself)."""
 import numpy as np
 import pytest
 
@@ -132,13 +131,18 @@ def test_kmer_records_in_a_batch(chunk):
 
 
 @pytest.mark.parametrize("k", [31, 45])
-def test_exact_counts_that_leave_super_kmers(k):
-    """300 bases a read, all alike: with the counts copied out such a minimizer's could pass what an entry
-    of a part holds, and the build goes by other records; without, it stays"""
-    n = (1 << 25) // (300 - k - 1) + 2000
+def test_exact_counts_past_what_an_entry_holds(k):
+    """300 bases a read, all alike, counted more than 2^26 times in all: by super-k-mers whether the counts
+    are copied out or not, to the last occurrence"""
+    n = (1 << 26) // (300 - k - 1) + 2000
     data = fastq(np.zeros((n, 300), dtype=np.int8))
     assert path_of(data, k)[0] == "super_kmers"
-    assert path_of(data, k, keep_k2=True)[0] != "super_kmers"
+    with bg.Graph(k=k, thresh=bg.thresholds([2]), min_update=True, keep_k2=True, keep_filtered=True) as g:
+        g.build_and_compact(data)
+        assert g.counting_path()[0] == "super_kmers"
+        for keys, edges, counts in (g.k2(), g.filtered()):
+            assert int(counts.max()) == n * (300 - k - 1) and counts.dtype == np.uint32
+        assert int(g.k2()[2].sum()) == n * (300 - k + 1)
 
 
 @pytest.mark.parametrize("steps", [False, True])

@@ -202,7 +202,8 @@ def test_crowded_partitions_cleaned():
 @pytest.mark.parametrize("k", [31, 45])
 def test_a_count_past_what_a_block_may_hold(k):
     """one biedge of one k-mer counted more than 2^25 times (300 bases a read, all alike, beside a
-    genome's reads): capped where only the filter reads it, exact where the counts are copied out"""
+    genome's reads): capped where only the filter reads it, exact where the counts are copied out, by the side
+    table of counts past an entry's own"""
     n = (1 << 25) // (300 - k - 1) + 2000
     rng = np.random.default_rng(k)
     data = fastq(np.zeros((n, 300), dtype=np.int8)) + fastq(rand_reads(rng, rng.integers(0, 4, 30_000), 6_000, 100, 0.003))
