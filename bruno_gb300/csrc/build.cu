@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
   const long long E = ctr->last_nonws + 1;  /* effective end (exclusive) */
   uint64_t base = tile_base[blockIdx.x];
   unsigned long long nl_eff = 0;  /* newlines ending lines before E, max over this thread */
-  unsigned long long seq = 0;     /* sequence ends less sequence starts: over all reads, their bases */
   if (blockIdx.x == 0 && threadIdx.x == 0 && E > 0 && buf[0] != '@') atomicMin(&ctr->bad_line, 0ull);
   /* stripes of TPB*64 bytes, 64 consecutive bytes per thread (four 16-byte loads in flight),
    * in byte order: one block scan per stripe */
@@ -197,12 +196,11 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
         nl_eff = ln + 1;
         const uint64_t r = ln >> 2;
         const unsigned role = (unsigned)(ln & 3);
-        if (role == 0 && rbase + r < rcap) { rstart[rbase + r] = (uint64_t)(buf + p + 1); seq -= p + 1; }
+        if (role == 0 && rbase + r < rcap) rstart[rbase + r] = (uint64_t)(buf + p + 1);
         if (role == 1 && rbase + r < rcap) {
           uint64_t e = p;
           if (e > 0 && buf[e - 1] == '\r') --e;
           rend[rbase + r] = (uint64_t)(buf + e);
-          seq += e;
         }
         /* the first byte of line ln+1 */
         const unsigned nrole = (unsigned)((ln + 1) & 3);
@@ -216,14 +214,8 @@ __global__ void __launch_bounds__(TPB) k_index_lines(const unsigned char *buf, u
     base += total;
   }
   __shared__ unsigned long long snl[TPB / 32];
-  for (int o = 16; o > 0; o >>= 1) {
-    nl_eff = max(nl_eff, __shfl_down_sync(~0u, nl_eff, o));
-    seq += __shfl_down_sync(~0u, seq, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    snl[threadIdx.x >> 5] = nl_eff;
-    if (seq) atomicAdd(&ctr->n_seq, seq);
-  }
+  for (int o = 16; o > 0; o >>= 1) nl_eff = max(nl_eff, __shfl_down_sync(~0u, nl_eff, o));
+  if ((threadIdx.x & 31) == 0) snl[threadIdx.x >> 5] = nl_eff;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long m = 0;
@@ -2661,8 +2653,9 @@ bruno_status extract_begin(Ctx *c, uint64_t upper, int max_blocks);
 void extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 int wx_blocks(uint64_t nr);
 bool sk_takes(const Ctx *c);
-bool sk_pays(const Ctx *c, double length);
-constexpr double BATCH_READS = 100.0;   /* a batch's choice of records comes before its reads are known */
+bool sk_pays(const Ctx *c, double kmers);
+double batch_kmers(const Ctx *c);
+bruno_status sk_pays_for(Ctx *c, uint64_t r0, uint64_t r1, uint64_t bytes, bool &yes);
 bruno_status sk_begin(Ctx *c, const std::vector<uint64_t> &bytes, uint64_t records = 0);
 void sk_extract_reads(Ctx *c, uint64_t r0, uint64_t r1);
 bruno_status sk_extract_samples(Ctx *c, uint32_t q0, uint32_t q1, const std::vector<uint64_t> &f);
@@ -2684,7 +2677,7 @@ bruno_status run_index_reads(Ctx *c) {
   if ((st = ensure(c, c->tile_base, std::max<uint64_t>(1, total_tiles) * 8)) != BRUNO_OK) return st;
   bool piped = false;
   for (auto &sg : c->segs) piped |= sg.ev >= 0;
-  c->sk_on = sk_takes(c) && (c->S == 1 || sk_pays(c, BATCH_READS));
+  c->sk_on = sk_takes(c) && (c->S == 1 || sk_pays(c, batch_kmers(c)));
   c->pre_extracted = false;
   const bool pieces = piped && c->S == 1 && c->force_direct_count != 1;
   const bool batch_hook = piped && c->S > 1 && c->batch_piped;   /* a batch extracts group by group */
@@ -2730,7 +2723,7 @@ bruno_status run_index_reads(Ctx *c) {
       return set_err(c, BRUNO_ERR_BAD_INPUT, "malformed FASTQ in file " + std::to_string(si) + " near line " +
                                                  std::to_string(h.bad_line != ~0ull ? h.bad_line : lines));
     if (pieces && rcap == 0) {   /* the first reads say which records these are going to be */
-      c->sk_on = c->sk_on && sk_pays(c, (double)h.n_seq / (double)(lines / 4));
+      if ((st = sk_pays_for(c, 0, lines / 4, sg.n, c->sk_on)) != BRUNO_OK) return st;
       c->pre_extracted = c->sk_on || (c->W == 1 && !c->cfg.edge_filter);
     }
     if (c->pre_extracted && rcap == 0) {
@@ -2749,8 +2742,7 @@ bruno_status run_index_reads(Ctx *c) {
     rcap += lines / 4;
   }
   c->n_reads = rcap;
-  if (c->S == 1 && !c->pre_extracted && rcap) c->sk_on = c->sk_on && sk_pays(c, (double)c->hctr->n_seq / (double)rcap);
-  return BRUNO_OK;
+  return c->S == 1 && !c->pre_extracted ? sk_pays_for(c, 0, rcap, total_bytes, c->sk_on) : BRUNO_OK;
 }
 
 /* ------------------------------------------------------------ counting */
@@ -3250,17 +3242,37 @@ bool sk_takes(const Ctx *c) {
 }
 /* Where every k-mer is kept the count has nothing to leave out, and the k-mer records' shorter runs in
  * the table win unless a super-k-mer record stands for several k-mers: from 5 on for reads of the given
- * mean length, which k = 24 has with 100 bases and k = 31 with 45 (200 kbp at 60x, 100 bases, steps: k =
- * 19, 3.9 a record, 1.04 ms against 1.13 by super-k-mers; 21, 4.4, 1.05 and 1.15; 23, 4.8, 1.08 and 1.12;
- * 24, 5.2, 1.14 and 1.09; k = 31 with 36 bases, 3.9: 3.4 and 3.8); from 6.2 with a target load above 0.6
- * (unthresholded, load 0.7: k = 25, 5.6, 1.39 and 1.48; 27, 6.5, 1.44 and 1.40).  Small builds are a
- * chain of launches, fewer of them here (0.8 MB: 0.7 ms and 0.5). */
+ * mean number of k-mers, which k = 24 has with 100 bases and k = 31 with 45 (200 kbp at 60x, 100 bases,
+ * steps: k = 19, 3.9 a record, 1.04 ms against 1.13 by super-k-mers; 21, 4.4, 1.05 and 1.15; 23, 4.8, 1.08
+ * and 1.12; 24, 5.2, 1.14 and 1.09; k = 31 with 36 bases, 3.9: 3.4 and 3.8); from 6.2 with a target load
+ * above 0.6 (unthresholded, load 0.7: k = 25, 5.6, 1.39 and 1.48; 27, 6.5, 1.44 and 1.40).  Small builds
+ * are a chain of launches, fewer of them here (0.8 MB: 0.7 ms and 0.5). */
 constexpr uint64_t SK_SMALL = 2ull << 20;   /* bytes a sample */
-bool sk_pays(const Ctx *c, double length) {
-  if (!sk_keeps_all(c) || c->cfg.edge_filter || fastq_bytes(c) / c->S < SK_SMALL) return true;
-  const double kmers = std::max(1.0, length - c->cfg.k + 1.0), w = c->cfg.k - MZ_M + 1;
-  const double records = 1.0 + (kmers - 1.0) * 2.0 / (w + 1.0);
-  return kmers / records >= (c->cfg.max_load > 0.6 ? 6.2 : 5.0);
+bool sk_always(const Ctx *c) { return !sk_keeps_all(c) || c->cfg.edge_filter || fastq_bytes(c) / c->S < SK_SMALL; }
+bool sk_pays(const Ctx *c, double kmers) {
+  if (sk_always(c)) return true;
+  const double w = c->cfg.k - MZ_M + 1, records = 1.0 + (std::max(1.0, kmers) - 1.0) * 2.0 / (w + 1.0);
+  return std::max(1.0, kmers) / records >= (c->cfg.max_load > 0.6 ? 6.2 : 5.0);
+}
+/* a batch's choice of records comes before its reads are known: 100 bases */
+double batch_kmers(const Ctx *c) { return 101.0 - c->cfg.k; }
+/* yes: stays so if it pays for the reads [r0, r1) of so many FASTQ bytes, which are looked at where it
+ * depends on their lengths: where some length pays and their records are not so long that most of them
+ * must be sequence and quality (up to 128 bytes of names; 36-base reads with longer ones pass for longer
+ * reads) */
+bruno_status sk_pays_for(Ctx *c, uint64_t r0, uint64_t r1, uint64_t bytes, bool &yes) {
+  if (!yes || r1 == r0 || sk_always(c)) return BRUNO_OK;
+  int kmers = 1;
+  while (kmers < 2000 && !sk_pays(c, kmers)) ++kmers;
+  yes = kmers < 2000;
+  if (!yes || bytes >= (r1 - r0) * (uint64_t)(2 * (kmers + c->cfg.k) + 128)) return BRUNO_OK;
+  cudaMemsetAsync(&c->dctr->n_upper, 0, 8, c->stream);
+  k_kmer_upper<<<num_sms() * 4, TPB, 0, c->stream>>>((const uint64_t *)c->rstart.p + r0, (const uint64_t *)c->rend.p + r0,
+                                                     r1 - r0, c->cfg.k, c->dctr);
+  c->launches += 1;
+  const bruno_status st = sync_counters(c);
+  yes = sk_pays(c, (double)c->hctr->n_upper / (double)(r1 - r0));
+  return st;
 }
 
 template <class KT, int BL, bool EDGES>
@@ -4316,7 +4328,7 @@ bruno_status run_count_samples(Ctx *c) {
   cudaMemsetAsync(c->s_used.p, 0, (size_t)S * 8, c->stream);
   cudaMemsetAsync(c->s_tally.p, 0, (size_t)S * T_NUM * 8, c->stream);
   bool indexed = false;
-  if (sk_takes(c) && sk_pays(c, BATCH_READS)) {   /* by super-k-mers */
+  if (sk_takes(c) && sk_pays(c, batch_kmers(c))) {   /* by super-k-mers */
     std::vector<uint64_t> bytes(S);
     for (uint32_t q = 0; q < S; ++q) bytes[q] = c->samp_off[q + 1] - c->samp_off[q];
     if ((st = sk_begin(c, bytes)) != BRUNO_OK) return st;

@@ -28,7 +28,6 @@ struct DevCounters {
   long long last_nonws;                /* index of the last byte that is not \n or \r, -1 if none */
   unsigned long long bad_line;         /* first malformed line, ~0 if none */
   unsigned long long n_records;
-  unsigned long long n_seq;            /* bases of the reads indexed */
   unsigned long long n_sk, n_sk_est;   /* super-k-mer record places taken, records listed for the estimate */
   unsigned long long n_sk_edges;       /* k-mers of reads of k + 1 bases, under the (k+1)-mer filter */
   unsigned long long n_instances, n_reads_used;
