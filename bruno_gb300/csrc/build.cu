@@ -3501,10 +3501,11 @@ constexpr uint64_t SK_PART_KMERS = 4096;
 uint64_t sk_parts_room(const Ctx *c, uint64_t n_rec) { return n_rec * (uint64_t)(c->cfg.k - MZ_M + 1) / (SK_PART_KMERS / 2); }
 
 /* The n partitions listed at `list` (superkmer.cuh, crowded partitions) by parts; NO if their parts do
- * not do either. */
+ * not do either, AGAIN if so many overflow that the estimate must have been too low (and `retry` is
+ * left).  (Partitions of too many records say nothing about it.) */
 template <class KT>
 bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vector<SGeom> &sg, const uint32_t *list,
-                              uint32_t n, uint64_t room, SkCounted &out) {
+                              uint32_t n, uint64_t room, bool retry, SkCounted &out) {
   constexpr int NW = SkRec<KT>::NW;
   bruno_status st;
   out = SkCounted::NO;
@@ -3516,6 +3517,12 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
   cudaMemcpyAsync(rec.data(), c->sk_items.p, (size_t)n * sizeof(uint2), cudaMemcpyDeviceToHost, c->stream);
   c->launches += 1;
   if ((st = cuda_check(c, cudaStreamSynchronize(c->stream), "crowded partitions")) != BRUNO_OK) return st;
+  uint32_t overflowed = 0;
+  for (const uint2 &r : rec) overflowed += r.y <= SK_MAX_RECORDS;
+  if (retry && overflowed > parts / 2) {
+    out = SkCounted::AGAIN;
+    return BRUNO_OK;
+  }
   std::vector<SkCrowd> crowd(n);
   std::vector<SkChunk> chunks;
   uint64_t subs = 0, most = 0;
@@ -3524,8 +3531,9 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
     most = std::max(most, kmers);
     uint32_t lg = 1;
     while (kmers >> lg > SK_PART_KMERS) ++lg;
-    uint32_t smp = 0;
-    while (smp + 1 < sg.size() && sg[smp + 1].pbase <= part[i]) ++smp;
+    const uint32_t smp = (uint32_t)(std::upper_bound(sg.begin(), sg.end(), part[i], [](uint32_t P, const SGeom &x) {
+                           return P < x.pbase;
+                         }) - sg.begin()) - 1u;
     crowd[i] = SkCrowd{part[i], (uint32_t)subs, lg, smp};
     for (uint32_t r = 0; r < rec[i].y; r += SK_CHUNK<NW>)
       chunks.push_back(SkChunk{rec[i].x + r, std::min(SK_CHUNK<NW>, rec[i].y - r), (uint32_t)subs, lg});
@@ -3601,8 +3609,7 @@ bruno_status sk_count_crowded(Ctx *c, SkCount a, uint32_t parts, const std::vect
 
 /* The partitions counted (records in partition order), those that overflow their block's slots
  * once more with as many as fit, and those that these do not do for either, or that hold too many
- * records for one block, by parts.  AGAIN: the table is too small, or so many overflow that the
- * estimate must have been too low (and `retry` is left). */
+ * records for one block, by parts.  AGAIN: the table is too small, or the estimate was too low. */
 template <class KT>
 bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector<SkLaunch<KT>> &launches,
                             const std::vector<SGeom> &sg, uint64_t room, bool retry, SkCounted &out) {
@@ -3635,9 +3642,7 @@ bruno_status sk_count_parts(Ctx *c, SkCount a, uint32_t parts, const std::vector
     if ((st = sync_counters(c)) != BRUNO_OK) return st;
     const uint32_t crowded = (uint32_t)c->hctr->n_over;
     if (crowded && !c->hctr->err) {
-      out = SkCounted::AGAIN;
-      if (retry && crowded > parts / 2) return BRUNO_OK;
-      return sk_count_crowded<KT>(c, a, parts, sg, b.over, crowded, room, out);
+      return sk_count_crowded<KT>(c, a, parts, sg, b.over, crowded, room, retry, out);
     }
   }
   out = c->hctr->err ? SkCounted::AGAIN : SkCounted::DONE;

@@ -324,3 +324,12 @@ def test_estimates_within_the_table(thr):
             assert g.counting_path()[0] == "super_kmers"
             launches.append(g.sizes()["launches"])
     assert len(set(launches)) == 1, launches
+
+
+def test_every_partition_crowded_by_records():
+    """a genome of 2200 bases at 60000x: more than half of the partitions hold more records than a block counts,
+    which says nothing about the estimate, so that the plan stays (a further attempt shows as launches)"""
+    rng = np.random.default_rng(6)
+    data = fastq(rand_reads(rng, rng.integers(0, 4, 2200), 1_300_000, 100))
+    s = check(data, 31, bg.thresholds([2]))
+    assert s["n_nodes"] <= 2170 and s["table_partitions"] == 256 and s["launches"] < 48, s["launches"]
