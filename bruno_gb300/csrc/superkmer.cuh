@@ -182,7 +182,7 @@ struct SkExtract {
  * inside one block.  Where the minimum changes a run starts; the tile's runs are listed, and each
  * lane builds the records of every 32nd run from the packed words.  Everything stays inside the
  * warp: with one tile a block of 256 threads the block's barriers cost a quarter of its time (6.4 ms
- * at 1.2G k-mers, now 4.9).  Bound by issue (0.64 of the SMs' peak, 133 instructions a k-mer); four
+ * at 1.2G k-mers, now 4.9).  Bound by issue (0.64 of the SMs' peak, 104 instructions a k-mer); four
  * blocks an SM instead of three spill (5.2 ms).  Output places come in chunks that a warp reserves (one counter
  * cannot take an atomic per tile); a chunk's unused end is marked SK_NONE.  EDGES: the (k+1)-mer
  * filter's, with reads of k + 1 bases (as a switch it cost the others 2%). */
@@ -1101,7 +1101,9 @@ __device__ __forceinline__ unsigned sk_code(bool fwd, unsigned in5, unsigned out
  * 2^lg parts, first counted, then placed; a part holds some thousand k-mers, is counted by a block and
  * has a region of its own, which lookups find by the key.  160M k-mers, adapters in 2% of the reads:
  * 5.9 ms a build (4.9 without the adapters); by k-mer records, where such an input used to go after the
- * count had been tried at three sizes, 29.9, of which the k-mer records themselves take 17.1. */
+ * count had been tried at three sizes, 29.9, of which the k-mer records themselves take 17.1.  Bound by
+ * the latency of few blocks: these adapters' 70 chunks take 0.04 ms to count and 0.05 to place, their
+ * parts 0.15 to count. */
 struct SkChunk { uint32_t r0, n, sub0, lg; };   /* records, first part, log2 of the parts */
 template <int NW> constexpr uint32_t SK_CHUNK = 2048 / NW;
 /* records of a partition at most that one block counts (a typical one: 500), and below 2^26 k-mers */
