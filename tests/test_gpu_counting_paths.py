@@ -167,3 +167,44 @@ def test_second_attempt_over_records_in_order(steps):
         assert path == "super_kmers" and records > 1 << 20 and g.sizes()["table_partitions"] >= 1 << 12
         assert_same(sort_nodes(*g.nodes()), ref["nodes"], "graph nodes")
         assert chain_set(*g.chains()) == chain_set(*ref["chains"])
+
+
+def test_a_bin_past_its_tally():
+    """more than 2^26 records of one minimizer (8.6M reads of 150 A): by other records, with the same graph; a
+    batch with such a sample is declined, as its hash bucket always was, and the context builds on"""
+    import torch
+    reads, length, k = 8_600_000, 150, 31
+    rec = fastq(np.zeros((100, length), dtype=np.int8))
+    d = torch.from_numpy(np.frombuffer(rec, dtype=np.uint8).copy()).cuda().repeat(reads // 100)
+    torch.cuda.synchronize()
+    rng = np.random.default_rng(9)
+    small = fastq(rand_reads(rng, rng.integers(0, 4, 20_000), 4_000, 100, 0.005))
+    e = torch.from_numpy(np.frombuffer(small, dtype=np.uint8).copy()).cuda()
+    torch.cuda.synchronize()
+    want = plain(small, k=k, thresh=bg.thresholds([2]), min_update=True)["sizes"]
+    with bg.Graph(k=k, thresh=bg.thresholds([2]), min_update=True) as g:
+        g.build_and_compact(d.data_ptr(), d.numel(), is_device=True)
+        s = g.sizes()
+        assert g.counting_path()[0] in ("l2_partitions", "whole_table")
+        assert s["n_instances"] == reads * (length - k + 1) and s["n_k2"] == 3 and s["n_nodes"] == 1
+        with pytest.raises(bg.BrunoError) as err:
+            g.build_samples([e.data_ptr(), d.data_ptr()], is_device=True, nbytes=[e.numel(), d.numel()])
+        assert err.value.status == 4
+        g.build_samples([e.data_ptr(), e.data_ptr()], is_device=True, nbytes=[e.numel(), e.numel()])
+        for i in range(2):
+            assert all(g.sample_sizes(i)[n] == want[n] for n in ("n_k2", "n_nodes", "n_chains", "n_chain_chars"))
+
+
+@pytest.mark.parametrize("chunk", [0, 1 << 20])
+@pytest.mark.parametrize("k,want", [(21, "kmer_records"), (31, "super_kmers")])
+def test_path_of_an_unthresholded_batch(k, want, chunk):
+    """samples of more than 2 MB on average, every k-mer kept, in one copy and in groups"""
+    rng = np.random.default_rng(k)
+    samples = [fastq(rand_reads(rng, rng.integers(0, 4, 40_000), n, 100, 0.005)) for n in (16_000, 9_000, 12_000)]
+    cfg = dict(k=k, thresholding=False, min_update=True)
+    got, _ = batch(samples, h2d_chunk=chunk, **cfg)
+    for i, data in enumerate(samples):
+        same_as_plain(got[i], plain(data, **cfg), f"sample {i}")
+    with bg.Graph(h2d_chunk=chunk, **cfg) as g:
+        g.build_samples(samples)
+        assert g.counting_path()[0] == want
