@@ -333,3 +333,25 @@ def test_every_partition_crowded_by_records():
     data = fastq(rand_reads(rng, rng.integers(0, 4, 2200), 1_300_000, 100))
     s = check(data, 31, bg.thresholds([2]))
     assert s["n_nodes"] <= 2170 and s["table_partitions"] == 256 and s["launches"] < 48, s["launches"]
+
+
+@pytest.mark.parametrize("k", [31, 45])
+def test_crowded_partitions_with_wide_kmers_and_other_thresholds(k):
+    """a k-mer between every pair of bases in a crowded partition (more biedges than a slot holds), and the
+    filter with other thresholds than the count's, which reads every slot"""
+    rng = np.random.default_rng(k)
+    c = crowded_reads("poly-A", k)
+    wide = np.array([np.concatenate([rng.integers(0, 4, 50 - k // 2), [a], np.zeros(k, dtype=int), [b],
+                                     rng.integers(0, 4, 100)])[:100] for a in range(4) for b in range(4)] * 3)
+    data = fastq(np.concatenate([c, wide]))
+    check(data, k, bg.thresholds([2]))
+    for thr in ([3], [1], [1, 2, 3]):
+        t = bg.thresholds(thr)
+        ref = oracle.run(data, k=k, thresh=t, min_update=True, threads=16)
+        with bg.Graph(k=k, thresh=bg.thresholds([2]), min_update=True) as g:
+            g.load_fastq(data)
+            g.compute_biedge_freqencies()
+            assert g.counting_path()[0] == "super_kmers"
+            g.local_insert_by_freqencies(t)
+            assert g.sizes()["n_nodes"] == ref["n_nodes"] and g.sizes()["filter_flag_hist"] == ref["filter_flag_hist"]
+            assert_same(sort_nodes(*g.nodes()), ref["nodes"], f"graph nodes, {thr}")
