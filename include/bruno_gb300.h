@@ -367,7 +367,8 @@ bruno_status bruno_counting_path(bruno_ctx *ctx, int32_t *path, uint64_t *record
  * are copied one after another into one device buffer, and every kernel of the path runs once
  * over all of them: each sample counts into hash-table partitions of its own (sized from its own
  * distinct-count estimate), is filtered, chained and ranked, so that each sample's graph, chains
- * and counts are exactly what bruno_build_and_compact gives for that sample alone.  The whole
+ * and counts are exactly what bruno_build_and_compact gives for that sample alone (one sample
+ * alone is that build).  The whole
  * path of one sample is the reference driver's build_index_thresholded -> extract_chains ->
  * list_rank[_min_update] -> to_ranked_chain_nodes (compact_dbg_freq_construct_clean.cpp:
  * 295-348, 549-737).  Needs k <= 31, no edge filter, no raw or filtered count copies, and
